@@ -22,6 +22,7 @@
 //    ∇²(Π+ψ) plus Σ_gp dL x∂X₀ᵀ δf_gp + vₛₘ∂X₀ᵀ δmₑ (load variation).
 // Output layout: R[12], K[i + 12 j] = ∂R_i/∂X_j (column-major, like asm[2]).
 #pragma once
+#include "beam_spin.hpp"
 #include "tj.hpp"
 
 namespace mgpu {
@@ -271,28 +272,6 @@ MG_HD void mul_ac(const TJ<D, N> A[9], const double M[9], TJ<D, N> C[9]) {
       C[i + 3 * j] = tj_fma(A[i + 6], real(M[2 + 3 * j]), tj_fma(A[i + 3], real(M[1 + 3 * j]), A[i] * real(M[3 * j])));
 }
 
-// ---- per-element constants, precomputed at create time ----------------------
-struct BeamConst {
-  double rm[9];   // as-meshed frame (column-major)
-  double tgm[3];  // c₂ − c₁
-  double L;
-  // strain energy Π = ½kε ε² + ½kt θt² + ½k3v θb² + k3uv wn θb + ½k3u wn²
-  //                 + ½k2v θn² − k2uv wb θn + ½k2u wb²
-  double ke, kt, k3u, k3uv, k3v, k2u, k2uv, k2v;
-  double S0;                                    // Σ dL
-  double dL[4], ya[4], yu[4], yv[4];            // Gauss data
-  double mu, iota1, w, Ca[3], Cl[3], Cq[3];     // cross section (dynamic part)
-};
-
-// Newton variation of the state: X₀ += p0 δ, X₁ += p1 δ, X₂ += p2 δ
-// (SweepX{0}: 1,0,0;  Newmark: 1,a₁,b₁;  diffed K/C/M: unit vectors).
-struct Perturb {
-  double p0, p1, p2;
-};
-
-// rotation-dof index (0..5) of element dof j, or -1 for translations
-MG_HD int rot_index(int j) { return (j >= 3 && j < 6) ? j - 3 : (j >= 9 ? j - 6 : -1); }
-
 // Full element evaluation.
 //   X0,X1,X2: element dofs and their first/second time derivatives (X1,X2 ignored if !D)
 //   U: U-dof loads per unit length (nullptr if none)
@@ -302,6 +281,10 @@ template <bool D>
 MG_HD void beam_element(const BeamConst& c, const double* X0, const double* X1, const double* X2, const double* U,
                         Perturb pt, const double* av, const double* bv, double* R, double* K, double* rdir,
                         double* H) {
+  if constexpr (!D) {
+    beam_static(c, X0, U, R, [&](int i, int j, real v) { K[i + 12 * j] = K[j + 12 * i] = to_d(pt.p0 * v); }, H);
+    return;
+  }
   // ---- rotation core
   // the nodal rotations depend on their own node's three dofs only
   TJ<D, 3> r1[9];

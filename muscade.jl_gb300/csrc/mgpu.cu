@@ -73,7 +73,7 @@ __device__ __forceinline__ void flag_nan(int* errflag, int64_t gid, bool bad) {
   if (bad) atomicMin(errflag, int(gid < INT_MAX ? gid : INT_MAX - 1));
 }
 
-// EulerBeam3D: one thread per element.  DYN selects the Newmark form.
+// EulerBeam3D: one thread per element.
 // EI-scale A-dof of the wrapper element EulerBeam3D{adof}: the bending
 // constants (EI2, EI3 times Gauss sums of the curvature shapes) scale with it
 __device__ __forceinline__ void scale_bending(BeamConst& bc, double s) {
@@ -85,9 +85,61 @@ __device__ __forceinline__ void scale_bending(BeamConst& bc, double s) {
   bc.k2v *= s;
 }
 
-// Launched with 64, 128 (default) or 256 threads per block (mgpu_autotune
-// picks); the bound of 256 leaves the register cap at 255 either way.
-template <bool DYN>
+// NaN test on the bits: an FP64 compare would hold the FP64 pipe like any other
+// FP64 instruction.
+__device__ __forceinline__ bool nan_bits(double v) {
+  const unsigned lo = unsigned(__double2loint(v)), hi = unsigned(__double2hiint(v)) & 0x7fffffffu;
+  return (hi | unsigned(lo != 0u)) > 0x7ff00000u;
+}
+
+// SweepX{0}.  Launched with 64, 128 (default) or 256 threads per block
+// (mgpu_autotune picks).  GEN: with dof scales or p0 != 1 (a factor for every
+// entry, which the models without them need not multiply by).
+template <bool GEN>
+__global__ void __launch_bounds__(256) beam_static_kernel(int64_t nele, const int32_t* __restrict__ idx,
+                                                          const int32_t* __restrict__ uidx,
+                                                          const double* __restrict__ cdata,
+                                                          const int32_t* __restrict__ aidx,
+                                                          const double* __restrict__ Avec, AsmArgs a,
+                                                          double* __restrict__ rout, double* __restrict__ kout,
+                                                          int64_t gid0) {
+  const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (e >= nele) return;
+  BeamConst bc;
+  load_soa(bc, cdata, nele, e);
+  if (aidx) scale_bending(bc, __ldg(Avec + __ldg(aidx + e)));
+  double X0[12], s[12];
+#pragma unroll
+  for (int i = 0; i < 12; ++i) {
+    const int dof = __ldg(idx + i * nele + e);
+    X0[i] = __ldg(a.x0 + dof);
+    if constexpr (GEN) s[i] = a.scale ? __ldg(a.scale + dof) : 1.0;
+  }
+  double U[3];
+  const bool has_u = uidx != nullptr;
+  if (has_u)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) U[k] = __ldg(a.u + __ldg(uidx + k * nele + e));
+  double R[12];
+  bool bad = false;
+  auto store = [&](int i, int j, double v) {
+    if constexpr (GEN) v *= a.p0 * s[i] * s[j];
+    bad |= nan_bits(v);
+    kout[(i + 12 * j) * nele + e] = v;
+    if (i != j) kout[(j + 12 * i) * nele + e] = v;
+  };
+  beam_static(bc, X0, has_u ? U : nullptr, R, store, nullptr);
+#pragma unroll
+  for (int i = 0; i < 12; ++i) {
+    const double r = GEN ? R[i] * s[i] : R[i];
+    bad |= nan_bits(r);
+    rout[i * nele + e] = r;
+  }
+  flag_nan(a.errflag, gid0 + e, bad);
+}
+
+// SweepX{2}; the same launch sizes, and the bound of 256 leaves the register
+// cap at 255.
 __global__ void __launch_bounds__(256) beam_kernel(int64_t nele, const int32_t* __restrict__ idx,
                                                    const int32_t* __restrict__ uidx, const double* __restrict__ cdata,
                                                    const int32_t* __restrict__ aidx, const double* __restrict__ Avec,
@@ -104,7 +156,7 @@ __global__ void __launch_bounds__(256) beam_kernel(int64_t nele, const int32_t* 
   for (int i = 0; i < 12; ++i) {
     dof[i] = __ldg(idx + i * nele + e);
     X0[i] = __ldg(a.x0 + dof[i]);
-    if constexpr (DYN) {
+    {
       X1[i] = __ldg(a.x1 + dof[i]);
       X2[i] = __ldg(a.x2 + dof[i]);
       if (a.mission == MGPU_ASM_STEP) {
@@ -119,9 +171,9 @@ __global__ void __launch_bounds__(256) beam_kernel(int64_t nele, const int32_t* 
 #pragma unroll
     for (int k = 0; k < 3; ++k) U[k] = __ldg(a.u + __ldg(uidx + k * nele + e));
   double R[12], K[144], rd[12];
-  const bool step = DYN && a.mission == MGPU_ASM_STEP;
-  const Perturb pt{a.p0, DYN ? a.sc[1] : 0.0, DYN ? a.sc[4] : 0.0};  // K + a1 C + b1 M
-  beam_element<DYN>(bc, X0, X1, X2, has_u ? U : nullptr, pt, av, bv, R, K, step ? rd : nullptr, nullptr);
+  const bool step = a.mission == MGPU_ASM_STEP;
+  const Perturb pt{a.p0, a.sc[1], a.sc[4]};  // K + a1 C + b1 M
+  beam_element<true>(bc, X0, X1, X2, has_u ? U : nullptr, pt, av, bv, R, K, step ? rd : nullptr, nullptr);
   double s[12];
 #pragma unroll
   for (int i = 0; i < 12; ++i) s[i] = a.scale ? __ldg(a.scale + dof[i]) : 1.0;
@@ -451,11 +503,14 @@ int launch_assembly(mgpu_ctx* c, int mission, cudaEvent_t* ev_groups, double p0)
     switch (G.kind) {
       case MGPU_EULERBEAM3D:
         if (dyn)
-          beam_kernel<true><<<nblk(G.nele, c->elem_block), c->elem_block, 0, c->stream>>>(G.nele, G.idx, G.uidx, G.cdata, G.aidx,
-                                                                      c->Avec, ag, rout, kout, gid0);
+          beam_kernel<<<nblk(G.nele, c->elem_block), c->elem_block, 0, c->stream>>>(
+              G.nele, G.idx, G.uidx, G.cdata, G.aidx, c->Avec, ag, rout, kout, gid0);
+        else if (ag.scale || p0 != 1.0)
+          beam_static_kernel<true><<<nblk(G.nele, c->elem_block), c->elem_block, 0, c->stream>>>(
+              G.nele, G.idx, G.uidx, G.cdata, G.aidx, c->Avec, ag, rout, kout, gid0);
         else
-          beam_kernel<false><<<nblk(G.nele, c->elem_block), c->elem_block, 0, c->stream>>>(G.nele, G.idx, G.uidx, G.cdata, G.aidx,
-                                                                       c->Avec, ag, rout, kout, gid0);
+          beam_static_kernel<false><<<nblk(G.nele, c->elem_block), c->elem_block, 0, c->stream>>>(
+              G.nele, G.idx, G.uidx, G.cdata, G.aidx, c->Avec, ag, rout, kout, gid0);
         break;
       case MGPU_BAR3D:
         bar_kernel<<<nblk(G.nele, c->elem_block), c->elem_block, 0, c->stream>>>(G.nele, dyn ? 3 : 1, G.idx, G.uidx, G.cdata, ag, rout,
