@@ -27,11 +27,13 @@
 //    second variation of Π+ψ is a 9 × 9 quadratic form in (δd, p, r), summed once
 //    with the moments of the frozen stresses, and goes to the dofs with two 3 × 3
 //    matrices, Rod(n)T(v₁) and Rod(n)ᵀT(v₂).
-//    What bounds the element on GB300 is the number of FP64 instructions (a warp
-//    instruction holds a sub-partition's FP64 pipe for 64 cycles), and this form
-//    needs a sixth of those of second-order Taylor arithmetic through every
-//    rotation matrix (21 Hessian entries of each of nine components), which is
-//    how the derivative was taken before; csrc/flopcount.cpp counts them.
+//    What bounds the element on GB300 is the number of FP64 instructions: a warp
+//    instruction holds a sub-partition's FP64 pipe for 64 cycles.  This form needs
+//    2,500 flops a beam and 11,700 with time derivatives (csrc/flopcount.cpp);
+//    second-order Taylor arithmetic through every rotation matrix, which took the
+//    derivative before, needed 16,200 and 44,200 (and spilled 16 KB a thread).
+//    Measured: 210,000 static beams 3.70 -> 0.62 ms, 50,000 Newmark beams
+//    2.84 -> 0.85 ms, and a model of one warp 350 -> 57 µs and 1,010 -> 282 µs.
 // Output layout: R[12], K[i + 12 j] = ∂R_i/∂X_j (column-major, like asm[2]).
 #pragma once
 #include "tj.hpp"
@@ -237,7 +239,17 @@ MG_HD void beam_state(const BeamConst& c, const double* X0, SinFun& q1, SinFun& 
   const real dn = sqrt(dot3(g.d, g.d));
   g.idn = 1.0 / dn;
   for (int i = 0; i < 3; ++i) g.dh[i] = g.d[i] * g.idn;
-  g.eps = dn * 2.0 / c.L - 1.0;
+  // ε = 2|d|/L − 1 as (|2d|² − L²)/(L (2|d| + L)), the numerator from (2d − tgₘ)·(2d + tgₘ)
+  // (2d − tgₘ is exact for small strains; |tgₘ|² − L² is rounding only): the
+  // difference from 1 would add the rounding of the root and the quotient, EA·2⁻⁵³
+  // of axial force, different at every state, which keeps the Newton iterations of
+  // stiff beams from settling (5,000 beams of EA = 1e10, Σ Δx² to 1e-14: 8.4
+  // iterations a step; 4.1 this way).  d keeps its own rounding, as in the
+  // reference: time stepping amplifies it in the rates of the multipliers.
+  const real tg[3] = {c.tgm[0], c.tgm[1], c.tgm[2]}, L = c.L;
+  real l2 = fma(tg[2], tg[2], fma(tg[1], tg[1], fma(tg[0], tg[0], -(L * L))));
+  for (int i = 0; i < 3; ++i) l2 = fma(fma(2.0, g.d[i], -tg[i]), fma(2.0, g.d[i], tg[i]), l2);
+  g.eps = l2 / fma(L, 2.0 * dn, L * L);
   for (int k = 0; k < 3; ++k) g.th[k] = dot3(g.rs + 3 * k, g.n);
   g.wn = dot3(g.rs + 3, g.d);
   g.wb = dot3(g.rs + 6, g.d);
@@ -249,12 +261,22 @@ struct BeamLoads {
   real u[3], a[3], v[3], o[3], m[3];
 };
 
+// x' = X₁ δv₁ and y' = Y₂ δv₂
+MG_HD void beam_maps(const double* X0, const SinFun& q1, const SinFun& q2, const BeamState& g, real X1[9], real Y2[9]) {
+  const real v1[3] = {X0[3], X0[4], X0[5]}, v2[3] = {X0[9], X0[10], X0[11]};
+  real T[9];
+  tan_matrix(v1, q1, T);
+  mul33(g.rd, T, X1);
+  tan_matrix(v2, q2, T);
+  mul33t(g.rd, T, Y2);
+}
+
 // The residual, and the second variation with the loads held: the 9 × 9 form in
 // (δd, p, r), then its dof entries through out(i, j, v), each pair i <= j of the
-// symmetric matrix once.  ROT: with the moment term mₑ·vₛₘ.
+// symmetric matrix once.  ROT and rot: with the moment term mₑ·vₛₘ.
 template <bool ROT, class Out>
 MG_HD void beam_frozen(const BeamConst& c, const double* X0, const SinFun& q1, const SinFun& q2, const BeamState& g,
-                       const BeamLoads& f, double* R, Out&& out) {
+                       const BeamLoads& f, bool rot, const real X1[9], const real Y2[9], double* R, Out&& out) {
   const real *t = g.rs, *nn = g.rs + 3, *bb = g.rs + 6, *n = g.n, *d = g.d;
   // stresses σ = ∂Π/∂q, q = (ε, θ, w)
   const real s_e = c.ke * g.eps;
@@ -303,7 +325,7 @@ MG_HD void beam_frozen(const BeamConst& c, const double* X0, const SinFun& q1, c
         }
       }
   }
-  if constexpr (ROT) {  // mₑ·vₛₘ, vₛₘ = Rod⁻¹(rₛₘ) = ι(x) q, with ι = 1/scac, x = (tr−1)/2, q = spin⁻¹
+  if (ROT && rot) {  // mₑ·vₛₘ, vₛₘ = Rod⁻¹(rₛₘ) = ι(x) q, with ι = 1/scac, x = (tr−1)/2, q = spin⁻¹
     const real* M = g.rs;
     const real tr = M[0] + M[4] + M[8];
     real io[3];
@@ -460,14 +482,8 @@ MG_HD void beam_frozen(const BeamConst& c, const double* X0, const SinFun& q1, c
       }
   }
   // ---- to the dofs
-  real X1[9], Y2[9];
   const real v1[3] = {X0[3], X0[4], X0[5]}, v2[3] = {X0[9], X0[10], X0[11]};
   {
-    real T[9];
-    tan_matrix(v1, q1, T);
-    mul33(g.rd, T, X1);
-    tan_matrix(v2, q2, T);
-    mul33t(g.rd, T, Y2);
     real gx[3], gy[3];
     for (int i = 0; i < 3; ++i) {
       gx[i] = fma(0.5, gO[i], -h[i]);
@@ -549,52 +565,39 @@ MG_HD void beam_frozen(const BeamConst& c, const double* X0, const SinFun& q1, c
 }
 
 
-// Columns of ∂m/∂v and ∂(n×t)/∂v over the six rotation dofs, m = (t·d) t
-MG_HD void beam_modes(const double* X0, const SinFun& q1, const SinFun& q2, const BeamState& g, real Jm[6][3],
-                      real Jw[6][3]) {
-  const real *t = g.rs, *n = g.n;
-  const real k0 = 0.5 / g.q.a, k1 = g.q.c * k0, be = g.q.b * k0, td = dot3(t, g.d);
-  for (int a = 0; a < 2; ++a) {
-    const real v[3] = {X0[3 + 6 * a], X0[4 + 6 * a], X0[5 + 6 * a]};
-    real T[9], X[9];
-    tan_matrix(v, a ? q2 : q1, T);
-    if (a)
-      mul33t(g.rd, T, X);
-    else
-      mul33(g.rd, T, X);
-    const real sg = a ? 1.0 : -1.0;
-    for (int j = 0; j < 3; ++j) {
-      const real* x = X + 3 * j;
-      real *jm = Jm[3 * a + j], *jw = Jw[3 * a + j], w[3] = {0.5 * x[0], 0.5 * x[1], 0.5 * x[2]}, dn[3], jt[3];
-      cross3_add(sg * be, n, x, w);
-      const real nx = sg * k1 * dot3(n, x);
-      for (int i = 0; i < 3; ++i) dn[i] = fma(sg * k0, x[i], -(nx * n[i]));
-      cross3(w, t, jt);
-      const real jd = dot3(jt, g.d);
-      for (int i = 0; i < 3; ++i) jm[i] = fma(t[i], jd, td * jt[i]);
-      cross3(dn, t, jw);
-      cross3_add(1.0, n, jt, jw);
-    }
-  }
+// Spin of rₛₘ and δn along x' = x (sg = −1) or y' = x (sg = 1)
+MG_HD void beam_spin(real sg, const real n[3], real k0, real k1, real be, const real x[3], real w[3], real dn[3]) {
+  for (int i = 0; i < 3; ++i) w[i] = 0.5 * x[i];
+  cross3_add(sg * be, n, x, w);
+  const real nx = sg * k1 * dot3(n, x);
+  for (int i = 0; i < 3; ++i) dn[i] = fma(sg * k0, x[i], -(nx * n[i]));
 }
 
 // ∂R/∂U of loads −U per unit length at the Gauss points, H[i + 12 k]
-MG_HD void beam_uload(const BeamConst& c, const double* X0, const SinFun& q1, const SinFun& q2, const BeamState& g,
-                      double* H) {
-  real Jm[6][3], Jw[6][3], su = 0.0, sa = 0.0, sv = 0.0;
-  beam_modes(X0, q1, q2, g, Jm, Jw);
+MG_HD void beam_uload(const BeamConst& c, const BeamState& g, const real X1[9], const real Y2[9], double* H) {
+  const real *t = g.rs, *n = g.n;
+  const real k0 = 0.5 / g.q.a, k1 = g.q.c * k0, be = g.q.b * k0, td = dot3(t, g.d);
+  real su = 0.0, sa = 0.0, sv = 0.0;
   for (int k = 0; k < 4; ++k) {
     su += c.dL[k] * c.yu[k];
     sa += c.dL[k] * (c.ya[k] - c.yu[k]);
     sv += c.dL[k] * c.yv[k];
   }
+  for (int j = 0; j < 6; ++j) {
+    real w[3], dn[3], jt[3], jw[3];
+    beam_spin(j < 3 ? -1.0 : 1.0, n, k0, k1, be, j < 3 ? X1 + 3 * j : Y2 + 3 * (j - 3), w, dn);
+    cross3(w, t, jt);
+    cross3(dn, t, jw);
+    cross3_add(1.0, n, jt, jw);
+    const real jd = dot3(jt, g.d);
+    for (int k = 0; k < 3; ++k)
+      H[(j < 3 ? 3 + j : 6 + j) + 12 * k] = to_d(-fma(sa, fma(t[k], jd, td * jt[k]), sv * jw[k]));
+  }
   for (int k = 0; k < 3; ++k)
     for (int j = 0; j < 3; ++j) {
-      const real m = fma(sa * g.rs[k], g.rs[j], k == j ? su : real(0.0)), o = k == j ? c.S0 : 0.0;
+      const real m = fma(sa * t[k], t[j], k == j ? su : real(0.0)), o = k == j ? c.S0 : 0.0;
       H[j + 12 * k] = to_d(0.5 * (m - o));
       H[6 + j + 12 * k] = to_d(-0.5 * (m + o));
-      H[3 + j + 12 * k] = to_d(-fma(sa, Jm[j][k], sv * Jw[j][k]));
-      H[9 + j + 12 * k] = to_d(-fma(sa, Jm[3 + j][k], sv * Jw[3 + j][k]));
     }
 }
 
@@ -622,8 +625,549 @@ MG_HD void beam_static(const BeamConst& c, const double* X0, const double* U, do
       f.m[i] = 0.0;
     }
   }
-  beam_frozen<false>(c, X0, q1, q2, g, f, R, out);
-  if (H) beam_uload(c, X0, q1, q2, g, H);
+  real X1[9], Y2[9];
+  beam_maps(X0, q1, q2, g, X1, Y2);
+  beam_frozen<false>(c, X0, q1, q2, g, f, false, X1, Y2, R, out);
+  if (H) beam_uload(c, g, X1, Y2, H);
+}
+
+// ---- time derivatives ---------------------------------------------------------
+MG_HD void axpy3(real a, const real x[3], real y[3]) {
+  for (int i = 0; i < 3; ++i) y[i] = fma(a, x[i], y[i]);
+}
+
+// e_s and f_s, from the next remainders (e = 1/24 − s e', f = 1/120 − s f'):
+// e_s = 2e' − f/2, f_s = (5f'−e')/2
+template <int K>
+MG_HD void sin_series_next(real s, real& e, real& f) {
+  real ee = inv_fact(2 * K + 4), ff = inv_fact(2 * K + 5);
+#pragma unroll
+  for (int k = K - 2; k >= 0; --k) {
+    ee = fma(-s, ee, inv_fact(2 * k + 6));
+    ff = fma(-s, ff, inv_fact(2 * k + 7));
+  }
+  e = ee;
+  f = ff;
+}
+MG_HD void sin_next(real s, const SinFun& q, real& es, real& fs) {
+  if (s < 10.0) {
+    real e1, f1;
+    if (s < 1.0)
+      sin_series_next<7>(s, e1, f1);
+    else
+      sin_series_next<14>(s, e1, f1);
+    es = fma(2.0, e1, -0.5 * q.f);
+    fs = 0.5 * fma(5.0, f1, -e1);
+  } else {
+    const real is = 1.0 / s;
+    es = is * fma(0.5, q.c, -2.0 * q.e);
+    fs = 0.5 * is * fma(-5.0, q.f, q.e);
+  }
+}
+
+// T(v) and its first two time derivatives.  Where |v| < 1e-14 the
+// reference takes sinc1 for a constant: there Rod = I + S + S²/2, whose third
+// derivative is that of T with a = 1, b = c = 1/2 held.
+MG_HD void tan_jets(const real v[3], const real v1[3], const real v2[3], real s, const SinFun& q, real T[9],
+                    real Td[9], real Tdd[9]) {
+  tan_matrix(v, q, T);
+  const real s1 = 2.0 * dot3(v, v1), s2 = 2.0 * (dot3(v1, v1) + dot3(v, v2));
+  real a1 = 0.0, b1 = 0.0, c1 = 0.0, a2 = 0.0, b2 = 0.0, c2 = 0.0, c0 = 0.5;
+  if (!(s < 1e-28)) {
+    real es, fs;
+    sin_next(s, q, es, fs);
+    const real as = sin_as(q), bs = sin_bs(q), cs = sin_cs(q);
+    const real bss = fma(-0.5, cs, es), ass = 0.5 * (cs - bs), css = 0.5 * fma(3.0, fs, -es);
+    a1 = as * s1;
+    b1 = bs * s1;
+    c1 = cs * s1;
+    a2 = fma(ass * s1, s1, as * s2);
+    b2 = fma(bss * s1, s1, bs * s2);
+    c2 = fma(css * s1, s1, cs * s2);
+    c0 = q.c;
+  }
+  for (int j = 0; j < 3; ++j)
+    for (int i = 0; i < 3; ++i) {
+      const real vv = v[i] * v[j], v1v = fma(v1[i], v[j], v[i] * v1[j]);
+      const real vx = fma(2.0 * v1[i], v1[j], fma(v2[i], v[j], v[i] * v2[j]));
+      Td[i + 3 * j] = fma(c1, vv, c0 * v1v);
+      Tdd[i + 3 * j] = fma(c2, vv, fma(2.0 * c1, v1v, c0 * vx));
+    }
+  const int up[3] = {5, 6, 1}, dw[3] = {7, 2, 3};  // +v_k and −v_k of [v]
+  for (int k = 0; k < 3; ++k) {
+    Td[4 * k] += a1;
+    Tdd[4 * k] += a2;
+    const real x = fma(b1, v[k], q.b * v1[k]), y = fma(b2, v[k], fma(2.0 * b1, v1[k], q.b * v2[k]));
+    Td[up[k]] += x;
+    Td[dw[k]] -= x;
+    Tdd[up[k]] += y;
+    Tdd[dw[k]] -= y;
+  }
+}
+
+// SweepX{2}: residual and Newton matrix p0 ∂R/∂X + p1 ∂R/∂X′ + p2 ∂R/∂X″.
+// out(i, j, v) receives all 144 entries once, column by column (first the
+// rotations' columns).  rdir (optional): ∂R along X′ += av, X″ += bv.
+// The loads' variation Σ dL x∂X₀ᵀ δf goes through the modes of a Gauss point's
+// position, x = yᵤ d + (yₐ−yᵤ) m + yᵥ w + ½(u₁+u₂), m = (t·d)t, w = n×t: per
+// direction the modes' velocity and acceleration vary (∂ẋ/∂X = J̇, ∂ẍ/∂X = J̈,
+// ∂ẍ/∂X′ = 2J̇ for a Jacobian J), the forces are summed over the Gauss points per
+// mode, and the six rotation rows come from the two sums' moment and couple alone.
+// Without drag that needs the modes' Gram sums only.
+template <class Out>
+MG_HD void beam_newmark(const BeamConst& c, const double* X0, const double* X1, const double* X2, const double* U,
+                        Perturb pt, const double* av, const double* bv, double* R, Out&& out, double* rdir, double* H) {
+  SinFun q1, q2;
+  BeamState g;
+  beam_state(c, X0, q1, q2, g);
+  const real *t = g.rs, *n = g.n, *d = g.d;
+  const SinFun& q = g.q;
+  const real k0 = 0.5 / q.a, k1 = q.c * k0, be = q.b * k0;
+  // ---- nodes: maps X = Rod(±n) T of (x', y') and of the derivatives of T
+  real X[2][9], Xd[2][9], Xdd[2][9];
+  for (int a = 0; a < 2; ++a) {
+    const int o = 3 + 6 * a;
+    const real v[3] = {X0[o], X0[o + 1], X0[o + 2]}, v1[3] = {X1[o], X1[o + 1], X1[o + 2]},
+               v2[3] = {X2[o], X2[o + 1], X2[o + 2]};
+    real T[9], Td[9], Tdd[9];
+    tan_jets(v, v1, v2, dot3(v, v), a ? q2 : q1, T, Td, Tdd);
+    if (a) {
+      mul33t(g.rd, T, X[1]);
+      mul33t(g.rd, Td, Xd[1]);
+      mul33t(g.rd, Tdd, Xdd[1]);
+    } else {
+      mul33(g.rd, T, X[0]);
+      mul33(g.rd, Td, Xd[0]);
+      mul33(g.rd, Tdd, Xdd[0]);
+    }
+  }
+  // ---- time derivatives of n and of the spin of rₛₘ
+  real n1[3], n2[3], om[3], om1[3], sp[2][3], sp1[2][3];  // ṅ, n̈, ω, ω̇, spins of Rod(±n) and their rates
+  {
+    real w[2][3], wd[2][3];  // w = X v̇, X v̈ + Ẋ v̇ (the frame's own turn apart)
+    for (int a = 0; a < 2; ++a)
+      for (int i = 0; i < 3; ++i) {
+        const int o = 3 + 6 * a;
+        w[a][i] = fma(X[a][i], X1[o], fma(X[a][i + 3], X1[o + 1], X[a][i + 6] * X1[o + 2]));
+        wd[a][i] = fma(X[a][i], X2[o], fma(X[a][i + 3], X2[o + 1], X[a][i + 6] * X2[o + 2])) +
+                   fma(Xd[a][i], X1[o], fma(Xd[a][i + 3], X1[o + 1], Xd[a][i + 6] * X1[o + 2]));
+      }
+    real r[3], p[3], o[3], r1[3], p1[3], o1[3], x[3];
+    for (int i = 0; i < 3; ++i) {
+      r[i] = w[1][i] - w[0][i];
+      p[i] = 0.5 * (w[0][i] + w[1][i]);
+      r1[i] = wd[1][i] - wd[0][i];
+      p1[i] = 0.5 * (wd[0][i] + wd[1][i]);
+    }
+    cross3(n, r, x);
+    for (int i = 0; i < 3; ++i) o[i] = be * x[i];
+    cross3_add(1.0, p, r, r1);
+    cross3_add(1.0, o, r, r1);
+    cross3_add(1.0, o, p, p1);
+    const real nr = dot3(n, r), as = sin_as(q) / q.a;
+    const real k0d = -k0 * as * nr, k1d = fma(sin_cs(q), k0, -(k1 * as)) * nr, bed = fma(sin_bs(q), k0, -(be * as)) * nr;
+    for (int i = 0; i < 3; ++i) n1[i] = fma(k0, r[i], -(k1 * nr * n[i]));
+    const real nrd = dot3(n1, r) + dot3(n, r1);
+    for (int i = 0; i < 3; ++i)
+      n2[i] = fma(k0, r1[i], fma(k0d, r[i], -fma(fma(k1d, nr, k1 * nrd), n[i], k1 * nr * n1[i])));
+    for (int i = 0; i < 3; ++i) o1[i] = bed * x[i];
+    cross3_add(be, n1, r, o1);
+    cross3_add(be, n, r1, o1);
+    for (int i = 0; i < 3; ++i) {
+      om[i] = p[i] + o[i];
+      om1[i] = p1[i] + o1[i];
+      sp[0][i] = fma(0.5, r[i], o[i]);
+      sp[1][i] = fma(-0.5, r[i], o[i]);
+      sp1[0][i] = fma(0.5, r1[i], o1[i]);
+      sp1[1][i] = fma(-0.5, r1[i], o1[i]);
+    }
+  }
+  // rates of κ0, κ1, β with n (of their second derivatives in s too)
+  real k01, k11, be1, k02, k12, be2;
+  {
+    real es, fs;
+    sin_next(g.s, q, es, fs);
+    const real s1 = 2.0 * dot3(n, n1), s2 = 2.0 * (dot3(n1, n1) + dot3(n, n2));
+    const real ia = 1.0 / q.a, as = sin_as(q), bs = sin_bs(q), cs = sin_cs(q);
+    const real bss = fma(-0.5, cs, es), ass = 0.5 * (cs - bs), css = 0.5 * fma(3.0, fs, -es);
+    // z/(2a) for z = 1, c, b: derivative (z_s/2 − as·(z/2a))/a, and again
+    const real p = as * ia, k0s = -k0 * p, k1s = fma(0.5 * cs, ia, -(k1 * p)), bes = fma(0.5 * bs, ia, -(be * p));
+    const real k0ss = -(2.0 * p * k0s + ass * ia * k0);
+    const real k1ss = 0.5 * css * ia - (2.0 * p * k1s + ass * ia * k1);
+    const real bess = 0.5 * bss * ia - (2.0 * p * bes + ass * ia * be);
+    k01 = k0s * s1;
+    k11 = k1s * s1;
+    be1 = bes * s1;
+    k02 = fma(k0ss * s1, s1, k0s * s2);
+    k12 = fma(k1ss * s1, s1, k1s * s2);
+    be2 = fma(bess * s1, s1, bes * s2);
+  }
+  // ---- modes and their rates
+  real t1[3], t2[3], d1[3], d2[3], m1[3], m2[3], w1[3], w2[3];
+  cross3(om, t, t1);
+  cross3(om1, t, t2);
+  cross3_add(1.0, om, t1, t2);
+  for (int i = 0; i < 3; ++i) {
+    d1[i] = 0.5 * (X1[6 + i] - X1[i]);
+    d2[i] = 0.5 * (X2[6 + i] - X2[i]);
+  }
+  const real xi = dot3(t, d), xi1 = dot3(t1, d) + dot3(t, d1),
+             xi2 = dot3(t2, d) + fma(2.0, dot3(t1, d1), dot3(t, d2));
+  for (int i = 0; i < 3; ++i) {
+    m1[i] = fma(xi1, t[i], xi * t1[i]);
+    m2[i] = fma(xi2, t[i], fma(2.0 * xi1, t1[i], xi * t2[i]));
+  }
+  cross3(n1, t, w1);
+  cross3_add(1.0, n, t1, w1);
+  cross3(n2, t, w2);
+  cross3_add(2.0, n1, t1, w2);
+  cross3_add(1.0, n, t2, w2);
+  const bool rot = c.iota1 != 0.0;
+  const bool drag = c.Ca[0] != 0.0 || c.Ca[1] != 0.0 || c.Ca[2] != 0.0 || c.Cl[0] != 0.0 || c.Cl[1] != 0.0 ||
+                    c.Cl[2] != 0.0 || c.Cq[0] != 0.0 || c.Cq[1] != 0.0 || c.Cq[2] != 0.0;
+  real yd[4], cv[3], ca[3];
+  for (int k = 0; k < 4; ++k) yd[k] = c.ya[k] - c.yu[k];
+  for (int i = 0; i < 3; ++i) {
+    cv[i] = 0.5 * (X1[i] + X1[6 + i]);
+    ca[i] = 0.5 * (X2[i] + X2[6 + i]);
+  }
+  auto point = [&](int k, real xd[3], real xdd[3]) {  // velocity and acceleration of Gauss point k
+    for (int i = 0; i < 3; ++i) {
+      xd[i] = fma(c.yu[k], d1[i], fma(yd[k], m1[i], fma(c.yv[k], w1[i], cv[i])));
+      xdd[i] = fma(c.yu[k], d2[i], fma(yd[k], m2[i], fma(c.yv[k], w2[i], ca[i])));
+    }
+  };
+  // ---- loads and their sums
+  const real vi = dot3(om1, t);  // vᵢ₂ of the rotational inertia: the spin acceleration about the axis
+  BeamLoads f;
+  for (int i = 0; i < 3; ++i) {
+    f.u[i] = f.a[i] = f.v[i] = f.o[i] = 0.0;
+    f.m[i] = rot ? c.S0 * c.iota1 * vi * t[i] : real(0.0);
+  }
+  for (int k = 0; k < 4; ++k) {
+    real xd[3], xdd[3];
+    point(k, xd, xdd);
+    real fe[3];
+    for (int i = 0; i < 3; ++i) fe[i] = fma(c.mu, xdd[i], (i == 2 ? c.w : 0.0) - (U ? U[i] : 0.0));
+    if (drag)
+      for (int i = 0; i < 3; ++i) {
+        const real x1 = dot3(g.rs + 3 * i, xd), x2 = dot3(g.rs + 3 * i, xdd);
+        axpy3(fma(c.Ca[i], x2, x1 * fma(c.Cq[i], fabs(x1), c.Cl[i])), g.rs + 3 * i, fe);
+      }
+    for (int i = 0; i < 3; ++i) {
+      const real w = c.dL[k] * fe[i];
+      f.u[i] = fma(c.yu[k], w, f.u[i]);
+      f.a[i] = fma(yd[k], w, f.a[i]);
+      f.v[i] = fma(c.yv[k], w, f.v[i]);
+      f.o[i] += w;
+    }
+  }
+  // ---- the symmetric part, packed by columns: (i, j), i <= j at i + j (j + 1)/2
+  real Ks[78];
+  beam_frozen<true>(c, X0, q1, q2, g, f, rot, X[0], X[1], R, [&](int i, int j, real v) { Ks[i + j * (j + 1) / 2] = pt.p0 * v; });
+  if (H) beam_uload(c, g, X[0], X[1], H);
+  // Dₛᵀ of vₛₘ: ∂vₛₘ = Dₛ ω, Dₛ = ι B − ι' q qᵀ, B = ½(tr I − rₛₘ)
+  real io[3] = {0.0, 0.0, 0.0}, vq[3], tau[3];
+  const real trs = g.rs[0] + g.rs[4] + g.rs[8];
+  if (rot) inv_scac2(0.5 * (trs - 1.0), io);
+  vq[0] = 0.5 * (g.rs[5] - g.rs[7]);
+  vq[1] = 0.5 * (g.rs[6] - g.rs[2]);
+  vq[2] = 0.5 * (g.rs[1] - g.rs[3]);
+  auto DsT = [&](const real y[3], real z[3]) {
+    const real qy = io[1] * dot3(vq, y);
+    for (int i = 0; i < 3; ++i) z[i] = fma(0.5 * io[0], fma(trs, y[i], -dot3(g.rs + 3 * i, y)), -(qy * vq[i]));
+  };
+  DsT(t, tau);
+  // Gram sums over (yᵤ, y_d, yᵥ, 1), with the mass
+  real Guu = 0.0, Gud = 0.0, Guv = 0.0, Gu = 0.0, Gdd = 0.0, Gdv = 0.0, Gd = 0.0, Gvv = 0.0, Gv = 0.0;
+  for (int k = 0; k < 4; ++k) {
+    const real l = c.mu * c.dL[k], lu = l * c.yu[k], ld = l * yd[k], lv = l * c.yv[k];
+    Guu = fma(lu, c.yu[k], Guu);
+    Gud = fma(lu, yd[k], Gud);
+    Guv = fma(lu, c.yv[k], Guv);
+    Gu += lu;
+    Gdd = fma(ld, yd[k], Gdd);
+    Gdv = fma(ld, c.yv[k], Gdv);
+    Gd += ld;
+    Gvv = fma(lv, c.yv[k], Gvv);
+    Gv += lv;
+  }
+  const real G1 = c.mu * c.S0;
+  // forces of a direction with drag, from the point's velocity and acceleration
+  // variation mk(k, V, A) and the spin sg of rₛₘ (nullptr: none)
+  auto dragsum = [&](auto&& mk, const real* sg, real Fu[3], real Fm[3], real Fv[3], real F1[3]) {
+    for (int i = 0; i < 3; ++i) Fu[i] = Fm[i] = Fv[i] = F1[i] = 0.0;
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) {
+      real xd[3], xdd[3], V[3], A[3], df[3];
+      point(k, xd, xdd);
+      mk(k, V, A);
+      for (int i = 0; i < 3; ++i) df[i] = c.mu * A[i];
+      if (sg) {
+        cross3_add(-1.0, sg, xd, V);
+        cross3_add(-1.0, sg, xdd, A);
+      }
+      for (int i = 0; i < 3; ++i) {
+        const real* col = g.rs + 3 * i;
+        const real x1 = dot3(col, xd);
+        real y = c.Ca[i] * dot3(col, A);
+        y = fma(fma(2.0 * c.Cq[i], fabs(x1), c.Cl[i]), dot3(col, V), y);
+        axpy3(y, col, df);
+        if (sg) {
+          const real fl = fma(c.Ca[i], dot3(col, xdd), x1 * fma(c.Cq[i], fabs(x1), c.Cl[i]));
+          cross3_add(fl, sg, col, df);
+        }
+      }
+      for (int i = 0; i < 3; ++i) {
+        const real w = c.dL[k] * df[i];
+        Fu[i] = fma(c.yu[k], w, Fu[i]);
+        Fm[i] = fma(yd[k], w, Fm[i]);
+        Fv[i] = fma(c.yv[k], w, Fv[i]);
+        F1[i] += w;
+      }
+    }
+  };
+  // rows of a column from its forces per mode and its couple rho on the spin:
+  // col[12], the translations' rows, and x·z of the rotations'
+  auto rows = [&](const real Fu[3], const real Fm[3], const real Fv[3], const real F1[3], const real rho[3], real col[12]) {
+    const real tF = dot3(t, Fm);
+    real y[3], la[3], cp[3], z[3], s[3];
+    for (int i = 0; i < 3; ++i) {
+      const real a = fma(tF, t[i], Fu[i]);
+      col[i] = 0.5 * (F1[i] - a);
+      col[6 + i] = 0.5 * (F1[i] + a);
+      y[i] = fma(tF, d[i], xi * Fm[i]);
+      la[i] = rho[i];
+    }
+    cross3_add(1.0, Fv, n, y);
+    cross3_add(1.0, t, y, la);
+    cross3(t, Fv, cp);
+    const real nc = k1 * dot3(n, cp);
+    for (int i = 0; i < 3; ++i) z[i] = fma(k0, cp[i], -(nc * n[i]));
+    cross3_add(be, la, n, z);
+    for (int a = 0; a < 2; ++a) {
+      for (int i = 0; i < 3; ++i) s[i] = fma(0.5, la[i], a ? z[i] : -z[i]);
+      for (int i = 0; i < 3; ++i) col[3 + 6 * a + i] = dot3(X[a] + 3 * i, s);
+    }
+  };
+  auto put = [&](int j, const real col[12]) {
+    for (int i = 0; i < 12; ++i) out(i, j, Ks[i <= j ? i + j * (j + 1) / 2 : j + i * (i + 1) / 2] + col[i]);
+  };
+  // sums of the rdir direction
+  real rVm[3] = {0, 0, 0}, rAm[3] = {0, 0, 0}, rVw[3] = {0, 0, 0}, rAw[3] = {0, 0, 0}, rvi = 0.0;
+  const real zero[3] = {0.0, 0.0, 0.0};
+  // ---- rotation columns
+  for (int a = 0; a < 2; ++a) {
+    const real sg = a ? 1.0 : -1.0;
+    for (int j = 0; j < 3; ++j) {
+      const real* x = X[a] + 3 * j;
+      const real* y1 = Xd[a] + 3 * j;
+      real x1[3], x2[3];  // ẋ, ẍ of the column: the frame turns with sp
+      for (int i = 0; i < 3; ++i) {
+        x1[i] = y1[i];
+        x2[i] = Xdd[a][3 * j + i];
+      }
+      cross3_add(1.0, sp[a], x, x1);
+      cross3_add(1.0, sp1[a], x, x2);
+      cross3_add(1.0, sp[a], x1, x2);
+      cross3_add(1.0, sp[a], y1, x2);
+      // spin σ = ½x ± β n×x and δn = ±(κ0 x − κ1 n (n·x)), with their rates
+      real s0[3], s1[3], s2[3], e0[3], e1[3], e2[3], z[3];
+      cross3(n, x, z);
+      for (int i = 0; i < 3; ++i) {
+        s0[i] = fma(sg * be, z[i], 0.5 * x[i]);
+        s1[i] = fma(sg * be1, z[i], 0.5 * x1[i]);
+        s2[i] = fma(sg * be2, z[i], 0.5 * x2[i]);
+      }
+      cross3(n1, x, z);
+      cross3_add(1.0, n, x1, z);  // (n×x)˙
+      axpy3(sg * be, z, s1);
+      axpy3(2.0 * sg * be1, z, s2);
+      cross3(n2, x, z);
+      cross3_add(2.0, n1, x1, z);
+      cross3_add(1.0, n, x2, z);
+      axpy3(sg * be, z, s2);
+      const real h0 = dot3(n, x), h1 = dot3(n1, x) + dot3(n, x1),
+                 h2 = dot3(n2, x) + fma(2.0, dot3(n1, x1), dot3(n, x2));
+      const real p0_ = k1 * h0, p1_ = fma(k11, h0, k1 * h1), p2_ = fma(k12, h0, fma(2.0 * k11, h1, k1 * h2));
+      for (int i = 0; i < 3; ++i) {
+        e0[i] = sg * fma(k0, x[i], -(p0_ * n[i]));
+        e1[i] = sg * (fma(k01, x[i], k0 * x1[i]) - fma(p1_, n[i], p0_ * n1[i]));
+        e2[i] = sg * (fma(k02, x[i], fma(2.0 * k01, x1[i], k0 * x2[i])) - fma(p2_, n[i], fma(2.0 * p1_, n1[i], p0_ * n2[i])));
+      }
+      if (g.s < 1e-28) {  // Rod(n) = I + S + S²/2 there (see tan_jets)
+        const real a2 = dot3(n1, n1) * (1.0 / 3.0), b2 = dot3(n1, e0) * (2.0 / 3.0);
+        for (int i = 0; i < 3; ++i) s2[i] += fma(a2, e0[i], b2 * n1[i]);
+      }
+      // m and w: Jacobian column and its rates
+      real jt[3], jt1[3], jt2[3], jm[3], jm1[3], jm2[3], jw[3], jw1[3], jw2[3];
+      cross3(s0, t, jt);
+      cross3(s1, t, jt1);
+      cross3_add(1.0, s0, t1, jt1);
+      cross3(s2, t, jt2);
+      cross3_add(2.0, s1, t1, jt2);
+      cross3_add(1.0, s0, t2, jt2);
+      const real u0 = dot3(jt, d), u1 = dot3(jt1, d) + dot3(jt, d1),
+                 u2 = dot3(jt2, d) + fma(2.0, dot3(jt1, d1), dot3(jt, d2));
+      for (int i = 0; i < 3; ++i) {
+        jm[i] = fma(u0, t[i], xi * jt[i]);
+        jm1[i] = fma(u1, t[i], fma(u0, t1[i], fma(xi1, jt[i], xi * jt1[i])));
+        jm2[i] = fma(u2, t[i], fma(2.0 * u1, t1[i], fma(u0, t2[i], fma(xi2, jt[i], fma(2.0 * xi1, jt1[i], xi * jt2[i])))));
+      }
+      cross3(e0, t, jw);
+      cross3_add(1.0, n, jt, jw);
+      cross3(e1, t, jw1);
+      cross3_add(1.0, e0, t1, jw1);
+      cross3_add(1.0, n1, jt, jw1);
+      cross3_add(1.0, n, jt1, jw1);
+      cross3(e2, t, jw2);
+      cross3_add(2.0, e1, t1, jw2);
+      cross3_add(1.0, e0, t2, jw2);
+      cross3_add(1.0, n2, jt, jw2);
+      cross3_add(2.0, n1, jt1, jw2);
+      cross3_add(1.0, n, jt2, jw2);
+      const real ts0 = dot3(t, s0), ts1 = fma(2.0, dot3(t, s1), dot3(t1, s0));
+      if (rdir) {
+        const real aj = av[3 + 6 * a + j], bj = bv[3 + 6 * a + j];
+        axpy3(aj, jm, rVm);
+        axpy3(2.0 * aj, jm1, rAm);
+        axpy3(bj, jm, rAm);
+        axpy3(aj, jw, rVw);
+        axpy3(2.0 * aj, jw1, rAw);
+        axpy3(bj, jw, rAw);
+        rvi = fma(aj, ts1, fma(bj, ts0, rvi));
+      }
+      real Am[3], Aw[3], Fu[3], Fm[3], Fv[3], F1[3], rho[3] = {0.0, 0.0, 0.0}, col[12];
+      for (int i = 0; i < 3; ++i) {
+        Am[i] = fma(pt.p0, jm2[i], fma(2.0 * pt.p1, jm1[i], pt.p2 * jm[i]));
+        Aw[i] = fma(pt.p0, jw2[i], fma(2.0 * pt.p1, jw1[i], pt.p2 * jw[i]));
+      }
+      if (drag) {
+        real Vm[3], Vw[3];
+        const real s[3] = {pt.p0 * s0[0], pt.p0 * s0[1], pt.p0 * s0[2]};
+        for (int i = 0; i < 3; ++i) {
+          Vm[i] = fma(pt.p0, jm1[i], pt.p1 * jm[i]);
+          Vw[i] = fma(pt.p0, jw1[i], pt.p1 * jw[i]);
+        }
+        dragsum(
+            [&](int k, real V[3], real A[3]) {
+              for (int i = 0; i < 3; ++i) {
+                V[i] = fma(yd[k], Vm[i], c.yv[k] * Vw[i]);
+                A[i] = fma(yd[k], Am[i], c.yv[k] * Aw[i]);
+              }
+            },
+            s, Fu, Fm, Fv, F1);
+      } else {
+        for (int i = 0; i < 3; ++i) {
+          Fu[i] = fma(Gud, Am[i], Guv * Aw[i]);
+          Fm[i] = fma(Gdd, Am[i], Gdv * Aw[i]);
+          Fv[i] = fma(Gdv, Am[i], Gvv * Aw[i]);
+          F1[i] = fma(Gd, Am[i], Gv * Aw[i]);
+        }
+      }
+      if (rot) {  // δmₑ = ι₁ (δvᵢ t + vᵢ δt), δvᵢ = p0 (t·σ̈ + ṫ·σ̇) + p1 (2 t·σ̇ + ṫ·σ) + p2 t·σ
+        const real dv = fma(pt.p0, dot3(t, s2) + dot3(t1, s1), fma(pt.p1, ts1, pt.p2 * ts0));
+        const real sc = c.S0 * c.iota1;
+        DsT(jt, z);
+        for (int i = 0; i < 3; ++i) rho[i] = sc * fma(dv, tau[i], pt.p0 * vi * z[i]);
+      }
+      rows(Fu, Fm, Fv, F1, rho, col);
+      put(3 + 6 * a + j, col);
+    }
+  }
+  // ---- translation columns: d moves by ∓½, the midpoint by ½
+  for (int j = 0; j < 3; ++j) {
+    real Am[3], Fu[3], Fm[3], Fv[3], F1[3], c1[12], c2[12], ca_[12], cb_[12];
+    for (int i = 0; i < 3; ++i) {
+      const real M = t[i] * t[j], M1 = fma(t1[i], t[j], t[i] * t1[j]),
+                 M2 = fma(t2[i], t[j], fma(2.0 * t1[i], t1[j], t[i] * t2[j]));
+      Am[i] = fma(pt.p0, M2, fma(2.0 * pt.p1, M1, pt.p2 * M));
+    }
+    if (rdir) {
+      const real aj = 0.5 * (av[6 + j] - av[j]), bj = 0.5 * (bv[6 + j] - bv[j]);
+      for (int i = 0; i < 3; ++i) {
+        rVm[i] = fma(aj * t[j], t[i], rVm[i]);
+        rAm[i] = fma(2.0 * aj, fma(t1[i], t[j], t[i] * t1[j]), fma(bj * t[j], t[i], rAm[i]));
+      }
+    }
+    if (drag) {
+      dragsum(
+          [&](int k, real V[3], real A[3]) {
+            for (int i = 0; i < 3; ++i) {
+              const real M = t[i] * t[j], M1 = fma(t1[i], t[j], t[i] * t1[j]);
+              V[i] = yd[k] * fma(pt.p0, M1, pt.p1 * M);
+              A[i] = yd[k] * Am[i];
+              if (i == j) {
+                V[i] = fma(c.yu[k], pt.p1, V[i]);
+                A[i] = fma(c.yu[k], pt.p2, A[i]);
+              }
+            }
+          },
+          nullptr, Fu, Fm, Fv, F1);
+      rows(Fu, Fm, Fv, F1, zero, c1);
+      dragsum(
+          [&](int, real V[3], real A[3]) {
+            for (int i = 0; i < 3; ++i) {
+              V[i] = i == j ? pt.p1 : 0.0;
+              A[i] = i == j ? pt.p2 : 0.0;
+            }
+          },
+          nullptr, Fu, Fm, Fv, F1);
+    } else {
+      for (int i = 0; i < 3; ++i) {
+        const real A = i == j ? pt.p2 : 0.0;
+        Fu[i] = fma(Gud, Am[i], Guu * A);
+        Fm[i] = fma(Gdd, Am[i], Gud * A);
+        Fv[i] = fma(Gdv, Am[i], Guv * A);
+        F1[i] = fma(Gd, Am[i], Gu * A);
+      }
+      rows(Fu, Fm, Fv, F1, zero, c1);
+      for (int i = 0; i < 3; ++i) {
+        const real A = i == j ? pt.p2 : 0.0;
+        Fu[i] = Gu * A;
+        Fm[i] = Gd * A;
+        Fv[i] = Gv * A;
+        F1[i] = G1 * A;
+      }
+    }
+    rows(Fu, Fm, Fv, F1, zero, c2);
+    for (int i = 0; i < 12; ++i) {
+      ca_[i] = 0.5 * (c2[i] - c1[i]);
+      cb_[i] = 0.5 * (c2[i] + c1[i]);
+    }
+    put(j, ca_);
+    put(6 + j, cb_);
+  }
+  // ---- the direction X′ += av, X″ += bv
+  if (rdir) {
+    real Fu[3], Fm[3], Fv[3], F1[3], col[12], rho[3], dv1[3], dv2[3], cv1[3], cv2[3];
+    for (int i = 0; i < 3; ++i) {
+      dv1[i] = 0.5 * (av[6 + i] - av[i]);
+      dv2[i] = 0.5 * (bv[6 + i] - bv[i]);
+      cv1[i] = 0.5 * (av[i] + av[6 + i]);
+      cv2[i] = 0.5 * (bv[i] + bv[6 + i]);
+      rho[i] = rot ? c.S0 * c.iota1 * rvi * tau[i] : real(0.0);
+    }
+    if (drag) {
+      dragsum(
+          [&](int k, real V[3], real A[3]) {
+            for (int i = 0; i < 3; ++i) {
+              V[i] = fma(c.yu[k], dv1[i], fma(yd[k], rVm[i], fma(c.yv[k], rVw[i], cv1[i])));
+              A[i] = fma(c.yu[k], dv2[i], fma(yd[k], rAm[i], fma(c.yv[k], rAw[i], cv2[i])));
+            }
+          },
+          nullptr, Fu, Fm, Fv, F1);
+    } else {
+      for (int i = 0; i < 3; ++i) {
+        Fu[i] = fma(Guu, dv2[i], fma(Gud, rAm[i], fma(Guv, rAw[i], Gu * cv2[i])));
+        Fm[i] = fma(Gud, dv2[i], fma(Gdd, rAm[i], fma(Gdv, rAw[i], Gd * cv2[i])));
+        Fv[i] = fma(Guv, dv2[i], fma(Gdv, rAm[i], fma(Gvv, rAw[i], Gv * cv2[i])));
+        F1[i] = fma(Gu, dv2[i], fma(Gd, rAm[i], fma(Gv, rAw[i], G1 * cv2[i])));
+      }
+    }
+    rows(Fu, Fm, Fv, F1, rho, col);
+    for (int i = 0; i < 12; ++i) rdir[i] = to_d(col[i]);
+  }
 }
 
 }  // namespace mgpu

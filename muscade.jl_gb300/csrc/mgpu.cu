@@ -138,8 +138,9 @@ __global__ void __launch_bounds__(256) beam_static_kernel(int64_t nele, const in
   flag_nan(a.errflag, gid0 + e, bad);
 }
 
-// SweepX{2}; the same launch sizes, and the bound of 256 leaves the register
-// cap at 255.
+// SweepX{2}; the same launch sizes.  STEP: a step's first iteration, with the
+// residual's part along the Newmark vectors a and b taken off.
+template <bool STEP>
 __global__ void __launch_bounds__(256) beam_kernel(int64_t nele, const int32_t* __restrict__ idx,
                                                    const int32_t* __restrict__ uidx, const double* __restrict__ cdata,
                                                    const int32_t* __restrict__ aidx, const double* __restrict__ Avec,
@@ -150,48 +151,41 @@ __global__ void __launch_bounds__(256) beam_kernel(int64_t nele, const int32_t* 
   BeamConst bc;
   load_soa(bc, cdata, nele, e);
   if (aidx) scale_bending(bc, __ldg(Avec + __ldg(aidx + e)));
-  int dof[12];
-  double X0[12], X1[12], X2[12], av[12], bv[12];
+  double X0[12], X1[12], X2[12], av[12], bv[12], s[12];
+  const bool scaled = a.scale != nullptr;
 #pragma unroll
   for (int i = 0; i < 12; ++i) {
-    dof[i] = __ldg(idx + i * nele + e);
-    X0[i] = __ldg(a.x0 + dof[i]);
-    {
-      X1[i] = __ldg(a.x1 + dof[i]);
-      X2[i] = __ldg(a.x2 + dof[i]);
-      if (a.mission == MGPU_ASM_STEP) {
-        av[i] = __ldg(a.av + dof[i]);
-        bv[i] = __ldg(a.bv + dof[i]);
-      }
+    const int dof = __ldg(idx + i * nele + e);
+    X0[i] = __ldg(a.x0 + dof);
+    X1[i] = __ldg(a.x1 + dof);
+    X2[i] = __ldg(a.x2 + dof);
+    if constexpr (STEP) {
+      av[i] = __ldg(a.av + dof);
+      bv[i] = __ldg(a.bv + dof);
     }
+    if (scaled) s[i] = __ldg(a.scale + dof);
   }
   double U[3];
   const bool has_u = uidx != nullptr;
   if (has_u)
 #pragma unroll
     for (int k = 0; k < 3; ++k) U[k] = __ldg(a.u + __ldg(uidx + k * nele + e));
-  double R[12], K[144], rd[12];
-  const bool step = a.mission == MGPU_ASM_STEP;
+  double R[12], rd[12];
   const Perturb pt{a.p0, a.sc[1], a.sc[4]};  // K + a1 C + b1 M
-  beam_element<true>(bc, X0, X1, X2, has_u ? U : nullptr, pt, av, bv, R, K, step ? rd : nullptr, nullptr);
-  double s[12];
-#pragma unroll
-  for (int i = 0; i < 12; ++i) s[i] = a.scale ? __ldg(a.scale + dof[i]) : 1.0;
   bool bad = false;
+  auto store = [&](int i, int j, double v) {
+    if (scaled) v *= s[i] * s[j];
+    bad |= nan_bits(v);
+    kout[(i + 12 * j) * nele + e] = v;
+  };
+  beam_newmark(bc, X0, X1, X2, has_u ? U : nullptr, pt, av, bv, R, store, STEP ? rd : nullptr, nullptr);
 #pragma unroll
   for (int i = 0; i < 12; ++i) {
-    const double r = (step ? R[i] - rd[i] : R[i]) * s[i];
-    bad |= isnan(r);
+    double r = STEP ? R[i] - rd[i] : R[i];
+    if (scaled) r *= s[i];
+    bad |= nan_bits(r);
     rout[i * nele + e] = r;
   }
-#pragma unroll
-  for (int j = 0; j < 12; ++j)
-#pragma unroll
-    for (int i = 0; i < 12; ++i) {
-      const double k = K[i + 12 * j] * s[i] * s[j];
-      bad |= isnan(k);
-      kout[(i + 12 * j) * nele + e] = k;
-    }
   flag_nan(a.errflag, gid0 + e, bad);
 }
 
@@ -502,8 +496,11 @@ int launch_assembly(mgpu_ctx* c, int mission, cudaEvent_t* ev_groups, double p0)
     if (G.tval_base >= 0) ag.tv = c->tv + G.tval_base;
     switch (G.kind) {
       case MGPU_EULERBEAM3D:
-        if (dyn)
-          beam_kernel<<<nblk(G.nele, c->elem_block), c->elem_block, 0, c->stream>>>(
+        if (mission == MGPU_ASM_STEP)
+          beam_kernel<true><<<nblk(G.nele, c->elem_block), c->elem_block, 0, c->stream>>>(
+              G.nele, G.idx, G.uidx, G.cdata, G.aidx, c->Avec, ag, rout, kout, gid0);
+        else if (dyn)
+          beam_kernel<false><<<nblk(G.nele, c->elem_block), c->elem_block, 0, c->stream>>>(
               G.nele, G.idx, G.uidx, G.cdata, G.aidx, c->Avec, ag, rout, kout, gid0);
         else if (ag.scale || p0 != 1.0)
           beam_static_kernel<true><<<nblk(G.nele, c->elem_block), c->elem_block, 0, c->stream>>>(
