@@ -24,6 +24,7 @@
 #include <string>
 #include <vector>
 
+#include "band_block.cuh"
 #include "band_rows.cuh"
 #include "ctx.hpp"
 #include "solver.hpp"
@@ -32,6 +33,21 @@ using namespace mgpu;
 
 namespace mgpu {
 
+
+// whether the device schedules clusters of more than 8 blocks of band_lu
+static bool cluster_fits(int cl) {
+  if (cudaFuncSetAttribute(band_lu, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return false;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim = {unsigned(cl), 1, 1};
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(cl));
+  cfg.blockDim = dim3(kBlkThreads);
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int m = 0;
+  return cudaOccupancyMaxActiveClusters(&m, band_lu, &cfg) == cudaSuccess && m > 0;
+}
 
 // ---------------------------------------------------------------- host analysis
 static void analyse(mgpu_ctx* c, Solver& S) {
@@ -519,142 +535,23 @@ static void analyse(mgpu_ctx* c, Solver& S) {
     S.why = "device allocation failed for the solver";
     return;
   }
+  // blocks per component of the block kernels: as many (a power of two, up to 16) as
+  // leave each its own SM, one where the panels are too low to share (a 6 x 5 x 4
+  // frame of band 143: see band_block.cuh)
+  int nsm = 152;
+  if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess) nsm = 152;
+  S.blkc = 1;
+  while (S.blkc < 16 && 2 * S.blkc * ncomp <= nsm && 16 * S.blkc <= S.maxkl) S.blkc *= 2;
+  if (S.blkc > 8 && !cluster_fits(S.blkc)) S.blkc = 8;
+  if (cudaFuncSetAttribute(band_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           int(band_solve_smem(kBlkMaxBand, 2 * kBlkMaxBand))) != cudaSuccess) {
+    S.why = "the block solver's shared memory is not available";
+    return;
+  }
   S.ok = true;
 }
 
 // ---------------------------------------------------------------- kernels
-__global__ void band_gather(int64_t nnz, const int64_t* __restrict__ bmap, const double* __restrict__ nzval,
-                            double* __restrict__ AB) {
-  const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k < nnz) AB[bmap[k]] = nzval[k];
-}
-
-// Banded LU with partial pivoting (LAPACK gbtf2 algorithm), one block per
-// component.  Also writes the reciprocal pivots, which the backward
-// substitution multiplies by (gbtrs divides; the results differ by rounding).
-__global__ void __launch_bounds__(128) band_lu(const int64_t* cbase, const int32_t* cn, const int32_t* ckl,
-                                               const int32_t* cku, const int32_t* cdof0, double* AB, int32_t* ipiv,
-                                               double* rdg, int* info) {
-  const int cc = blockIdx.x;
-  const int n = cn[cc], kl = ckl[cc], ku = cku[cc];
-  const int kv = kl + ku, ld = 2 * kl + ku + 1;
-  double* A = AB + cbase[cc];
-  int32_t* piv = ipiv + cdof0[cc];
-  double* rdiag = rdg + cdof0[cc];  // reciprocal pivots for the backward substitution
-  __shared__ double sval[128];
-  __shared__ int sidx[128];
-  __shared__ int s_jp, s_ju;
-  __shared__ double s_piv;
-  if (threadIdx.x == 0) s_ju = 0;
-  __syncthreads();
-  for (int k = 0; k < n; ++k) {
-    const int km = min(kl, n - 1 - k);
-    // pivot search over rows k..k+km of column k (first index of max |a|)
-    double best = -1.0;
-    int bi = 0;
-    for (int i = threadIdx.x; i <= km; i += blockDim.x) {
-      const double v = fabs(A[kv + i + int64_t(ld) * k]);
-      if (v > best) {
-        best = v;
-        bi = i;
-      }
-    }
-    sval[threadIdx.x] = best;
-    sidx[threadIdx.x] = bi;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-      if (threadIdx.x < s) {
-        const double v2 = sval[threadIdx.x + s];
-        const int i2 = sidx[threadIdx.x + s];
-        if (v2 > sval[threadIdx.x] || (v2 == sval[threadIdx.x] && i2 < sidx[threadIdx.x])) {
-          sval[threadIdx.x] = v2;
-          sidx[threadIdx.x] = i2;
-        }
-      }
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-      const int jp = sidx[0];
-      s_jp = jp;
-      piv[k] = k + jp;
-      const double p = A[kv + jp + int64_t(ld) * k];
-      s_piv = p;
-      if (p == 0.0 && *info == 0) atomicCAS(info, 0, cc + 1);
-      rdiag[k] = 1.0 / p;
-      s_ju = max(s_ju, min(k + ku + jp, n - 1));
-    }
-    __syncthreads();
-    const int jp = s_jp, ju = s_ju;
-    const double p = s_piv;
-    if (p != 0.0) {
-      // swap rows k and k+jp in columns k..ju
-      if (jp != 0)
-        for (int j = k + threadIdx.x; j <= ju; j += blockDim.x) {
-          double* a = A + kv + (k - j) + int64_t(ld) * j;
-          double* b = A + kv + (k + jp - j) + int64_t(ld) * j;
-          const double t = *a;
-          *a = *b;
-          *b = t;
-        }
-      __syncthreads();
-      // multipliers (scaled by the reciprocal pivot, like gbtf2)
-      const double rp = 1.0 / p;
-      for (int i = 1 + threadIdx.x; i <= km; i += blockDim.x) A[kv + i + int64_t(ld) * k] *= rp;
-      __syncthreads();
-      // rank-1 update of columns k+1..ju, rows k+1..k+km
-      const int w = ju - k;
-      const int tot = w * km;
-      for (int q = threadIdx.x; q < tot; q += blockDim.x) {
-        const int jj = q / km + 1, i = q % km + 1;
-        const int j = k + jj;
-        const double u = A[kv - jj + int64_t(ld) * j];  // row k of column j
-        if (u != 0.0) A[kv + i - jj + int64_t(ld) * j] -= A[kv + i + int64_t(ld) * k] * u;
-      }
-    }
-    __syncthreads();
-  }
-}
-
-// Solve with the band factors: permute, L with interchanges, U; one block per component.
-__global__ void __launch_bounds__(128) band_solve(const int64_t* cbase, const int32_t* cn, const int32_t* ckl,
-                                                  const int32_t* cku, const int32_t* cdof0, const int32_t* perm,
-                                                  const double* AB, const int32_t* ipiv, const double* rdg,
-                                                  const double* Ll, double* rhs, double* dx) {
-  const int cc = blockIdx.x;
-  const int n = cn[cc], kl = ckl[cc], ku = cku[cc];
-  const int kv = kl + ku, ld = 2 * kl + ku + 1;
-  const double* A = AB + cbase[cc];
-  const int32_t* piv = ipiv + cdof0[cc];
-  const int32_t* pm = perm + cdof0[cc];
-  double* b = rhs + cdof0[cc];
-  for (int k = threadIdx.x; k < n; k += blockDim.x) b[k] = Ll[pm[k]];
-  __syncthreads();
-  // forward: L y = P b
-  for (int k = 0; k < n; ++k) {
-    const int km = min(kl, n - 1 - k);
-    const int p = piv[k];
-    if (threadIdx.x == 0 && p != k) {
-      const double t = b[k];
-      b[k] = b[p];
-      b[p] = t;
-    }
-    __syncthreads();
-    const double bk = b[k];
-    for (int i = 1 + threadIdx.x; i <= km; i += blockDim.x) b[k + i] -= A[kv + i + int64_t(ld) * k] * bk;
-    __syncthreads();
-  }
-  // backward: U x = y  (U has kl+ku superdiagonals)
-  for (int k = n - 1; k >= 0; --k) {
-    if (threadIdx.x == 0) b[k] *= rdg[cdof0[cc] + k];  // reciprocal pivot from band_lu
-    __syncthreads();
-    const double bk = b[k];
-    const int m = min(kv, k);
-    for (int i = 1 + threadIdx.x; i <= m; i += blockDim.x) b[k - i] -= A[kv - i + int64_t(ld) * k] * bk;
-    __syncthreads();
-  }
-  for (int k = threadIdx.x; k < n; k += blockDim.x) dx[pm[k]] = b[k];
-}
-
 // Σ Δx², Σ Lλ²: kNormBlocks partial sums (fixed assignment and tree order), then
 // one block adds the partials in index order -- deterministic for a given n
 __global__ void __launch_bounds__(256) norms_partial(int64_t n, const double* dx, const double* Ll, double* part) {
@@ -1248,9 +1145,19 @@ int factor_solve(mgpu_ctx* c, int* info) {
   } else if (S.path == PATH_BLOCK) {
     MG_CUDA(cudaMemsetAsync(S.AB, 0, S.band_total * sizeof(double), st));
     band_gather<<<nb(c->pat.nnz, 256), 256, 0, st>>>(c->pat.nnz, S.bmap, c->nzval, S.AB);
-    band_lu<<<S.ncomp, 128, 0, st>>>(S.cbase, S.cn, S.ckl, S.cku, S.cdof0, S.AB, S.ipiv, S.rdiag, info);
-    band_solve<<<S.ncomp, 128, 0, st>>>(S.cbase, S.cn, S.ckl, S.cku, S.cdof0, S.perm, S.AB, S.ipiv, S.rdiag, c->Ll,
-                                        S.rhs, S.dx);
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim = {unsigned(S.blkc), 1, 1};
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(unsigned(S.ncomp) * unsigned(S.blkc));
+    cfg.blockDim = dim3(kBlkThreads);
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    MG_CUDA(cudaLaunchKernelEx(&cfg, band_lu, (const int64_t*)S.cbase, (const int32_t*)S.cn, (const int32_t*)S.ckl,
+                               (const int32_t*)S.cku, (const int32_t*)S.cdof0, S.AB, S.ipiv, S.rdiag, info, S.blkc));
+    band_solve<<<S.ncomp, kBlkThreads, band_solve_smem(S.maxkl, S.maxkl + S.maxku), st>>>(
+        S.cbase, S.cn, S.ckl, S.cku, S.cdof0, S.perm, S.AB, S.ipiv, S.rdiag, c->Ll, S.rhs, S.dx);
   } else {
     // one warp per component, one per block, so that the components spread over all SMs
     const RbComp cp{S.rbase, S.lbase, S.cn, S.ckl, S.cku, S.cdof0};

@@ -110,6 +110,7 @@ struct Solver {
   int32_t* perm = nullptr;    // [nX] dofs of component c in band order: perm[cdof0[c] + k]
   int64_t* bmap = nullptr;    // [nnz] band position of each nnz
   double* AB = nullptr;       // band storage
+  int blkc = 1;               // blocks per component of the block factorisation (band_block.cuh)
   int32_t* ipiv = nullptr;    // [nX] pivot offsets (band order)
   double* rhs = nullptr;      // [nX] permuted right-hand side / solution
   double* rdiag = nullptr;    // [nX] reciprocal pivots (block kernels)
