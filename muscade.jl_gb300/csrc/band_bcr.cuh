@@ -19,12 +19,14 @@
 //
 // Storage (per separator k, global index; component offset sep0, local index
 // k - sep0; SS = 16 x 16 doubles per block whatever s):
-//   DLU[lvl][k] D, L, U of level lvl     FA[k]: LU factors of D at elimination, pivots PV[k]
+//   DLU[lvl][k] D, L, U of level lvl     FA[k]: LU factors of D at elimination (bcr_factor), PV[k]: the row at each pivoted place
 //   WL[k], WU[k]: D^-1 L and D^-1 U      rhs / z / x: vectors of N s entries per component
 #pragma once
 #include <cuda_runtime.h>
 
 #include <cstdint>
+
+#include "band_rows.cuh"
 
 namespace mgpu {
 
@@ -47,136 +49,130 @@ __device__ __forceinline__ int bcr_role(int kloc, int N, int l) {
   return ((kloc / h) & 1) ? 1 : 2;
 }
 
-// dense helpers, one warp; A row-major s x s with leading dimension BCR_S
-template <typename T>
-__device__ void bcr_lu(T* A, int* piv, int s, int lane, int* singular) {
-  for (int j = 0; j < s; ++j) {
-    // pivot: first largest |A[i][j]|, i >= j
-    T best = T(-1);
-    int bi = j;
-    for (int i = j; i < s; ++i) {
-      const T v = fabs(A[i * BCR_S + j]);
-      if (v > best) best = v, bi = i;
+// 1/pivot in the factors' type
+__device__ __forceinline__ double bcr_rcp(double p) { return rb_rcp(p); }
+__device__ __forceinline__ float bcr_rcp(float p) { return __frcp_rn(p); }
+
+// The dense work of one block, one warp, a matrix row per lane in registers:
+// what bounds it is the chain of s pivots and, in FP64, the instructions issued
+// (64 cycles each), so every step is one multiply-add per remaining column for all
+// rows at once and nothing goes through memory.  One chain of 490 separators, a level
+// (FP64): bcr_eliminate 58 -> 25 us (L and U sides on a warp each; blocks of 13 and
+// then 11), bcr_update 21 -> 6, bcr_fwd_elim 12.6 -> 3.2, against blocks in shared
+// memory, row by row, with divisions on the chain.
+//
+// LU with partial pivoting of d (ties to the first row), x <- d^-1 x for s columns.
+// Rows stay on their lanes: *pos is the place of the lane's row in the pivoted
+// order.  On return the row holds L left of the diagonal, 1/pivot on it and
+// U(i, j)/U(j, j) right of it.  Returns whether a pivot was zero.
+template <typename T, bool RHS>
+__device__ __forceinline__ bool bcr_factor(T d[BCR_S], T x[BCR_S], int s, int lane, int* pos_out) {
+  int pos = lane < s ? lane : (1 << 30);
+  T rpo = T(0);
+  bool singular = false;
+#pragma unroll
+  for (int j = 0; j < BCR_S; ++j) {
+    if (j >= s) break;
+    int pl;
+    const int jp = rb_argmax(d[j], pos >= j && pos < s, pos, &pl);
+    const T p = __shfl_sync(RB_FULL, d[j], pl);
+    if (lane == pl)
+      pos = j;
+    else if (pos == j)
+      pos = jp;
+    const bool zero = p == T(0);
+    singular = singular || zero;
+    const T rp = zero ? T(0) : bcr_rcp(p);
+    if (lane == pl) rpo = rp;
+    T l = T(0);
+    if (pos > j && pos < s && !zero) l = d[j] = d[j] * rp;
+#pragma unroll
+    for (int c = j + 1; c < BCR_S; ++c) {
+      if (c >= s) break;
+      d[c] = fma(-l, __shfl_sync(RB_FULL, d[c], pl), d[c]);
     }
-    if (lane == 0) piv[j] = bi;
-    if (bi != j)
-      for (int c = lane; c < s; c += 32) {
-        const T t = A[j * BCR_S + c];
-        A[j * BCR_S + c] = A[bi * BCR_S + c];
-        A[bi * BCR_S + c] = t;
+    if constexpr (RHS)
+#pragma unroll
+      for (int c = 0; c < BCR_S; ++c) {
+        if (c >= s) break;
+        x[c] = fma(-l, __shfl_sync(RB_FULL, x[c], pl), x[c]);
       }
-    __syncwarp();
-    const T p = A[j * BCR_S + j];
-    if (p == T(0)) {
-      if (lane == 0) *singular = 1;
-      continue;
-    }
-    const T rp = T(1) / p;
-    for (int i = j + 1 + lane; i < s; i += 32) A[i * BCR_S + j] *= rp;
-    __syncwarp();
-    const int m = s - j - 1;
-    for (int e = lane; e < m * m; e += 32) {
-      const int i = j + 1 + e / m, c = j + 1 + e % m;
-      A[i * BCR_S + c] = fma(-A[i * BCR_S + j], A[j * BCR_S + c], A[i * BCR_S + c]);
-    }
-    __syncwarp();
   }
-}
-
-// B (s x nrhs, row-major, ld BCR_S) <- (LU)^-1 P B; lanes over right-hand sides
-template <typename T>
-__device__ void bcr_lu_solve(const T* F, const int* piv, T* B, int s, int nrhs, int lane) {
-  for (int r = lane; r < nrhs; r += 32) {
-    for (int j = 0; j < s; ++j)
-      if (piv[j] != j) {
-        const T t = B[j * BCR_S + r];
-        B[j * BCR_S + r] = B[piv[j] * BCR_S + r];
-        B[piv[j] * BCR_S + r] = t;
+#pragma unroll
+  for (int j = BCR_S - 1; j >= 0; --j) {
+    if (j >= s) continue;
+    const int pl = __ffs(__ballot_sync(RB_FULL, pos == j)) - 1;
+    const T rp = __shfl_sync(RB_FULL, rpo, pl);
+    T e = T(0);
+    if (pos < j) e = d[j] = d[j] * rp;
+    if (pos == j) d[j] = rpo;
+    if constexpr (RHS)
+#pragma unroll
+      for (int c = 0; c < BCR_S; ++c) {
+        if (c >= s) break;
+        x[c] = fma(-e, __shfl_sync(RB_FULL, x[c], pl), x[c]);
       }
-    for (int i = 1; i < s; ++i) {
-      T v = B[i * BCR_S + r];
-      for (int j = 0; j < i; ++j) v = fma(-F[i * BCR_S + j], B[j * BCR_S + r], v);
-      B[i * BCR_S + r] = v;
-    }
-    for (int i = s - 1; i >= 0; --i) {
-      T v = B[i * BCR_S + r];
-      for (int j = i + 1; j < s; ++j) v = fma(-F[i * BCR_S + j], B[j * BCR_S + r], v);
-      B[i * BCR_S + r] = v / F[i * BCR_S + i];
-    }
   }
-  __syncwarp();
+  if constexpr (RHS)
+#pragma unroll
+    for (int c = 0; c < BCR_S; ++c) x[c] *= rpo;
+  *pos_out = pos;
+  return singular;
+}
+template <typename T>
+__device__ __forceinline__ void bcr_row_load(T v[BCR_S], const T* M, int s, int row) {
+#pragma unroll
+  for (int c = 0; c < BCR_S; ++c) v[c] = (row < s && c < s) ? M[row * BCR_S + c] : T(0);
+}
+template <typename T>
+__device__ __forceinline__ void bcr_row_store(const T v[BCR_S], T* M, int s, int row) {
+  if (row < s)
+#pragma unroll
+    for (int c = 0; c < BCR_S; ++c)
+      if (c < s) M[row * BCR_S + c] = v[c];
 }
 
-// C (+)= alpha * A B, s x s, lanes over entries of C
+// level l, eliminated blocks: factor D_k, W_L = D^-1 L (first warp), W_U = D^-1 U (second)
 template <typename T>
-__device__ void bcr_gemm(const T* A, const T* B, T* C, int s, T alpha, bool accumulate, int lane) {
-  for (int e = lane; e < s * s; e += 32) {
-    const int i = e / s, j = e % s;
-    T v = T(0);
-    for (int q = 0; q < s; ++q) v = fma(A[i * BCR_S + q], B[q * BCR_S + j], v);
-    C[i * BCR_S + j] = accumulate ? fma(alpha, v, C[i * BCR_S + j]) : alpha * v;
-  }
-  __syncwarp();
-}
-
-// level l, eliminated blocks: factor D_k, W_L = D^-1 L, W_U = D^-1 U
-template <typename T>
-__global__ void __launch_bounds__(32) bcr_eliminate(int nsep, const BcrSep* __restrict__ bs, int l,
+__global__ void __launch_bounds__(64) bcr_eliminate(int nsep, const BcrSep* __restrict__ bs, int l,
                                                     const T* __restrict__ DLU, T* __restrict__ FA,
                                                     int* __restrict__ PV, T* __restrict__ WL, T* __restrict__ WU,
                                                     const int* __restrict__ only, int* __restrict__ info) {
-  __shared__ T sA[BCR_SS];
-  __shared__ T sB[BCR_S * BCR_S * 2];
-  __shared__ int sp[BCR_S];
-  __shared__ int sing;
-  const int k = blockIdx.x, lane = threadIdx.x;
+  const int k = blockIdx.x, lane = threadIdx.x & 31, side = threadIdx.x >> 5;
   if (k >= nsep) return;
   const BcrSep B = bs[k];
   if (only && only[B.comp] == 0) return;
   const int role = l < B.nlev ? bcr_role(B.kloc, B.N, l) : 0;
   if (role != 1) return;
   const int s = B.s, h = 1 << l;
-  const int64_t lvl = int64_t(l) * nsep * 3;
-  const T* D = DLU + (lvl + 3 * int64_t(k)) * BCR_SS;
-  for (int e = lane; e < BCR_SS; e += 32) sA[e] = D[e];
-  // right-hand sides [L | U] side by side in sB (row-major, ld BCR_S, columns 0..s-1 L, the next s U)
-  const bool hasU = B.kloc + h < B.N;
-  for (int e = lane; e < s * s; e += 32) {
-    const int i = e / s, j = e % s;
-    sB[i * BCR_S + j] = D[BCR_SS + i * BCR_S + j];  // L
+  const T* D = DLU + (int64_t(l) * nsep * 3 + 3 * int64_t(k)) * BCR_SS;
+  T* W = (side ? WU : WL) + int64_t(k) * BCR_SS;
+  T d[BCR_S], x[BCR_S];
+  if (side && B.kloc + h >= B.N) {  // no block above
+#pragma unroll
+    for (int c = 0; c < BCR_S; ++c) x[c] = T(0);
+    bcr_row_store(x, W, s, lane);
+    return;
   }
-  if (lane == 0) sing = 0;
-  __syncwarp();
-  bcr_lu(sA, sp, s, lane, &sing);
-  bcr_lu_solve(sA, sp, sB, s, s, lane);
-  T* wl = WL + int64_t(k) * BCR_SS;
-  for (int e = lane; e < BCR_SS; e += 32) wl[e] = sB[e];
-  __syncwarp();
-  T* wu = WU + int64_t(k) * BCR_SS;
-  if (hasU) {
-    for (int e = lane; e < s * s; e += 32) {
-      const int i = e / s, j = e % s;
-      sB[i * BCR_S + j] = D[2 * BCR_SS + i * BCR_S + j];  // U
-    }
-    __syncwarp();
-    bcr_lu_solve(sA, sp, sB, s, s, lane);
-    for (int e = lane; e < BCR_SS; e += 32) wu[e] = sB[e];
-  } else {
-    for (int e = lane; e < BCR_SS; e += 32) wu[e] = T(0);
-  }
-  T* fa = FA + int64_t(k) * BCR_SS;
-  for (int e = lane; e < BCR_SS; e += 32) fa[e] = sA[e];
-  if (lane < s) PV[int64_t(k) * BCR_S + lane] = sp[lane];
+  bcr_row_load(d, D, s, lane);
+  bcr_row_load(x, D + (1 + side) * BCR_SS, s, lane);
+  int pos;
+  const bool sing = bcr_factor<T, true>(d, x, s, lane, &pos);
+  bcr_row_store(x, W, s, pos);
+  if (side) return;
+  bcr_row_store(d, FA + int64_t(k) * BCR_SS, s, pos);
+  if (lane < s) PV[int64_t(k) * BCR_S + pos] = lane;
   if (lane == 0 && sing && info) atomicCAS(info, 0, B.comp + 1);
 }
 
-// level l, kept blocks: D, L, U of level l+1
+// level l, kept blocks: D' = D - U W_L(k+h) - L W_U(k-h), U' = -U W_U(k+h), L' = -L W_L(k-h)
+// into level l + 1.  The six blocks in shared memory, a thread per two entries.
 template <typename T>
-__global__ void __launch_bounds__(32) bcr_update(int nsep, const BcrSep* __restrict__ bs, int l, T* __restrict__ DLU,
-                                                 const T* __restrict__ WL, const T* __restrict__ WU,
-                                                 const int* __restrict__ only) {
-  __shared__ T sD[BCR_SS], sL[BCR_SS], sU[BCR_SS];
-  const int k = blockIdx.x, lane = threadIdx.x;
+__global__ void __launch_bounds__(128) bcr_update(int nsep, const BcrSep* __restrict__ bs, int l, T* __restrict__ DLU,
+                                                  const T* __restrict__ WL, const T* __restrict__ WU,
+                                                  const int* __restrict__ only) {
+  __shared__ T sU[BCR_SS], sL[BCR_SS], uL[BCR_SS], uU[BCR_SS], dL[BCR_SS], dU[BCR_SS];
+  const int k = blockIdx.x, tid = threadIdx.x;
   if (k >= nsep) return;
   const BcrSep B = bs[k];
   if (only && only[B.comp] == 0) return;
@@ -185,35 +181,33 @@ __global__ void __launch_bounds__(32) bcr_update(int nsep, const BcrSep* __restr
   const int s = B.s, h = 1 << l;
   const T* cur = DLU + (int64_t(l) * nsep * 3 + 3 * int64_t(k)) * BCR_SS;
   T* nxt = DLU + (int64_t(l + 1) * nsep * 3 + 3 * int64_t(k)) * BCR_SS;
-  for (int e = lane; e < BCR_SS; e += 32) {
-    sD[e] = cur[e];
-    sL[e] = cur[BCR_SS + e];
-    sU[e] = cur[2 * BCR_SS + e];
-  }
-  __syncwarp();
   const bool up = B.kloc + h < B.N, dn = B.kloc >= h;
-  const int64_t kup = k + h, kdn = k - h;
-  // D' = D - U W_L(k+h) - L W_U(k-h)
-  if (up) bcr_gemm(sU, WL + kup * BCR_SS, sD, s, T(-1), true, lane);
-  if (dn) bcr_gemm(sL, WU + kdn * BCR_SS, sD, s, T(-1), true, lane);
-  for (int e = lane; e < BCR_SS; e += 32) nxt[e] = sD[e];
-  __syncwarp();  // sD is reused as scratch below, with another lane-to-entry assignment
-  // U' = -U W_U(k+h), L' = -L W_L(k-h)
-  T* nU = nxt + 2 * BCR_SS;
-  T* nL = nxt + BCR_SS;
-  if (up) {
-    bcr_gemm(sU, WU + kup * BCR_SS, sD, s, T(-1), false, lane);  // sD reused as scratch
-    for (int e = lane; e < BCR_SS; e += 32) nU[e] = sD[e];
-    __syncwarp();
-  } else {
-    for (int e = lane; e < BCR_SS; e += 32) nU[e] = T(0);
+  const int64_t kup = int64_t(k + h) * BCR_SS, kdn = int64_t(k - h) * BCR_SS;
+#pragma unroll
+  for (int q = 0; q < BCR_SS / 128; ++q) {
+    const int e = tid + 128 * q;
+    const bool in = e / BCR_S < s && e % BCR_S < s;
+    sL[e] = in && dn ? cur[BCR_SS + e] : T(0);
+    sU[e] = in && up ? cur[2 * BCR_SS + e] : T(0);
+    uL[e] = in && up ? WL[kup + e] : T(0);
+    uU[e] = in && up ? WU[kup + e] : T(0);
+    dL[e] = in && dn ? WL[kdn + e] : T(0);
+    dU[e] = in && dn ? WU[kdn + e] : T(0);
   }
-  __syncwarp();
-  if (dn) {
-    bcr_gemm(sL, WL + kdn * BCR_SS, sD, s, T(-1), false, lane);
-    for (int e = lane; e < BCR_SS; e += 32) nL[e] = sD[e];
-  } else {
-    for (int e = lane; e < BCR_SS; e += 32) nL[e] = T(0);
+  __syncthreads();
+  for (int t = tid; t < s * s; t += 128) {
+    const int i = t / s, j = t % s, e = i * BCR_S + j;
+    T a = T(0), b = T(0), u = T(0), v = T(0);
+    for (int q = 0; q < s; ++q) {
+      const T x = sU[i * BCR_S + q], y = sL[i * BCR_S + q];
+      a = fma(x, uL[q * BCR_S + j], a);
+      b = fma(y, dU[q * BCR_S + j], b);
+      u = fma(x, uU[q * BCR_S + j], u);
+      v = fma(y, dL[q * BCR_S + j], v);
+    }
+    nxt[e] = (cur[e] - a) - b;
+    nxt[BCR_SS + e] = -v;
+    nxt[2 * BCR_SS + e] = -u;
   }
 }
 
@@ -222,21 +216,16 @@ template <typename T>
 __global__ void __launch_bounds__(32) bcr_root(int nsep, const BcrSep* __restrict__ bs, const T* __restrict__ DLU,
                                                T* __restrict__ FA, int* __restrict__ PV, const int* __restrict__ only,
                                                int* __restrict__ info) {
-  __shared__ T sA[BCR_SS];
-  __shared__ int sp[BCR_S];
-  __shared__ int sing;
   const int k = blockIdx.x, lane = threadIdx.x;
   if (k >= nsep) return;
   const BcrSep B = bs[k];
   if (B.kloc != 0 || (only && only[B.comp] == 0)) return;
-  const T* D = DLU + (int64_t(B.nlev) * nsep * 3 + 3 * int64_t(k)) * BCR_SS;
-  for (int e = lane; e < BCR_SS; e += 32) sA[e] = D[e];
-  if (lane == 0) sing = 0;
-  __syncwarp();
-  bcr_lu(sA, sp, B.s, lane, &sing);
-  T* fa = FA + int64_t(k) * BCR_SS;
-  for (int e = lane; e < BCR_SS; e += 32) fa[e] = sA[e];
-  if (lane < B.s) PV[int64_t(k) * BCR_S + lane] = sp[lane];
+  T d[BCR_S], x[BCR_S];
+  bcr_row_load(d, DLU + (int64_t(B.nlev) * nsep * 3 + 3 * int64_t(k)) * BCR_SS, B.s, lane);
+  int pos;
+  const bool sing = bcr_factor<T, false>(d, x, B.s, lane, &pos);
+  bcr_row_store(d, FA + int64_t(k) * BCR_SS, B.s, pos);
+  if (lane < B.s) PV[int64_t(k) * BCR_S + pos] = lane;
   if (lane == 0 && sing && info) atomicCAS(info, 0, B.comp + 1);
 }
 
@@ -246,112 +235,78 @@ __global__ void __launch_bounds__(32) bcr_root(int nsep, const BcrSep* __restric
 // functions shared by the level-by-level kernels below and by the fused
 // per-component solve (band_torn.cuh).
 
-// shared scratch of one warp
-template <typename T>
-struct BcrWarp {
-  T A[BCR_SS];
-  T B[BCR_SS];
-  T v[BCR_S];
-  T w[BCR_S];
-  int p[BCR_S];
-};
-
-// v <- (LU)^-1 P v for one block: F and v in shared memory, the triangular
-// sweeps lane-parallel over rows (one column step per warp-synchronous step)
-template <typename T>
-__device__ void bcr_block_solve(const T* F, const int* piv, T* v, int s, int lane) {
-  if (lane == 0)
-    for (int j = 0; j < s; ++j)
-      if (piv[j] != j) {
-        const T t = v[j];
-        v[j] = v[piv[j]];
-        v[piv[j]] = t;
-      }
-  __syncwarp();
-  for (int j = 0; j < s; ++j) {  // unit lower
-    if (lane > j && lane < s) v[lane] = fma(-F[lane * BCR_S + j], v[j], v[lane]);
-    __syncwarp();
-  }
-  for (int j = s - 1; j >= 0; --j) {  // upper
-    if (lane == j) v[j] /= F[j * BCR_S + j];
-    __syncwarp();
-    if (lane < j) v[lane] = fma(-F[lane * BCR_S + j], v[j], v[lane]);
-    __syncwarp();
-  }
-}
-
-template <typename T>
-__device__ void bcr_stage(T* dst, const T* src, int lane) {
-  for (int e = lane; e < BCR_SS; e += 32) dst[e] = src[e];
-}
-
-// z_k = D_k^-1 r_k with the factors FA[k] (an eliminated block at its level, or the root)
+// z_k = D_k^-1 r_k with the factors FA[k] (an eliminated block at its level, or the
+// root): row `lane` of the factors and entry `lane` of the vector in registers, the
+// substitutions by shuffles
 template <typename T>
 __device__ void bcr_diag_solve_warp(const BcrSep& B, int k, const T* __restrict__ FA, const int* __restrict__ PV,
-                                    const int64_t* __restrict__ row0, const double* r, double* z,
-                                    BcrWarp<T>* sw, int lane) {
+                                    const int64_t* __restrict__ row0, const double* r, double* z, int lane) {
   const int s = B.s;
   const int64_t o = row0[k];
-  bcr_stage(sw->A, FA + int64_t(k) * BCR_SS, lane);
-  if (lane < s) {
-    sw->v[lane] = T(r[o + lane]);
-    sw->p[lane] = PV[int64_t(k) * BCR_S + lane];
+  T f[BCR_S];
+  bcr_row_load(f, FA + int64_t(k) * BCR_SS, s, lane);
+  T v = lane < s ? T(r[o + PV[int64_t(k) * BCR_S + lane]]) : T(0);
+  T rp = T(0);
+#pragma unroll
+  for (int j = 0; j < BCR_S; ++j) {  // unit lower
+    if (j >= s) break;
+    const T y = __shfl_sync(RB_FULL, v, j);
+    if (lane > j) v = fma(-f[j], y, v);
+    if (lane == j) rp = f[j];
   }
+#pragma unroll
+  for (int j = BCR_S - 1; j >= 0; --j) {  // upper, rows over their pivots at the end
+    if (j >= s) continue;
+    const T y = __shfl_sync(RB_FULL, v, j);
+    if (lane < j) v = fma(-f[j], y, v);
+  }
+  if (lane < s) z[o + lane] = double(v * rp);
   __syncwarp();
-  bcr_block_solve(sw->A, sw->p, sw->v, s, lane);
-  if (lane < s) z[o + lane] = double(sw->v[lane]);
-  __syncwarp();
+}
+
+// v − M1 w1 − M2 w2 for row `lane` of two blocks and the entries `lane` of two vectors
+template <typename T>
+__device__ __forceinline__ T bcr_row_sub(T v, const T m1[BCR_S], T w1, const T m2[BCR_S], T w2, int s) {
+  T a = T(0);
+#pragma unroll
+  for (int q = 0; q < BCR_S; ++q) {
+    if (q >= s) break;
+    v = fma(-m1[q], __shfl_sync(RB_FULL, w1, q), v);
+    a = fma(-m2[q], __shfl_sync(RB_FULL, w2, q), a);
+  }
+  return v + a;
 }
 
 // kept block e at level l: r_e -= U_e z_{e+h} + L_e z_{e-h}
 template <typename T>
 __device__ void bcr_keep_warp(const BcrSep& B, int k, int l, int nsep, const T* __restrict__ DLU,
-                              const int64_t* __restrict__ row0, double* r, const double* z, BcrWarp<T>* sw,
-                              int lane) {
+                              const int64_t* __restrict__ row0, double* r, const double* z, int lane) {
   const int s = B.s, h = 1 << l;
   const T* cur = DLU + (int64_t(l) * nsep * 3 + 3 * int64_t(k)) * BCR_SS;
   const bool up = B.kloc + h < B.N, dn = B.kloc >= h;
-  if (up) bcr_stage(sw->B, cur + 2 * BCR_SS, lane);
-  if (dn) bcr_stage(sw->A, cur + BCR_SS, lane);
-  if (lane < s) {
-    sw->v[lane] = up ? T(z[row0[k + h] + lane]) : T(0);
-    sw->w[lane] = dn ? T(z[row0[k - h] + lane]) : T(0);
-  }
-  __syncwarp();
-  if (lane < s) {
-    const int64_t o = row0[k];
-    T v = T(r[o + lane]);
-    for (int q = 0; q < s; ++q) {
-      if (up) v = fma(-sw->B[lane * BCR_S + q], sw->v[q], v);
-      if (dn) v = fma(-sw->A[lane * BCR_S + q], sw->w[q], v);
-    }
-    r[o + lane] = double(v);
-  }
+  T u[BCR_S], d[BCR_S];
+  bcr_row_load(u, cur + 2 * BCR_SS, up ? s : 0, lane);
+  bcr_row_load(d, cur + BCR_SS, dn ? s : 0, lane);
+  const T wu = up && lane < s ? T(z[row0[k + h] + lane]) : T(0), wd = dn && lane < s ? T(z[row0[k - h] + lane]) : T(0);
+  const int64_t o = row0[k];
+  const T v = bcr_row_sub(lane < s ? T(r[o + lane]) : T(0), u, wu, d, wd, s);
+  if (lane < s) r[o + lane] = double(v);
   __syncwarp();
 }
 
 // eliminated block k at level l: x_k = z_k - W_L(k) x_{k-h} - W_U(k) x_{k+h}  (z holds z_k and the kept x)
 template <typename T>
 __device__ void bcr_back_warp(const BcrSep& B, int k, int l, const T* __restrict__ WL, const T* __restrict__ WU,
-                              const int64_t* __restrict__ row0, double* z, BcrWarp<T>* sw, int lane) {
+                              const int64_t* __restrict__ row0, double* z, int lane) {
   const int s = B.s, h = 1 << l;
   const bool up = B.kloc + h < B.N;
   const int64_t o = row0[k];
-  bcr_stage(sw->A, WL + int64_t(k) * BCR_SS, lane);
-  if (up) bcr_stage(sw->B, WU + int64_t(k) * BCR_SS, lane);
-  if (lane < s) {
-    sw->w[lane] = T(z[row0[k - h] + lane]);
-    sw->v[lane] = up ? T(z[row0[k + h] + lane]) : T(0);
-  }
-  __syncwarp();
-  if (lane < s) {
-    T a = T(z[o + lane]);
-    for (int q = 0; q < s; ++q) {
-      a = fma(-sw->A[lane * BCR_S + q], sw->w[q], a);
-      if (up) a = fma(-sw->B[lane * BCR_S + q], sw->v[q], a);
-    }
-    z[o + lane] = double(a);
-  }
+  T wl[BCR_S], wu[BCR_S];
+  bcr_row_load(wl, WL + int64_t(k) * BCR_SS, s, lane);
+  bcr_row_load(wu, WU + int64_t(k) * BCR_SS, up ? s : 0, lane);
+  const T xl = lane < s ? T(z[row0[k - h] + lane]) : T(0), xu = up && lane < s ? T(z[row0[k + h] + lane]) : T(0);
+  const T v = bcr_row_sub(lane < s ? T(z[o + lane]) : T(0), wl, xl, wu, xu, s);
+  if (lane < s) z[o + lane] = double(v);
   __syncwarp();
 }
 
@@ -362,13 +317,12 @@ __global__ void __launch_bounds__(32) bcr_fwd_elim(int nsep, const BcrSep* __res
                                                    const T* __restrict__ FA, const int* __restrict__ PV,
                                                    const int64_t* __restrict__ row0, const double* __restrict__ r,
                                                    double* __restrict__ z, const int* __restrict__ only) {
-  __shared__ BcrWarp<T> sw;
   const int k = blockIdx.x;
   if (k >= nsep) return;
   const BcrSep B = bs[k];
   if (only && only[B.comp] == 0) return;
   if (!(l < B.nlev && bcr_role(B.kloc, B.N, l) == 1)) return;
-  bcr_diag_solve_warp(B, k, FA, PV, row0, r, z, &sw, threadIdx.x);
+  bcr_diag_solve_warp(B, k, FA, PV, row0, r, z, threadIdx.x);
 }
 
 // forward, level l: kept r_e -= U_e z_{e+h} + L_e z_{e-h}
@@ -377,13 +331,12 @@ __global__ void __launch_bounds__(32) bcr_fwd_keep(int nsep, const BcrSep* __res
                                                    const T* __restrict__ DLU, const int64_t* __restrict__ row0,
                                                    double* __restrict__ r, const double* __restrict__ z,
                                                    const int* __restrict__ only) {
-  __shared__ BcrWarp<T> sw;
   const int k = blockIdx.x;
   if (k >= nsep) return;
   const BcrSep B = bs[k];
   if (only && only[B.comp] == 0) return;
   if (!(l < B.nlev && bcr_role(B.kloc, B.N, l) == 2)) return;
-  bcr_keep_warp(B, k, l, nsep, DLU, row0, r, z, &sw, threadIdx.x);
+  bcr_keep_warp(B, k, l, nsep, DLU, row0, r, z, threadIdx.x);
 }
 
 // root: x_0 = D_0^-1 r_0 (into z, which then holds x for every block as the back-substitution proceeds)
@@ -392,12 +345,11 @@ __global__ void __launch_bounds__(32) bcr_root_solve(int nsep, const BcrSep* __r
                                                      const T* __restrict__ FA, const int* __restrict__ PV,
                                                      const int64_t* __restrict__ row0, const double* __restrict__ r,
                                                      double* __restrict__ z, const int* __restrict__ only) {
-  __shared__ BcrWarp<T> sw;
   const int k = blockIdx.x;
   if (k >= nsep) return;
   const BcrSep B = bs[k];
   if (B.kloc != 0 || (only && only[B.comp] == 0)) return;
-  bcr_diag_solve_warp(B, k, FA, PV, row0, r, z, &sw, threadIdx.x);
+  bcr_diag_solve_warp(B, k, FA, PV, row0, r, z, threadIdx.x);
 }
 
 // backward, level l
@@ -406,13 +358,12 @@ __global__ void __launch_bounds__(32) bcr_back(int nsep, const BcrSep* __restric
                                                const T* __restrict__ WL, const T* __restrict__ WU,
                                                const int64_t* __restrict__ row0, double* __restrict__ z,
                                                const int* __restrict__ only) {
-  __shared__ BcrWarp<T> sw;
   const int k = blockIdx.x;
   if (k >= nsep) return;
   const BcrSep B = bs[k];
   if (only && only[B.comp] == 0) return;
   if (!(l < B.nlev && bcr_role(B.kloc, B.N, l) == 1)) return;
-  bcr_back_warp(B, k, l, WL, WU, row0, z, &sw, threadIdx.x);
+  bcr_back_warp(B, k, l, WL, WU, row0, z, threadIdx.x);
 }
 
 }  // namespace mgpu

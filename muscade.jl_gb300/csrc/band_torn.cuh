@@ -368,7 +368,7 @@ struct TbFusedFactors {
 
 template <typename T, int WM>
 __host__ __device__ constexpr int tb_fused_warp_bytes() {
-  return ((RbSmem<T, WM>::bytes > int(sizeof(BcrWarp<T>)) ? RbSmem<T, WM>::bytes : int(sizeof(BcrWarp<T>))) + 15) /
+  return (RbSmem<T, WM>::bytes + 15) /
          16 * 16;
 }
 
@@ -462,7 +462,6 @@ __global__ void __launch_bounds__(kTbFusedMaxThreads, 2) tb_fused(TbFusedArgs A,
   if (A.only && A.only[cc] == 0) return;
   const int W = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   unsigned char* my = tb_dyn + size_t(w) * tb_fused_warp_bytes<T, WM>();
-  BcrWarp<T>* sw = reinterpret_cast<BcrWarp<T>*>(my);
   const int a0 = A.cint0[cc], a1 = A.cint0[cc + 1], k0 = A.csep0[cc], k1 = A.csep0[cc + 1];
   const int nc = A.ccn[cc];
   const int64_t q0 = A.ccdof0[cc];
@@ -492,21 +491,21 @@ __global__ void __launch_bounds__(kTbFusedMaxThreads, 2) tb_fused(TbFusedArgs A,
       for (int l = 0; l < nlev; ++l) {
         for (int k = k0 + w; k < k1; k += W) {
           const BcrSep B = A.bs[k];
-          if (bcr_role(B.kloc, B.N, l) == 1) bcr_diag_solve_warp(B, k, F.FA, F.PV, A.brow, A.trhs, A.txs, sw, lane);
+          if (bcr_role(B.kloc, B.N, l) == 1) bcr_diag_solve_warp(B, k, F.FA, F.PV, A.brow, A.trhs, A.txs, lane);
         }
         __syncthreads();
         for (int k = k0 + w; k < k1; k += W) {
           const BcrSep B = A.bs[k];
-          if (bcr_role(B.kloc, B.N, l) == 2) bcr_keep_warp(B, k, l, A.nsep, F.DLU, A.brow, A.trhs, A.txs, sw, lane);
+          if (bcr_role(B.kloc, B.N, l) == 2) bcr_keep_warp(B, k, l, A.nsep, F.DLU, A.brow, A.trhs, A.txs, lane);
         }
         __syncthreads();
       }
-      if (w == 0) bcr_diag_solve_warp(A.bs[k0], k0, F.FA, F.PV, A.brow, A.trhs, A.txs, sw, lane);
+      if (w == 0) bcr_diag_solve_warp(A.bs[k0], k0, F.FA, F.PV, A.brow, A.trhs, A.txs, lane);
       __syncthreads();
       for (int l = nlev - 1; l >= 0; --l) {
         for (int k = k0 + w; k < k1; k += W) {
           const BcrSep B = A.bs[k];
-          if (bcr_role(B.kloc, B.N, l) == 1) bcr_back_warp(B, k, l, F.WL, F.WU, A.brow, A.txs, sw, lane);
+          if (bcr_role(B.kloc, B.N, l) == 1) bcr_back_warp(B, k, l, F.WL, F.WU, A.brow, A.txs, lane);
         }
         __syncthreads();
       }

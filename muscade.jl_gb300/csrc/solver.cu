@@ -983,8 +983,8 @@ static void torn_factor(mgpu_ctx* c, bool tr, const int* cflag, int* info) {
     tb_spikes<T, 64, 32><<<S.nint, 32, 0, st>>>(S.nint, ti, B.uc, B.lm, S.tpiv, blk, B.y, cflag);
   tb_schur<T><<<S.nsep, 32, 0, st>>>(S.nsep, S.d_ts, ti, blk, B.y, B.dlu, cflag);
   for (int l = 0; l < S.bcr_levels; ++l) {
-    bcr_eliminate<T><<<S.nsep, 32, 0, st>>>(S.nsep, S.d_bsep, l, B.dlu, B.fa, S.PV, B.wl, B.wu, cflag, info);
-    bcr_update<T><<<S.nsep, 32, 0, st>>>(S.nsep, S.d_bsep, l, B.dlu, B.wl, B.wu, cflag);
+    bcr_eliminate<T><<<S.nsep, 64, 0, st>>>(S.nsep, S.d_bsep, l, B.dlu, B.fa, S.PV, B.wl, B.wu, cflag, info);
+    bcr_update<T><<<S.nsep, 128, 0, st>>>(S.nsep, S.d_bsep, l, B.dlu, B.wl, B.wu, cflag);
   }
   bcr_root<T><<<S.nsep, 32, 0, st>>>(S.nsep, S.d_bsep, B.dlu, B.fa, S.PV, cflag, info);
 }
