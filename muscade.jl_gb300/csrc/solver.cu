@@ -49,6 +49,133 @@ static bool cluster_fits(int cl) {
   return cudaOccupancyMaxActiveClusters(&m, band_lu, &cfg) == cudaSuccess && m > 0;
 }
 
+// Reverse Cuthill-McKee over single dofs leaves the ends of a chain wider than its
+// middle: a Hold's multiplier is a leaf next to one dof, so breadth-first levels
+// mix the first nodes' dofs (bands 13 to 16 for chains of 6-dof nodes that need
+// 11, and the band sets the spikes, the separators and the register windows of
+// every interior).  Here each component is also ordered by nodes: leaf multipliers
+// (dofs with one neighbour) set aside, dofs of equal closed neighbourhood grouped,
+// the groups in reverse Cuthill-McKee order, and each group's leaves before it at
+// the start of the order, else behind it.  The narrower of the two is kept.
+static void narrow_by_nodes(int64_t n, const std::vector<int64_t>& deg, const std::vector<int32_t>& adj,
+                            const std::vector<std::vector<int32_t>>& members, const std::vector<int32_t>& comp_start,
+                            std::vector<int32_t>& order, std::vector<int32_t>& pos) {
+  auto width = [&](const std::vector<int32_t>& M) {
+    int32_t w = 0;
+    for (int32_t v : M)
+      for (int64_t q = deg[v]; q < deg[v + 1]; ++q) w = std::max(w, std::abs(pos[adj[q]] - pos[v]));
+    return w;
+  };
+  std::vector<int32_t> todo, wid(members.size());
+#pragma omp parallel for schedule(dynamic, 16)
+  for (int64_t cc = 0; cc < int64_t(members.size()); ++cc) wid[cc] = width(members[cc]);
+  // one 6-dof node next to another needs 11; wider than 48 is no chain
+  for (size_t cc = 0; cc < members.size(); ++cc)
+    if (wid[cc] > 11 && wid[cc] <= 48 && members[cc].size() > 2) todo.push_back(int32_t(cc));
+  if (todo.empty()) return;
+  std::vector<int32_t> nb(adj.size()), cnt(n, 0), grp(n, -1), host(n, -1);  // sorted neighbours, each once
+#pragma omp parallel for schedule(dynamic, 16)
+  for (int64_t t = 0; t < int64_t(todo.size()); ++t) {
+    const auto& M = members[todo[t]];
+    const int32_t c0 = comp_start[todo[t]], w0 = wid[todo[t]];
+    for (int32_t v : M) {
+      std::copy(adj.begin() + deg[v], adj.begin() + deg[v + 1], nb.begin() + deg[v]);
+      std::sort(nb.begin() + deg[v], nb.begin() + deg[v + 1]);
+      cnt[v] = int32_t(std::unique(nb.begin() + deg[v], nb.begin() + deg[v + 1]) - (nb.begin() + deg[v]));
+    }
+    for (int32_t v : M) {
+      const int32_t u = cnt[v] == 1 ? nb[deg[v]] : -1;
+      host[v] = u >= 0 && cnt[u] > 1 ? u : -1;
+    }
+    // groups of equal closed neighbourhood (leaves left out), by a hash of the list
+    auto closed = [&](int32_t v, std::vector<int32_t>& k) {
+      k.clear();
+      for (int32_t q = 0; q < cnt[v]; ++q)
+        if (host[nb[deg[v] + q]] < 0) k.push_back(nb[deg[v] + q]);
+      k.insert(std::lower_bound(k.begin(), k.end(), v), v);
+    };
+    std::vector<std::pair<uint64_t, int32_t>> key;
+    std::vector<int32_t> ka, kb;
+    for (int32_t v : M)
+      if (host[v] < 0) {
+        closed(v, ka);
+        uint64_t h = 1469598103934665603ull;
+        for (int32_t u : ka) h = (h ^ uint64_t(uint32_t(u))) * 1099511628211ull;
+        key.push_back({h, v});
+      }
+    std::sort(key.begin(), key.end());
+    std::vector<std::vector<int32_t>> G;  // dofs of each group
+    for (size_t q = 0; q < key.size(); ++q) {
+      bool same = q > 0 && key[q].first == key[q - 1].first;
+      if (same) {
+        closed(key[q].second, ka);
+        closed(G.back()[0], kb);
+        same = ka == kb;
+      }
+      if (!same) G.push_back({});
+      G.back().push_back(key[q].second);
+    }
+    // numbered by their first dof, so that a model orders alike alone and among others
+    std::sort(G.begin(), G.end());
+    const int ng = int(G.size());
+    for (int g = 0; g < ng; ++g)
+      for (int32_t v : G[g]) grp[v] = g;
+    std::vector<std::vector<int32_t>> ga(ng);
+    for (int g = 0; g < ng; ++g) {
+      for (int32_t q = 0, v = G[g][0]; q < cnt[v]; ++q) {
+        const int32_t u = nb[deg[v] + q];
+        if (host[u] < 0 && grp[u] != g) ga[g].push_back(grp[u]);
+      }
+      std::sort(ga[g].begin(), ga[g].end());
+      ga[g].erase(std::unique(ga[g].begin(), ga[g].end()), ga[g].end());
+    }
+    // breadth-first order from an end of the group graph (the farthest group, three times)
+    std::vector<int32_t> seen(ng, -1), bfs;
+    auto sweep = [&](int32_t s0, int32_t tag) {
+      bfs.assign(1, s0);
+      seen[s0] = tag;
+      for (size_t h = 0; h < bfs.size(); ++h) {
+        const size_t from = bfs.size();
+        for (int32_t u : ga[bfs[h]])
+          if (seen[u] != tag) seen[u] = tag, bfs.push_back(u);
+        std::sort(bfs.begin() + from, bfs.end(), [&](int32_t x, int32_t y) {
+          return ga[x].size() != ga[y].size() ? ga[x].size() < ga[y].size() : x < y;
+        });
+      }
+    };
+    int32_t start = 0;
+    for (int32_t tag = 0; tag < 3; ++tag) {
+      sweep(start, tag);
+      start = bfs.back();
+    }
+    sweep(start, 3);
+    if (int(bfs.size()) != ng) continue;
+    std::vector<std::vector<int32_t>> leaves(ng);
+    for (int32_t v : M)
+      if (host[v] >= 0) leaves[grp[host[v]]].push_back(v);
+    std::vector<int32_t> ord;
+    ord.reserve(M.size());
+    for (size_t h = 0; h < bfs.size(); ++h) {
+      const int32_t g = bfs[bfs.size() - 1 - h];
+      auto& lv = leaves[g];
+      std::sort(lv.begin(), lv.end(), [&](int32_t x, int32_t y) { return host[x] != host[y] ? host[x] < host[y] : x < y; });
+      if (h == 0) ord.insert(ord.end(), lv.begin(), lv.end());
+      ord.insert(ord.end(), G[g].begin(), G[g].end());
+      if (h > 0) ord.insert(ord.end(), lv.begin(), lv.end());
+    }
+    const std::vector<int32_t> keep(order.begin() + c0, order.begin() + c0 + M.size());
+    for (size_t k = 0; k < ord.size(); ++k) {
+      order[c0 + k] = ord[k];
+      pos[ord[k]] = c0 + int32_t(k);
+    }
+    if (width(M) >= w0)  // no narrower: as it was
+      for (size_t k = 0; k < keep.size(); ++k) {
+        order[c0 + k] = keep[k];
+        pos[keep[k]] = c0 + int32_t(k);
+      }
+  }
+}
+
 // ---------------------------------------------------------------- host analysis
 static void analyse(mgpu_ctx* c, Solver& S) {
   const Pattern& P = c->pat;
@@ -163,6 +290,7 @@ static void analyse(mgpu_ctx* c, Solver& S) {
   comp_start[ncomp] = int32_t(order.size());
   std::vector<int32_t> pos(n);
   for (int64_t k = 0; k < n; ++k) pos[order[k]] = int32_t(k);
+  narrow_by_nodes(n, deg, adj, members, comp_start, order, pos);
   // bandwidths per component
   std::vector<int32_t> kl(ncomp, 0), ku(ncomp, 0);
   for (int64_t j = 0; j < n; ++j)
