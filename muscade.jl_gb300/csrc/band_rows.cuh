@@ -35,6 +35,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 namespace mgpu {
 
@@ -203,6 +204,115 @@ __global__ void __launch_bounds__(32) rb_lu(RbComp cp, const T* __restrict__ Aro
     }
     pos = me ? kl : pos - 1;
   }
+  rb_cp_wait<0>();
+  if (singular && lane == 0) {
+    if (mode == RB_PRIMARY)
+      flag[cc] = 1;
+    else if (info)
+      atomicCAS(info, 0, cc + 1);
+  }
+}
+
+// The same for kl <= 15 and kv + 1 <= 2 NC (chains of 6-dof nodes: kl = ku = 11, NC =
+// 12): rb_lu leaves lanes kl+1..31 idle in every FP64 instruction, so here 16 lanes
+// hold a row each and the half-warps share its columns, half h those of parity h
+// (slot s of half h: column 2(⌊k/2⌋ + s) + h), which needs a shift only every
+// second step.  12 instead of 22 multiply-adds a column; 132 dofs of one cantilever
+// 218 -> 139 us.  The arithmetic of an entry is that of rb_lu.
+template <typename T, int NC>
+__global__ void __launch_bounds__(32) rb_lu_half(RbComp cp, const T* __restrict__ Arows, T* __restrict__ UC,
+                                                 T* __restrict__ LM, int32_t* __restrict__ ipiv, int mode,
+                                                 int* __restrict__ flag, int* __restrict__ info) {
+  __shared__ __align__(16) T sR[2][32 * 2 * NC];
+  const int cc = cp.list ? cp.list[blockIdx.x] : int(blockIdx.x), lane = threadIdx.x;
+  if (mode == RB_FALLBACK && flag[cc] == 0) return;
+  const int n = cp.cn[cc], kl = cp.ckl[cc], kv = kl + cp.cku[cc], w = kv + 1;
+  const T* Ac = Arows + cp.rbase[cc];
+  T* U = UC + cp.rbase[cc];
+  T* L = LM + cp.lbase[cc];
+  int32_t* piv = ipiv + cp.cdof0[cc];
+  const int row = lane & 15, half = lane >> 4;
+  auto issue = [&](int ch) {  // rows [32 ch, 32 ch + 32) of the component into buffer ch & 1
+    const int r0 = ch * 32, r1 = min(n, r0 + 32);
+    T* dst = sR[ch & 1];
+    for (int e = lane; e < (r1 - r0) * w; e += 32) rb_cp_async(dst + e, Ac + int64_t(r0) * w + e, sizeof(T));
+  };
+  issue((kl + 1) >> 5);
+  rb_cp_commit();
+  T a[NC];
+  int pos = (row <= kl) ? row : (1 << 30);  // rows above kl stay empty
+#pragma unroll
+  for (int s = 0; s < NC; ++s) {
+    const int c = 2 * s + half, q = c - row + kl;  // column c of row `row` in its storage row
+    a[s] = (row <= kl && row < n && c <= kv && q >= 0 && q <= kv) ? Ac[int64_t(row) * w + q] : T(0);
+  }
+  bool singular = false;
+  auto step = [&](auto parity, int k) {
+    constexpr int KP = decltype(parity)::value;  // k & 1
+    const int km = min(kl, n - 1 - k);
+    const int rn = k + 1 + kl;  // row that enters after this column
+    if (rn < n && (k == 0 || (rn & 31) == 0)) {
+      __syncwarp();
+      issue((rn >> 5) + 1);
+      rb_cp_commit();
+      rb_cp_wait<1>();
+      __syncwarp();
+    }
+    int pl;
+    const int jp = rb_argmax(a[0], half == KP && pos <= km, pos, &pl);
+    const T pv = __shfl_sync(RB_FULL, a[0], pl);
+    if (lane == 0) piv[k] = k + jp;
+    const bool me = row == (pl & 15);  // both halves of the pivot row
+    if (me)
+      pos = 0;
+    else if (pos == 0)
+      pos = jp;
+    const bool zero = (pv == T(0));
+    singular = singular || zero;
+    T rp = T(0);
+    if (!zero) {
+      if constexpr (sizeof(T) == 8)
+        rp = rb_rcp(pv);
+      else
+        rp = __frcp_rn(pv);
+    }
+    const bool below = pos >= 1 && pos <= km;
+    T l = (!zero && below) ? a[0] * rp : a[0];
+    if (half == KP && below) L[int64_t(k) * kl + pos - 1] = l;
+    l = __shfl_sync(RB_FULL, l, row + 16 * KP);
+    const T le = (!zero && below) ? l : T(0);
+    const int src = (pl & 15) + (lane & 16);
+    T cap = T(0);
+#pragma unroll
+    for (int s = 0; s < NC; ++s) {
+      const T u = __shfl_sync(RB_FULL, a[s], src);
+      if (row == s) cap = u;
+      a[s] = fma(-le, u, a[s]);
+    }
+    const int j = 2 * row + half - KP;  // column k + j of the pivot row is this lane's cap
+    if (row < NC && j >= 0 && j <= kv && k + j < n) U[int64_t(k + j) * w + j] = (j == 0) ? rp : cap;
+    // advance to column k + 1: a shift after an odd step, and the pivot lanes take row rn
+    if constexpr (KP == 1) {
+#pragma unroll
+      for (int s = 0; s + 1 < NC; ++s) a[s] = a[s + 1];
+      a[NC - 1] = T(0);
+    }
+    if (me) {
+      const T* r = sR[(rn >> 5) & 1] + (rn & 31) * w;
+#pragma unroll
+      for (int s = 0; s < NC; ++s) {
+        const int q = 2 * s + half - (KP == 1 ? 0 : 1);  // its column less k + 1
+        a[s] = (rn < n && q >= 0 && q <= kv) ? r[q] : T(0);
+      }
+    }
+    pos = me ? kl : pos - 1;
+  };
+  int k = 0;
+  for (; k + 1 < n; k += 2) {
+    step(std::integral_constant<int, 0>{}, k);
+    step(std::integral_constant<int, 1>{}, k + 1);
+  }
+  if (k < n) step(std::integral_constant<int, 0>{}, k);
   rb_cp_wait<0>();
   if (singular && lane == 0) {
     if (mode == RB_PRIMARY)

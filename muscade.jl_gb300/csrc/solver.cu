@@ -49,6 +49,15 @@ static bool cluster_fits(int cl) {
   return cudaOccupancyMaxActiveClusters(&m, band_lu, &cfg) == cudaSuccess && m > 0;
 }
 
+// class of a row-band factorisation by s = max(kl, ku) and w = kl + ku + 1 (lu_launch);
+// the half-warp kernels take 16 rows and 2 NC − 1 columns
+constexpr int kLuClasses = 6;
+static int lu_class(int s, int w) {
+  if (s <= 15 && w <= 23) return 0;
+  if (s <= 15 && w <= 31) return 1;
+  return w <= 32 ? 2 : w <= 40 ? 3 : w <= 48 ? 4 : 5;
+}
+
 // Reverse Cuthill-McKee over single dofs leaves the ends of a chain wider than its
 // middle: a Hold's multiplier is a leaf next to one dof, so breadth-first levels
 // mix the first nodes' dofs (bands 13 to 16 for chains of 6-dof nodes that need
@@ -346,17 +355,17 @@ static void analyse(mgpu_ctx* c, Solver& S) {
   if (S.maxkl <= 31 && maxw <= 64) {
     S.wm = maxw <= 32 ? 32 : 64;
     {
-      std::vector<int32_t> l32, l64, lu[4];
+      std::vector<int32_t> l32, l64, lu[kLuClasses];
       for (int cc = 0; cc < ncomp; ++cc) {
         const int w = kl[cc] + ku[cc] + 1;
         (w <= 32 ? l32 : l64).push_back(cc);
-        lu[w <= 32 ? 0 : w <= 40 ? 1 : w <= 48 ? 2 : 3].push_back(cc);
+        lu[lu_class(std::max(kl[cc], ku[cc]), w)].push_back(cc);
       }
       S.n32 = int(l32.size());
       S.n64 = int(l64.size());
       if (!l32.empty()) good = good && up(&S.list32, l32);
       if (!l64.empty()) good = good && up(&S.list64, l64);
-      for (int q = 0; q < 4; ++q) {
+      for (int q = 0; q < kLuClasses; ++q) {
         S.nlu[q] = int(lu[q].size());
         if (!lu[q].empty()) good = good && up(&S.lulist[q], lu[q]);
       }
@@ -524,6 +533,7 @@ static void analyse(mgpu_ctx* c, Solver& S) {
       cint0[ncomp] = S.nint;
       csep0[ncomp] = S.nsep;
       S.twmI = maxwI <= 32 ? 32 : 64;
+      S.tlu = lu_class(*std::max_element(sc.begin(), sc.end()), maxwI);
       // fused per-component solve (one block per component) when every component has
       // few interiors; warps per block bounded by ~112 KB of shared memory (two blocks per SM)
       {
@@ -1020,8 +1030,9 @@ extern "C" void mgpu_solver_destroy(mgpu_ctx* c) {
                 S->FA, S->WL, S->WU, S->PV, S->trhs, S->txs, S->tpiv, S->TALL32, S->TUC32, S->TLM32, S->TY32,
                 S->DLU32, S->FA32, S->WL32, S->WU32, S->i_comp,
                 S->iflag, S->nbad, S->info32, S->dtmp, S->rtmp, S->rptr, S->rq, S->rcol, S->dcolptr,
-                S->drowval, S->c_int0, S->c_sep0, S->list32, S->list64, S->lulist[0], S->lulist[1], S->lulist[2], S->lulist[3]};
+                S->drowval, S->c_int0, S->c_sep0, S->list32, S->list64};
   for (void* p : ps) cudaFree(p);
+  for (int32_t* p : S->lulist) cudaFree(p);
   if (S->hbuf) cudaFreeHost(S->hbuf);
   delete S;
   c->solver = nullptr;
@@ -1029,6 +1040,22 @@ extern "C" void mgpu_solver_destroy(mgpu_ctx* c) {
 
 namespace mgpu {
 unsigned nb(int64_t n, int b) { return unsigned((n + b - 1) / b); }
+
+// Row-band factorisation of `count` components (or interiors) of one class: the
+// half-warp kernels where every band fits them, else a register window of 32, 40,
+// 48 or 64 (registers, and so resident warps, follow the window)
+template <typename T>
+static void lu_launch(int cls, int count, const RbComp& cp, cudaStream_t st, const T* rows, T* uc, T* lm, int32_t* piv,
+                      int mode, int* flag, int* info) {
+  switch (cls) {
+    case 0: rb_lu_half<T, 12><<<count, 32, 0, st>>>(cp, rows, uc, lm, piv, mode, flag, info); break;
+    case 1: rb_lu_half<T, 16><<<count, 32, 0, st>>>(cp, rows, uc, lm, piv, mode, flag, info); break;
+    case 2: rb_lu<T, 32><<<count, 32, 0, st>>>(cp, rows, uc, lm, piv, mode, flag, info); break;
+    case 3: rb_lu<T, 40><<<count, 32, 0, st>>>(cp, rows, uc, lm, piv, mode, flag, info); break;
+    case 4: rb_lu<T, 48><<<count, 32, 0, st>>>(cp, rows, uc, lm, piv, mode, flag, info); break;
+    default: rb_lu<T, 64><<<count, 32, 0, st>>>(cp, rows, uc, lm, piv, mode, flag, info);
+  }
+}
 
 // one Newton correction: factor Lλx, Δx = Lλx \ Lλ, norms -> S.red (device);
 // a singular factorisation writes its component+1 to *info.  Capturable.
@@ -1039,23 +1066,11 @@ unsigned nb(int64_t n, int b) { return unsigned((n + b - 1) / b); }
 template <typename T>
 static void rb_launch(Solver& S, RbComp cp, cudaStream_t st, const T* rows, T* uc, T* lm, const double* rhs, T* tw,
                       double* out, int nref, int mode, int* nsweep, int* info) {
-  // factorisation: windows of 32, 40, 48 or 64 (registers, and so resident warps, follow the window)
-  if (S.nlu[0] > 0) {
-    cp.list = S.lulist[0];
-    rb_lu<T, 32><<<S.nlu[0], 32, 0, st>>>(cp, rows, uc, lm, S.ipiv, mode, S.flag, info);
-  }
-  if (S.nlu[1] > 0) {
-    cp.list = S.lulist[1];
-    rb_lu<T, 40><<<S.nlu[1], 32, 0, st>>>(cp, rows, uc, lm, S.ipiv, mode, S.flag, info);
-  }
-  if (S.nlu[2] > 0) {
-    cp.list = S.lulist[2];
-    rb_lu<T, 48><<<S.nlu[2], 32, 0, st>>>(cp, rows, uc, lm, S.ipiv, mode, S.flag, info);
-  }
-  if (S.nlu[3] > 0) {
-    cp.list = S.lulist[3];
-    rb_lu<T, 64><<<S.nlu[3], 32, 0, st>>>(cp, rows, uc, lm, S.ipiv, mode, S.flag, info);
-  }
+  for (int q = 0; q < kLuClasses; ++q)
+    if (S.nlu[q] > 0) {
+      cp.list = S.lulist[q];
+      lu_launch<T>(q, S.nlu[q], cp, st, rows, uc, lm, S.ipiv, mode, S.flag, info);
+    }
   // substitution: circular windows of 32 or 64 (a power of two)
   if (S.n32 > 0) {
     cp.list = S.list32;
@@ -1094,10 +1109,7 @@ static void torn_factor(mgpu_ctx* c, bool tr, const int* cflag, int* info) {
   const TornInt* ti = tr ? S.d_tiT : S.d_ti;
   const int mode = cflag ? RB_FALLBACK : RB_PLAIN;
   const T* blk = B.rows + S.tb_rows;
-  if (S.twmI == 32)
-    rb_lu<T, 32><<<S.nint, 32, 0, st>>>(cpI, B.rows, B.uc, B.lm, S.tpiv, mode, S.iflag, info);
-  else
-    rb_lu<T, 64><<<S.nint, 32, 0, st>>>(cpI, B.rows, B.uc, B.lm, S.tpiv, mode, S.iflag, info);
+  lu_launch<T>(S.tlu, S.nint, cpI, st, B.rows, B.uc, B.lm, S.tpiv, mode, S.iflag, info);
   if (S.nsep == 0) return;
   // forward window: kl+1 of the matrix being factorised (ku for the transpose); both <= s <= 16
   const bool narrow = S.tmaxs <= 15;

@@ -35,8 +35,8 @@ struct Solver {
   int wm = 0;            // row-band register window (32 or 64), 0 if the row-band kernels do not apply
   int n32 = 0, n64 = 0;  // components whose band fits a 32- / needs a 64-wide window (substitution)
   int32_t *list32 = nullptr, *list64 = nullptr;
-  int nlu[4] = {0, 0, 0, 0};  // components by factorisation window: 32, 40, 48, 64
-  int32_t* lulist[4] = {nullptr, nullptr, nullptr, nullptr};
+  int nlu[6] = {0, 0, 0, 0, 0, 0};  // components by factorisation class (lu_class)
+  int32_t* lulist[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   int nref = 8;          // refinement sweeps allowed on the FP32 path
   // row-band layout
   int64_t* rbase = nullptr;   // [ncomp] offset in RB / UC*
@@ -61,6 +61,7 @@ struct Solver {
   int tearable = 0;           // some component is long enough to be cut
   int nint = 0, nsep = 0;
   int twmI = 0;               // register window of the interior kernels
+  int tlu = 0;                // their factorisation class
   int bcr_levels = 0;         // cyclic-reduction levels of the longest separator chain
   int tmaxs = 0;              // largest max(kl, ku) over all components
   TornInt* d_ti = nullptr;    // [nint] interiors (bands of Lλx)
