@@ -714,9 +714,18 @@ MG_HD void tan_jets(const real v[3], const real v1[3], const real v2[3], real s,
 // ∂ẍ/∂X′ = 2J̇ for a Jacobian J), the forces are summed over the Gauss points per
 // mode, and the six rotation rows come from the two sums' moment and couple alone.
 // Without drag that needs the modes' Gram sums only.
-template <class Out>
-MG_HD void beam_newmark(const BeamConst& c, const double* X0, const double* X1, const double* X2, const double* U,
-                        Perturb pt, const double* av, const double* bv, double* R, Out&& out, double* rdir, double* H) {
+// PART splits an element over four threads that repeat its state and share the
+// rest: 1 the residual and the symmetric part (out receives pairs i <= j), 2 to 4 a
+// third of the columns each (out receives the loads' part alone) and of rdir's sums,
+// which `sum` adds up: it returns whether this thread goes on with their total.
+// 0 is the whole element on one thread.
+struct BeamDirSums {
+  real Vm[3], Am[3], Vw[3], Aw[3], vi;
+};
+template <int PART, class Out, class Sum>
+MG_HD void beam_newmark_part(const BeamConst& c, const double* X0, const double* X1, const double* X2, const double* U,
+                             Perturb pt, const double* av, const double* bv, double* R, Out&& out, Sum&& sum,
+                             double* rdir, double* H) {
   SinFun q1, q2;
   BeamState g;
   beam_state(c, X0, q1, q2, g);
@@ -839,33 +848,40 @@ MG_HD void beam_newmark(const BeamConst& c, const double* X0, const double* X1, 
   };
   // ---- loads and their sums
   const real vi = dot3(om1, t);  // vᵢ₂ of the rotational inertia: the spin acceleration about the axis
-  BeamLoads f;
-  for (int i = 0; i < 3; ++i) {
-    f.u[i] = f.a[i] = f.v[i] = f.o[i] = 0.0;
-    f.m[i] = rot ? c.S0 * c.iota1 * vi * t[i] : real(0.0);
-  }
-  for (int k = 0; k < 4; ++k) {
-    real xd[3], xdd[3];
-    point(k, xd, xdd);
-    real fe[3];
-    for (int i = 0; i < 3; ++i) fe[i] = fma(c.mu, xdd[i], (i == 2 ? c.w : 0.0) - (U ? U[i] : 0.0));
-    if (drag)
-      for (int i = 0; i < 3; ++i) {
-        const real x1 = dot3(g.rs + 3 * i, xd), x2 = dot3(g.rs + 3 * i, xdd);
-        axpy3(fma(c.Ca[i], x2, x1 * fma(c.Cq[i], fabs(x1), c.Cl[i])), g.rs + 3 * i, fe);
-      }
+  real Ks[PART == 0 ? 78 : 1];  // the symmetric part, packed by columns: (i, j), i <= j at i + j (j + 1)/2
+  if constexpr (PART <= 1) {
+    BeamLoads f;
     for (int i = 0; i < 3; ++i) {
-      const real w = c.dL[k] * fe[i];
-      f.u[i] = fma(c.yu[k], w, f.u[i]);
-      f.a[i] = fma(yd[k], w, f.a[i]);
-      f.v[i] = fma(c.yv[k], w, f.v[i]);
-      f.o[i] += w;
+      f.u[i] = f.a[i] = f.v[i] = f.o[i] = 0.0;
+      f.m[i] = rot ? c.S0 * c.iota1 * vi * t[i] : real(0.0);
     }
+    for (int k = 0; k < 4; ++k) {
+      real xd[3], xdd[3];
+      point(k, xd, xdd);
+      real fe[3];
+      for (int i = 0; i < 3; ++i) fe[i] = fma(c.mu, xdd[i], (i == 2 ? c.w : 0.0) - (U ? U[i] : 0.0));
+      if (drag)
+        for (int i = 0; i < 3; ++i) {
+          const real x1 = dot3(g.rs + 3 * i, xd), x2 = dot3(g.rs + 3 * i, xdd);
+          axpy3(fma(c.Ca[i], x2, x1 * fma(c.Cq[i], fabs(x1), c.Cl[i])), g.rs + 3 * i, fe);
+        }
+      for (int i = 0; i < 3; ++i) {
+        const real w = c.dL[k] * fe[i];
+        f.u[i] = fma(c.yu[k], w, f.u[i]);
+        f.a[i] = fma(yd[k], w, f.a[i]);
+        f.v[i] = fma(c.yv[k], w, f.v[i]);
+        f.o[i] += w;
+      }
+    }
+    beam_frozen<true>(c, X0, q1, q2, g, f, rot, X[0], X[1], R, [&](int i, int j, real v) {
+      if constexpr (PART == 0)
+        Ks[i + j * (j + 1) / 2] = pt.p0 * v;
+      else
+        out(i, j, pt.p0 * v);
+    });
+    if (H) beam_uload(c, g, X[0], X[1], H);
+    if constexpr (PART == 1) return;
   }
-  // ---- the symmetric part, packed by columns: (i, j), i <= j at i + j (j + 1)/2
-  real Ks[78];
-  beam_frozen<true>(c, X0, q1, q2, g, f, rot, X[0], X[1], R, [&](int i, int j, real v) { Ks[i + j * (j + 1) / 2] = pt.p0 * v; });
-  if (H) beam_uload(c, g, X[0], X[1], H);
   // Dₛᵀ of vₛₘ: ∂vₛₘ = Dₛ ω, Dₛ = ι B − ι' q qᵀ, B = ½(tr I − rₛₘ)
   real io[3] = {0.0, 0.0, 0.0}, vq[3], tau[3];
   const real trs = g.rs[0] + g.rs[4] + g.rs[8];
@@ -951,15 +967,22 @@ MG_HD void beam_newmark(const BeamConst& c, const double* X0, const double* X1, 
     }
   };
   auto put = [&](int j, const real col[12]) {
-    for (int i = 0; i < 12; ++i) out(i, j, Ks[i <= j ? i + j * (j + 1) / 2 : j + i * (i + 1) / 2] + col[i]);
+    for (int i = 0; i < 12; ++i) {
+      if constexpr (PART == 0)
+        out(i, j, Ks[i <= j ? i + j * (j + 1) / 2 : j + i * (i + 1) / 2] + col[i]);
+      else
+        out(i, j, col[i]);
+    }
   };
-  // sums of the rdir direction
-  real rVm[3] = {0, 0, 0}, rAm[3] = {0, 0, 0}, rVw[3] = {0, 0, 0}, rAw[3] = {0, 0, 0}, rvi = 0.0;
+  BeamDirSums r{};
   const real zero[3] = {0.0, 0.0, 0.0};
-  // ---- rotation columns
+  // ---- rotation columns (one thread's whole element keeps the loops: fewer spills)
+#pragma unroll (PART == 0 ? 1 : 2)
   for (int a = 0; a < 2; ++a) {
     const real sg = a ? 1.0 : -1.0;
+#pragma unroll (PART == 0 ? 1 : 3)
     for (int j = 0; j < 3; ++j) {
+      if (PART > 1 && (3 * a + j) / 2 != PART - 2) continue;
       const real* x = X[a] + 3 * j;
       const real* y1 = Xd[a] + 3 * j;
       real x1[3], x2[3];  // ẋ, ẍ of the column: the frame turns with sp
@@ -1029,13 +1052,13 @@ MG_HD void beam_newmark(const BeamConst& c, const double* X0, const double* X1, 
       const real ts0 = dot3(t, s0), ts1 = fma(2.0, dot3(t, s1), dot3(t1, s0));
       if (rdir) {
         const real aj = av[3 + 6 * a + j], bj = bv[3 + 6 * a + j];
-        axpy3(aj, jm, rVm);
-        axpy3(2.0 * aj, jm1, rAm);
-        axpy3(bj, jm, rAm);
-        axpy3(aj, jw, rVw);
-        axpy3(2.0 * aj, jw1, rAw);
-        axpy3(bj, jw, rAw);
-        rvi = fma(aj, ts1, fma(bj, ts0, rvi));
+        axpy3(aj, jm, r.Vm);
+        axpy3(2.0 * aj, jm1, r.Am);
+        axpy3(bj, jm, r.Am);
+        axpy3(aj, jw, r.Vw);
+        axpy3(2.0 * aj, jw1, r.Aw);
+        axpy3(bj, jw, r.Aw);
+        r.vi = fma(aj, ts1, fma(bj, ts0, r.vi));
       }
       real Am[3], Aw[3], Fu[3], Fm[3], Fv[3], F1[3], rho[3] = {0.0, 0.0, 0.0}, col[12];
       for (int i = 0; i < 3; ++i) {
@@ -1076,7 +1099,9 @@ MG_HD void beam_newmark(const BeamConst& c, const double* X0, const double* X1, 
     }
   }
   // ---- translation columns: d moves by ∓½, the midpoint by ½
+#pragma unroll (PART == 0 ? 1 : 3)
   for (int j = 0; j < 3; ++j) {
+    if (PART > 1 && j != PART - 2) continue;
     real Am[3], Fu[3], Fm[3], Fv[3], F1[3], c1[12], c2[12], ca_[12], cb_[12];
     for (int i = 0; i < 3; ++i) {
       const real M = t[i] * t[j], M1 = fma(t1[i], t[j], t[i] * t1[j]),
@@ -1086,8 +1111,8 @@ MG_HD void beam_newmark(const BeamConst& c, const double* X0, const double* X1, 
     if (rdir) {
       const real aj = 0.5 * (av[6 + j] - av[j]), bj = 0.5 * (bv[6 + j] - bv[j]);
       for (int i = 0; i < 3; ++i) {
-        rVm[i] = fma(aj * t[j], t[i], rVm[i]);
-        rAm[i] = fma(2.0 * aj, fma(t1[i], t[j], t[i] * t1[j]), fma(bj * t[j], t[i], rAm[i]));
+        r.Vm[i] = fma(aj * t[j], t[i], r.Vm[i]);
+        r.Am[i] = fma(2.0 * aj, fma(t1[i], t[j], t[i] * t1[j]), fma(bj * t[j], t[i], r.Am[i]));
       }
     }
     if (drag) {
@@ -1139,35 +1164,41 @@ MG_HD void beam_newmark(const BeamConst& c, const double* X0, const double* X1, 
     put(6 + j, cb_);
   }
   // ---- the direction X′ += av, X″ += bv
-  if (rdir) {
+  if (rdir && sum(r)) {
     real Fu[3], Fm[3], Fv[3], F1[3], col[12], rho[3], dv1[3], dv2[3], cv1[3], cv2[3];
     for (int i = 0; i < 3; ++i) {
       dv1[i] = 0.5 * (av[6 + i] - av[i]);
       dv2[i] = 0.5 * (bv[6 + i] - bv[i]);
       cv1[i] = 0.5 * (av[i] + av[6 + i]);
       cv2[i] = 0.5 * (bv[i] + bv[6 + i]);
-      rho[i] = rot ? c.S0 * c.iota1 * rvi * tau[i] : real(0.0);
+      rho[i] = rot ? c.S0 * c.iota1 * r.vi * tau[i] : real(0.0);
     }
     if (drag) {
       dragsum(
           [&](int k, real V[3], real A[3]) {
             for (int i = 0; i < 3; ++i) {
-              V[i] = fma(c.yu[k], dv1[i], fma(yd[k], rVm[i], fma(c.yv[k], rVw[i], cv1[i])));
-              A[i] = fma(c.yu[k], dv2[i], fma(yd[k], rAm[i], fma(c.yv[k], rAw[i], cv2[i])));
+              V[i] = fma(c.yu[k], dv1[i], fma(yd[k], r.Vm[i], fma(c.yv[k], r.Vw[i], cv1[i])));
+              A[i] = fma(c.yu[k], dv2[i], fma(yd[k], r.Am[i], fma(c.yv[k], r.Aw[i], cv2[i])));
             }
           },
           nullptr, Fu, Fm, Fv, F1);
     } else {
       for (int i = 0; i < 3; ++i) {
-        Fu[i] = fma(Guu, dv2[i], fma(Gud, rAm[i], fma(Guv, rAw[i], Gu * cv2[i])));
-        Fm[i] = fma(Gud, dv2[i], fma(Gdd, rAm[i], fma(Gdv, rAw[i], Gd * cv2[i])));
-        Fv[i] = fma(Guv, dv2[i], fma(Gdv, rAm[i], fma(Gvv, rAw[i], Gv * cv2[i])));
-        F1[i] = fma(Gu, dv2[i], fma(Gd, rAm[i], fma(Gv, rAw[i], G1 * cv2[i])));
+        Fu[i] = fma(Guu, dv2[i], fma(Gud, r.Am[i], fma(Guv, r.Aw[i], Gu * cv2[i])));
+        Fm[i] = fma(Gud, dv2[i], fma(Gdd, r.Am[i], fma(Gdv, r.Aw[i], Gd * cv2[i])));
+        Fv[i] = fma(Guv, dv2[i], fma(Gdv, r.Am[i], fma(Gvv, r.Aw[i], Gv * cv2[i])));
+        F1[i] = fma(Gu, dv2[i], fma(Gd, r.Am[i], fma(Gv, r.Aw[i], G1 * cv2[i])));
       }
     }
     rows(Fu, Fm, Fv, F1, rho, col);
     for (int i = 0; i < 12; ++i) rdir[i] = to_d(col[i]);
   }
+}
+
+template <class Out>
+MG_HD void beam_newmark(const BeamConst& c, const double* X0, const double* X1, const double* X2, const double* U,
+                        Perturb pt, const double* av, const double* bv, double* R, Out&& out, double* rdir, double* H) {
+  beam_newmark_part<0>(c, X0, X1, X2, U, pt, av, bv, R, out, [](BeamDirSums&) { return true; }, rdir, H);
 }
 
 }  // namespace mgpu

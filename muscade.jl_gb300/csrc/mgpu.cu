@@ -189,6 +189,108 @@ __global__ void __launch_bounds__(256) beam_kernel(int64_t nele, const int32_t* 
   flag_nan(a.errflag, gid0 + e, bad);
 }
 
+// The same for models that leave sub-partitions idle: 32 beams a block, their four
+// parts (beam_newmark_part) on a warp each, joined in shared memory.  A warp's FP64
+// stream is what a small model waits for (each instruction holds its sub-partition
+// for 64 cycles), and the parts' streams are less than half of the whole element's.
+// Newmark kernel, µs (a thread per beam / split; a wave of the first is 19,456 beams):
+//   beams       20       1,000      5,000     10,000     15,000     30,000
+//   mass only   328/168  314/133    309/211   310/318    312/420    564/723
+//   with drag   508/228  498/189    494/303   495/459    497/609    933/1064
+constexpr int64_t kSplitMaxBeams = 9000;
+constexpr int kSplitEntries = 144 + 78 + 12 + 3 * 13;  // columns, symmetric part, direction, its sums
+constexpr size_t kSplitSmem = size_t(kSplitEntries) * 32 * sizeof(double);
+
+template <bool STEP>
+__global__ void __launch_bounds__(128) beam_split_kernel(int64_t nele, const int32_t* __restrict__ idx,
+                                                         const int32_t* __restrict__ uidx,
+                                                         const double* __restrict__ cdata,
+                                                         const int32_t* __restrict__ aidx,
+                                                         const double* __restrict__ Avec, AsmArgs a,
+                                                         double* __restrict__ rout, double* __restrict__ kout,
+                                                         int64_t gid0) {
+  extern __shared__ double sh[];
+  const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
+  double* col = sh + lane;                // entry q of this lane's beam at 32 q
+  double* sym = col + 32 * 144;           // (i, j), i <= j at i + j (j + 1)/2
+  double* dir = sym + 32 * 78;
+  double* dsum = dir + 32 * 12;           // [part − 1][13]
+  const int64_t e0 = int64_t(blockIdx.x) * 32 + lane;
+  const bool live = e0 < nele;
+  const int64_t e = live ? e0 : nele - 1;  // the last block's spare lanes repeat a beam and store nothing
+  BeamConst bc;
+  load_soa(bc, cdata, nele, e);
+  if (aidx) scale_bending(bc, __ldg(Avec + __ldg(aidx + e)));
+  double X0[12], X1[12], X2[12], av[12], bv[12];
+#pragma unroll
+  for (int i = 0; i < 12; ++i) {
+    const int dof = __ldg(idx + i * nele + e);
+    X0[i] = __ldg(a.x0 + dof);
+    X1[i] = __ldg(a.x1 + dof);
+    X2[i] = __ldg(a.x2 + dof);
+    if constexpr (STEP) {
+      av[i] = __ldg(a.av + dof);
+      bv[i] = __ldg(a.bv + dof);
+    }
+  }
+  double U[3];
+  const bool has_u = uidx != nullptr;
+  if (has_u)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) U[k] = __ldg(a.u + __ldg(uidx + k * nele + e));
+  const Perturb pt{a.p0, a.sc[1], a.sc[4]};
+  const double* u = has_u ? U : nullptr;
+  double R[12], rd[12];
+  auto put = [&](int i, int j, double v) { col[32 * (i + 12 * j)] = v; };
+  auto puts = [&](int i, int j, double v) { sym[32 * (i + j * (j + 1) / 2)] = v; };
+  auto nosum = [](BeamDirSums&) { return false; };
+  // the three column warps' sums of the direction; the first goes on with the total
+  auto sum = [&](BeamDirSums& r) {
+    double* p = reinterpret_cast<double*>(&r);
+#pragma unroll
+    for (int q = 0; q < 13; ++q) dsum[32 * (13 * (part - 1) + q)] = p[q];
+    __syncthreads();
+    if (part != 1) return false;
+#pragma unroll
+    for (int q = 0; q < 13; ++q) p[q] = (p[q] + dsum[32 * (13 + q)]) + dsum[32 * (26 + q)];
+    return true;
+  };
+  if (part == 0) {
+    beam_newmark_part<1>(bc, X0, X1, X2, u, pt, av, bv, R, puts, nosum, nullptr, nullptr);
+    if constexpr (STEP) __syncthreads();  // the sums'
+  } else if (part == 1) {
+    beam_newmark_part<2>(bc, X0, X1, X2, u, pt, av, bv, R, put, sum, STEP ? rd : nullptr, nullptr);
+    if constexpr (STEP)
+#pragma unroll
+      for (int i = 0; i < 12; ++i) dir[32 * i] = rd[i];
+  } else if (part == 2) {
+    beam_newmark_part<3>(bc, X0, X1, X2, u, pt, av, bv, R, put, sum, STEP ? rd : nullptr, nullptr);
+  } else {
+    beam_newmark_part<4>(bc, X0, X1, X2, u, pt, av, bv, R, put, sum, STEP ? rd : nullptr, nullptr);
+  }
+  __syncthreads();
+  if (!live) return;
+  bool bad = false;
+  // 36 entries of the matrix a warp
+#pragma unroll 4
+  for (int q = 36 * part; q < 36 * part + 36; ++q) {
+    const int i = q % 12, j = q / 12;
+    double v = sym[32 * (i <= j ? i + j * (j + 1) / 2 : j + i * (i + 1) / 2)] + col[32 * q];
+    if (a.scale) v *= __ldg(a.scale + __ldg(idx + i * nele + e)) * __ldg(a.scale + __ldg(idx + j * nele + e));
+    bad |= nan_bits(v);
+    kout[q * nele + e] = v;
+  }
+  if (part == 0)
+#pragma unroll
+    for (int i = 0; i < 12; ++i) {
+      double r = STEP ? R[i] - dir[32 * i] : R[i];
+      if (a.scale) r *= __ldg(a.scale + __ldg(idx + i * nele + e));
+      bad |= nan_bits(r);
+      rout[i * nele + e] = r;
+    }
+  flag_nan(a.errflag, gid0 + e, bad);
+}
+
 __global__ void bar_kernel(int64_t nele, int nder, const int32_t* __restrict__ idx, const int32_t* __restrict__ uidx,
                            const double* __restrict__ cdata, AsmArgs a, double* __restrict__ rout,
                            double* __restrict__ kout, int64_t gid0) {
@@ -496,7 +598,11 @@ int launch_assembly(mgpu_ctx* c, int mission, cudaEvent_t* ev_groups, double p0)
     if (G.tval_base >= 0) ag.tv = c->tv + G.tval_base;
     switch (G.kind) {
       case MGPU_EULERBEAM3D:
-        if (mission == MGPU_ASM_STEP)
+        if (dyn && G.nele <= kSplitMaxBeams) {
+          const auto kern = mission == MGPU_ASM_STEP ? beam_split_kernel<true> : beam_split_kernel<false>;
+          kern<<<nblk(G.nele, 32), 128, kSplitSmem, c->stream>>>(G.nele, G.idx, G.uidx, G.cdata, G.aidx, c->Avec, ag,
+                                                                 rout, kout, gid0);
+        } else if (mission == MGPU_ASM_STEP)
           beam_kernel<true><<<nblk(G.nele, c->elem_block), c->elem_block, 0, c->stream>>>(
               G.nele, G.idx, G.uidx, G.cdata, G.aidx, c->Avec, ag, rout, kout, gid0);
         else if (dyn)
@@ -612,6 +718,8 @@ extern "C" int mgpu_create(mgpu_ctx** out, const mgpu_model_desc* d) {
   c->device = d->device;
   MG_CUDA(cudaSetDevice(d->device));
   MG_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
+  for (auto kern : {beam_split_kernel<false>, beam_split_kernel<true>})
+    MG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSplitSmem)));
   c->nX = d->nX;
   c->nU = d->nU;
   if (d->nX < 0 || d->nU < 0 || d->ngroup < 0 || (d->ngroup > 0 && !d->groups))

@@ -76,14 +76,14 @@ static void narrow_by_nodes(int64_t n, const std::vector<int64_t>& deg, const st
     return w;
   };
   std::vector<int32_t> todo, wid(members.size());
-#pragma omp parallel for schedule(dynamic, 16)
+#pragma omp parallel for schedule(dynamic, 16) if (n > 50000)
   for (int64_t cc = 0; cc < int64_t(members.size()); ++cc) wid[cc] = width(members[cc]);
   // one 6-dof node next to another needs 11; wider than 48 is no chain
   for (size_t cc = 0; cc < members.size(); ++cc)
     if (wid[cc] > 11 && wid[cc] <= 48 && members[cc].size() > 2) todo.push_back(int32_t(cc));
   if (todo.empty()) return;
   std::vector<int32_t> nb(adj.size()), cnt(n, 0), grp(n, -1), host(n, -1);  // sorted neighbours, each once
-#pragma omp parallel for schedule(dynamic, 16)
+#pragma omp parallel for schedule(dynamic, 16) if (n > 50000)
   for (int64_t t = 0; t < int64_t(todo.size()); ++t) {
     const auto& M = members[todo[t]];
     const int32_t c0 = comp_start[todo[t]], w0 = wid[todo[t]];
