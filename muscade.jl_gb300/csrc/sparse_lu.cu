@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <type_traits>
+#include <utility>
 
 #include "ctx.hpp"
 #include "sparse_analysis.hpp"
@@ -41,6 +42,16 @@ __device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) {
 constexpr size_t kUpd32Smem = size_t(2) * 64 * (128 + 4) * sizeof(float);  // sp_update_f32<64> tiles
 constexpr double kRefineTol = 1e-14;   // scaled correction / scaled solution: converged
 constexpr double kRefineStall = 1e-10;  // ... or stalled below this
+
+// f(0), f(1), .., f(N − 1) with constant arguments
+template <class F, int... K>
+__device__ __forceinline__ void unrolled(std::integer_sequence<int, K...>, F&& f) {
+  (f(std::integral_constant<int, K>{}), ...);
+}
+template <int N, class F>
+__device__ __forceinline__ void unrolled(F&& f) {
+  unrolled(std::make_integer_sequence<int, N>{}, f);
+}
 
 inline unsigned nblocks(int64_t n, int b) { return unsigned((n + b - 1) / b); }
 
@@ -105,8 +116,8 @@ __global__ void __launch_bounds__(kThreads) sp_extend_add(const SpFrontDev* __re
 // Stage the kb × kb block at (k0, k0) of a column-major front (leading
 // dimension m) into Dg, 8 loads per thread in flight before their stores (a
 // load-then-store loop would wait for each load in turn).
-template <class T, int NB>
-__device__ __forceinline__ void stage_diag_block(const T* __restrict__ A, int m, int k0, int kb, T (*Dg)[NB + 1]) {
+template <class T, int NB, int LD = NB + 1>
+__device__ __forceinline__ void stage_diag_block(const T* __restrict__ A, int m, int k0, int kb, T (*Dg)[LD]) {
   const int n = kb * kb, nt = int(blockDim.x);
   for (int t0 = int(threadIdx.x); t0 < n; t0 += 8 * nt) {
     T v[8];
@@ -223,7 +234,7 @@ __global__ void __launch_bounds__(kThreads) sp_panel(const SpFrontDev* __restric
 // [nrc, nrc + ncc) 64 columns of the U panel, a warp taking eight columns at
 // once (lanes over rows) so that eight substitution chains interleave.
 template <class T, int NB>
-__global__ void __launch_bounds__(kThreads) sp_panel_f(const SpFrontDev* __restrict__ fr,
+__global__ void __launch_bounds__(kThreads, 2) sp_panel_f(const SpFrontDev* __restrict__ fr,
                                                        const int32_t* __restrict__ flist, int k0,
                                                        T* __restrict__ F) {
   const SpFrontDev Fr = fr[flist[blockIdx.y]];
@@ -234,61 +245,36 @@ __global__ void __launch_bounds__(kThreads) sp_panel_f(const SpFrontDev* __restr
   const int nrc = (rest + kThreads - 1) / kThreads, ncc = (rest + 63) / 64;
   if (int(blockIdx.x) >= nrc + ncc) return;
   T* A = F + Fr.off;
-  __shared__ T Dg[NB][NB + 1];
+  __shared__ __align__(16) T Dg[NB][NB + 4];
   __shared__ T rdg[NB];  // reciprocal pivots: no division on the rows' substitution chains
   const int tid = threadIdx.x;
-  stage_diag_block<T, NB>(A, m, k0, kb, Dg);
+  if (kb < NB) {
+    for (int t = tid; t < NB * NB; t += kThreads) Dg[t / NB][t % NB] = T(0);
+    __syncthreads();
+  }
+  stage_diag_block<T, NB, NB + 4>(A, m, k0, kb, Dg);
   if (tid < kb) rdg[tid] = T(1) / A[(k0 + tid) + int64_t(k0 + tid) * m];
   __syncthreads();
   const int b = blockIdx.x;
   if (b < nrc) {
-    // one row per thread, x U₁₁ = a; for NB = 64 in two halves of 32 columns
-    // (the second half first takes the first half's products, in the same
-    // order as a single pass), so that 32 values, not 64, are live
+    // one row per thread in registers, x U₁₁ = a; the rows of U₁₁ are read 16 bytes at
+    // a time (one shared-memory read per product bound these blocks before)
     const int i = r0 + b * kThreads + tid;
     if (i < m) {
       T* row = A + i;
-      constexpr int H = NB > 32 ? NB / 2 : NB;
-      {
-        T x[H];
+      T x[NB];
 #pragma unroll
-        for (int c = 0; c < H; ++c) x[c] = c < kb ? row[int64_t(k0 + c) * m] : T(0);
+      for (int c = 0; c < NB; ++c) x[c] = c < kb ? row[int64_t(k0 + c) * m] : T(0);
 #pragma unroll
-        for (int c = 0; c < H; ++c) {
-          if (c < kb) {
-            x[c] *= rdg[c];
+      for (int c = 0; c < NB; ++c) {
+        if (c >= kb) break;
+        x[c] *= rdg[c];
 #pragma unroll
-            for (int t = c + 1; t < H; ++t)
-              if (t < kb) x[t] -= x[c] * Dg[c][t];
-          }
-        }
-#pragma unroll
-        for (int c = 0; c < H; ++c)
-          if (c < kb) row[int64_t(k0 + c) * m] = x[c];
+        for (int t = c + 1; t < NB; ++t) x[t] -= x[c] * Dg[c][t];  // zero beyond kb
       }
-      if constexpr (NB > H) {
-        T y[NB - H];
 #pragma unroll
-        for (int t = 0; t < NB - H; ++t) y[t] = H + t < kb ? row[int64_t(k0 + H + t) * m] : T(0);
-        for (int c = 0; c < H && c < kb; ++c) {
-          const T xc = row[int64_t(k0 + c) * m];
-#pragma unroll
-          for (int t = 0; t < NB - H; ++t)
-            if (H + t < kb) y[t] -= xc * Dg[c][H + t];
-        }
-#pragma unroll
-        for (int c = 0; c < NB - H; ++c) {
-          if (H + c < kb) {
-            y[c] *= rdg[H + c];
-#pragma unroll
-            for (int t = c + 1; t < NB - H; ++t)
-              if (H + t < kb) y[t] -= y[c] * Dg[H + c][H + t];
-          }
-        }
-#pragma unroll
-        for (int t = 0; t < NB - H; ++t)
-          if (H + t < kb) row[int64_t(k0 + H + t) * m] = y[t];
-      }
+      for (int c = 0; c < NB; ++c)
+        if (c < kb) row[int64_t(k0 + c) * m] = x[c];
     }
     return;
   }
@@ -665,10 +651,10 @@ __global__ void __launch_bounds__(tc::kTcThreads) sp_rect_tc(const SpFrontDev* _
 
 // the diagonal block of pivot block k0 factored in place in every listed front
 // (before sp_panel_f, which reads it factored), with the arithmetic of
-// factor_diag: NB threads, thread i owning row i of the staged block; one
-// block barrier per step (after it, row k is final).  Every thread applies the
-// pivot rule to its read of the pivot itself (the rule is idempotent, so the
-// owner's write-back of a raised pivot cannot change what another reads).
+// factor_diag: NB threads, thread i owning row i in registers; the owner of the
+// pivot row hands it round through shared memory (two buffers, one block barrier
+// per step).  Bound by that chain of NB steps: with the block in shared memory a
+// step also waited for its row's loads and stores (NB = 64: 45 -> 22 us).
 template <class T, int NB>
 __global__ void __launch_bounds__(NB) sp_diag_store(const SpFrontDev* __restrict__ fr,
                                                     const int32_t* __restrict__ flist, int k0, T* __restrict__ F,
@@ -677,44 +663,53 @@ __global__ void __launch_bounds__(NB) sp_diag_store(const SpFrontDev* __restrict
   const int m = Fr.m, p = Fr.p;
   if (k0 >= p) return;
   const int kb = min(NB, p - k0);
-  T* A = F + Fr.off;
-  __shared__ T Dg[NB][NB + 1];
   const int i = threadIdx.x;
-  stage_diag_block<T, NB>(A, m, k0, kb, Dg);
-  for (int k = 0; k < kb; ++k) {
-    __syncthreads();
-    const T d = Dg[k][k];
-    const bool bad = !isfinite(d) || (d == T(0) && tau == T(0));
-    const bool raise = !bad && fabs(d) < tau;
-    const T piv = raise ? (d < T(0) ? -tau : tau) : d;
+  T* A = F + Fr.off + (k0 + i) + int64_t(k0) * m;  // row i of the block
+  constexpr int V = 16 / sizeof(T);  // entries of a 16-byte access
+  struct __align__(16) Quad {
+    T e[V];
+  };
+  __shared__ Quad row[2][NB / V];
+  T a[NB];
+#pragma unroll
+  for (int j = 0; j < NB; ++j) a[j] = (i < kb && j < kb) ? A[int64_t(j) * m] : T(0);
+  unrolled<NB>([&](auto step) {  // the steps written out: a[] stays in registers
+    constexpr int k = decltype(step)::value;
+    if (k >= kb) return;
     if (i == k) {
+      const T d = a[k];
+      const bool bad = !isfinite(d) || (d == T(0) && tau == T(0));
       if (bad) atomicOr(flags + 3, 1);
-      if (raise) {
-        Dg[k][k] = piv;
+      if (!bad && fabs(d) < tau) {
+        a[k] = d < T(0) ? -tau : tau;
         atomicAdd(flags + 2, 1);
       }
-    } else if (i > k && i < kb) {
-      const T l = Dg[i][k] / piv;
-      Dg[i][k] = l;
-      // eight entries of row k and of row i loaded before any is stored (the
-      // compiler cannot tell the rows apart, so a plain loop would wait for
-      // each load behind the previous store)
-      for (int j0 = k + 1; j0 < kb; j0 += 8) {
-        T u[8], r[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          u[q] = j0 + q < kb ? Dg[k][j0 + q] : T(0);
-          r[q] = j0 + q < kb ? Dg[i][j0 + q] : T(0);
-        }
+      for (int q = k / V; q < NB / V; ++q) {
+        Quad v;
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
-          if (j0 + q < kb) Dg[i][j0 + q] = r[q] - l * u[q];
+        for (int e = 0; e < V; ++e) v.e[e] = a[V * q + e];
+        row[k & 1][q] = v;
       }
     }
-  }
-  __syncthreads();
-  for (int j = 0; j < kb; ++j)
-    if (i < kb) A[(k0 + i) + int64_t(k0 + j) * m] = Dg[i][j];
+    __syncthreads();
+    if (i > k) {
+      Quad u = row[k & 1][k / V];
+      const T l = a[k] / u.e[k % V];
+      a[k] = l;
+#pragma unroll
+      for (int q = k / V; q < NB / V; ++q) {
+        if (q > k / V) u = row[k & 1][q];
+#pragma unroll
+        for (int e = 0; e < V; ++e)
+          if (V * q + e > k) a[V * q + e] -= l * u.e[e];
+      }
+    }
+  });
+  if (i < kb)
+#pragma unroll
+    for (int j = 0; j < NB; ++j)
+      if (j < kb) A[int64_t(j) * m] = a[j];
 }
 
 // FP32 trailing update on the tensor cores: one 128 × 128 tile per block
@@ -773,7 +768,7 @@ __global__ void __launch_bounds__(tc::kTcThreads) tc_gemm_check(const float* __r
 // rectangular part (L₂₁ y or U₁₂ x_u), one row per thread summing in column
 // order.  Vectors are FP64, factors T.
 constexpr int kTriThreads = 512;
-constexpr int kGemvRows = 256;
+constexpr int kGemvThreads = 256;
 
 // forward, triangle: v = the front's pivot entries plus the children's update
 // vectors (in child order); y = L₁₁⁻¹ v[0:p] -> w; v[p:m] (the children's part of
@@ -832,51 +827,70 @@ __global__ void __launch_bounds__(kTriThreads) sp_fwd_tri(const SpFrontDev* __re
     for (int t = p + tid; t < m; t += kTriThreads) cvec[Fr.eoff + (t - p)] = v[t];
 }
 
-// forward, rectangle: cvec[f][t] -= Σ_c L₂₁[t, c] y_c for the update rows t of
-// every front of the height (y staged in shared memory)
+// Σ_c M[c ld] y[c] of 32 rows (one per lane; row < 32 rows valid when `in`) by the
+// block's warps, each a run of columns in FP64, the runs added in order: a row's
+// products are FP64 instructions (64 cycles each, and the conversions), and one
+// thread a row left all but a few warps idle on the small fronts (12 x 12 x 6
+// lattice: bwd_gemv 40 -> 9 us a launch, fwd_gemv 13 -> 4).  Only the first warp
+// gets the sum.
 template <class T>
-__global__ void __launch_bounds__(kGemvRows) sp_fwd_gemv(const SpFrontDev* __restrict__ fr,
-                                                         const int32_t* __restrict__ flist, const T* __restrict__ F,
-                                                         const double* __restrict__ w, double* __restrict__ cvec,
-                                                         const int* __restrict__ conv) {
+__device__ __forceinline__ double sp_rows_dot(const T* __restrict__ M, int64_t ld, int n, const double* __restrict__ y,
+                                              bool in, double (*part)[32]) {
+  constexpr int NW = kGemvThreads / 32;
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int c0 = int(int64_t(n) * wp / NW), c1 = int(int64_t(n) * (wp + 1) / NW);
+  double s = 0.0;
+  if (in)
+#pragma unroll 8
+    for (int c = c0; c < c1; ++c) s += double(M[int64_t(c) * ld]) * y[c];
+  part[wp][lane] = s;
+  __syncthreads();
+  double t = 0.0;
+  if (wp == 0)
+#pragma unroll
+    for (int q = 0; q < NW; ++q) t += part[q][lane];
+  return t;
+}
+
+// forward, rectangle: cvec[f][t] -= Σ_c L₂₁[t, c] y_c for the update rows t of
+// every front of the height (y staged in shared memory), 32 rows a block
+template <class T>
+__global__ void __launch_bounds__(kGemvThreads) sp_fwd_gemv(const SpFrontDev* __restrict__ fr,
+                                                            const int32_t* __restrict__ flist,
+                                                            const T* __restrict__ F, const double* __restrict__ w,
+                                                            double* __restrict__ cvec, const int* __restrict__ conv) {
   if (*conv) return;
   const SpFrontDev Fr = fr[flist[blockIdx.y]];
   const int m = Fr.m, p = Fr.p, u = m - p;
-  if (Fr.parent < 0 || int(blockIdx.x) * kGemvRows >= u) return;
+  if (Fr.parent < 0 || int(blockIdx.x) * 32 >= u) return;
   extern __shared__ double y[];
-  for (int c = threadIdx.x; c < p; c += kGemvRows) y[c] = w[Fr.pos0 + c];
+  __shared__ double part[kGemvThreads / 32][32];
+  for (int c = threadIdx.x; c < p; c += kGemvThreads) y[c] = w[Fr.pos0 + c];
   __syncthreads();
-  const int t = blockIdx.x * kGemvRows + threadIdx.x;
-  if (t >= u) return;
-  const T* L = F + Fr.off + p + t;  // row p+t of the front, column c at L[c*m]
-  double s = 0.0;
-#pragma unroll 8
-  for (int c = 0; c < p; ++c) s += double(L[int64_t(c) * m]) * y[c];
-  cvec[Fr.eoff + t] -= s;
+  const int t = blockIdx.x * 32 + (threadIdx.x & 31);
+  const double s = sp_rows_dot(F + Fr.off + p + t, m, p, y, t < u, part);  // row p+t of the front
+  if (threadIdx.x < 32 && t < u) cvec[Fr.eoff + t] -= s;
 }
 
 // backward, rectangle: tw[pos0 + r] = Σ_{j ≥ p} U₁₂[r, j] x_j for the pivot rows r
-// (x_u the ancestors' solved values, staged in shared memory)
+// (x_u the ancestors' solved values, staged in shared memory), 32 rows a block
 template <class T>
-__global__ void __launch_bounds__(kGemvRows) sp_bwd_gemv(const SpFrontDev* __restrict__ fr,
-                                                         const int32_t* __restrict__ flist,
-                                                         const int32_t* __restrict__ fidx, const T* __restrict__ F,
-                                                         const double* __restrict__ w, double* __restrict__ tw,
-                                                         const int* __restrict__ conv) {
+__global__ void __launch_bounds__(kGemvThreads) sp_bwd_gemv(const SpFrontDev* __restrict__ fr,
+                                                            const int32_t* __restrict__ flist,
+                                                            const int32_t* __restrict__ fidx, const T* __restrict__ F,
+                                                            const double* __restrict__ w, double* __restrict__ tw,
+                                                            const int* __restrict__ conv) {
   if (*conv) return;
   const SpFrontDev Fr = fr[flist[blockIdx.y]];
   const int m = Fr.m, p = Fr.p, u = m - p;
-  if (int(blockIdx.x) * kGemvRows >= p) return;
+  if (int(blockIdx.x) * 32 >= p) return;
   extern __shared__ double xu[];
-  for (int j = threadIdx.x; j < u; j += kGemvRows) xu[j] = w[fidx[Fr.idx + p + j]];
+  __shared__ double part[kGemvThreads / 32][32];
+  for (int j = threadIdx.x; j < u; j += kGemvThreads) xu[j] = w[fidx[Fr.idx + p + j]];
   __syncthreads();
-  const int r = blockIdx.x * kGemvRows + threadIdx.x;
-  if (r >= p) return;
-  const T* U = F + Fr.off + r + int64_t(p) * m;  // row r, column p+j at U[j*m]
-  double s = 0.0;
-#pragma unroll 8
-  for (int j = 0; j < u; ++j) s += double(U[int64_t(j) * m]) * xu[j];
-  tw[Fr.pos0 + r] = s;
+  const int r = blockIdx.x * 32 + (threadIdx.x & 31);
+  const double s = sp_rows_dot(F + Fr.off + r + int64_t(p) * m, m, u, xu, r < p, part);  // columns p..m−1 of row r
+  if (threadIdx.x < 32 && r < p) tw[Fr.pos0 + r] = s;
 }
 
 // backward, triangle: x[0:p] = U₁₁⁻¹ (y − U₁₂ x_u) -> w
@@ -1695,9 +1709,9 @@ cudaError_t refine(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, int 
         sp_fwd_tri<T><<<unsigned(nsmall), kTriThreads, smem, st>>>(sp.d_fr, fs, sp.d_clist, sp.d_emap, F, sp.w,
                                                                     sp.cvec, sp.flags);
         ++c->launches;
-        const int ur = (sp.h_sumax[h] + kGemvRows - 1) / kGemvRows;
+        const int ur = (sp.h_sumax[h] + 31) / 32;
         for (int f0 = 0; f0 < nsmall && ur > 0; f0 += kMaxGridY) {
-          sp_fwd_gemv<T><<<dim3(unsigned(ur), unsigned(std::min(kMaxGridY, nsmall - f0))), kGemvRows,
+          sp_fwd_gemv<T><<<dim3(unsigned(ur), unsigned(std::min(kMaxGridY, nsmall - f0))), kGemvThreads,
                            size_t(sp.h_spmax[h]) * sizeof(double), st>>>(sp.d_fr, fs + f0, F, sp.w, sp.cvec, sp.flags);
           ++c->launches;
         }
@@ -1739,9 +1753,9 @@ cudaError_t refine(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, int 
       const int nbig = sp.h_nbig[h], nsmall = sp.h_nlf[h] - nbig;
       if (nsmall > 0) {
         const int32_t* fs = fl + nbig;
-        const int pr = (sp.h_spmax[h] + kGemvRows - 1) / kGemvRows;
+        const int pr = (sp.h_spmax[h] + 31) / 32;
         for (int f0 = 0; f0 < nsmall; f0 += kMaxGridY) {
-          sp_bwd_gemv<T><<<dim3(unsigned(pr), unsigned(std::min(kMaxGridY, nsmall - f0))), kGemvRows,
+          sp_bwd_gemv<T><<<dim3(unsigned(pr), unsigned(std::min(kMaxGridY, nsmall - f0))), kGemvThreads,
                            size_t(std::max(sp.h_sumax[h], 1)) * sizeof(double), st>>>(sp.d_fr, fs + f0, sp.d_fidx, F,
                                                                                       sp.w, sp.tw, sp.flags);
           ++c->launches;
