@@ -335,73 +335,85 @@ __global__ void bar_kernel(int64_t nele, int nder, const int32_t* __restrict__ i
   flag_nan(a.errflag, gid0 + e, bad);
 }
 
+// The element types of a few operations per element (constraints, loads, costs), all
+// of a model's groups in one launch: apart they were up to ten launches of 2 µs each
+// in an assembly, a tenth of a small model's Newton iteration.
+struct SmallGroup {
+  int32_t kind, nX;
+  int64_t nele, gid0;
+  const int32_t* idx;
+  const int32_t* uidx;
+  const double* cdata;
+  const double* tv;
+  double* rout;
+  double* kout;
+  unsigned block0;  // first block of the group
+};
+constexpr int kSmallGroups = 32;  // per launch
+struct SmallGroups {
+  int n;
+  SmallGroup g[kSmallGroups];
+};
+static_assert(sizeof(SmallGroups) + sizeof(AsmArgs) < 4000, "kernel parameters");
+
 // DofConstraint{:X} in equal mode with gap g = Σ aᵢ xᵢ − c(t):
 // R = [−aᵢ λ ; −g]  (src/BasicElements.jl:426-438)
-__global__ void constraint_kernel(int64_t nele, int nX, const int32_t* __restrict__ idx,
-                                  const double* __restrict__ cdata, const double* __restrict__ tv, AsmArgs a,
-                                  double* __restrict__ rout, double* __restrict__ kout, int64_t gid0) {
-  const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (e >= nele) return;
-  const int nx = nX - 1;
-  const int dl = __ldg(idx + nx * nele + e);
+__device__ bool constraint_element(const SmallGroup& G, const AsmArgs& a, int64_t e) {
+  const int64_t nele = G.nele;
+  const int nX = G.nX, nx = nX - 1;
+  const int dl = __ldg(G.idx + nx * nele + e);
   const double lam = __ldg(a.x0 + dl);
   const double sl = a.scale ? __ldg(a.scale + dl) : 1.0;
-  double gap = -__ldg(tv + e);
+  double gap = -__ldg(G.tv + e);
   bool bad = false;
   for (int i = 0; i < nx; ++i) {
-    const int di = __ldg(idx + i * nele + e);
-    const double ci = __ldg(cdata + i * nele + e);
+    const int di = __ldg(G.idx + i * nele + e);
+    const double ci = __ldg(G.cdata + i * nele + e);
     gap += ci * __ldg(a.x0 + di);
     const double si = a.scale ? __ldg(a.scale + di) : 1.0;
     const double r = -ci * lam * si;
     bad |= isnan(r);
-    rout[i * nele + e] = r;
-    for (int j = 0; j < nX; ++j) kout[(i + nX * j) * nele + e] = (j == nx) ? -ci * si * sl * a.p0 : 0.0;
+    G.rout[i * nele + e] = r;
+    for (int j = 0; j < nX; ++j) G.kout[(i + nX * j) * nele + e] = (j == nx) ? -ci * si * sl * a.p0 : 0.0;
   }
-  rout[nx * nele + e] = -gap * sl;
+  G.rout[nx * nele + e] = -gap * sl;
   bad |= isnan(gap);
   for (int j = 0; j < nX; ++j) {
     double k = 0.0;
     if (j < nx) {
-      const int dj = __ldg(idx + j * nele + e);
+      const int dj = __ldg(G.idx + j * nele + e);
       const double sj = a.scale ? __ldg(a.scale + dj) : 1.0;
-      k = -__ldg(cdata + j * nele + e) * sl * sj * a.p0;
+      k = -__ldg(G.cdata + j * nele + e) * sl * sj * a.p0;
     }
-    kout[(nx + nX * j) * nele + e] = k;
+    G.kout[(nx + nX * j) * nele + e] = k;
   }
-  flag_nan(a.errflag, gid0 + e, bad);
+  return bad;
 }
 
-// DofLoad: R = −F(t), zero tangent entry (src/BasicElements.jl:281-284)
-__global__ void load_kernel(int64_t nele, const int32_t* __restrict__ idx, const double* __restrict__ tv, AsmArgs a,
-                            double* __restrict__ rout, double* __restrict__ kout, int64_t gid0) {
-  const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (e >= nele) return;
-  const int d = __ldg(idx + e);
-  const double s = a.scale ? __ldg(a.scale + d) : 1.0;
-  const double r = -__ldg(tv + e) * s;
-  rout[e] = r;
-  kout[e] = 0.0;
-  flag_nan(a.errflag, gid0 + e, isnan(r));
-}
-
-// SingleDofCost and SingleUdof in SweepX: the residual of a Lagrangian
-// element is ∂L/∂Λ (src/Assemble.jl:661-677), 0 for a cost and −u for the
-// U-dof load of SingleUdof (L = cost(u,t) − λu); the tangents are zero.
-__global__ void cost_kernel(int64_t nele, int udof, const int32_t* __restrict__ idx,
-                            const int32_t* __restrict__ uidx, AsmArgs a, double* __restrict__ rout,
-                            double* __restrict__ kout, int64_t gid0) {
-  const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (e >= nele) return;
+// DofLoad: R = −F(t), zero tangent entry (src/BasicElements.jl:281-284).
+// SingleDofCost and SingleUdof in SweepX: the residual of a Lagrangian element is
+// ∂L/∂Λ (src/Assemble.jl:661-677), 0 for a cost and −u for the U-dof load of
+// SingleUdof (L = cost(u,t) − λu); the tangents are zero.
+__device__ bool dof_element(const SmallGroup& G, const AsmArgs& a, int64_t e) {
   double r = 0.0;
-  if (udof) {
-    const int d = __ldg(idx + e);
-    const double s = a.scale ? __ldg(a.scale + d) : 1.0;
-    r = -__ldg(a.u + __ldg(uidx + e)) * s;
+  if (G.kind != MGPU_DOFCOST) {
+    const double s = a.scale ? __ldg(a.scale + __ldg(G.idx + e)) : 1.0;
+    r = -(G.kind == MGPU_DOFLOAD ? __ldg(G.tv + e) : __ldg(a.u + __ldg(G.uidx + e))) * s;
   }
-  rout[e] = r;
-  kout[e] = 0.0;
-  flag_nan(a.errflag, gid0 + e, isnan(r));
+  G.rout[e] = r;
+  G.kout[e] = 0.0;
+  return isnan(r);
+}
+
+__global__ void __launch_bounds__(256) small_groups_kernel(const __grid_constant__ SmallGroups S,
+                                                           const __grid_constant__ AsmArgs a) {
+  int q = 0;
+  while (q + 1 < S.n && blockIdx.x >= S.g[q + 1].block0) ++q;
+  const SmallGroup& G = S.g[q];
+  const int64_t e = int64_t(blockIdx.x - G.block0) * blockDim.x + threadIdx.x;
+  if (e >= G.nele) return;
+  const bool bad = G.kind == MGPU_DOFCONSTRAINT_X ? constraint_element(G, a, e) : dof_element(G, a, e);
+  flag_nan(a.errflag, G.gid0 + e, bad);
 }
 
 // Deterministic gather-sum:
@@ -429,16 +441,27 @@ __device__ __forceinline__ double plus_zero(double v) {
   return __double_as_longlong(v) == (long long)0x8000000000000000ULL ? 0.0 : v;
 }
 
-__global__ void __launch_bounds__(kGatherThreads) scatter_kernel(int64_t n, const uint32_t* __restrict__ seg,
-                                                                 const uint32_t* __restrict__ src,
-                                                                 const double* __restrict__ buf,
-                                                                 double* __restrict__ out) {
+// One launch for the matrix (the first bm blocks) and the vector.
+struct GatherPlan {
+  int64_t n;
+  const uint32_t* seg;
+  const uint32_t* src;
+  const double* buf;
+  double* out;
+};
+__global__ void __launch_bounds__(kGatherThreads) scatter_kernel(GatherPlan mat, GatherPlan vec, unsigned bm) {
+  const bool isv = blockIdx.x >= bm;
+  const int64_t n = isv ? vec.n : mat.n;
+  const uint32_t* __restrict__ seg = isv ? vec.seg : mat.seg;
+  const uint32_t* __restrict__ src = isv ? vec.src : mat.src;
+  const double* __restrict__ buf = isv ? vec.buf : mat.buf;
+  double* __restrict__ out = isv ? vec.out : mat.out;
   __shared__ uint32_t sseg[kGatherOut + 1];
   __shared__ double sval[kGatherStage];
   __shared__ int16_t slist[kGatherOut];
   __shared__ int nlist;
   const int tid = threadIdx.x, lane = tid & 31;
-  const int64_t k0 = int64_t(blockIdx.x) * kGatherOut;
+  const int64_t k0 = int64_t(blockIdx.x - (isv ? bm : 0u)) * kGatherOut;
   const int nk = int(n - k0 < kGatherOut ? n - k0 : kGatherOut);
   for (int t = tid; t <= nk; t += kGatherThreads) sseg[t] = __ldg(seg + k0 + t);
   if (tid == 0) nlist = 0;
@@ -586,6 +609,16 @@ int launch_assembly(mgpu_ctx* c, int mission, cudaEvent_t* ev_groups, double p0)
     ++c->launches;
   }
   int64_t gid0 = 0;
+  SmallGroups small;  // the groups that share a launch (each its own when it is timed)
+  small.n = 0;
+  unsigned sblocks = 0;
+  auto flush_small = [&] {
+    if (small.n == 0) return;
+    small_groups_kernel<<<sblocks, 256, 0, c->stream>>>(small, a);
+    ++c->launches;
+    small.n = 0;
+    sblocks = 0;
+  };
   for (size_t g = 0; g < c->groups.size(); ++g) {
     const DevGroup& G = c->groups[g];
     if (G.nele == 0) {
@@ -620,31 +653,25 @@ int launch_assembly(mgpu_ctx* c, int mission, cudaEvent_t* ev_groups, double p0)
                                                              kout, gid0);
         break;
       case MGPU_DOFCONSTRAINT_X:
-        constraint_kernel<<<nblk(G.nele, 256), 256, 0, c->stream>>>(G.nele, G.nX, G.idx, G.cdata, ag.tv, ag, rout,
-                                                                    kout, gid0);
-        break;
       case MGPU_DOFLOAD:
-        load_kernel<<<nblk(G.nele, 256), 256, 0, c->stream>>>(G.nele, G.idx, ag.tv, ag, rout, kout, gid0);
-        break;
       case MGPU_DOFCOST:
       case MGPU_SINGLEUDOF:
-        cost_kernel<<<nblk(G.nele, 256), 256, 0, c->stream>>>(G.nele, G.kind == MGPU_SINGLEUDOF, G.idx, G.uidx, ag,
-                                                              rout, kout, gid0);
+        small.g[small.n++] = SmallGroup{G.kind, G.nX, G.nele, gid0, G.idx, G.uidx, G.cdata, ag.tv, rout, kout, sblocks};
+        sblocks += nblk(G.nele, 256);
+        if (ev_groups || small.n == kSmallGroups) flush_small();
         break;
       case MGPU_ACOST:  // no X-dofs: nothing in SweepX's Lλ and Lλx
         break;
     }
-    if (G.kind != MGPU_ACOST) ++c->launches;
+    if (G.kind == MGPU_EULERBEAM3D || G.kind == MGPU_BAR3D) ++c->launches;
     gid0 += G.nele;
     if (ev_groups) cudaEventRecord(ev_groups[g], c->stream);
   }
-  if (c->pat.nnz > 0) {
-    scatter_kernel<<<nblk(c->pat.nnz, kGatherOut), kGatherThreads, 0, c->stream>>>(c->pat.nnz, c->mseg, c->msrc,
-                                                                                  c->kbuf, c->nzval);
-    ++c->launches;
-  }
-  if (nX > 0) {
-    scatter_kernel<<<nblk(nX, kGatherOut), kGatherThreads, 0, c->stream>>>(nX, c->vseg, c->vsrc, c->rbuf, c->Ll);
+  flush_small();
+  const unsigned bm = nblk(c->pat.nnz, kGatherOut), bv = nblk(nX, kGatherOut);
+  if (bm + bv > 0) {
+    scatter_kernel<<<bm + bv, kGatherThreads, 0, c->stream>>>(
+        GatherPlan{c->pat.nnz, c->mseg, c->msrc, c->kbuf, c->nzval}, GatherPlan{nX, c->vseg, c->vsrc, c->rbuf, c->Ll}, bm);
     ++c->launches;
   }
   cudaError_t e = cudaGetLastError();

@@ -656,7 +656,8 @@ static void analyse(mgpu_ctx* c, Solver& S) {
   good = good && cudaMalloc(&S.rhs, n * sizeof(double)) == cudaSuccess;
   good = good && cudaMalloc(&S.rdiag, n * sizeof(double)) == cudaSuccess;
   good = good && cudaMalloc(&S.dx, n * sizeof(double)) == cudaSuccess;
-  good = good && cudaMalloc(&S.red, 4 * sizeof(double)) == cudaSuccess;
+  good = good && cudaMalloc(&S.red, 4 * sizeof(double)) == cudaSuccess &&
+         cudaMemsetAsync(S.red, 0, 4 * sizeof(double), c->stream) == cudaSuccess;
   good = good && cudaMalloc(&S.part, 2 * kNormBlocks * sizeof(double)) == cudaSuccess;
   good = good && cudaMalloc(&S.info, kInfoSlots * sizeof(int)) == cudaSuccess &&
          cudaMemset(S.info, 0, kInfoSlots * sizeof(int)) == cudaSuccess;
@@ -690,39 +691,47 @@ static void analyse(mgpu_ctx* c, Solver& S) {
 }
 
 // ---------------------------------------------------------------- kernels
-// Σ Δx², Σ Lλ²: kNormBlocks partial sums (fixed assignment and tree order), then
-// one block adds the partials in index order -- deterministic for a given n
-__global__ void __launch_bounds__(256) norms_partial(int64_t n, const double* dx, const double* Ll, double* part) {
+// Σ Δx², Σ Lλ²: partial sums of up to kNormBlocks blocks (fixed assignment and tree
+// order); the block that ends last adds the partials, again by a fixed tree, so the
+// sums are deterministic for a given n.  (A second kernel's single thread adding 128
+// partials took 11 µs of every Newton iteration.)  done: zero between launches.
+__global__ void __launch_bounds__(256) norms_kernel(int64_t n, const double* dx, const double* Ll, double* part,
+                                                    unsigned* done, double* red) {
   __shared__ double s1[256], s2[256];
+  __shared__ bool last;
+  auto tree = [&](double a, double b) {
+    s1[threadIdx.x] = a;
+    s2[threadIdx.x] = b;
+    __syncthreads();
+    for (int s = 128; s > 0; s >>= 1) {
+      if (threadIdx.x < s) {
+        s1[threadIdx.x] += s1[threadIdx.x + s];
+        s2[threadIdx.x] += s2[threadIdx.x + s];
+      }
+      __syncthreads();
+    }
+  };
   double a = 0.0, b = 0.0;
   for (int64_t i = int64_t(blockIdx.x) * 256 + threadIdx.x; i < n; i += int64_t(gridDim.x) * 256) {
     a += dx[i] * dx[i];
     b += Ll[i] * Ll[i];
   }
-  s1[threadIdx.x] = a;
-  s2[threadIdx.x] = b;
-  __syncthreads();
-  for (int s = 128; s > 0; s >>= 1) {
-    if (threadIdx.x < s) {
-      s1[threadIdx.x] += s1[threadIdx.x + s];
-      s2[threadIdx.x] += s2[threadIdx.x + s];
-    }
-    __syncthreads();
-  }
+  tree(a, b);
   if (threadIdx.x == 0) {
     part[2 * blockIdx.x] = s1[0];
     part[2 * blockIdx.x + 1] = s2[0];
+    __threadfence();
+    last = atomicInc(done, gridDim.x - 1) == gridDim.x - 1;  // wraps to zero
   }
-}
-__global__ void norms_final(int nb, const double* part, double* red) {
-  if (threadIdx.x != 0) return;
-  double a = 0.0, b = 0.0;
-  for (int k = 0; k < nb; ++k) {
-    a += part[2 * k];
-    b += part[2 * k + 1];
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const bool in = threadIdx.x < gridDim.x;
+  tree(in ? __ldcg(part + 2 * threadIdx.x) : 0.0, in ? __ldcg(part + 2 * threadIdx.x + 1) : 0.0);
+  if (threadIdx.x == 0) {
+    red[0] = s1[0];
+    red[1] = s2[0];
   }
-  red[0] = a;
-  red[1] = b;
 }
 
 // Per-component convergence for independent models solved together: ΣΔx² and
@@ -798,7 +807,10 @@ static int ensure_sparse(mgpu_ctx* c, Solver& S) {
   // the Newton loop's buffers (the banded analysis allocates them only when it applies)
   const int64_t n = std::max<int64_t>(c->nX, 1);
   if (!S.dx) MG_CUDA(cudaMalloc(&S.dx, n * sizeof(double)));
-  if (!S.red) MG_CUDA(cudaMalloc(&S.red, 4 * sizeof(double)));
+  if (!S.red) {
+    MG_CUDA(cudaMalloc(&S.red, 4 * sizeof(double)));
+    MG_CUDA(cudaMemsetAsync(S.red, 0, 4 * sizeof(double), c->stream));
+  }
   if (!S.part) MG_CUDA(cudaMalloc(&S.part, 2 * kNormBlocks * sizeof(double)));
   if (!S.info) {
     MG_CUDA(cudaMalloc(&S.info, kInfoSlots * sizeof(int)));
@@ -1311,9 +1323,9 @@ int factor_solve(mgpu_ctx* c, int* info) {
     // FP64: the whole solve (PATH_F64ROWS) or the components flagged above
     rb_launch<double>(S, cp, st, S.RB, S.UC64, S.LM64, c->Ll, S.tw64, S.dx, 0, mode64, nullptr, info);
   }
-  norms_partial<<<kNormBlocks, 256, 0, st>>>(c->nX, S.dx, c->Ll, S.part);
-  norms_final<<<1, 32, 0, st>>>(kNormBlocks, S.part, S.red);
-  c->launches += 2;
+  norms_kernel<<<std::max(1u, std::min(unsigned(kNormBlocks), nb(c->nX, 256))), 256, 0, st>>>(
+      c->nX, S.dx, c->Ll, S.part, reinterpret_cast<unsigned*>(S.red + 2), S.red);
+  ++c->launches;
   MG_CUDA(cudaGetLastError());
   return MGPU_OK;
 }
