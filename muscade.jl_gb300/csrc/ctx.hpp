@@ -25,6 +25,7 @@ struct DevGroup {
   std::vector<int64_t> h_indexA;  // host copy (1-based)
   double* cdata = nullptr;  // [nfield][nele] kernel constants (structure of arrays)
   int32_t nfield = 0;
+  double* fields = nullptr;  // EULERBEAM3D: the element records [nele][69], after the first mgpu_beam_results
   int64_t tval_base = -1;   // offset in the time-value vector (loads, constraints, cost targets)
   int32_t maxder = 0;       // DOFCOST: highest time derivative a cost reads
   bool distinct = true;     // cost groups: no two elements write the same gradient entry
@@ -67,6 +68,8 @@ struct mgpu_ctx {
   double* flush = nullptr;  // L2 flush buffer
   size_t flush_bytes = 0;
   int nXder_resident = 1;
+  double* res_work = nullptr;  // mgpu_beam_results: states and results of a call
+  size_t res_bytes = 0;
   // host: coordinates of each X-dof's node from the beam and bar elements'
   // geometry (NaN where no element gives one) and the constraint multipliers;
   // the sparse solver's ordering uses them
