@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -70,6 +71,7 @@ struct mgpu_ctx {
   int nXder_resident = 1;
   double* res_work = nullptr;  // mgpu_beam_results: states and results of a call
   size_t res_bytes = 0;
+  std::mutex res_lock;  // its owner
   // host: coordinates of each X-dof's node from the beam and bar elements'
   // geometry (NaN where no element gives one) and the constraint multipliers;
   // the sparse solver's ordering uses them

@@ -1330,6 +1330,7 @@ extern "C" int mgpu_beam_results(mgpu_ctx* c, int32_t g, int64_t nstate, const d
   const int64_t n = G.nele * nstate;
   if (n == 0) return MGPU_OK;
   MG_CUDA(cudaSetDevice(c->device));
+  std::lock_guard<std::mutex> own(c->res_lock);
   // workspace [X | results], kept for the next call up to kResKeep bytes
   constexpr size_t kResKeep = size_t(256) << 20;
   const size_t nx = size_t(nstate) * c->nX, bytes = (nx + size_t(n) * kRes) * sizeof(double);
