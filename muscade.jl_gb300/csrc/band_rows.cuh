@@ -101,6 +101,19 @@ enum RbMode : int {
   RB_PLAIN = 2      // all components; a zero pivot is an error (info)
 };
 
+// per interior of a partitioned component (band_torn.cuh): where its data lives
+struct TornInt {
+  int64_t rbase, lbase;  // row-band storage and multipliers (as RbComp)
+  int32_t n, kl, ku;     // size and bands of the interior
+  int32_t dof0;          // offset of its dofs in perm
+  int32_t s;             // separator width of its component
+  int64_t eL, eR, fL, fR;  // offsets of E^L, E^R, F^L, F^R in the block array, -1 if absent
+  int64_t yL, yR;          // offsets of Y^L, Y^R (m x s), -1 if absent
+  int32_t sepL, sepR;      // global index of the left / right separator, -1 if absent
+  int32_t comp;            // connected component it belongs to
+  int32_t end;             // 1: an end of its component, held as [factors | coupling] (tb_end)
+};
+
 struct RbComp {
   const int64_t* rbase;  // [ncomp] offset of the component in A and UC
   const int64_t* lbase;  // [ncomp] offset in LM
@@ -331,7 +344,8 @@ struct RbSmem {
   static constexpr int bytes = (kL > kU ? kL : kU) * int(sizeof(T));
 };
 
-// t = (LU)^-1 P in for one component, by one warp.  `in` is FP64 (the
+// t = (LU)^-1 P in for one component, by one warp (rb_fb), in its two halves:
+// t = L^-1 P in (rb_fwd), t = U^-1 t (rb_bwd).  `in` is FP64 (the
 // right-hand side or a residual), `t` receives the result in T.  L and U
 // stream through shared memory in chunks of 32 columns (cp.async, double
 // buffered).  The vector entries ride in circular register windows; the lane
@@ -339,13 +353,10 @@ struct RbSmem {
 // (backward), and since each lane refills once per chunk, those values and
 // the pivots are loaded a whole chunk ahead into registers no per-column
 // instruction reads.
-template <typename T, int WM>
-__device__ void rb_fb(int n, int kl, int kv, int w, const T* __restrict__ U, const T* __restrict__ L,
-                      const int32_t* __restrict__ piv, const double* __restrict__ in, T* __restrict__ t,
-                      unsigned char* smem, int lane) {
-  constexpr int NS = WM / 32, M = WM;  // backward window modulus (a power of two, >= kv + 1)
+template <typename T>
+__device__ void rb_fwd(int n, int kl, const T* __restrict__ L, const int32_t* __restrict__ piv,
+                       const double* __restrict__ in, T* __restrict__ t, unsigned char* smem, int lane) {
   T* sL = reinterpret_cast<T*>(smem);
-  T* sU = reinterpret_cast<T*>(smem);
   const int nch = (n + 31) >> 5;
   // ---- forward: entry k' lives on lane k' & 31; window k..k+kl
   auto load_fchunk = [&](int c) {
@@ -398,6 +409,14 @@ __device__ void rb_fb(int n, int kl, int kv, int w, const T* __restrict__ U, con
   rb_cp_wait<0>();
   __threadfence_block();
   __syncwarp();
+}
+
+// t = U^-1 t
+template <typename T, int WM>
+__device__ void rb_bwd(int n, int kv, int w, const T* __restrict__ U, T* t, unsigned char* smem, int lane) {
+  constexpr int NS = WM / 32, M = WM;  // window modulus (a power of two, >= kv + 1)
+  T* sU = reinterpret_cast<T*>(smem);
+  const int nch = (n + 31) >> 5;
   // ---- backward: entry k' lives on lane k' & 31, slot (k' mod M) >> 5; window k-kv..k
   auto load_bchunk = [&](int c, int buf) {
     const int k0 = c * 32, k1 = min(n, k0 + 32);
@@ -453,6 +472,14 @@ __device__ void rb_fb(int n, int kl, int kv, int w, const T* __restrict__ U, con
   __syncwarp();
 }
 
+template <typename T, int WM>
+__device__ void rb_fb(int n, int kl, int kv, int w, const T* __restrict__ U, const T* __restrict__ L,
+                      const int32_t* __restrict__ piv, const double* __restrict__ in, T* __restrict__ t,
+                      unsigned char* smem, int lane) {
+  rb_fwd<T>(n, kl, L, piv, in, t, smem, lane);
+  rb_bwd<T, WM>(n, kv, w, U, t, smem, lane);
+}
+
 // Δx for every component: b = P_rcm Lλ, x = (LU)^-1 b, then (T = float)
 // sweeps of iterative refinement r = b - A x (FP64, unfactorised rows),
 // x += (LU)^-1 r until the correction is below 1e-12 of x (max norms).  The
@@ -468,7 +495,7 @@ __global__ void __launch_bounds__(32) rb_solve(RbComp cp, const int32_t* __restr
                                               const double* __restrict__ Ll, double* __restrict__ bw,
                                               double* __restrict__ xw, double* __restrict__ rw, T* __restrict__ tw,
                                               double* __restrict__ dx, int nref, int mode, int* __restrict__ flag,
-                                              int* __restrict__ nsweep) {
+                                              int* __restrict__ nsweep, const TornInt* __restrict__ ti) {
   __shared__ __align__(16) unsigned char smem[RbSmem<T, WM>::bytes];
   const int cc = cp.list ? cp.list[blockIdx.x] : int(blockIdx.x), lane = threadIdx.x;
   if (mode == RB_FALLBACK && flag[cc] == 0) return;
@@ -486,7 +513,10 @@ __global__ void __launch_bounds__(32) rb_solve(RbComp cp, const int32_t* __restr
   T* t = tw + d0;
   for (int k = lane; k < n; k += 32) b[k] = Ll[pm[k]];
   __syncwarp();
-  rb_fb<T, WM>(n, kl, kv, w, U, L, piv, b, t, smem, lane);
+  if (ti && ti[cc].end)  // an end interior of a partitioned component: L^-1 P b only
+    rb_fwd<T>(n, kl, L, piv, b, t, smem, lane);
+  else
+    rb_fb<T, WM>(n, kl, kv, w, U, L, piv, b, t, smem, lane);
   double xn = 0.0, dn = 0.0;
   for (int k = lane; k < n; k += 32) {
     const double v = double(t[k]);

@@ -33,18 +33,6 @@
 
 namespace mgpu {
 
-// per interior: where its data lives
-struct TornInt {
-  int64_t rbase, lbase;  // row-band storage and multipliers (as RbComp)
-  int32_t n, kl, ku;     // size and bands of the interior
-  int32_t dof0;          // offset of its dofs in perm
-  int32_t s;             // separator width of its component
-  int64_t eL, eR, fL, fR;  // offsets of E^L, E^R, F^L, F^R in the block array, -1 if absent
-  int64_t yL, yR;          // offsets of Y^L, Y^R (m x s), -1 if absent
-  int32_t sepL, sepR;      // global index of the left / right separator, -1 if absent
-  int32_t comp;            // connected component it belongs to
-};
-
 // per separator
 struct TornSep {
   int32_t s;
@@ -60,6 +48,89 @@ struct TornSep {
 // only[comp] == 0 skips the component (FP64 fallback after an FP32 factorisation);
 // only == nullptr runs all
 __device__ __forceinline__ bool tb_skip(const int* only, int comp) { return only && only[comp] == 0; }
+
+// ---------------------------------------------------------------- end interiors
+// An interior with one separator needs no spike: with the separator after its last
+// row (the last interior of a component is numbered backwards for that), the
+// separator is only the next rows of the same elimination,
+//     T_kk -= G Z,   r_k -= G z,   x_a = U^-1 (z - Z x_S),   z = L^-1 P b_a,
+// with Z = L^-1 P E^R, nonzero in the last s + kl rows, and G = F^R U^-1, from the
+// last s rows of U alone.  Both come from the last s + kl pivot steps, where the
+// spikes cost kl + kv FMAs a row over the whole interior, half as much again as its
+// LU (512 frame chains of 60 to 2,400 dofs, five interiors each: 1.7 of 3.9 ms).  Y^R's room holds G (rows 0..s) and Z (its own rows); n >= 2 s + kl, since
+// interiors have at least 48 rows and s <= 16.
+template <typename T, int KLW>
+__device__ void tb_end(const TornInt& I, const T* __restrict__ U, const T* __restrict__ L,
+                       const int32_t* __restrict__ piv, const T* __restrict__ blk, T* __restrict__ Y, T* sU, T* sL,
+                       int* sP, int lane) {
+  const int m = I.n, kl = I.kl, w = I.kl + I.ku + 1, s = I.s, k0 = m - s - kl;
+  for (int e = lane; e < (m - k0) * kl; e += 32) sL[e] = L[int64_t(k0) * kl + e];
+  for (int e = lane; e < s * w; e += 32) sU[e] = U[int64_t(m - s) * w + e];
+  if (lane < m - k0) sP[lane] = piv[k0 + lane] - (k0 + lane);
+  __syncwarp();
+  if (lane >= s) return;
+  // Z, a column per lane: window rows k..k+kl, the first of E^R entering at row m - s
+  const T* eR = blk + I.eR + lane;
+  T* Yr = Y + I.yR + lane;
+  T yw[KLW];
+#pragma unroll
+  for (int p = 0; p < KLW; ++p) yw[p] = p == kl ? eR[0] : T(0);
+  for (int k = k0; k < m; ++k) {
+    const int km = min(kl, m - 1 - k), jp = sP[k - k0];
+    if (jp != 0) {
+      T v = yw[0];
+#pragma unroll
+      for (int p = 1; p < KLW; ++p) v = (p == jp) ? yw[p] : v;
+      const T y0 = yw[0];
+      yw[0] = v;
+#pragma unroll
+      for (int p = 1; p < KLW; ++p) yw[p] = (p == jp) ? y0 : yw[p];
+    }
+    const T yk = yw[0];
+    Yr[int64_t(k) * s] = yk;
+    const T* lk = sL + (k - k0) * kl;
+#pragma unroll
+    for (int p = 1; p < KLW; ++p)
+      if (p <= km) yw[p] = fma(-lk[p - 1], yk, yw[p]);
+    const int r = k + 1 + kl - (m - s);  // row entering the window
+    const T nx = r < s ? eR[int64_t(r) * s] : T(0);
+#pragma unroll
+    for (int p = 0; p < KLW; ++p) yw[p] = p < kl ? yw[min(p + 1, KLW - 1)] : p == kl ? nx : yw[p];
+  }
+  // G, a row per lane
+  T g[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    if (j < s) {
+      T v = blk[I.fR + lane * s + j];
+#pragma unroll
+      for (int q = 0; q < j; ++q) v = fma(-sU[j * w + j - q], g[q], v);
+      g[j] = v * sU[j * w];  // 1/U(j,j)
+      Y[I.yR + lane * s + j] = g[j];
+    }
+  }
+}
+
+// F^R (or G) of a separator's left interior and the rows it meets, and the same of its
+// right interior (F^L, or G of one numbered backwards)
+template <typename T>
+struct TornSides {
+  const T *fl, *fr;  // s x s
+  int64_t yl, yr;    // offsets in Y of the s rows next to the separator
+  int32_t pl, pr;    // band positions of these rows
+};
+template <typename T>
+__device__ __forceinline__ TornSides<T> tb_sides(const TornInt& IL, const TornInt& IR, const T* blk, const T* Y) {
+  TornSides<T> r;
+  const int s = IL.s;
+  r.fl = IL.end ? Y + IL.yR : blk + IL.fR;
+  r.yl = IL.yR + int64_t(IL.n - s) * s;
+  r.pl = IL.dof0 + IL.n - s;
+  r.fr = IR.end ? Y + IR.yR : blk + IR.fL;
+  r.yr = IR.end ? IR.yR + int64_t(IR.n - s) * s : IR.yL;
+  r.pr = IR.end ? IR.dof0 + IR.n - s : IR.dof0;
+  return r;
+}
 
 // ---------------------------------------------------------------- spikes
 // One warp per interior with at least one separator.  Lane r < s computes
@@ -88,6 +159,10 @@ __global__ void __launch_bounds__(32) tb_spikes(int nint, const TornInt* __restr
   const T* U = UC + I.rbase;
   const T* L = LM + I.lbase;
   const int32_t* piv = ipiv + I.dof0;
+  if (I.end) {
+    tb_end<T, KLW>(I, U, L, piv, blk, Y, sU, sL, sP, lane);
+    return;
+  }
   const bool isL = lane < s, isR = lane >= s && lane < 2 * s;
   const bool act = (isL && I.sepL >= 0) || (isR && I.sepR >= 0);
   const int col = isL ? lane : lane - s;
@@ -193,16 +268,17 @@ __global__ void __launch_bounds__(32) tb_schur(int nsep, const TornSep* __restri
   if (tb_skip(only, S.comp)) return;
   const int s = S.s;
   const TornInt IL = ti[S.intL], IR = ti[S.intR];
+  const TornSides<T> sd = tb_sides<T>(IL, IR, blk, Y);
   T* Dk = DLU + 3 * int64_t(k) * BCR_SS;
   T* Uk = Dk + 2 * BCR_SS;
   T* Lk1 = DLU + (3 * int64_t(k + 1) + 1) * BCR_SS;  // L of the next separator (only when !S.last)
   for (int e = lane; e < s * s; e += 32) {
     const int i = e / s, j = e % s;
     // T_kk = D - F^R_{left} Y^R_{left}[last s rows] - F^L_{right} Y^L_{right}[first s rows]
-    const T* FR = blk + IL.fR;
-    const T* YR = Y + IL.yR + int64_t(IL.n - s) * s;
-    const T* FL = blk + IR.fL;
-    const T* YL = Y + IR.yL;
+    const T* FR = sd.fl;
+    const T* YR = Y + sd.yl;
+    const T* FL = sd.fr;
+    const T* YL = Y + sd.yr;
     T a1 = T(0), a2 = T(0);
     for (int q = 0; q < s; ++q) {
       a1 = fma(FR[i * s + q], YR[q * s + j], a1);
@@ -231,20 +307,20 @@ __global__ void __launch_bounds__(32) tb_schur(int nsep, const TornSep* __restri
 // the factors' type, stored in FP64.  One warp; yl, yr: s entries of scratch.
 template <typename T>
 __device__ void tb_sep_rhs_warp(const TornSep& S, const TornInt* __restrict__ ti, const T* __restrict__ blk,
-                                const int32_t* __restrict__ perm, const double* b, const double* x, double* tr,
+                                const T* __restrict__ Y, const int32_t* __restrict__ perm, const double* b, const double* x, double* tr,
                                 T* yl, T* yr, int lane) {
   const int s = S.s;
-  const TornInt IL = ti[S.intL], IR = ti[S.intR];
+  const TornSides<T> sd = tb_sides<T>(ti[S.intL], ti[S.intR], blk, Y);
   if (lane < s) {
-    yl[lane] = T(x[perm[IL.dof0 + IL.n - s + lane]]);
-    yr[lane] = T(x[perm[IR.dof0 + lane]]);
+    yl[lane] = T(x[perm[sd.pl + lane]]);
+    yr[lane] = T(x[perm[sd.pr + lane]]);
   }
   __syncwarp();
   if (lane < s) {
     T v = T(b[perm[S.dof0 + lane]]);
     for (int q = 0; q < s; ++q) {
-      v -= blk[IL.fR + lane * s + q] * yl[q];
-      v -= blk[IR.fL + lane * s + q] * yr[q];
+      v -= sd.fl[lane * s + q] * yl[q];
+      v -= sd.fr[lane * s + q] * yr[q];
     }
     tr[S.trow + lane] = double(v);
   }
@@ -254,7 +330,8 @@ __device__ void tb_sep_rhs_warp(const TornSep& S, const TornInt* __restrict__ ti
 template <typename T>
 __global__ void __launch_bounds__(32) tb_sep_rhs(int nsep, const TornSep* __restrict__ ts,
                                                  const TornInt* __restrict__ ti, const T* __restrict__ blk,
-                                                 const int32_t* __restrict__ perm, const double* __restrict__ b,
+                                                 const T* __restrict__ Y, const int32_t* __restrict__ perm,
+                                                 const double* __restrict__ b,
                                                  const double* __restrict__ x, double* __restrict__ tr,
                                                  const int* __restrict__ only) {
   __shared__ T yl[BCR_S], yr[BCR_S];
@@ -262,16 +339,17 @@ __global__ void __launch_bounds__(32) tb_sep_rhs(int nsep, const TornSep* __rest
   if (k >= nsep) return;
   const TornSep S = ts[k];
   if (tb_skip(only, S.comp)) return;
-  tb_sep_rhs_warp(S, ti, blk, perm, b, x, tr, yl, yr, threadIdx.x);
+  tb_sep_rhs_warp(S, ti, blk, Y, perm, b, x, tr, yl, yr, threadIdx.x);
 }
 
 // x_a -= Y^L_a x_S_a + Y^R_a x_S_a+1 (interior dofs), x_S = T solution (separator dofs);
 // arithmetic in the factors' type (with FP32 factors this is a refinement
-// correction).  One warp; xl, xr: s entries of scratch.
-template <typename T>
-__device__ void tb_back_warp(const TornInt& I, const TornSep* __restrict__ ts, const T* __restrict__ Y,
-                             const int32_t* __restrict__ perm, const double* txs, double* x, T* xl, T* xr,
-                             int lane) {
+// correction).  An end interior: its last s + kl rows of z in tw, then the backward
+// substitution.  One warp; xl, xr: s entries of scratch.
+template <typename T, int WM>
+__device__ void tb_back_warp(const TornInt& I, int a, const TornSep* __restrict__ ts, const T* __restrict__ UC,
+                             const T* __restrict__ Y, const int32_t* __restrict__ perm, const double* txs, T* tw,
+                             double* x, T* xl, T* xr, unsigned char* smem, int lane) {
   const int s = I.s;
   const bool hl = I.sepL >= 0, hr = I.sepR >= 0;
   if (!(hl || hr)) return;
@@ -280,32 +358,42 @@ __device__ void tb_back_warp(const TornInt& I, const TornSep* __restrict__ ts, c
     xr[lane] = hr ? T(txs[ts[I.sepR].trow + lane]) : T(0);
   }
   __syncwarp();
-  for (int i = lane; i < I.n; i += 32) {
+  for (int i = (I.end ? I.n - s - I.kl : 0) + lane; i < I.n; i += 32) {
     T v = T(x[perm[I.dof0 + i]]);
     for (int q = 0; q < s; ++q) {
       if (hl) v -= Y[I.yL + int64_t(i) * s + q] * xl[q];
       if (hr) v -= Y[I.yR + int64_t(i) * s + q] * xr[q];
     }
-    x[perm[I.dof0 + i]] = double(v);
+    if (I.end)
+      tw[I.dof0 + i] = v;
+    else
+      x[perm[I.dof0 + i]] = double(v);
   }
-  if (hr) {
+  if (I.end) {
+    __syncwarp();
+    rb_bwd<T, WM>(I.n, I.kl + I.ku, I.kl + I.ku + 1, UC + I.rbase, tw + I.dof0, smem, lane);
+    for (int i = lane; i < I.n; i += 32) x[perm[I.dof0 + i]] = double(tw[I.dof0 + i]);
+  }
+  if (hr && ts[I.sepR].intL == a) {
     const TornSep S = ts[I.sepR];
     if (lane < s) x[perm[S.dof0 + lane]] = txs[S.trow + lane];
   }
   __syncwarp();
 }
 
-template <typename T>
+template <typename T, int WM>
 __global__ void __launch_bounds__(32) tb_back(int nint, const TornInt* __restrict__ ti,
-                                              const TornSep* __restrict__ ts, const T* __restrict__ Y,
-                                              const int32_t* __restrict__ perm, const double* __restrict__ txs,
+                                              const TornSep* __restrict__ ts, const T* __restrict__ UC,
+                                              const T* __restrict__ Y, const int32_t* __restrict__ perm,
+                                              const double* __restrict__ txs, T* __restrict__ tw,
                                               double* __restrict__ x, const int* __restrict__ only) {
   __shared__ T xl[BCR_S], xr[BCR_S];
+  __shared__ __align__(16) unsigned char smem[2 * 32 * WM * sizeof(T)];
   const int a = blockIdx.x;
   if (a >= nint) return;
   const TornInt I = ti[a];
   if (tb_skip(only, I.comp)) return;
-  tb_back_warp(I, ts, Y, perm, txs, x, xl, xr, threadIdx.x);
+  tb_back_warp<T, WM>(I, a, ts, UC, Y, perm, txs, tw, x, xl, xr, smem, threadIdx.x);
 }
 
 // ---------------------------------------------------------------- fused per-component solve
@@ -373,18 +461,19 @@ __host__ __device__ constexpr int tb_fused_warp_bytes() {
 }
 
 // separator right-hand side in band order: r_S = b_S - F^R_{left} t_{left}[last s] - F^L_{right} t_{right}[first s]
+// (G and z of an end interior in their place)
 template <typename T>
 __device__ void tb_sep_rhs_band(const TornSep& S, const TornInt* __restrict__ ti, const T* __restrict__ blk,
-                                const double* b, const T* t, double* tr, int lane) {
+                                const T* __restrict__ Y, const double* b, const T* t, double* tr, int lane) {
   const int s = S.s;
   if (lane < s) {
-    const TornInt IL = ti[S.intL], IR = ti[S.intR];
-    const T* yl = t + IL.dof0 + IL.n - s;
-    const T* yr = t + IR.dof0;
+    const TornSides<T> sd = tb_sides<T>(ti[S.intL], ti[S.intR], blk, Y);
+    const T* yl = t + sd.pl;
+    const T* yr = t + sd.pr;
     T v = T(b[S.dof0 + lane]);
     for (int q = 0; q < s; ++q) {
-      v -= blk[IL.fR + lane * s + q] * yl[q];
-      v -= blk[IR.fL + lane * s + q] * yr[q];
+      v -= sd.fl[lane * s + q] * yl[q];
+      v -= sd.fr[lane * s + q] * yr[q];
     }
     tr[S.trow + lane] = double(v);
   }
@@ -392,9 +481,10 @@ __device__ void tb_sep_rhs_band(const TornSep& S, const TornInt* __restrict__ ti
 
 // back-substitution in band order: t_a -= Y^L_a x_S_a + Y^R_a x_S_a+1, t_S = x_S.
 // One warp; the rows of Y go through shared memory 32 at a time (contiguous
-// loads), each lane then takes one row.  sc: scratch of 2*32*16 + 32 T.
+// loads), each lane then takes one row.  An end interior's last s + kl rows only
+// (z -= Z x_S; its backward substitution follows).  sc: scratch of 2*32*16 + 32 T.
 template <typename T>
-__device__ void tb_back_band(const TornInt& I, const TornSep* __restrict__ ts, const T* __restrict__ Y,
+__device__ void tb_back_band(const TornInt& I, int a, const TornSep* __restrict__ ts, const T* __restrict__ Y,
                              const double* txs, T* t, T* sc, int lane) {
   const int s = I.s;
   const bool hl = I.sepL >= 0, hr = I.sepR >= 0;
@@ -408,7 +498,7 @@ __device__ void tb_back_band(const TornInt& I, const TornSep* __restrict__ ts, c
     xr[lane] = hr ? T(txs[ts[I.sepR].trow + lane]) : T(0);
   }
 #pragma unroll 1
-  for (int i0 = 0; i0 < I.n; i0 += 32) {
+  for (int i0 = I.end ? I.n - s - I.kl : 0; i0 < I.n; i0 += 32) {
     const int m = min(32, I.n - i0);
     __syncwarp();
     if (hl)
@@ -425,7 +515,7 @@ __device__ void tb_back_band(const TornInt& I, const TornSep* __restrict__ ts, c
       t[I.dof0 + i0 + lane] = v;
     }
   }
-  if (hr && lane < s) t[ts[I.sepR].dof0 + lane] = xr[lane];
+  if (hr && ts[I.sepR].intL == a && lane < s) t[ts[I.sepR].dof0 + lane] = xr[lane];
   __syncwarp();
 }
 
@@ -480,13 +570,13 @@ __global__ void __launch_bounds__(kTbFusedMaxThreads, 2) tb_fused(TbFusedArgs A,
     for (int a = a0 + w; a < a1; a += W) {
       const int n = A.cpI.cn[a], kl = A.cpI.ckl[a], kv = kl + A.cpI.cku[a];
       const int64_t d0 = A.cpI.cdof0[a];
-      rb_fb<T, WM>(n, kl, kv, kv + 1, F.UC + A.cpI.rbase[a], F.LM + A.cpI.lbase[a], A.tpiv + d0, in + d0, t + d0,
-                   my, lane);
+      rb_fwd<T>(n, kl, F.LM + A.cpI.lbase[a], A.tpiv + d0, in + d0, t + d0, my, lane);
+      if (!A.ti[a].end) rb_bwd<T, WM>(n, kv, kv + 1, F.UC + A.cpI.rbase[a], t + d0, my, lane);
       __syncwarp();
     }
     __syncthreads();
     if (k1 > k0) {
-      for (int k = k0 + w; k < k1; k += W) tb_sep_rhs_band(A.ts[k], A.ti, F.blk, in, t, A.trhs, lane);
+      for (int k = k0 + w; k < k1; k += W) tb_sep_rhs_band(A.ts[k], A.ti, F.blk, F.Y, in, t, A.trhs, lane);
       __syncthreads();
       for (int l = 0; l < nlev; ++l) {
         for (int k = k0 + w; k < k1; k += W) {
@@ -509,7 +599,14 @@ __global__ void __launch_bounds__(kTbFusedMaxThreads, 2) tb_fused(TbFusedArgs A,
         }
         __syncthreads();
       }
-      for (int a = a0 + w; a < a1; a += W) tb_back_band(A.ti[a], A.ts, F.Y, A.txs, t, reinterpret_cast<T*>(my), lane);
+      for (int a = a0 + w; a < a1; a += W) {
+        tb_back_band(A.ti[a], a, A.ts, F.Y, A.txs, t, reinterpret_cast<T*>(my), lane);
+        if (A.ti[a].end) {
+          const int64_t d0 = A.cpI.cdof0[a];
+          const int kv = A.cpI.ckl[a] + A.cpI.cku[a];
+          rb_bwd<T, WM>(A.cpI.cn[a], kv, kv + 1, F.UC + A.cpI.rbase[a], t + d0, my, lane);
+        }
+      }
       __syncthreads();
     }
     ++sweeps;
@@ -600,7 +697,8 @@ __global__ void __launch_bounds__(kTbFusedMaxThreads, 2) tb_fused(TbFusedArgs A,
         double v = A.bw[q];
         v = tb_dot16_sub(blk64 + IL.fR + lane * s, A.xw + IL.dof0 + IL.n - s, s, v);
         v = tb_dot16_sub(blk64 + S.d + lane * s, A.xw + S.dof0, s, v);
-        v = tb_dot16_sub(blk64 + IR.fL + lane * s, A.xw + IR.dof0, s, v);
+        v = tb_dot16_sub(blk64 + (IR.end ? IR.fR : IR.fL) + lane * s,
+                         A.xw + (IR.end ? IR.dof0 + IR.n - s : IR.dof0), s, v);
         A.rw[q] = v;
       }
     }

@@ -415,7 +415,11 @@ static void analyse(mgpu_ctx* c, Solver& S) {
     // max(2s, 48) dofs (the separators cost log2(P) cyclic-reduction levels),
     // but no more than needed to give every SM sub-partition ~4 warps: with
     // many components (batched models) the GPU is already full and cutting only
-    // adds work
+    // adds work.  Two interiors need no spikes (band_torn.cuh, tb_end), so where that
+    // cap is 5 or less (487 components or more on 152 SMs) two are better than 3 to 5:
+    // sweep of 512 frame chains (FP64 factors) 108.8 -> 79.1 ms, 1,024: 207 -> 131,
+    // 608 risers (FP32 factors) 59.4 -> 55.4; below it FP32 factors want the shorter
+    // chains, 304 risers 32.1 against 37.9 (256 frame chains 73.6 against 67.0)
     int nsm = 0;
     if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess || nsm <= 0) nsm = 152;
     const int64_t target_warps = int64_t(16) * nsm;
@@ -427,7 +431,7 @@ static void analyse(mgpu_ctx* c, Solver& S) {
       sc[cc] = sw;
       if (sw > 16 || nc < kTornMinDofs) continue;
       const int64_t mmin = std::max(2 * sw, 48);
-      const int64_t pmax = std::min((nc + sw) / (mmin + sw), pcap);
+      const int64_t pmax = std::min((nc + sw) / (mmin + sw), pcap > 5 ? pcap : std::min<int64_t>(pcap, 2));
       Pc[cc] = int(std::max<int64_t>(1, pmax));
       if (Pc[cc] > 1) S.tearable = 1;
     }
@@ -441,6 +445,7 @@ static void analyse(mgpu_ctx* c, Solver& S) {
       // segment of each band position: >= 0 interior index (global), < 0 -(separator index + 1)
       std::vector<int32_t> seg(n), loc(n);
       int maxwI = 0;
+      std::vector<int32_t> tperm(order.begin(), order.end());
       std::vector<int32_t> cint0(ncomp + 1, 0), csep0(ncomp + 1, 0);
       for (int cc = 0; cc < ncomp; ++cc) {
         const int64_t c0 = comp_start[cc], nc = comp_start[cc + 1] - c0;
@@ -466,6 +471,13 @@ static void analyse(mgpu_ctx* c, Solver& S) {
           I.sepL = a > 0 ? sep0 + a - 1 : -1;
           I.sepR = a < P - 1 ? sep0 + a : -1;
           I.comp = cc;
+          I.end = P > 1 && (a == 0 || a == P - 1);
+          const bool back = I.end && a > 0;  // numbered backwards, its separator after its last row
+          if (back) {
+            std::swap(I.sepL, I.sepR);
+            std::swap(I.kl, I.ku);
+            std::reverse(tperm.begin() + I.dof0, tperm.begin() + I.dof0 + m);
+          }
           if (I.sepL >= 0) {
             I.eL = oblk, oblk += int64_t(sw) * sw;
             I.fL = oblk, oblk += int64_t(sw) * sw;
@@ -480,7 +492,7 @@ static void analyse(mgpu_ctx* c, Solver& S) {
           olm += m * std::max(kl[cc], ku[cc]);
           for (int64_t q = 0; q < m; ++q) {
             seg[c0 + p0 + q] = int32_t(ti.size());
-            loc[c0 + p0 + q] = int32_t(q);
+            loc[c0 + p0 + q] = int32_t(back ? m - 1 - q : q);
           }
           irb.push_back(I.rbase), ilb.push_back(I.lbase), in_.push_back(I.n), ikl.push_back(I.kl),
               iku.push_back(I.ku), idof.push_back(I.dof0), icomp.push_back(cc);
@@ -596,7 +608,7 @@ static void analyse(mgpu_ctx* c, Solver& S) {
           if (tbmap[q] < 0 || tbmapT[q] < 0) S.tearable = 0;  // an entry outside the bands (cannot happen)
         }
       auto upv = [&](auto** dst, const auto& v) -> bool { return v.empty() ? true : up(dst, v); };
-      good = good && upv(&S.d_ti, ti) && upv(&S.d_tiT, tiT) && upv(&S.d_ts, ts) && upv(&S.i_rbase, irb) &&
+      good = good && upv(&S.d_ti, ti) && upv(&S.d_tiT, tiT) && upv(&S.d_ts, ts) && up(&S.tperm, tperm) && upv(&S.i_rbase, irb) &&
              upv(&S.i_lbase, ilb) && upv(&S.i_n, in_) && upv(&S.i_kl, ikl) && upv(&S.i_ku, iku) &&
              upv(&S.i_dof0, idof) && upv(&S.d_bsep, bsep) && upv(&S.d_brow, brow) && up(&S.tbmap, tbmap) &&
              up(&S.tbmapT, tbmapT) && up(&S.c_int0, cint0) && up(&S.c_sep0, csep0);
@@ -1037,7 +1049,7 @@ extern "C" void mgpu_solver_destroy(mgpu_ctx* c) {
   void* ps[] = {S->cbase, S->cn, S->ckl, S->cku, S->cdof0, S->perm, S->bmap, S->AB, S->ipiv, S->rhs, S->dx,
                 S->red, S->info, S->rbase, S->lbase, S->rbmap, S->rbmapT, S->RB, S->RB32, S->UC32, S->LM32, S->UC64, S->LM64,
                 S->bw, S->xw, S->rw, S->tw32, S->tw64, S->flag, S->nsweep, S->rdiag, S->part, S->cod, S->frozen,
-                S->nactive, S->d_ti, S->d_tiT, S->d_ts, S->i_rbase, S->i_lbase, S->i_n, S->i_kl, S->i_ku,
+                S->nactive, S->d_ti, S->d_tiT, S->d_ts, S->tperm, S->i_rbase, S->i_lbase, S->i_n, S->i_kl, S->i_ku,
                 S->i_dof0, S->d_bsep, S->d_brow, S->tbmap, S->tbmapT, S->TALL, S->TUC, S->TLM, S->TY, S->DLU,
                 S->FA, S->WL, S->WU, S->PV, S->trhs, S->txs, S->tpiv, S->TALL32, S->TUC32, S->TLM32, S->TY32,
                 S->DLU32, S->FA32, S->WL32, S->WU32, S->i_comp,
@@ -1087,12 +1099,12 @@ static void rb_launch(Solver& S, RbComp cp, cudaStream_t st, const T* rows, T* u
   if (S.n32 > 0) {
     cp.list = S.list32;
     rb_solve<T, 32><<<S.n32, 32, 0, st>>>(cp, S.perm, S.RB, uc, lm, S.ipiv, rhs, S.bw, S.xw, S.rw, tw, out, nref, mode,
-                                          S.flag, nsweep);
+                                          S.flag, nsweep, nullptr);
   }
   if (S.n64 > 0) {
     cp.list = S.list64;
     rb_solve<T, 64><<<S.n64, 32, 0, st>>>(cp, S.perm, S.RB, uc, lm, S.ipiv, rhs, S.bw, S.xw, S.rw, tw, out, nref, mode,
-                                          S.flag, nsweep);
+                                          S.flag, nsweep, nullptr);
   }
 }
 
@@ -1154,13 +1166,13 @@ static void torn_apply(mgpu_ctx* c, bool tr, const double* rhs, double* out, con
   const T* blk = B.rows + S.tb_rows;
   T* tw = sizeof(T) == 4 ? reinterpret_cast<T*>(S.tw32) : reinterpret_cast<T*>(S.tw64);
   if (S.twmI == 32)
-    rb_solve<T, 32><<<S.nint, 32, 0, st>>>(cpI, S.perm, S.TALL, B.uc, B.lm, S.tpiv, rhs, S.bw, S.xw, S.rw, tw, out, 0,
-                                           mode, S.iflag, nullptr);
+    rb_solve<T, 32><<<S.nint, 32, 0, st>>>(cpI, S.tperm, S.TALL, B.uc, B.lm, S.tpiv, rhs, S.bw, S.xw, S.rw, tw, out, 0,
+                                           mode, S.iflag, nullptr, ti);
   else
-    rb_solve<T, 64><<<S.nint, 32, 0, st>>>(cpI, S.perm, S.TALL, B.uc, B.lm, S.tpiv, rhs, S.bw, S.xw, S.rw, tw, out, 0,
-                                           mode, S.iflag, nullptr);
+    rb_solve<T, 64><<<S.nint, 32, 0, st>>>(cpI, S.tperm, S.TALL, B.uc, B.lm, S.tpiv, rhs, S.bw, S.xw, S.rw, tw, out, 0,
+                                           mode, S.iflag, nullptr, ti);
   if (S.nsep == 0) return;
-  tb_sep_rhs<T><<<S.nsep, 32, 0, st>>>(S.nsep, S.d_ts, ti, blk, S.perm, rhs, out, S.trhs, cflag);
+  tb_sep_rhs<T><<<S.nsep, 32, 0, st>>>(S.nsep, S.d_ts, ti, blk, B.y, S.tperm, rhs, out, S.trhs, cflag);
   // separators: block cyclic reduction (trhs reduced in place, txs receives z and then x)
   for (int l = 0; l < S.bcr_levels; ++l) {
     bcr_fwd_elim<T><<<S.nsep, 32, 0, st>>>(S.nsep, S.d_bsep, l, B.fa, S.PV, S.d_brow, S.trhs, S.txs, cflag);
@@ -1169,7 +1181,10 @@ static void torn_apply(mgpu_ctx* c, bool tr, const double* rhs, double* out, con
   bcr_root_solve<T><<<S.nsep, 32, 0, st>>>(S.nsep, S.d_bsep, B.fa, S.PV, S.d_brow, S.trhs, S.txs, cflag);
   for (int l = S.bcr_levels - 1; l >= 0; --l)
     bcr_back<T><<<S.nsep, 32, 0, st>>>(S.nsep, S.d_bsep, l, B.wl, B.wu, S.d_brow, S.txs, cflag);
-  tb_back<T><<<S.nint, 32, 0, st>>>(S.nint, ti, S.d_ts, B.y, S.perm, S.txs, out, cflag);
+  if (S.twmI == 32)
+    tb_back<T, 32><<<S.nint, 32, 0, st>>>(S.nint, ti, S.d_ts, B.uc, B.y, S.tperm, S.txs, tw, out, cflag);
+  else
+    tb_back<T, 64><<<S.nint, 32, 0, st>>>(S.nint, ti, S.d_ts, B.uc, B.y, S.tperm, S.txs, tw, out, cflag);
 }
 
 // Fused per-component partitioned solve (band_torn.cuh tb_fused): nref
@@ -1190,7 +1205,7 @@ static void torn_fused(mgpu_ctx* c, bool tr, const double* rhs, double* out, int
   A.ts = S.d_ts;
   A.bs = S.d_bsep;
   A.nsep = S.nsep;
-  A.perm = S.perm;
+  A.perm = S.tperm;
   A.tpiv = S.tpiv;
   A.brow = S.d_brow;
   A.tall = S.TALL;

@@ -67,6 +67,7 @@ struct Solver {
   TornInt* d_ti = nullptr;    // [nint] interiors (bands of Lλx)
   TornInt* d_tiT = nullptr;   // [nint] the same with kl and ku exchanged (the transpose)
   TornSep* d_ts = nullptr;    // [nsep]
+  int32_t* tperm = nullptr;   // [nX] perm with the last interiors numbered backwards
   int64_t *i_rbase = nullptr, *i_lbase = nullptr;
   int32_t *i_n = nullptr, *i_kl = nullptr, *i_ku = nullptr, *i_dof0 = nullptr;
   BcrSep* d_bsep = nullptr;   // [nsep] cyclic-reduction roles
