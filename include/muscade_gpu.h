@@ -131,6 +131,11 @@ int64_t mgpu_launch_count(const mgpu_ctx *ctx);
 int mgpu_assemble(mgpu_ctx *ctx, int32_t mission, int32_t nXder, const double *x, const double *u, double t,
                   const double *tvals, const mgpu_newmark *c, double *Ll, double *nzval);
 
+/* The same with the state's derivatives where they lie, x[0..nXder), each nX long
+ * (mgpu_assemble wants them one after the other). */
+int mgpu_assemble_parts(mgpu_ctx *ctx, int32_t mission, int32_t nXder, const double *const *x, const double *u,
+                        double t, const double *tvals, const mgpu_newmark *c, double *Ll, double *nzval);
+
 /* The same assembly, pipelined: enqueues it and returns a ticket.  The inputs
  * are copied before the call returns (the caller may reuse x, u, tvals at
  * once).  Ll and nzval receive the outputs by the time mgpu_assemble_wait

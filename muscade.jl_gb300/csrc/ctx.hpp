@@ -11,6 +11,8 @@
 
 namespace mgpu {
 
+constexpr int kDownChunks = 8;  // parts of a matrix on its way to the host (mgpu_assemble)
+
 template <class T>
 struct DevBuf {
   T* p = nullptr;
@@ -85,11 +87,14 @@ struct mgpu_ctx {
   // that a captured step replays with new values: t, a1, a2, a3, b1, b2, b3
   double* stepc = nullptr;   // [8] device
   double* hstepc = nullptr;  // pinned upload ring [kStepcSlots][8]
+  int* herr = nullptr;       // pinned copy of the NaN flag (mgpu_download), behind the ring
   cudaEvent_t stepc_ev[8] = {};
   int stepc_slot = 0;
   // pipelined assembly (mgpu_assemble_async): two slots of device outputs and
   // host input staging; a copy stream returns each slot's outputs while the
   // next slot computes
+  cudaStream_t dstream = nullptr;             // mgpu_assemble: the matrix's way back, part by part
+  cudaEvent_t down_ev[mgpu::kDownChunks] = {};
   cudaStream_t cstream = nullptr;
   double* anz[2] = {nullptr, nullptr};   // [nnz] device outputs per slot
   double* aLl[2] = {nullptr, nullptr};   // [nX]
@@ -112,7 +117,7 @@ int upload_stepc(mgpu_ctx* c, double t, const mgpu_newmark* nm);
 // from the step constants (p0 = 1 in the Newton loops; 0 to assemble the
 // damping or mass matrix alone).  Enqueues no copy and no synchronisation
 // (capturable).
-int launch_assembly(mgpu_ctx* c, int mission, cudaEvent_t* ev_groups, double p0 = 1.0);
+int launch_assembly(mgpu_ctx* c, int mission, cudaEvent_t* ev_groups, double p0 = 1.0, double* host_nz = nullptr);
 // errflag <- INT_MAX on ctx->stream (capturable)
 void launch_reset_errflag(mgpu_ctx* c);
 int set_err(mgpu_ctx* c, int code, const std::string& msg);

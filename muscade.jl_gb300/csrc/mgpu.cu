@@ -441,7 +441,8 @@ __device__ __forceinline__ double plus_zero(double v) {
   return __double_as_longlong(v) == (long long)0x8000000000000000ULL ? 0.0 : v;
 }
 
-// One launch for the matrix (the first bm blocks) and the vector.
+// One launch for the matrix (the first bm blocks) and the vector, or several, each of
+// some of their blocks (from b0).
 struct GatherPlan {
   int64_t n;
   const uint32_t* seg;
@@ -449,8 +450,10 @@ struct GatherPlan {
   const double* buf;
   double* out;
 };
-__global__ void __launch_bounds__(kGatherThreads) scatter_kernel(GatherPlan mat, GatherPlan vec, unsigned bm) {
-  const bool isv = blockIdx.x >= bm;
+__global__ void __launch_bounds__(kGatherThreads) scatter_kernel(GatherPlan mat, GatherPlan vec, unsigned bm,
+                                                                 unsigned b0) {
+  const unsigned blk = b0 + blockIdx.x;
+  const bool isv = blk >= bm;
   const int64_t n = isv ? vec.n : mat.n;
   const uint32_t* __restrict__ seg = isv ? vec.seg : mat.seg;
   const uint32_t* __restrict__ src = isv ? vec.src : mat.src;
@@ -461,7 +464,7 @@ __global__ void __launch_bounds__(kGatherThreads) scatter_kernel(GatherPlan mat,
   __shared__ int16_t slist[kGatherOut];
   __shared__ int nlist;
   const int tid = threadIdx.x, lane = tid & 31;
-  const int64_t k0 = int64_t(blockIdx.x - (isv ? bm : 0u)) * kGatherOut;
+  const int64_t k0 = int64_t(blk - (isv ? bm : 0u)) * kGatherOut;
   const int nk = int(n - k0 < kGatherOut ? n - k0 : kGatherOut);
   for (int t = tid; t <= nk; t += kGatherThreads) sseg[t] = __ldg(seg + k0 + t);
   if (tid == 0) nlist = 0;
@@ -587,7 +590,11 @@ void launch_reset_errflag(mgpu_ctx* c) {
   ++c->launches;
 }
 
-int launch_assembly(mgpu_ctx* c, int mission, cudaEvent_t* ev_groups, double p0) {
+// host_nz: the matrix's values go there too, on a stream of their own: the gather-sum
+// runs in kDownChunks parts, and the copy of one part overlaps the next ones (18
+// million entries: gather-sum and copy 212 + 761 µs one after the other).
+constexpr int64_t kDownMin = int64_t(1) << 20;  // entries; 8 MB, 42 µs of copy, against 4 µs a launch
+int launch_assembly(mgpu_ctx* c, int mission, cudaEvent_t* ev_groups, double p0, double* host_nz) {
   const int64_t nX = c->nX;
   AsmArgs a;
   a.x0 = c->x;
@@ -669,10 +676,21 @@ int launch_assembly(mgpu_ctx* c, int mission, cudaEvent_t* ev_groups, double p0)
   }
   flush_small();
   const unsigned bm = nblk(c->pat.nnz, kGatherOut), bv = nblk(nX, kGatherOut);
-  if (bm + bv > 0) {
-    scatter_kernel<<<bm + bv, kGatherThreads, 0, c->stream>>>(
-        GatherPlan{c->pat.nnz, c->mseg, c->msrc, c->kbuf, c->nzval}, GatherPlan{nX, c->vseg, c->vsrc, c->rbuf, c->Ll}, bm);
+  const GatherPlan mat{c->pat.nnz, c->mseg, c->msrc, c->kbuf, c->nzval}, vec{nX, c->vseg, c->vsrc, c->rbuf, c->Ll};
+  const int parts = host_nz && c->pat.nnz >= kDownMin ? kDownChunks : 1;
+  for (int q = 0; q < parts && bm + bv > 0; ++q) {
+    const unsigned b0 = unsigned(uint64_t(bm) * q / parts);
+    const unsigned b1 = q + 1 < parts ? unsigned(uint64_t(bm) * (q + 1) / parts) : bm + bv;
+    scatter_kernel<<<b1 - b0, kGatherThreads, 0, c->stream>>>(mat, vec, bm, b0);
     ++c->launches;
+    if (host_nz) MG_CUDA(cudaEventRecord(c->down_ev[q], c->stream));
+  }
+  for (int q = 0; host_nz && q < parts && bm > 0; ++q) {
+    const int64_t k0 = int64_t(uint64_t(bm) * q / parts) * kGatherOut;
+    const int64_t k1 = q + 1 < parts ? int64_t(uint64_t(bm) * (q + 1) / parts) * kGatherOut : c->pat.nnz;
+    MG_CUDA(cudaStreamWaitEvent(c->dstream, c->down_ev[q], 0));
+    MG_CUDA(cudaMemcpyAsync(host_nz + k0, c->nzval + k0, size_t(k1 - k0) * sizeof(double), cudaMemcpyDeviceToHost,
+                            c->dstream));
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_err(c, MGPU_ERR_CUDA, std::string("assembly launch: ") + cudaGetErrorString(e));
@@ -951,7 +969,8 @@ extern "C" int mgpu_create(mgpu_ctx** out, const mgpu_model_desc* d) {
   }
   MG_TRY(dalloc(c, &c->stepc, 8));
   MG_CUDA(cudaMemset(c->stepc, 0, 8 * sizeof(double)));
-  MG_CUDA(cudaMallocHost(&c->hstepc, kStepcSlots * 8 * sizeof(double)));
+  MG_CUDA(cudaMallocHost(&c->hstepc, (kStepcSlots * 8 + 1) * sizeof(double)));
+  c->herr = reinterpret_cast<int*>(c->hstepc + kStepcSlots * 8);
   for (int k = 0; k < kStepcSlots; ++k) MG_CUDA(cudaEventCreateWithFlags(&c->stepc_ev[k], cudaEventDisableTiming));
   if (d->scaleX) {
     bool ones = true;
@@ -987,6 +1006,9 @@ extern "C" void mgpu_destroy(mgpu_ctx* c) {
     cudaFree(G.fields);
   }
   if (c->cstream) cudaStreamSynchronize(c->cstream);
+  if (c->dstream) cudaStreamDestroy(c->dstream);
+  for (cudaEvent_t e : c->down_ev)
+    if (e) cudaEventDestroy(e);
   void* ps[] = {c->kbuf, c->rbuf, c->mseg, c->msrc, c->vseg, c->vsrc, c->nzval, c->Ll, c->x,
                 c->u,    c->tv,   c->ab,   c->scale, c->errflag, c->flush, c->stepc, c->Avec,
                 c->anz[0], c->anz[1], c->aLl[0], c->aLl[1], c->aerr, c->res_work};
@@ -1047,12 +1069,17 @@ extern "C" int mgpu_get_asm(const mgpu_ctx* cc, int32_t g, int64_t* asm1, int64_
   return MGPU_OK;
 }
 
-extern "C" int mgpu_upload_state(mgpu_ctx* c, int32_t nXder, const double* x, const double* u, const double* tvals) {
-  if (!c || !x || nXder < 1 || nXder > 3) return set_err(c, MGPU_ERR_ARG, "mgpu_upload_state: bad arguments");
+// the state's nXder parts, each nX long
+static int upload_parts(mgpu_ctx* c, int32_t nXder, const double* const* x, const double* u, const double* tvals) {
   MG_CUDA(cudaSetDevice(c->device));
-  MG_CUDA(cudaMemcpyAsync(c->x, x, nXder * c->nX * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  if (nXder < 3)
-    MG_CUDA(cudaMemsetAsync(c->x + nXder * c->nX, 0, (3 - nXder) * c->nX * sizeof(double), c->stream));
+  const size_t nb = size_t(c->nX) * sizeof(double);
+  for (int32_t k = 0; k < nXder;) {
+    int32_t m = 1;  // parts that lie one after the other are one copy
+    while (k + m < nXder && x[k + m] == x[k] + m * c->nX) ++m;
+    MG_CUDA(cudaMemcpyAsync(c->x + k * c->nX, x[k], m * nb, cudaMemcpyHostToDevice, c->stream));
+    k += m;
+  }
+  if (nXder < 3) MG_CUDA(cudaMemsetAsync(c->x + nXder * c->nX, 0, (3 - nXder) * nb, c->stream));
   if (c->nU > 0 && u) MG_CUDA(cudaMemcpyAsync(c->u, u, c->nU * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   if (c->ntval > 0 && tvals)
     MG_CUDA(cudaMemcpyAsync(c->tv, tvals, c->ntval * sizeof(double), cudaMemcpyHostToDevice, c->stream));
@@ -1060,30 +1087,68 @@ extern "C" int mgpu_upload_state(mgpu_ctx* c, int32_t nXder, const double* x, co
   return MGPU_OK;
 }
 
-extern "C" int mgpu_assemble_resident(mgpu_ctx* c, int32_t mission, double t, const mgpu_newmark* nm) {
+extern "C" int mgpu_upload_state(mgpu_ctx* c, int32_t nXder, const double* x, const double* u, const double* tvals) {
+  if (!c || !x || nXder < 1 || nXder > 3) return set_err(c, MGPU_ERR_ARG, "mgpu_upload_state: bad arguments");
+  const double* part[3] = {x, x + c->nX, x + 2 * c->nX};
+  return upload_parts(c, nXder, part, u, tvals);
+}
+
+static int assemble_resident(mgpu_ctx* c, int32_t mission, double t, const mgpu_newmark* nm, double* host_nz) {
   if (!c || mission < 0 || mission > 2 || (mission != MGPU_ASM_STATIC && !nm))
     return set_err(c, MGPU_ERR_ARG, "mgpu_assemble_resident: bad arguments");
   MG_CUDA(cudaSetDevice(c->device));
   MG_TRY(upload_stepc(c, t, mission != MGPU_ASM_STATIC ? nm : nullptr));
-  return launch_assembly(c, mission, nullptr, 1.0);
+  return launch_assembly(c, mission, nullptr, 1.0, host_nz);
 }
 
+extern "C" int mgpu_assemble_resident(mgpu_ctx* c, int32_t mission, double t, const mgpu_newmark* nm) {
+  return assemble_resident(c, mission, t, nm, nullptr);
+}
+
+// the NaN flag comes back with the results: one wait instead of two
 extern "C" int mgpu_download(mgpu_ctx* c, double* Ll, double* nzval) {
   if (!c) return MGPU_ERR_ARG;
   MG_CUDA(cudaSetDevice(c->device));
   if (Ll) MG_CUDA(cudaMemcpyAsync(Ll, c->Ll, c->nX * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   if (nzval) MG_CUDA(cudaMemcpyAsync(nzval, c->nzval, c->pat.nnz * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  MG_CUDA(cudaMemcpyAsync(c->herr, c->errflag, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   MG_CUDA(cudaStreamSynchronize(c->stream));
-  return check_nan(c);
+  return nan_error(c, *c->herr);
+}
+
+static int assemble_parts(mgpu_ctx* c, int32_t mission, int32_t nXder, const double* const* x, const double* u,
+                          double t, const double* tvals, const mgpu_newmark* nm, double* Ll, double* nzval) {
+  MG_CUDA(cudaSetDevice(c->device));
+  if (nzval && c->pat.nnz >= kDownMin && !c->dstream) {
+    for (cudaEvent_t& e : c->down_ev) MG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    MG_CUDA(cudaStreamCreateWithFlags(&c->dstream, cudaStreamNonBlocking));
+  }
+  MG_TRY(reset_errflag(c));
+  MG_TRY(upload_parts(c, nXder, x, u, tvals));
+  double* own = nzval && c->pat.nnz >= kDownMin ? nzval : nullptr;  // copied beside the gather-sum
+  const int rc = assemble_resident(c, mission, t, nm, own);
+  if (own && cudaStreamSynchronize(c->dstream) != cudaSuccess && rc == MGPU_OK)
+    return set_err(c, MGPU_ERR_CUDA, "mgpu_assemble: copy of the matrix failed");
+  MG_TRY(rc);
+  return mgpu_download(c, Ll, own ? nullptr : nzval);
 }
 
 extern "C" int mgpu_assemble(mgpu_ctx* c, int32_t mission, int32_t nXder, const double* x, const double* u, double t,
                              const double* tvals, const mgpu_newmark* nm, double* Ll, double* nzval) {
   if (!c) return MGPU_ERR_ARG;
-  MG_TRY(reset_errflag(c));
-  MG_TRY(mgpu_upload_state(c, nXder, x, u, tvals));
-  MG_TRY(mgpu_assemble_resident(c, mission, t, nm));
-  return mgpu_download(c, Ll, nzval);
+  if (!x || nXder < 1 || nXder > 3) return set_err(c, MGPU_ERR_ARG, "mgpu_upload_state: bad arguments");
+  const double* part[3] = {x, x + c->nX, x + 2 * c->nX};
+  return assemble_parts(c, mission, nXder, part, u, t, tvals, nm, Ll, nzval);
+}
+
+extern "C" int mgpu_assemble_parts(mgpu_ctx* c, int32_t mission, int32_t nXder, const double* const* x,
+                                   const double* u, double t, const double* tvals, const mgpu_newmark* nm, double* Ll,
+                                   double* nzval) {
+  if (!c) return MGPU_ERR_ARG;
+  bool bad = !x || nXder < 1 || nXder > 3;
+  for (int32_t k = 0; !bad && k < nXder; ++k) bad = !x[k];
+  if (bad) return set_err(c, MGPU_ERR_ARG, "mgpu_upload_state: bad arguments");
+  return assemble_parts(c, mission, nXder, x, u, t, tvals, nm, Ll, nzval);
 }
 
 // Pipelined assembly.  Slot s = ticket mod 2 owns a device copy of the outputs

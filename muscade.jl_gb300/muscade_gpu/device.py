@@ -275,16 +275,17 @@ class DeviceModel:
         return buf[:n]
 
     def assemble(self, X, U=None, t=0.0, mission=L.ASM_STATIC, c=None, want=(True, True), reuse=False):
-        """One assembly with host buffers (mgpu_assemble).  With reuse, the state
-        goes through and the outputs come back in page-locked arrays kept by the
-        model: the returned arrays are overwritten by the next reuse call."""
+        """One assembly with host buffers (mgpu_assemble_parts).  With reuse, the
+        outputs come back in page-locked arrays kept by the model: the returned
+        arrays are overwritten by the next reuse call."""
         X = [np.ascontiguousarray(x, dtype=np.float64) for x in X]
         nXder = len(X)
-        if reuse:
-            x = self._pinned("_xin", nXder * self.nX)
-            np.concatenate(X, out=x)
-        else:
-            x = np.ascontiguousarray(np.concatenate(X))
+        if not X or any(v.size != self.nX for v in X):
+            flat = np.concatenate(X)
+            if flat.size < nXder * self.nX or (reuse and flat.size > nXder * self.nX):
+                raise ValueError(f"a state of {flat.size} values for {nXder} times {self.nX} dofs")
+            X = [flat[k * self.nX:] for k in range(nXder)]
+        x = (ctypes.POINTER(ctypes.c_double) * nXder)(*[L.ptr(v) for v in X])
         u = np.ascontiguousarray(U if U is not None else np.zeros(self.nU), dtype=np.float64)
         tv = self.tvals(t)
         nm = L.Newmark(**(c or {})) if c else L.Newmark()
@@ -294,8 +295,8 @@ class DeviceModel:
         else:
             Ll = np.zeros(self.nX) if want[0] else None
             nz = np.zeros(self.nnz) if want[1] else None
-        rc = self.lib.mgpu_assemble(self.ctx, mission, nXder, L.ptr(x), L.ptr(u), float(t), L.ptr(tv),
-                                    ctypes.byref(nm), L.ptr(Ll), L.ptr(nz))
+        rc = self.lib.mgpu_assemble_parts(self.ctx, mission, nXder, x, L.ptr(u), float(t), L.ptr(tv),
+                                          ctypes.byref(nm), L.ptr(Ll), L.ptr(nz))
         self._check(rc)
         return Ll, nz
 
