@@ -1103,6 +1103,25 @@ __global__ void sp_fwdb_ext(const SpFrontDev* __restrict__ fr, const int32_t* __
   if (t < C.m - C.p) V[Fr.idx + emap[C.eoff + t]] += cvec[C.eoff + t];
 }
 
+// the two in one launch for fronts of up to kPrepRows rows, a block each
+constexpr int kPrepRows = 4096;
+__global__ void __launch_bounds__(1024) sp_fwdb_prep(const SpFrontDev* __restrict__ fr,
+                                                     const int32_t* __restrict__ flist,
+                                                     const int32_t* __restrict__ clist,
+                                                     const int32_t* __restrict__ emap, const double* __restrict__ w,
+                                                     const double* __restrict__ cvec, double* __restrict__ V,
+                                                     const int* __restrict__ conv) {
+  if (*conv) return;
+  const SpFrontDev Fr = fr[flist[blockIdx.x]];
+  double* v = V + Fr.idx;
+  for (int t = threadIdx.x; t < Fr.m; t += 1024) v[t] = t < Fr.p ? w[Fr.pos0 + t] : 0.0;
+  for (int k = 0; k < Fr.nc; ++k) {
+    __syncthreads();
+    const SpFrontDev C = fr[clist[Fr.c0 + k]];
+    for (int t = threadIdx.x; t < C.m - C.p; t += 1024) v[emap[C.eoff + t]] += cvec[C.eoff + t];
+  }
+}
+
 // forward: the triangle of pivot tile 0
 template <class T>
 __global__ void __launch_bounds__(kSBThreads) sp_fwdb_first(const SpFrontDev* __restrict__ fr,
@@ -1209,7 +1228,8 @@ __global__ void __launch_bounds__(kSBThreads) sp_bwdb_u12(const SpFrontDev* __re
 }
 
 __global__ void sp_bwdb_red(const SpFrontDev* __restrict__ fr, const int32_t* __restrict__ flist,
-                            const int64_t* __restrict__ poff, const double* __restrict__ P, double* __restrict__ V,
+                            const int64_t* __restrict__ poff, const double* __restrict__ P,
+                            const double* __restrict__ w, double* __restrict__ V,
                             const int* __restrict__ conv) {
   if (*conv) return;
   const int32_t f = flist[blockIdx.y];
@@ -1219,7 +1239,7 @@ __global__ void sp_bwdb_red(const SpFrontDev* __restrict__ fr, const int32_t* __
   const int nu = sb_nu(Fr.m, Fr.p);
   double s = 0.0;
   for (int b = 0; b < nu; ++b) s += P[poff[f] + int64_t(b) * Fr.p + r];
-  V[Fr.idx + r] -= s;
+  V[Fr.idx + r] = w[Fr.pos0 + r] - s;
 }
 
 // backward: the triangle of the last pivot tile, once the update columns are in
@@ -1354,6 +1374,7 @@ template <class T>
 __global__ void __launch_bounds__(kSBThreads) sp_fwdb_chain(const SpFrontDev* __restrict__ fr,
                                                             const int32_t* __restrict__ flist, int nf, int ntmax,
                                                             const T* __restrict__ F, double* __restrict__ V,
+                                                            double* __restrict__ w, double* __restrict__ cvec,
                                                             unsigned* __restrict__ tflag, unsigned epoch,
                                                             int* __restrict__ ctr, int* __restrict__ abort_word,
                                                             int* __restrict__ flags) {
@@ -1392,7 +1413,7 @@ __global__ void __launch_bounds__(kSBThreads) sp_fwdb_chain(const SpFrontDev* __
     }
     if (!ok) return;
     if (!piv) {
-      if (tid < kSB && r0 + tid < r1) Vf[r0 + tid] = v;
+      if (tid < kSB && r0 + tid < r1 && Fr.parent >= 0) cvec[Fr.eoff + (r0 + tid - p)] = v;
       continue;
     }
     const int nr = r1 - r0;
@@ -1406,8 +1427,8 @@ __global__ void __launch_bounds__(kSBThreads) sp_fwdb_chain(const SpFrontDev* __
         a0 = fma(-Dg[tid][c], yc, a0);
         a1 = fma(-Dg[tid + 32][c], yc, a1);
       }
-      if (tid < nr) Vf[r0 + tid] = double(a0);
-      if (tid + 32 < nr) Vf[r0 + tid + 32] = double(a1);
+      if (tid < nr) w[Fr.pos0 + r0 + tid] = Vf[r0 + tid] = double(a0);
+      if (tid + 32 < nr) w[Fr.pos0 + r0 + tid + 32] = Vf[r0 + tid + 32] = double(a1);
       __threadfence();
     }
     __syncthreads();
@@ -1419,6 +1440,7 @@ template <class T>
 __global__ void __launch_bounds__(kSBThreads) sp_bwdb_chain(const SpFrontDev* __restrict__ fr,
                                                             const int32_t* __restrict__ flist, int nf, int npmax,
                                                             const T* __restrict__ F, double* __restrict__ V,
+                                                            double* __restrict__ w,
                                                             unsigned* __restrict__ tflag, unsigned epoch,
                                                             int* __restrict__ ctr, int* __restrict__ abort_word,
                                                             int* __restrict__ flags) {
@@ -1459,6 +1481,8 @@ __global__ void __launch_bounds__(kSBThreads) sp_bwdb_chain(const SpFrontDev* __
     __syncthreads();
     if (tid < 32) {
       sb_solve_upper<T>(Dg, rd, vs, nr, r0, Vf);
+      if (tid < nr) w[Fr.pos0 + r0 + tid] = Vf[r0 + tid];
+      if (tid + 32 < nr) w[Fr.pos0 + r0 + tid + 32] = Vf[r0 + tid + 32];
       __threadfence();
     }
     __syncthreads();
@@ -1476,13 +1500,142 @@ __global__ void sp_bwdb_fin(const SpFrontDev* __restrict__ fr, const int32_t* __
 }
 
 // ---------------------------------------------------------------- refinement
-__global__ void sp_gather_scaled(int64_t n, const int32_t* __restrict__ perm, const double* __restrict__ D,
-                                 const double* __restrict__ r, double* __restrict__ w, const int* __restrict__ conv) {
+// Sweeps of the generalised conjugate residual method (Eisenstat, Elman, Schultz
+// 1983), preconditioned by the factors M and in FP64 throughout: a sweep's direction
+// z = M^-1 r, q = A z, is made conjugate to the earlier ones (q orthogonal to their
+// q), and the step along it leaves the smallest residual over all of them.  The
+// factors' error E = I − M^-1 A is large in a few soft modes of the structure only;
+// plain refinement carries each at its own rate, |E| a sweep, here each direction
+// takes one of them out.  A and r are scaled, A = D Lλx D; z in elimination order, q
+// and r in model order.  The directions of all sweeps are kept (kSparseSweeps at most).
+//   60 x 60 x 20 lattice: 11 -> 8 sweeps a solve; 12 x 12 x 6: 8 -> 5
+constexpr int kDotBlocks = 304;
+
+// r = D b, w = r in elimination order
+__global__ void sp_start(int64_t n, const int32_t* __restrict__ perm, const double* __restrict__ D,
+                         const double* __restrict__ b, double* __restrict__ r, double* __restrict__ w,
+                         const int* __restrict__ conv) {
   if (*conv) return;
   const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const int32_t d = perm[k];
-  w[k] = D[d] * r[d];
+  w[k] = r[d] = D[d] * b[d];
+}
+
+// z = w, and D z in model order
+__global__ void sp_direction(int64_t n, const int32_t* __restrict__ perm, const double* __restrict__ D,
+                             const double* __restrict__ w, double* __restrict__ z, double* __restrict__ dz,
+                             const int* __restrict__ conv) {
+  if (*conv) return;
+  const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const int32_t d = perm[k];
+  const double v = w[k];
+  z[k] = v;
+  dz[d] = D[d] * v;
+}
+
+// Sums over all blocks of acc[0..NV), nv of them: each block's to part, and the block
+// that ends last adds the blocks' (in a fixed order) and is told so; sum[] then holds
+// the totals.  done is zero between launches.
+template <int NV>
+__device__ __forceinline__ bool sp_sums(double (&acc)[NV], int nv, double* __restrict__ part, unsigned* done,
+                                        double* sum) {
+  __shared__ double sh[kThreads / 32][NV];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  auto block_sum = [&] {
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      if (j < nv) {
+        double v = acc[j];
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) sh[wp][j] = v;
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x < nv) {
+      double v = 0.0;
+      for (int q = 0; q < kThreads / 32; ++q) v += sh[q][threadIdx.x];
+      sum[threadIdx.x] = v;
+    }
+    __syncthreads();
+  };
+  block_sum();
+  if (threadIdx.x < nv) part[int64_t(blockIdx.x) * NV + threadIdx.x] = sum[threadIdx.x];
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicInc(done, gridDim.x - 1) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+#pragma unroll
+  for (int j = 0; j < NV; ++j) acc[j] = 0.0;
+  for (unsigned q = threadIdx.x; q < gridDim.x; q += blockDim.x)
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+      if (j < nv) acc[j] += __ldcg(part + int64_t(q) * NV + j);
+  block_sum();
+  return true;
+}
+
+// q = D Lλx dz, and beta_j = q·q_j / q_j·q_j for the it earlier directions (Q: [it][n])
+__global__ void __launch_bounds__(kThreads) sp_apply(int64_t n, int it, const int64_t* __restrict__ rptr,
+                                                     const int32_t* __restrict__ rq, const int32_t* __restrict__ rcol,
+                                                     const double* __restrict__ nzval, const double* __restrict__ D,
+                                                     const double* __restrict__ dz, const double* __restrict__ Q,
+                                                     double* __restrict__ q, double* __restrict__ part,
+                                                     unsigned* __restrict__ done, const double* __restrict__ qq,
+                                                     double* __restrict__ beta, const int* __restrict__ conv) {
+  if (*conv) return;
+  __shared__ double sum[kSparseSweeps];
+  double acc[kSparseSweeps];
+#pragma unroll
+  for (int j = 0; j < kSparseSweeps; ++j) acc[j] = 0.0;
+  for (int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x; i < n; i += int64_t(gridDim.x) * kThreads) {
+    double s = 0.0;
+    for (int64_t t = rptr[i]; t < rptr[i + 1]; ++t) s = fma(nzval[rq[t]], dz[rcol[t]], s);
+    s *= D[i];
+    q[i] = s;
+#pragma unroll
+    for (int j = 0; j < kSparseSweeps; ++j)
+      if (j < it) acc[j] = fma(s, Q[j * n + i], acc[j]);
+  }
+  if (it > 0 && sp_sums(acc, it, part, done, sum) && threadIdx.x < it)
+    beta[threadIdx.x] = qq[threadIdx.x] > 0.0 ? sum[threadIdx.x] / qq[threadIdx.x] : 0.0;
+}
+
+// q -= Σ beta_j q_j, z -= Σ beta_j z_j; qq = q·q, alpha = q·r / q·q
+__global__ void __launch_bounds__(kThreads) sp_conjugate(int64_t n, int it, const double* __restrict__ Q,
+                                                         const double* __restrict__ Z, double* __restrict__ q,
+                                                         double* __restrict__ z, const double* __restrict__ r,
+                                                         const double* __restrict__ beta, double* __restrict__ part,
+                                                         unsigned* __restrict__ done, double* __restrict__ qq,
+                                                         double* __restrict__ alpha, const int* __restrict__ conv) {
+  if (*conv) return;
+  __shared__ double sum[2];
+  double acc[2] = {0.0, 0.0}, be[kSparseSweeps];
+#pragma unroll
+  for (int j = 0; j < kSparseSweeps; ++j) be[j] = j < it ? beta[j] : 0.0;
+  for (int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x; i < n; i += int64_t(gridDim.x) * kThreads) {
+    double a = q[i], b = z[i];
+#pragma unroll
+    for (int j = 0; j < kSparseSweeps; ++j)
+      if (j < it) {
+        a = fma(-be[j], Q[j * n + i], a);
+        b = fma(-be[j], Z[j * n + i], b);
+      }
+    if (it > 0) {
+      q[i] = a;
+      z[i] = b;
+    }
+    acc[0] = fma(a, a, acc[0]);
+    acc[1] = fma(a, r[i], acc[1]);
+  }
+  if (sp_sums(acc, 2, part, done, sum) && threadIdx.x == 0) {
+    *qq = sum[0];
+    *alpha = sum[0] == 0.0 ? 0.0 : sum[1] / sum[0];  // zero only with a zero residual
+  }
 }
 
 __device__ __forceinline__ void max_bits(unsigned long long* dst, double v) {
@@ -1490,21 +1643,25 @@ __device__ __forceinline__ void max_bits(unsigned long long* dst, double v) {
   atomicMax(dst, (unsigned long long)__double_as_longlong(isnan(v) ? INFINITY : fabs(v)));
 }
 
-__global__ void __launch_bounds__(kThreads) sp_accumulate(int64_t n, int first, const int32_t* __restrict__ perm,
-                                                          const double* __restrict__ D, const double* __restrict__ w,
-                                                          double* __restrict__ yacc, double* __restrict__ x,
-                                                          unsigned long long* __restrict__ nrm,
-                                                          const int* __restrict__ conv) {
+// y += alpha z, x = D y, r -= alpha q; w: the new residual in elimination order
+__global__ void __launch_bounds__(kThreads) sp_step(int64_t n, int first, const int32_t* __restrict__ perm,
+                                                    const double* __restrict__ D, const double* __restrict__ alpha,
+                                                    const double* __restrict__ zv, const double* __restrict__ q,
+                                                    double* __restrict__ yacc, double* __restrict__ x,
+                                                    double* __restrict__ r, double* __restrict__ w,
+                                                    unsigned long long* __restrict__ nrm,
+                                                    const int* __restrict__ conv) {
   if (*conv) return;
   __shared__ double smax[2][kThreads / 32];
   const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   double mw = 0.0, my = 0.0;
   if (k < n) {
-    const double z = w[k];
+    const double al = *alpha, z = al * zv[k];
     const double y = first ? z : yacc[k] + z;
     yacc[k] = y;
     const int32_t d = perm[k];
     x[d] = D[d] * y;
+    w[k] = r[d] = fma(-al, q[d], r[d]);
     mw = isnan(z) ? INFINITY : fabs(z);
     my = isnan(y) ? INFINITY : fabs(y);
   }
@@ -1527,32 +1684,22 @@ __global__ void __launch_bounds__(kThreads) sp_accumulate(int64_t n, int first, 
   }
 }
 
-// Converged when the scaled correction is below tol of the scaled solution,
-// or when it has stopped shrinking (no better than half the previous one)
+// Converged when the scaled correction is below tol of the scaled solution, or the
+// next one would be, by a factor of ten, at the rate of the last two (the rate only
+// improves from sweep to sweep), or when it has stopped shrinking (no better than half the previous one)
 // while below stall of the solution: the attainable accuracy of the FP64
 // residual is then reached.  prev holds the previous correction's norm.
 __global__ void sp_check(unsigned long long* nrm, double* prev, int* flags, double tol, double stall) {
   if (flags[0]) return;
   const double nw = __longlong_as_double((long long)nrm[0]), ny = __longlong_as_double((long long)nrm[1]);
   flags[1] += 1;
-  if (nw <= tol * ny || (flags[1] > 1 && nw >= 0.5 * *prev && nw <= stall * ny)) flags[0] = 1;
+  const bool again = flags[1] > 1;
+  if (nw <= tol * ny || (again && nw < *prev && nw * (nw / *prev) <= 0.1 * tol * ny) ||
+      (again && nw >= 0.5 * *prev && nw <= stall * ny))
+    flags[0] = 1;
   *prev = nw;
   nrm[0] = 0ull;
   nrm[1] = 0ull;
-}
-
-__global__ void __launch_bounds__(kThreads) sp_residual(int64_t n, const int64_t* __restrict__ rptr,
-                                                        const int32_t* __restrict__ rq,
-                                                        const int32_t* __restrict__ rcol,
-                                                        const double* __restrict__ nzval,
-                                                        const double* __restrict__ x, const double* __restrict__ b,
-                                                        double* __restrict__ r, const int* __restrict__ conv) {
-  if (*conv) return;
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double s = b[i];
-  for (int64_t t = rptr[i]; t < rptr[i + 1]; ++t) s -= nzval[rq[t]] * x[rcol[t]];
-  r[i] = s;
 }
 
 template <class T>
@@ -1691,15 +1838,10 @@ cudaError_t refine(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, int 
       const cudaError_t e = cudaMemsetAsync(sp.chain, 0, (2 * size_t(sp.nheight) + 1) * sizeof(int), st);
       if (e != cudaSuccess) return e;
     }
-    const double* r = b;
-    if (it > 0) {
-      sp_residual<<<nblocks(n, kThreads), kThreads, 0, st>>>(n, sp.d_rptr, sp.d_rq, sp.d_rcol, c->nzval, sp.xs, b,
-                                                             sp.r, sp.flags);
+    if (it == 0) {
+      sp_start<<<nblocks(n, kThreads), kThreads, 0, st>>>(n, sp.d_perm, sp.D, b, sp.r, sp.w, sp.flags);
       ++c->launches;
-      r = sp.r;
     }
-    sp_gather_scaled<<<nblocks(n, kThreads), kThreads, 0, st>>>(n, sp.d_perm, sp.D, r, sp.w, sp.flags);
-    ++c->launches;
     for (int h = 0; h < sp.nheight; ++h) {
       if (!sp.h_nlf[h]) continue;
       const int32_t* fl = sp.d_lf + sp.h_lf0[h];
@@ -1718,17 +1860,23 @@ cudaError_t refine(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, int 
       }
       if (nbig > 0) {
         const unsigned gm = nblocks(sp.h_mmax[h], kThreads);
-        sp_fwdb_init<<<dim3(gm, unsigned(nbig)), kThreads, 0, st>>>(sp.d_fr, fl, sp.w, sp.V, sp.flags);
-        ++c->launches;
-        for (size_t rk = 0; rk < sp.h_nea[h].size(); ++rk) {
-          sp_fwdb_ext<<<dim3(nblocks(std::max(sp.h_eumax[h][rk], 1), kThreads), unsigned(nbig)), kThreads, 0, st>>>(
-              sp.d_fr, fl, sp.d_clist, sp.d_emap, int(rk), sp.cvec, sp.V, sp.flags);
+        if (sp.h_mmax[h] <= kPrepRows) {
+          sp_fwdb_prep<<<unsigned(nbig), 1024, 0, st>>>(sp.d_fr, fl, sp.d_clist, sp.d_emap, sp.w, sp.cvec, sp.V,
+                                                        sp.flags);
           ++c->launches;
+        } else {
+          sp_fwdb_init<<<dim3(gm, unsigned(nbig)), kThreads, 0, st>>>(sp.d_fr, fl, sp.w, sp.V, sp.flags);
+          ++c->launches;
+          for (size_t rk = 0; rk < sp.h_nea[h].size(); ++rk) {
+            sp_fwdb_ext<<<dim3(nblocks(std::max(sp.h_eumax[h][rk], 1), kThreads), unsigned(nbig)), kThreads, 0, st>>>(
+                sp.d_fr, fl, sp.d_clist, sp.d_emap, int(rk), sp.cvec, sp.V, sp.flags);
+            ++c->launches;
+          }
         }
         if (sp.chained) {
           const int items = sp.h_bnt[h] * nbig;
           sp_fwdb_chain<T><<<unsigned(std::min(items, grid)), kSBThreads, 0, st>>>(
-              sp.d_fr, fl, nbig, sp.h_bnt[h], F, sp.V, sp.tflag, next_epoch(sp, st), sp.chain + h,
+              sp.d_fr, fl, nbig, sp.h_bnt[h], F, sp.V, sp.w, sp.cvec, sp.tflag, next_epoch(sp, st), sp.chain + h,
               sp.chain + 2 * sp.nheight, sp.flags);
           ++c->launches;
         } else {
@@ -1742,9 +1890,9 @@ cudaError_t refine(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, int 
               ++c->launches;
             }
           }
+          sp_fwdb_fin<<<dim3(gm, unsigned(nbig)), kThreads, 0, st>>>(sp.d_fr, fl, sp.V, sp.w, sp.cvec, sp.flags);
+          ++c->launches;
         }
-        sp_fwdb_fin<<<dim3(gm, unsigned(nbig)), kThreads, 0, st>>>(sp.d_fr, fl, sp.V, sp.w, sp.cvec, sp.flags);
-        ++c->launches;
       }
     }
     for (int h = sp.nheight - 1; h >= 0; --h) {
@@ -1765,18 +1913,20 @@ cudaError_t refine(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, int 
       }
       if (nbig > 0) {
         const unsigned gp = nblocks(sp.h_pmax[h], kThreads);
-        sp_bwdb_init<<<dim3(gp, unsigned(nbig)), kThreads, 0, st>>>(sp.d_fr, fl, sp.w, sp.V, sp.flags);
-        ++c->launches;
         if (sp.h_bnu[h] > 0) {
           sp_bwdb_u12<T><<<dim3(unsigned(sp.h_bnp[h]), unsigned(sp.h_bnu[h]), unsigned(nbig)), kSBThreads, 0, st>>>(
               sp.d_fr, fl, sp.d_poff, sp.d_fidx, F, sp.w, sp.P, sp.flags);
-          sp_bwdb_red<<<dim3(gp, unsigned(nbig)), kThreads, 0, st>>>(sp.d_fr, fl, sp.d_poff, sp.P, sp.V, sp.flags);
+          sp_bwdb_red<<<dim3(gp, unsigned(nbig)), kThreads, 0, st>>>(sp.d_fr, fl, sp.d_poff, sp.P, sp.w, sp.V,
+                                                                     sp.flags);
           c->launches += 2;
+        } else {
+          sp_bwdb_init<<<dim3(gp, unsigned(nbig)), kThreads, 0, st>>>(sp.d_fr, fl, sp.w, sp.V, sp.flags);
+          ++c->launches;
         }
         if (sp.chained) {
           const int items = sp.h_bnp[h] * nbig;
           sp_bwdb_chain<T><<<unsigned(std::min(items, grid)), kSBThreads, 0, st>>>(
-              sp.d_fr, fl, nbig, sp.h_bnp[h], F, sp.V, sp.tflag, next_epoch(sp, st), sp.chain + sp.nheight + h,
+              sp.d_fr, fl, nbig, sp.h_bnp[h], F, sp.V, sp.w, sp.tflag, next_epoch(sp, st), sp.chain + sp.nheight + h,
               sp.chain + 2 * sp.nheight, sp.flags);
           ++c->launches;
         } else {
@@ -1787,15 +1937,21 @@ cudaError_t refine(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, int 
                                                                                                 sp.V, sp.flags);
             ++c->launches;
           }
+          sp_bwdb_fin<<<dim3(gp, unsigned(nbig)), kThreads, 0, st>>>(sp.d_fr, fl, sp.V, sp.w, sp.flags);
+          ++c->launches;
         }
-        sp_bwdb_fin<<<dim3(nblocks(sp.h_pmax[h], kThreads), unsigned(nbig)), kThreads, 0, st>>>(sp.d_fr, fl, sp.V,
-                                                                                               sp.w, sp.flags);
-        ++c->launches;
       }
     }
-    sp_accumulate<<<nblocks(n, kThreads), kThreads, 0, st>>>(n, it == 0, sp.d_perm, sp.D, sp.w, sp.yacc, sp.xs, sp.nrm,
-                                                             sp.flags);
-    ++c->launches;
+    double *z = sp.dirz + it * n, *q = sp.dirq + it * n;
+    const unsigned gd = std::max(1u, std::min(unsigned(kDotBlocks), unsigned(nblocks(n, kThreads))));
+    sp_direction<<<nblocks(n, kThreads), kThreads, 0, st>>>(n, sp.d_perm, sp.D, sp.w, z, sp.dz, sp.flags);
+    sp_apply<<<gd, kThreads, 0, st>>>(n, it, sp.d_rptr, sp.d_rq, sp.d_rcol, c->nzval, sp.D, sp.dz, sp.dirq, q, sp.part,
+                                      sp.done, sp.coef, sp.coef + kSparseSweeps, sp.flags);
+    sp_conjugate<<<gd, kThreads, 0, st>>>(n, it, sp.dirq, sp.dirz, q, z, sp.r, sp.coef + kSparseSweeps, sp.part,
+                                          sp.done, sp.coef + it, sp.coef + 2 * kSparseSweeps, sp.flags);
+    sp_step<<<nblocks(n, kThreads), kThreads, 0, st>>>(n, it == 0, sp.d_perm, sp.D, sp.coef + 2 * kSparseSweeps, z, q,
+                                                       sp.yacc, sp.xs, sp.r, sp.w, sp.nrm, sp.flags);
+    c->launches += 4;
     sp_check<<<1, 1, 0, st>>>(sp.nrm, sp.prev, sp.flags, kRefineTol, kRefineStall);
     ++c->launches;
   }
@@ -1809,7 +1965,7 @@ template <class T>
 cudaError_t refine_batches(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, int sweeps, int first) {
   int done = 0;
   while (done < sweeps) {
-    const int nb_ = done == 0 ? std::min(first, sweeps) : std::min(2, sweeps - done);
+    const int nb_ = done == 0 ? std::min(first, sweeps) : 1;
     cudaError_t e = refine<T>(c, sp, F, b, done, done + nb_);
     if (e != cudaSuccess) return e;
     done += nb_;
@@ -2022,6 +2178,11 @@ int sparse_create(mgpu_ctx* c, SparseDev*& spp, const double* dof_xyz, const uin
   ok(cudaMalloc(&sp.tw, n * sizeof(double)));
   ok(cudaMalloc(&sp.yacc, n * sizeof(double)));
   ok(cudaMalloc(&sp.r, n * sizeof(double)));
+  ok(cudaMalloc(&sp.dirz, size_t(kSparseSweeps) * n * sizeof(double)));
+  ok(cudaMalloc(&sp.dirq, size_t(kSparseSweeps) * n * sizeof(double)));
+  ok(cudaMalloc(&sp.dz, n * sizeof(double)));
+  ok(cudaMalloc(&sp.part, size_t(kDotBlocks) * kSparseSweeps * sizeof(double)));
+  ok(cudaMalloc(&sp.coef, (2 * kSparseSweeps + 2) * sizeof(double)));  // q·q, beta, alpha, done
   ok(cudaMalloc(&sp.xs, n * sizeof(double)));
   ok(cudaMalloc(&sp.nrm, 2 * sizeof(unsigned long long)));
   ok(cudaMalloc(&sp.prev, sizeof(double)));
@@ -2044,6 +2205,8 @@ int sparse_create(mgpu_ctx* c, SparseDev*& spp, const double* dof_xyz, const uin
   }
   if (const char* ev = getenv("MGPU_SPARSE_CHAINED")) sp.chained = atoi(ev) != 0;
   ok(cudaMemset(sp.nrm, 0, 2 * sizeof(unsigned long long)));
+  ok(cudaMemsetAsync(sp.coef, 0, (2 * kSparseSweeps + 2) * sizeof(double), c->stream));
+  sp.done = reinterpret_cast<unsigned*>(sp.coef + 2 * kSparseSweeps + 1);
   for (cudaEvent_t& ev : sp.ev) ok(cudaEventCreate(&ev));
   const int smem = int(sp.max_m_small * sizeof(double));
   if (smem > 48 * 1024) {
@@ -2077,7 +2240,8 @@ void sparse_destroy(SparseDev*& sp) {
   void* ps[] = {sp->d_fr, sp->d_lf, sp->d_ea, sp->d_clist, sp->d_fidx, sp->d_emap, sp->d_amap, sp->d_aq,
                 sp->d_acol, sp->d_perm, sp->d_diag, sp->d_colptr, sp->d_rowval, sp->d_rptr, sp->d_rq, sp->d_rcol,
                 sp->F32, sp->F64, sp->prev,
-                sp->D, sp->cvec, sp->w, sp->V, sp->P, sp->d_poff, sp->tw, sp->yacc, sp->r, sp->xs, sp->nrm,
+                sp->D, sp->cvec, sp->w, sp->V, sp->P, sp->d_poff, sp->tw, sp->yacc, sp->r,
+                sp->dirz, sp->dirq, sp->dz, sp->part, sp->coef, sp->xs, sp->nrm,
                 sp->flags, sp->tflag, sp->chain};
   for (void* p : ps) cudaFree(p);
   if (sp->hflags) cudaFreeHost(sp->hflags);
@@ -2108,7 +2272,7 @@ int sparse_factor_solve(mgpu_ctx* c, SparseDev& sp, const double* rhs, double* o
     MG_CUDA(cudaEventRecord(sp.ev[0], st));
     MG_CUDA((factorise<float, kNB32>(c, sp, sp.F32, 1e-10f)));
     MG_CUDA(cudaEventRecord(sp.ev[1], st));
-    MG_CUDA(refine_batches<float>(c, sp, sp.F32, rhs, kSparseSweeps, 8));
+    MG_CUDA(refine_batches<float>(c, sp, sp.F32, rhs, kSparseSweeps, 4));
     MG_CUDA(cudaEventRecord(sp.ev[2], st));
     MG_CUDA(cudaMemcpyAsync(sp.hflags, sp.flags, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
     MG_CUDA(cudaStreamSynchronize(st));
@@ -2136,7 +2300,7 @@ int sparse_factor_solve(mgpu_ctx* c, SparseDev& sp, const double* rhs, double* o
     MG_CUDA(cudaEventRecord(sp.ev[0], st));
     MG_CUDA((factorise<double, kNB64>(c, sp, sp.F64, 0.0)));
     MG_CUDA(cudaEventRecord(sp.ev[1], st));
-    MG_CUDA(refine_batches<double>(c, sp, sp.F64, rhs, kSparseSweeps64, 4));
+    MG_CUDA(refine_batches<double>(c, sp, sp.F64, rhs, kSparseSweeps64, 2));
     MG_CUDA(cudaEventRecord(sp.ev[2], st));
     MG_CUDA(cudaMemcpyAsync(sp.hflags, sp.flags, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
     MG_CUDA(cudaStreamSynchronize(st));

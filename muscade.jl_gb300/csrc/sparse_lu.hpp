@@ -13,8 +13,9 @@
 //     dofs they constrain, so their zero diagonal is never a pivot) in blocks
 //     of NB columns: one kernel factors the diagonal block and solves the
 //     block's L and U panels, one updates the trailing block;
-//   * FP32 factors inside FP64 iterative refinement (residuals of the FP64
-//     Lλx), until the scaled correction is below 1e-14 of the scaled solution
+//   * FP32 factors inside FP64 sweeps of the conjugate residual method (residuals
+//     of the FP64 Lλx), until the scaled correction, or the next one at the rate
+//     of the last two and ten times over, is below 1e-14 of the scaled solution
 //     or stops shrinking below 1e-10 of it (the FP64 residual's attainable
 //     accuracy), at most kSparseSweeps sweeps; when that fails the same
 //     kernels factorise in FP64 (MGPU_LINSOLVE_SPARSE), or FP64 throughout
@@ -86,6 +87,9 @@ struct SparseDev {
   int64_t* d_poff = nullptr;    // [nfront] offset of each blocked front's partials in P
   double* tw = nullptr;         // [n] U₁₂ x_u of each pivot (backward substitution)
   double* yacc = nullptr;       // [n] accumulated scaled solution (elimination order)
+  double *dirz = nullptr, *dirq = nullptr;  // [kSparseSweeps][n] directions of the sweeps and A times them
+  double *dz = nullptr, *part = nullptr, *coef = nullptr;  // D z, blocks' sums, the sweeps' coefficients
+  unsigned* done = nullptr;                 // blocks that have added theirs
   double* r = nullptr;          // [n] residual (model order)
   double* xs = nullptr;         // [n] current solution (model order)
   unsigned long long* nrm = nullptr;  // [2] max |correction|, max |solution| (as ordered bits)
