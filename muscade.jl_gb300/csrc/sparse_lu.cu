@@ -616,6 +616,80 @@ __global__ void __launch_bounds__(tc::kTcThreads) sp_trail_tc(const SpFrontDev* 
   if (!ok && threadIdx.x == 0) atomicOr(flags + 3, 4);
 }
 
+// The same from packed operands (tc::tile_update_packed): sp_pack splits a group of
+// fronts' L and U parts of the super-panel, a front's share `stride` floats: its row
+// tiles of 128, then (from uoff) its column tiles of 256, kPackChunks chunks a tile.
+// 60 x 60 x 20 lattice, one factorisation: 85 ms by sp_trail_tc, 53 and 5 to pack.
+constexpr int kPackChunks = kSuper / tc::kPkK;
+constexpr int kPackThreads = 256, kPackZ = 4;
+constexpr int64_t kPackMax = int64_t(64) << 20;  // floats of the workspace at most: groups of fronts take turns
+
+// tiles of up to `rest` rows or columns, and the floats they take
+__host__ __device__ inline int64_t pack_uoff(int rest) {
+  return int64_t((rest + tc::kPkM - 1) / tc::kPkM) * kPackChunks * tc::kPkA;
+}
+inline int64_t pack_stride(int rest) {
+  return pack_uoff(rest) + int64_t((rest + tc::kPkN - 1) / tc::kPkN) * kPackChunks * tc::kPkB;
+}
+
+__global__ void __launch_bounds__(kPackThreads) sp_pack(const SpFrontDev* __restrict__ fr,
+                                                        const int32_t* __restrict__ flist, int s0, int nt,
+                                                        int64_t stride, int64_t uoff, const float* __restrict__ F,
+                                                        float* __restrict__ P) {
+  const SpFrontDev Fr = fr[flist[blockIdx.y]];
+  const int m = Fr.m, p = Fr.p, e0 = min(s0 + kSuper, p);
+  if (e0 <= s0) return;
+  const float* A = F + Fr.off;
+  const int nch = (e0 - s0 + tc::kPkK - 1) / tc::kPkK;
+  const int c0 = nch * blockIdx.z / kPackZ, c1 = nch * (blockIdx.z + 1) / kPackZ;
+  const bool isu = int(blockIdx.x) >= nt;
+  const int tile = isu ? blockIdx.x - nt : blockIdx.x, rows = isu ? tc::kPkN : tc::kPkM;
+  if (e0 + tile * rows >= m) return;
+  const int r = threadIdx.x % rows, x = e0 + tile * rows + r;  // row of L or column of U
+  const int64_t len = int64_t(rows) * tc::kPkK;
+  float* out = P + int64_t(blockIdx.y) * stride + (isu ? uoff : 0) + int64_t(tile) * kPackChunks * 2 * len;
+  for (int c = c0 + threadIdx.x / rows; c < c1; c += kPackThreads / rows) {
+    const int k0 = s0 + c * tc::kPkK;
+    float h[8], l[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const bool in = x < m && k0 + k < e0;
+      const float v = in ? (isu ? A[(k0 + k) + int64_t(x) * m] : A[x + int64_t(k0 + k) * m]) : 0.f;
+      tc::split_tf32(v, h[k], l[k]);
+    }
+    float* o = out + int64_t(c) * 2 * len + (r >> 3) * 64 + (r & 7) * 4;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      *reinterpret_cast<float4*>(o + 32 * q) = make_float4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
+      *reinterpret_cast<float4*>(o + len + 32 * q) = make_float4(l[4 * q], l[4 * q + 1], l[4 * q + 2], l[4 * q + 3]);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(tc::kPkThreads, 2) sp_trail_packed(const SpFrontDev* __restrict__ fr,
+                                                                     const int32_t* __restrict__ flist, int s0, int nt,
+                                                                     int64_t stride, int64_t uoff,
+                                                                     const float* __restrict__ P,
+                                                                     float* __restrict__ F, int* __restrict__ flags) {
+  const SpFrontDev Fr = fr[flist[blockIdx.y]];
+  const int m = Fr.m, p = Fr.p, e0 = min(s0 + kSuper, p);
+  if (e0 <= s0) return;
+  const int ti = blockIdx.x % nt, tj = blockIdx.x / nt;
+  const int i0 = e0 + ti * tc::kPkM, j0 = e0 + tj * tc::kPkN;
+  if (i0 >= m || j0 >= m) return;
+  if (ld_relaxed_i32(flags + 3) & 4) return;
+  extern __shared__ __align__(128) float smem_tc[];
+  __shared__ uint64_t bars[2 * tc::kPkStages + 1];
+  __shared__ uint32_t tslot;
+  __shared__ int fail;
+  const float* Pf = P + int64_t(blockIdx.y) * stride;
+  const int nch = (e0 - s0 + tc::kPkK - 1) / tc::kPkK;
+  const bool ok = tc::tile_update_packed(Pf + int64_t(ti) * kPackChunks * tc::kPkA,
+                                         Pf + uoff + int64_t(tj) * kPackChunks * tc::kPkB, nch, F + Fr.off, m, i0, j0,
+                                         m, m, smem_tc, bars, &tslot, &fail);
+  if (!ok && threadIdx.x == 0) atomicOr(flags + 3, 4);
+}
+
 // the left-looking column block (mode 0) or row block (mode 1) of pivot block
 // k0 inside a super-panel on the tensor cores: what sp_rect_f32 does in those
 // modes, one 128 × 128 tile per block (the 64-wide side masked)
@@ -1764,15 +1838,27 @@ cudaError_t factorise(mgpu_ctx* c, SparseDev& sp, T* F, T tau) {
           }
           int cnt = 0;
           while (cnt < int(lp.size()) && lp[cnt] > s0) ++cnt;
-          const int nt = (mmax - s0 + kTile32 - 1) / kTile32;
-          for (int f0 = 0; f0 < cnt; f0 += kMaxGridY) {
+          const int rest = mmax - s0, nt = (rest + kTile32 - 1) / kTile32;
+          const bool tcs = sp.tensor_cores && rest >= kTcMinRest;
+          const int64_t stride = pack_stride(rest), uoff = pack_uoff(rest);
+          const bool packed = tcs && sp.pack && stride <= sp.pack_len;
+          const int per = packed ? int(std::min<int64_t>(kMaxGridY, sp.pack_len / stride)) : kMaxGridY;
+          for (int f0 = 0; f0 < cnt; f0 += per) {
             const int32_t* fl = sp.d_lf + sp.h_lf0[h] + f0;
-            const unsigned gy = unsigned(std::min(kMaxGridY, cnt - f0));
-            if (sp.tensor_cores && mmax - s0 >= kTcMinRest)
+            const unsigned gy = unsigned(std::min(per, cnt - f0));
+            if (packed) {
+              const int ntu = (rest + tc::kPkN - 1) / tc::kPkN;
+              sp_pack<<<dim3(unsigned(nt + ntu), gy, kPackZ), kPackThreads, 0, st>>>(sp.d_fr, fl, s0, nt, stride, uoff,
+                                                                                   F, sp.pack);
+              sp_trail_packed<<<dim3(unsigned(nt * ntu), gy), tc::kPkThreads, tc::kPkSmem, st>>>(
+                  sp.d_fr, fl, s0, nt, stride, uoff, sp.pack, F, sp.flags);
+              ++c->launches;
+            } else if (tcs) {
               sp_trail_tc<<<dim3(unsigned(nt * nt), gy), tc::kTcThreads, tc::kTcSmem, st>>>(sp.d_fr, fl, s0, nt, F,
                                                                                           sp.flags);
-            else
+            } else {
               sp_rect_f32<<<dim3(unsigned(nt * nt), gy), kThreads, kUpd32Smem, st>>>(sp.d_fr, fl, 2, s0, 0, nt, F);
+            }
             ++c->launches;
           }
         }
@@ -2216,11 +2302,25 @@ int sparse_create(mgpu_ctx* c, SparseDev*& spp, const double* dof_xyz, const uin
   ok(cudaFuncSetAttribute(sp_update_f32<kNB32>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kUpd32Smem)));
   ok(cudaFuncSetAttribute(sp_update_tc<kNB32>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tc::kTcSmem)));
   ok(cudaFuncSetAttribute(sp_rect_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kUpd32Smem)));
+  ok(cudaFuncSetAttribute(sp_trail_packed, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tc::kPkSmem)));
   ok(cudaFuncSetAttribute(sp_trail_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tc::kTcSmem)));
   ok(cudaFuncSetAttribute(sp_rect_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tc::kTcSmem)));
   if (const char* ev = getenv("MGPU_SPARSE_TC_LEFT")) sp.tc_left = atoi(ev) != 0;
   if (const char* ev = getenv("MGPU_SPARSE_SUPER")) sp.super_panels = atoi(ev) != 0;
   if (const char* ev = getenv("MGPU_SPARSE_TC")) sp.tensor_cores = atoi(ev) != 0;
+  // workspace of the packed trailing updates; without it (MGPU_SPARSE_PACK=0, or no
+  // room) the trailing blocks take their operands from the fronts
+  const char* pe = getenv("MGPU_SPARSE_PACK");
+  if (sp.super_panels && sp.tensor_cores && !(pe && pe[0] == '0')) {
+    for (int h = 0; h < H; ++h)
+      if (sp.h_mmax[h] >= kTcMinRest)
+        sp.pack_len = std::max(sp.pack_len, std::min(kPackMax, pack_stride(sp.h_mmax[h]) * sp.h_nlf[h]));
+    if (e == cudaSuccess && sp.pack_len > 0 &&
+        cudaMalloc(&sp.pack, size_t(sp.pack_len) * sizeof(float)) != cudaSuccess) {
+      cudaGetLastError();
+      sp.pack = nullptr;
+    }
+  }
   if (e != cudaSuccess) {
     sp.why = std::string("device upload of the sparse solver: ") + cudaGetErrorString(e);
     return set_err(c, e == cudaErrorMemoryAllocation ? MGPU_ERR_NOMEM : MGPU_ERR_CUDA, sp.why);
@@ -2241,7 +2341,7 @@ void sparse_destroy(SparseDev*& sp) {
                 sp->d_acol, sp->d_perm, sp->d_diag, sp->d_colptr, sp->d_rowval, sp->d_rptr, sp->d_rq, sp->d_rcol,
                 sp->F32, sp->F64, sp->prev,
                 sp->D, sp->cvec, sp->w, sp->V, sp->P, sp->d_poff, sp->tw, sp->yacc, sp->r,
-                sp->dirz, sp->dirq, sp->dz, sp->part, sp->coef, sp->xs, sp->nrm,
+                sp->dirz, sp->dirq, sp->pack, sp->dz, sp->part, sp->coef, sp->xs, sp->nrm,
                 sp->flags, sp->tflag, sp->chain};
   for (void* p : ps) cudaFree(p);
   if (sp->hflags) cudaFreeHost(sp->hflags);

@@ -58,6 +58,8 @@ struct SparseDev {
   int big_pivots = 0;                          // fronts with this many pivots or more: blocked substitutions
   bool tensor_cores = true;                    // FP32 trailing updates on the tensor cores (TF32 ×3; MGPU_SPARSE_TC=0: SIMT)
   bool tc_left = false;                        // the super-panels' left-looking blocks on the tensor cores too (MGPU_SPARSE_TC_LEFT=1)
+  float* pack = nullptr;                       // operands of the trailing blocks, split for the tensor cores
+  int64_t pack_len = 0;
   bool super_panels = true;                    // FP32 factorisation by super-panels (MGPU_SPARSE_SUPER=0: per 64-column block)
   // per height and child rank: children to add
   std::vector<std::vector<int32_t>> h_ea0, h_nea, h_eumax;

@@ -300,5 +300,120 @@ __device__ __forceinline__ bool tile_update_tf32x3(const float* __restrict__ A, 
   return ok;
 }
 
+// ---- C tile −= A · B from packed operands
+// The operands of a large block's update are split and laid out once, in the order
+// the tensor core reads (kmajor_offset with 8 columns of K), hi then lo:
+//   A: [tile of 128 rows][chunk of 8 k][hi, lo][128 × 8]
+//   B: [tile of 256 columns][chunk][hi, lo][256 × 8]
+// so a chunk's operands are one bulk copy each and the threads stage nothing: in
+// tile_update_tf32x3 each of a tile row's and a tile column's operands is loaded and
+// split again by every tile, B in 4-byte loads of eight columns; that, not the
+// MMAs, took the time (9.5 TFLOP of a lattice front tree in 85 ms, three products
+// each, a third of half the bf16 rate).  Here one thread copies, one issues
+// MMAs of 128 × 256 (a 128 × 128 one reads 8 KB of shared memory in 69 cycles, all
+// that it delivers), kPkStages chunks in flight; two blocks an SM, so that one's
+// read and write of C runs beside the other's MMAs.  The products and their order
+// are tile_update_tf32x3's.  Zeros beyond the last row, column and k.
+constexpr int kPkM = 128, kPkN = 256, kPkK = 8, kPkStages = 4;
+constexpr int kPkA = 2 * kPkM * kPkK, kPkB = 2 * kPkN * kPkK;  // floats of a chunk, hi and lo
+constexpr size_t kPkSmem = size_t(kPkStages) * (kPkA + kPkB) * sizeof(float);
+constexpr int kPkThreads = 128;
+
+// one bulk copy (16-byte aligned, a multiple of 16 bytes) into shared memory
+__device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   smem_addr(dst)),
+               "l"(src), "r"(bytes), "r"(smem_addr(bar))
+               : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
+}
+
+// Pa, Pb: the tile's packed operands, nch chunks; C(i, j) for rows below mrows and
+// columns below ncols.  bars: 2 kPkStages + 1; smem: kPkSmem bytes, 128-byte aligned.
+// False when a bounded wait ran out (then C is left as it was).
+__device__ __forceinline__ bool tile_update_packed(const float* __restrict__ Pa, const float* __restrict__ Pb, int nch,
+                                                   float* __restrict__ C, int64_t ldc, int i0, int j0, int mrows,
+                                                   int ncols, float* smem, uint64_t* bars, uint32_t* tslot, int* fail) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  uint64_t *full = bars, *empty = bars + kPkStages, *done = bars + 2 * kPkStages;
+  if (warp == 0) {
+    tmem_alloc(tslot, kPkN);
+    tmem_relinquish();
+  }
+  if (tid == 0) {
+    for (int q = 0; q < 2 * kPkStages + 1; ++q) mbar_init(bars + q, 1);
+    *fail = 0;
+  }
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  const uint32_t tmem = *tslot;
+  auto stage = [&](int s) { return smem + s * (kPkA + kPkB); };
+  if (tid == 0) {  // copies
+    int c = 0;
+    for (; c < nch; ++c) {
+      const int s = c % kPkStages;
+      if (c >= kPkStages && !mbar_wait(empty + s, uint32_t((c / kPkStages - 1) & 1), kTcPolls)) break;
+      mbar_expect(full + s, (kPkA + kPkB) * 4);
+      bulk_copy(stage(s), Pa + int64_t(c) * kPkA, kPkA * 4, full + s);
+      bulk_copy(stage(s) + kPkA, Pb + int64_t(c) * kPkB, kPkB * 4, full + s);
+    }
+    if (c < nch) {  // no copy may be in flight when the block ends
+      *reinterpret_cast<volatile int*>(fail) = 1;
+      for (int q = c < kPkStages ? 0 : c - kPkStages; q < c; ++q)
+        mbar_wait(full + q % kPkStages, uint32_t((q / kPkStages) & 1), kTcPolls);
+    }
+  } else if (tid == 32) {  // MMAs
+    const uint32_t idesc = idesc_tf32(kPkM, ncols - j0 > kPkM ? kPkN : kPkM);
+    constexpr uint32_t kLbo = 128, kSbo = (kPkK / 4) * 128;
+    bool ok = true;
+    for (int c = 0; c < nch && ok; ++c) {
+      const int s = c % kPkStages;
+      ok = mbar_wait(full + s, uint32_t((c / kPkStages) & 1), kTcPolls);
+      if (!ok) break;
+      fence_after_sync();
+      const uint32_t a = smem_addr(stage(s)), b = a + kPkA * 4;
+      const uint64_t ah = smem_desc(a, kLbo, kSbo), al = smem_desc(a + kPkA * 2, kLbo, kSbo);
+      const uint64_t bh = smem_desc(b, kLbo, kSbo), bl = smem_desc(b + kPkB * 2, kLbo, kSbo);
+      mma_tf32(tmem, ah, bh, idesc, c > 0 ? 1u : 0u);
+      mma_tf32(tmem, ah, bl, idesc, 1u);
+      mma_tf32(tmem, al, bh, idesc, 1u);
+      mma_commit(empty + s);
+    }
+    if (ok)
+      mma_commit(done);
+    else
+      *reinterpret_cast<volatile int*>(fail) = 1;
+  }
+  __syncwarp();
+  const bool ok =
+      __syncthreads_and(mbar_wait(done, 0, kTcPolls) && !*reinterpret_cast<volatile int*>(fail) ? 1 : 0) != 0;
+  fence_after_sync();
+  const int i = i0 + 32 * warp + lane;
+  const bool row_ok = ok && i < mrows;
+  const int cend = min(kPkN, ncols - j0);
+  for (int c = 0; c < cend; c += 32) {
+    float cv[32], v0[16], v1[16];
+#pragma unroll
+    for (int q = 0; q < 32; ++q) {
+      const int j = j0 + c + q;
+      cv[q] = (row_ok && j < ncols) ? C[i + int64_t(j) * ldc] : 0.f;
+    }
+    tmem_ld16(tmem + (uint32_t(32 * warp) << 16) + uint32_t(c), v0);
+    tmem_ld16(tmem + (uint32_t(32 * warp) << 16) + uint32_t(c + 16), v1);
+#pragma unroll
+    for (int q = 0; q < 32; ++q) {
+      const int j = j0 + c + q;
+      if (row_ok && j < ncols) C[i + int64_t(j) * ldc] = cv[q] - (q < 16 ? v0[q] : v1[q - 16]);
+    }
+  }
+  fence_before_sync();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, kPkN);
+  return ok;
+}
+
 }  // namespace tc
 }  // namespace mgpu

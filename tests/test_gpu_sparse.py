@@ -198,3 +198,22 @@ def test_tensor_core_trailing_update(monkeypatch):
     ref = [(0.0, (out["0"][k, 0],)) for k in range(len(out["0"]))]
     errs = state_errors(out["1"], ref, st.dis.fieldX)
     assert all(e <= TOL_STATE for e in errs.values()), errs
+
+
+@pytest.mark.parametrize("grid, nstep", [((12, 12, 6), 1), ((14, 13, 9), 1), ((20, 20, 8), 2)])
+def test_packed_trailing_update_is_bitwise_the_tile_by_tile_one(monkeypatch, grid, nstep):
+    """The trailing blocks from operands split once and copied in bulk take the same
+    products in the same order as the kernel whose tiles each load and split their own
+    (MGPU_SPARSE_PACK=0), so the states are equal bit for bit: fronts from just above
+    the smallest trailing block of the tensor cores, ragged rows, columns and pivots."""
+    m, times = W.lattice(*grid)
+    st = m.initialize()
+    out = {}
+    for pack in ("1", "0"):
+        monkeypatch.setenv("MGPU_SPARSE_PACK", pack)
+        dm = DeviceModel(m, st.dis, linsolve="sparse")
+        rc, out[pack], _ = dm.sweepx(0, times[:nstep], st.time, list(st.X), fixed_iter=3)
+        info = dm.sparse_info()
+        dm.close()
+        assert rc == 0 and info["last_fallback"] == 0 and info["max_front"] >= 512
+    assert np.array_equal(out["1"], out["0"])
