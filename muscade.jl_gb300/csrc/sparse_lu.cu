@@ -619,7 +619,7 @@ __global__ void __launch_bounds__(tc::kTcThreads) sp_trail_tc(const SpFrontDev* 
 // The same from packed operands (tc::tile_update_packed): sp_pack splits a group of
 // fronts' L and U parts of the super-panel, a front's share `stride` floats: its row
 // tiles of 128, then (from uoff) its column tiles of 256, kPackChunks chunks a tile.
-// 60 x 60 x 20 lattice, one factorisation: 85 ms by sp_trail_tc, 53 and 5 to pack.
+// 60 x 60 x 20 lattice, one factorisation: 85 ms by sp_trail_tc, 52 and 5 to pack.
 constexpr int kPackChunks = kSuper / tc::kPkK;
 constexpr int kPackThreads = 256, kPackZ = 4;
 constexpr int64_t kPackMax = int64_t(64) << 20;  // floats of the workspace at most: groups of fronts take turns

@@ -317,7 +317,7 @@ __device__ __forceinline__ bool tile_update_tf32x3(const float* __restrict__ A, 
 constexpr int kPkM = 128, kPkN = 256, kPkK = 8, kPkStages = 4;
 constexpr int kPkA = 2 * kPkM * kPkK, kPkB = 2 * kPkN * kPkK;  // floats of a chunk, hi and lo
 constexpr size_t kPkSmem = size_t(kPkStages) * (kPkA + kPkB) * sizeof(float);
-constexpr int kPkThreads = 128;
+constexpr int kPkThreads = 256;
 
 // one bulk copy (16-byte aligned, a multiple of 16 bytes) into shared memory
 __device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
@@ -388,26 +388,30 @@ __device__ __forceinline__ bool tile_update_packed(const float* __restrict__ Pa,
       *reinterpret_cast<volatile int*>(fail) = 1;
   }
   __syncwarp();
+  // epilogue: row i, half the columns a warp, 16 at a time, the next 16 of C on their way
+  // (the first ones while the MMAs run)
+  const int i = i0 + 32 * (warp & 3) + lane;
+  const int c0 = (warp >> 2) * (kPkN / 2), cn = min(kPkN / 2, ncols - j0 - c0);
+  float* Ci = C + i + int64_t(j0 + c0) * ldc;
+  const uint32_t tm = tmem + (uint32_t(32 * (warp & 3)) << 16) + uint32_t(c0);
+  float cv[2][16];
+  auto load = [&](int c, float (&v)[16]) {
+#pragma unroll
+    for (int q = 0; q < 16; ++q) v[q] = (i < mrows && c + q < cn) ? Ci[int64_t(c + q) * ldc] : 0.f;
+  };
+  load(0, cv[0]);
   const bool ok =
       __syncthreads_and(mbar_wait(done, 0, kTcPolls) && !*reinterpret_cast<volatile int*>(fail) ? 1 : 0) != 0;
   fence_after_sync();
-  const int i = i0 + 32 * warp + lane;
-  const bool row_ok = ok && i < mrows;
-  const int cend = min(kPkN, ncols - j0);
-  for (int c = 0; c < cend; c += 32) {
-    float cv[32], v0[16], v1[16];
 #pragma unroll
-    for (int q = 0; q < 32; ++q) {
-      const int j = j0 + c + q;
-      cv[q] = (row_ok && j < ncols) ? C[i + int64_t(j) * ldc] : 0.f;
-    }
-    tmem_ld16(tmem + (uint32_t(32 * warp) << 16) + uint32_t(c), v0);
-    tmem_ld16(tmem + (uint32_t(32 * warp) << 16) + uint32_t(c + 16), v1);
+  for (int c = 0; c < kPkN / 2; c += 16) {
+    if (c >= cn) break;  // the same for a warp
+    if (c + 16 < kPkN / 2) load(c + 16, cv[(c / 16 + 1) & 1]);
+    float v[16];
+    tmem_ld16(tm + uint32_t(c), v);
 #pragma unroll
-    for (int q = 0; q < 32; ++q) {
-      const int j = j0 + c + q;
-      if (row_ok && j < ncols) C[i + int64_t(j) * ldc] = cv[q] - (q < 16 ? v0[q] : v1[q - 16]);
-    }
+    for (int q = 0; q < 16; ++q)
+      if (ok && i < mrows && c + q < cn) Ci[int64_t(c + q) * ldc] = cv[(c / 16) & 1][q] - v[q];
   }
   fence_before_sync();
   __syncthreads();
