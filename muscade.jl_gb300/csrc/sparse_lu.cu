@@ -481,42 +481,17 @@ __global__ void __launch_bounds__(kThreads) sp_update_f32(const SpFrontDev* __re
 // and written once per kSuper pivots instead of once per 64.
 constexpr int kSuper = 256;
 
-// C −= L U over 128 × 128 tiles of a rectangle of every listed front, K in
-// chunks of 64.  mode 0: rows [k0, m) × columns [k0, min(k0+64, p)), K [s0, k0)
-// (the column block); mode 1: rows [k0, min(k0+64, p)) × columns [min(k0+64, p), m),
-// K [s0, k0) (the row block); mode 2: rows and columns [e0, m) with
-// e0 = min(s0 + kSuper, p), K [s0, e0) (the trailing block).  The products
-// are summed apart from C and subtracted once: accumulating them into C would
+// C −= L U over the 128 × 128 tiles of every listed front's trailing block, rows and
+// columns [e0, m) with e0 = min(s0 + kSuper, p), K [s0, e0) in chunks of 64.  The
+// products are summed apart from C and subtracted once: accumulating them into C would
 // round every product at the scale of C, which leaves the FP32 factors of the
 // large lattice fronts too coarse for the refinement.
 __global__ void __launch_bounds__(kThreads, 2) sp_rect_f32(const SpFrontDev* __restrict__ fr,
-                                                        const int32_t* __restrict__ flist, int mode, int s0, int k0,
-                                                        int ntc, float* __restrict__ F) {
+                                                        const int32_t* __restrict__ flist, int s0, int ntc,
+                                                        float* __restrict__ F) {
   const SpFrontDev Fr = fr[flist[blockIdx.y]];
   const int m = Fr.m, p = Fr.p;
-  int ra, rb, ca, cb, ka, kz;
-  if (mode == 2) {
-    const int e0 = min(s0 + kSuper, p);
-    ra = ca = e0;
-    rb = cb = m;
-    ka = s0;
-    kz = e0;
-  } else {
-    if (k0 >= p) return;
-    ka = s0;
-    kz = k0;
-    if (mode == 0) {
-      ra = k0;
-      rb = m;
-      ca = k0;
-      cb = min(k0 + 64, p);
-    } else {
-      ra = k0;
-      rb = min(k0 + 64, p);
-      ca = rb;
-      cb = m;
-    }
-  }
+  const int ka = s0, kz = min(s0 + kSuper, p), ra = kz, ca = kz, rb = m, cb = m;
   if (kz <= ka) return;
   const int i0 = ra + int(blockIdx.x / ntc) * kTile32;
   const int j0 = ca + int(blockIdx.x % ntc) * kTile32;
@@ -595,8 +570,173 @@ __global__ void __launch_bounds__(kThreads, 2) sp_rect_f32(const SpFrontDev* __r
   }
 }
 
+// the diagonal block of pivot block k0 factored in place in every listed front
+// (before sp_panel_f, which reads it factored), with the arithmetic of
+// factor_diag: NB threads, thread i owning row i in registers; the owner of the
+// pivot row hands it round through shared memory (two buffers, one block barrier
+// per step).  Bound by that chain of NB steps: with the block in shared memory a
+// step also waited for its row's loads and stores (NB = 64: 45 -> 22 us).
+template <class T, int NB, class Sync>
+__device__ __forceinline__ void diag_rows(T (&a)[NB], int kb, int i, T tau, int* __restrict__ flags, Sync&& sync) {
+  constexpr int V = 16 / sizeof(T);  // entries of a 16-byte access
+  struct __align__(16) Quad {
+    T e[V];
+  };
+  __shared__ Quad row[2][NB / V];
+  unrolled<NB>([&](auto step) {  // the steps written out: a[] stays in registers
+    constexpr int k = decltype(step)::value;
+    if (k >= kb) return;
+    if (i == k) {
+      const T d = a[k];
+      const bool bad = !isfinite(d) || (d == T(0) && tau == T(0));
+      if (bad) atomicOr(flags + 3, 1);
+      if (!bad && fabs(d) < tau) {
+        a[k] = d < T(0) ? -tau : tau;
+        atomicAdd(flags + 2, 1);
+      }
+#pragma unroll
+      for (int q = k / V; q < NB / V; ++q) {
+        Quad v;
+#pragma unroll
+        for (int e = 0; e < V; ++e) v.e[e] = a[V * q + e];
+        row[k & 1][q] = v;
+      }
+    }
+    sync();
+    if (i > k) {
+      Quad u = row[k & 1][k / V];
+      const T l = a[k] / u.e[k % V];
+      a[k] = l;
+#pragma unroll
+      for (int q = k / V; q < NB / V; ++q) {
+        if (q > k / V) u = row[k & 1][q];
+#pragma unroll
+        for (int e = 0; e < V; ++e)
+          if (V * q + e > k) a[V * q + e] -= l * u.e[e];
+      }
+    }
+  });
+}
+
+template <class T, int NB>
+__global__ void __launch_bounds__(NB) sp_diag_store(const SpFrontDev* __restrict__ fr,
+                                                    const int32_t* __restrict__ flist, int k0, T* __restrict__ F,
+                                                    T tau, int* __restrict__ flags) {
+  const SpFrontDev Fr = fr[flist[blockIdx.x]];
+  const int m = Fr.m, p = Fr.p;
+  if (k0 >= p) return;
+  const int kb = min(NB, p - k0);
+  const int i = threadIdx.x;
+  T* A = F + Fr.off + (k0 + i) + int64_t(k0) * m;  // row i of the block
+  T a[NB];
+#pragma unroll
+  for (int j = 0; j < NB; ++j) a[j] = (i < kb && j < kb) ? A[int64_t(j) * m] : T(0);
+  diag_rows<T, NB>(a, kb, i, tau, flags, [] { __syncthreads(); });
+  if (i < kb)
+#pragma unroll
+    for (int j = 0; j < NB; ++j)
+      if (j < kb) A[int64_t(j) * m] = a[j];
+}
+
+// The left-looking part of pivot block k0 of a super-panel: the column block, rows
+// [k0, m) × columns [k0, min(k0+64, p)), and the row block, rows [k0, min(k0+64, p)) ×
+// the columns after them, minus the products of the super-panel's earlier pivots
+// [s0, k0), in 64 × 64 tiles (the first ntr blocks the column block's; 128 × 128 ones
+// left half of each idle, in two launches of 18 µs on a 12 x 12 x 6 lattice).  The
+// block of the first tile goes on to factor it, so that the chain of its 64 steps,
+// 22 µs in a launch of its own, runs beside the other tiles.  60 x 60 x 20 lattice,
+// one factorisation: 28 -> 16 ms.
+// The products are summed apart from C and subtracted once, as in sp_rect_f32.
+constexpr int kLeft = 64;
+__global__ void __launch_bounds__(kThreads, 2) sp_left_f32(const SpFrontDev* __restrict__ fr,
+                                                        const int32_t* __restrict__ flist, int s0, int k0, int ntr,
+                                                        float* __restrict__ F, float tau, int* __restrict__ flags) {
+  static_assert(kThreads == 256 && kNB32 == kLeft, "16 entries a thread");
+  const SpFrontDev Fr = fr[flist[blockIdx.y]];
+  const int m = Fr.m, p = Fr.p;
+  if (k0 >= p) return;
+  const int kb = min(kLeft, p - k0);
+  const bool col = int(blockIdx.x) < ntr;
+  const int i0 = col ? k0 + int(blockIdx.x) * kLeft : k0, rb = col ? m : k0 + kb;
+  const int j0 = col ? k0 : k0 + kb + (int(blockIdx.x) - ntr) * kLeft, cb = col ? k0 + kb : m;
+  if (i0 >= rb || j0 >= cb) return;
+  float* A = F + Fr.off;
+  __shared__ __align__(16) float As[kLeft][kLeft + 4], Bs[kLeft][kLeft + 4];
+  const int tid = threadIdx.x, tr = tid & 15, tc = tid >> 4;
+  float acc[4][4] = {}, va[16], vb[16];
+  auto load = [&](int kc) {  // rows of L, then columns of U, 64 of K
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int i = tid & 63, c = 4 * u + (tid >> 6);
+      va[u] = (kc + c < k0 && i0 + i < rb) ? A[(i0 + i) + int64_t(kc + c) * m] : 0.f;
+      vb[u] = (kc + i < k0 && j0 + c < cb) ? A[(kc + i) + int64_t(j0 + c) * m] : 0.f;
+    }
+  };
+  load(s0);
+  for (int kc = s0; kc < k0; kc += kLeft) {
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int i = tid & 63, c = 4 * u + (tid >> 6);
+      As[c][i] = va[u];
+      Bs[c][i] = vb[u];
+    }
+    __syncthreads();
+    if (kc + kLeft < k0) load(kc + kLeft);
+#pragma unroll 2
+    for (int c = 0; c < kLeft; c += 4) {
+      float4 y[4];
+#pragma unroll
+      for (int v = 0; v < 4; ++v) y[v] = *reinterpret_cast<const float4*>(&Bs[4 * tc + v][c]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float4 x = *reinterpret_cast<const float4*>(&As[c + q][4 * tr]);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          const float b = q == 0 ? y[v].x : q == 1 ? y[v].y : q == 2 ? y[v].z : y[v].w;
+          acc[0][v] = fmaf(x.x, b, acc[0][v]);
+          acc[1][v] = fmaf(x.y, b, acc[1][v]);
+          acc[2][v] = fmaf(x.z, b, acc[2][v]);
+          acc[3][v] = fmaf(x.w, b, acc[3][v]);
+        }
+      }
+    }
+    __syncthreads();
+  }
+  const bool first = blockIdx.x == 0;  // the pivot block is in this tile
+  float cv[4][4];
+#pragma unroll
+  for (int v = 0; v < 4; ++v)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 + 4 * tr + u, j = j0 + 4 * tc + v;
+      cv[v][u] = (i < rb && j < cb) ? A[i + int64_t(j) * m] : 0.f;
+    }
+#pragma unroll
+  for (int v = 0; v < 4; ++v)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 + 4 * tr + u, j = j0 + 4 * tc + v;
+      const float x = cv[v][u] - acc[u][v];
+      if (first && i < k0 + kb)
+        As[4 * tc + v][4 * tr + u] = x;
+      else if (i < rb && j < cb)
+        A[i + int64_t(j) * m] = x;
+    }
+  if (!first) return;
+  __syncthreads();
+  if (tid >= kLeft) return;
+  float a[kLeft];
+#pragma unroll
+  for (int j = 0; j < kLeft; ++j) a[j] = (tid < kb && j < kb) ? As[j][tid] : 0.f;
+  diag_rows<float, kLeft>(a, kb, tid, tau, flags, [] { asm volatile("bar.sync 1, 64;" ::: "memory"); });
+  if (tid < kb)
+#pragma unroll
+    for (int j = 0; j < kLeft; ++j)
+      if (j < kb) A[(k0 + tid) + int64_t(k0 + j) * m] = a[j];
+}
+
 // the trailing block of a super-panel on the tensor cores (what sp_rect_f32
-// does in mode 2: rows and columns [e0, m) −= the super-panel's L and U parts,
+// does: rows and columns [e0, m) −= the super-panel's L and U parts,
 // K [s0, e0)), one 128 × 128 tile per block
 __global__ void __launch_bounds__(tc::kTcThreads) sp_trail_tc(const SpFrontDev* __restrict__ fr,
                                                                const int32_t* __restrict__ flist, int s0, int nt,
@@ -691,8 +831,8 @@ __global__ void __launch_bounds__(tc::kPkThreads, 2) sp_trail_packed(const SpFro
 }
 
 // the left-looking column block (mode 0) or row block (mode 1) of pivot block
-// k0 inside a super-panel on the tensor cores: what sp_rect_f32 does in those
-// modes, one 128 × 128 tile per block (the 64-wide side masked)
+// k0 inside a super-panel on the tensor cores: what sp_left_f32 does before it
+// factors, one 128 × 128 tile per block (the 64-wide side masked)
 __global__ void __launch_bounds__(tc::kTcThreads) sp_rect_tc(const SpFrontDev* __restrict__ fr,
                                                               const int32_t* __restrict__ flist, int mode, int s0,
                                                               int k0, int ntc, float* __restrict__ F,
@@ -723,68 +863,6 @@ __global__ void __launch_bounds__(tc::kTcThreads) sp_rect_tc(const SpFrontDev* _
   if (!ok && threadIdx.x == 0) atomicOr(flags + 3, 4);
 }
 
-// the diagonal block of pivot block k0 factored in place in every listed front
-// (before sp_panel_f, which reads it factored), with the arithmetic of
-// factor_diag: NB threads, thread i owning row i in registers; the owner of the
-// pivot row hands it round through shared memory (two buffers, one block barrier
-// per step).  Bound by that chain of NB steps: with the block in shared memory a
-// step also waited for its row's loads and stores (NB = 64: 45 -> 22 us).
-template <class T, int NB>
-__global__ void __launch_bounds__(NB) sp_diag_store(const SpFrontDev* __restrict__ fr,
-                                                    const int32_t* __restrict__ flist, int k0, T* __restrict__ F,
-                                                    T tau, int* __restrict__ flags) {
-  const SpFrontDev Fr = fr[flist[blockIdx.x]];
-  const int m = Fr.m, p = Fr.p;
-  if (k0 >= p) return;
-  const int kb = min(NB, p - k0);
-  const int i = threadIdx.x;
-  T* A = F + Fr.off + (k0 + i) + int64_t(k0) * m;  // row i of the block
-  constexpr int V = 16 / sizeof(T);  // entries of a 16-byte access
-  struct __align__(16) Quad {
-    T e[V];
-  };
-  __shared__ Quad row[2][NB / V];
-  T a[NB];
-#pragma unroll
-  for (int j = 0; j < NB; ++j) a[j] = (i < kb && j < kb) ? A[int64_t(j) * m] : T(0);
-  unrolled<NB>([&](auto step) {  // the steps written out: a[] stays in registers
-    constexpr int k = decltype(step)::value;
-    if (k >= kb) return;
-    if (i == k) {
-      const T d = a[k];
-      const bool bad = !isfinite(d) || (d == T(0) && tau == T(0));
-      if (bad) atomicOr(flags + 3, 1);
-      if (!bad && fabs(d) < tau) {
-        a[k] = d < T(0) ? -tau : tau;
-        atomicAdd(flags + 2, 1);
-      }
-#pragma unroll
-      for (int q = k / V; q < NB / V; ++q) {
-        Quad v;
-#pragma unroll
-        for (int e = 0; e < V; ++e) v.e[e] = a[V * q + e];
-        row[k & 1][q] = v;
-      }
-    }
-    __syncthreads();
-    if (i > k) {
-      Quad u = row[k & 1][k / V];
-      const T l = a[k] / u.e[k % V];
-      a[k] = l;
-#pragma unroll
-      for (int q = k / V; q < NB / V; ++q) {
-        if (q > k / V) u = row[k & 1][q];
-#pragma unroll
-        for (int e = 0; e < V; ++e)
-          if (V * q + e > k) a[V * q + e] -= l * u.e[e];
-      }
-    }
-  });
-  if (i < kb)
-#pragma unroll
-    for (int j = 0; j < NB; ++j)
-      if (j < kb) A[int64_t(j) * m] = a[j];
-}
 
 // FP32 trailing update on the tensor cores: one 128 × 128 tile per block
 // (tc::tile_update_tf32x3, three TF32 products per k-step, FP32 accumulators in
@@ -1817,23 +1895,24 @@ cudaError_t factorise(mgpu_ctx* c, SparseDev& sp, T* F, T tau) {
             for (int f0 = 0; f0 < cnt; f0 += kMaxGridY) {
               const int32_t* fl = sp.d_lf + sp.h_lf0[h] + f0;
               const unsigned gy = unsigned(std::min(kMaxGridY, cnt - f0));
-              if (k0 > s0) {
-                const int ntr = (rest + kTile32 - 1) / kTile32;
-                const int ntc = (rest + kTile32 - 1) / kTile32;  // columns from min(k0 + 64, p)
-                if (sp.tensor_cores && sp.tc_left && rest >= kTcMinRest) {
-                  sp_rect_tc<<<dim3(unsigned(ntr), gy), tc::kTcThreads, tc::kTcSmem, st>>>(sp.d_fr, fl, 0, s0, k0, 1,
-                                                                                          F, sp.flags);
-                  sp_rect_tc<<<dim3(unsigned(ntc), gy), tc::kTcThreads, tc::kTcSmem, st>>>(sp.d_fr, fl, 1, s0, k0, ntc,
-                                                                                          F, sp.flags);
-                } else {
-                  sp_rect_f32<<<dim3(unsigned(ntr), gy), kThreads, kUpd32Smem, st>>>(sp.d_fr, fl, 0, s0, k0, 1, F);
-                  sp_rect_f32<<<dim3(unsigned(ntc), gy), kThreads, kUpd32Smem, st>>>(sp.d_fr, fl, 1, s0, k0, ntc, F);
-                }
-                c->launches += 2;
+              if (k0 > s0 && sp.tensor_cores && sp.tc_left && rest >= kTcMinRest) {
+                const int nt = (rest + kTile32 - 1) / kTile32;  // columns from min(k0 + 64, p)
+                sp_rect_tc<<<dim3(unsigned(nt), gy), tc::kTcThreads, tc::kTcSmem, st>>>(sp.d_fr, fl, 0, s0, k0, 1, F,
+                                                                                       sp.flags);
+                sp_rect_tc<<<dim3(unsigned(nt), gy), tc::kTcThreads, tc::kTcSmem, st>>>(sp.d_fr, fl, 1, s0, k0, nt, F,
+                                                                                       sp.flags);
+                sp_diag_store<T, NB><<<gy, NB, 0, st>>>(sp.d_fr, fl, k0, F, tau, sp.flags);
+                c->launches += 3;
+              } else if (k0 > s0) {
+                const int nt = (rest + kLeft - 1) / kLeft;
+                sp_left_f32<<<dim3(unsigned(2 * nt), gy), kThreads, 0, st>>>(sp.d_fr, fl, s0, k0, nt, F, tau, sp.flags);
+                ++c->launches;
+              } else {
+                sp_diag_store<T, NB><<<gy, NB, 0, st>>>(sp.d_fr, fl, k0, F, tau, sp.flags);
+                ++c->launches;
               }
-              sp_diag_store<T, NB><<<gy, NB, 0, st>>>(sp.d_fr, fl, k0, F, tau, sp.flags);
               sp_panel_f<T, NB><<<dim3(unsigned(nrc + ncc), gy), kThreads, 0, st>>>(sp.d_fr, fl, k0, F);
-              c->launches += 2;
+              ++c->launches;
             }
           }
           int cnt = 0;
@@ -1857,7 +1936,7 @@ cudaError_t factorise(mgpu_ctx* c, SparseDev& sp, T* F, T tau) {
               sp_trail_tc<<<dim3(unsigned(nt * nt), gy), tc::kTcThreads, tc::kTcSmem, st>>>(sp.d_fr, fl, s0, nt, F,
                                                                                           sp.flags);
             } else {
-              sp_rect_f32<<<dim3(unsigned(nt * nt), gy), kThreads, kUpd32Smem, st>>>(sp.d_fr, fl, 2, s0, 0, nt, F);
+              sp_rect_f32<<<dim3(unsigned(nt * nt), gy), kThreads, kUpd32Smem, st>>>(sp.d_fr, fl, s0, nt, F);
             }
             ++c->launches;
           }
