@@ -154,17 +154,16 @@ MG_HD void mul33nt(const real A[9], const real B[9], real C[9]) {  // A Bᵀ
 // diag·I + k [v] + m v vᵀ
 MG_HD void axis_matrix(real diag, real k, real m, const real v[3], real M[9]) {
   const real m0 = m * v[0], m1 = m * v[1], m2 = m * v[2];
-  const real p01 = m0 * v[1], p02 = m0 * v[2], p12 = m1 * v[2];
   const real k0 = k * v[0], k1 = k * v[1], k2 = k * v[2];
   M[0] = fma(m0, v[0], diag);
   M[4] = fma(m1, v[1], diag);
   M[8] = fma(m2, v[2], diag);
-  M[1] = p01 + k2;
-  M[3] = p01 - k2;
-  M[2] = p02 - k1;
-  M[6] = p02 + k1;
-  M[5] = p12 + k0;
-  M[7] = p12 - k0;
+  M[1] = fma(m0, v[1], k2);
+  M[3] = fma(m0, v[1], -k2);
+  M[2] = fma(m0, v[2], -k1);
+  M[6] = fma(m0, v[2], k1);
+  M[5] = fma(m1, v[2], k0);
+  M[7] = fma(m1, v[2], -k0);
 }
 // Rodrigues(v) = cosθ I + a [v] + b v vᵀ (Rotations.jl:131-135) and its left
 // tangent map T(v) = a I + b [v] + c v vᵀ
@@ -202,9 +201,6 @@ struct BeamConst {
 struct Perturb {
   double p0, p1, p2;
 };
-
-// rotation-dof index (0..5) of element dof j, or -1 for translations
-MG_HD int rot_index(int j) { return (j >= 3 && j < 6) ? j - 3 : (j >= 9 ? j - 6 : -1); }
 
 // Geometry of an element at a state: what both the residual and the tangent use.
 struct BeamState {
@@ -459,14 +455,14 @@ MG_HD void beam_frozen(const BeamConst& c, const double* X0, const SinFun& q1, c
     cross3(tA_, bn, tAN);
     const real Pbn = dot3(P, bn);
     const real sp[9] = {0.0, P[2], -P[1], -P[2], 0.0, P[0], P[1], -P[0], 0.0};  // [P]
-    const real se = s_e * i2L * g.idn, kd = fma(c.ke * i2L, i2L, -se);
+    const real s2 = s_e * i2L, kd = fma(c.ke * i2L, i2L, -(s2 * g.idn));
     int k = 0;
     for (int i = 0; i < 3; ++i)
       for (int j = 0; j < 3; ++j) {
         const real wi = c.k3u * nn[i], vi = c.k2u * bb[i];
         if (j >= i) {
           real v = fma(wi, nn[j], fma(vi, bb[j], kd * g.dh[i] * g.dh[j]));
-          if (i == j) v += se;
+          if (i == j) v = fma(s2, g.idn, v);
           Hdd[k] = v;
           v = fma(En[i], unp[j], fma(C[2][i], ubp[j], fma(Eb[i], vbp[j], fma(C[1][i], vnp[j], fma(C[0][i], ctp[j], K6[k])))));
           Hpp[k] = v;
@@ -548,14 +544,14 @@ MG_HD void beam_frozen(const BeamConst& c, const double* X0, const SinFun& q1, c
     for (int a = 0; a < 2; ++a) {
       const real *v = va[a], *G_ = Ga[a];
       const SinFun& qq = *qa[a];
-      const real gv_ = dot3(G_, v), cg = qq.c * gv_, kg = fma(2.0, qq.c, -qq.b), kx = 2.0 * sin_bs(qq), kv = 2.0 * sin_cs(qq) * gv_;
+      const real gv_ = dot3(G_, v), kg = fma(2.0, qq.c, -qq.b), kx = 2.0 * sin_bs(qq), kv = 2.0 * sin_cs(qq) * gv_;
       real gx[3], kk[3];
       cross3(G_, v, gx);
       for (int i = 0; i < 3; ++i) kk[i] = 0.5 * fma(kg, G_[i], fma(kx, gx[i], kv * v[i]));
       for (int i = 0; i < 3; ++i)
         for (int j = i; j < 3; ++j) {
           real w = dot3(Xa[a] + 3 * i, Sa[a] + 3 * j);
-          w = i == j ? fma(2.0 * v[i], kk[i], w + cg) : fma(v[i], kk[j], fma(v[j], kk[i], w));
+          w = i == j ? fma(2.0 * v[i], kk[i], fma(qq.c, gv_, w)) : fma(v[i], kk[j], fma(v[j], kk[i], w));
           out(3 + 6 * a + i, 3 + 6 * a + j, w);
         }
     }

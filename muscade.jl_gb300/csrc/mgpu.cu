@@ -138,6 +138,73 @@ __global__ void __launch_bounds__(256) beam_static_kernel(int64_t nele, const in
   flag_nan(a.errflag, gid0 + e, bad);
 }
 
+// The same for models that leave sub-partitions idle: the entries of 32 beams' matrices
+// in four parts, a warp each, with what each needs of the geometry and the second
+// variation (the compiler drops the rest): the translations' rows with the residual,
+// and the three blocks of the rotations.
+// A thread per beam / split, µs: 20 beams 56/38, 1,000 61/39, 4,800 61/40, 6,000 61/75
+// (four warps for 32 beams fill the 608 sub-partitions once at 4,864 beams).
+constexpr int64_t kStaticSplitMax = 4864;
+template <int PART, bool GEN>
+__device__ __forceinline__ void beam_static_part(const BeamConst& bc, const double* X0, const double* U,
+                                                 const double* s, double p0, int64_t nele, int64_t e,
+                                                 double* __restrict__ rout, double* __restrict__ kout, bool& bad) {
+  double R[12];
+  auto store = [&](int i, int j, double v) {
+    const bool ri = i % 6 >= 3, rj = j % 6 >= 3;
+    const int part = !ri || !rj ? 0 : j < 6 ? 1 : i >= 6 ? 2 : 3;
+    if (part != PART) return;
+    if constexpr (GEN) v *= p0 * s[i] * s[j];
+    bad |= nan_bits(v);
+    kout[(i + 12 * j) * nele + e] = v;
+    if (i != j) kout[(j + 12 * i) * nele + e] = v;
+  };
+  beam_static(bc, X0, U, R, store, nullptr);
+  if constexpr (PART == 0)
+#pragma unroll
+    for (int i = 0; i < 12; ++i) {
+      const double r = GEN ? R[i] * s[i] : R[i];
+      bad |= nan_bits(r);
+      rout[i * nele + e] = r;
+    }
+}
+
+template <bool GEN>
+__global__ void __launch_bounds__(128) beam_static_split_kernel(int64_t nele, const int32_t* __restrict__ idx,
+                                                                const int32_t* __restrict__ uidx,
+                                                                const double* __restrict__ cdata,
+                                                                const int32_t* __restrict__ aidx,
+                                                                const double* __restrict__ Avec, AsmArgs a,
+                                                                double* __restrict__ rout, double* __restrict__ kout,
+                                                                int64_t gid0) {
+  const int64_t e = int64_t(blockIdx.x) * 32 + (threadIdx.x & 31);
+  if (e >= nele) return;
+  BeamConst bc;
+  load_soa(bc, cdata, nele, e);
+  if (aidx) scale_bending(bc, __ldg(Avec + __ldg(aidx + e)));
+  double X0[12], s[12];
+#pragma unroll
+  for (int i = 0; i < 12; ++i) {
+    const int dof = __ldg(idx + i * nele + e);
+    X0[i] = __ldg(a.x0 + dof);
+    if constexpr (GEN) s[i] = a.scale ? __ldg(a.scale + dof) : 1.0;
+  }
+  double U[3];
+  const bool has_u = uidx != nullptr;
+  if (has_u)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) U[k] = __ldg(a.u + __ldg(uidx + k * nele + e));
+  const double* u = has_u ? U : nullptr;
+  bool bad = false;
+  switch (threadIdx.x >> 5) {
+    case 0: beam_static_part<0, GEN>(bc, X0, u, s, a.p0, nele, e, rout, kout, bad); break;
+    case 1: beam_static_part<1, GEN>(bc, X0, u, s, a.p0, nele, e, rout, kout, bad); break;
+    case 2: beam_static_part<2, GEN>(bc, X0, u, s, a.p0, nele, e, rout, kout, bad); break;
+    default: beam_static_part<3, GEN>(bc, X0, u, s, a.p0, nele, e, rout, kout, bad);
+  }
+  flag_nan(a.errflag, gid0 + e, bad);
+}
+
 // SweepX{2}; the same launch sizes.  STEP: a step's first iteration, with the
 // residual's part along the Newmark vectors a and b taken off.
 template <bool STEP>
@@ -648,7 +715,11 @@ int launch_assembly(mgpu_ctx* c, int mission, cudaEvent_t* ev_groups, double p0,
         else if (dyn)
           beam_kernel<false><<<nblk(G.nele, c->elem_block), c->elem_block, 0, c->stream>>>(
               G.nele, G.idx, G.uidx, G.cdata, G.aidx, c->Avec, ag, rout, kout, gid0);
-        else if (ag.scale || p0 != 1.0)
+        else if (G.nele <= kStaticSplitMax) {
+          const auto kern = ag.scale || p0 != 1.0 ? beam_static_split_kernel<true> : beam_static_split_kernel<false>;
+          kern<<<nblk(G.nele, 32), 128, 0, c->stream>>>(G.nele, G.idx, G.uidx, G.cdata, G.aidx, c->Avec, ag, rout, kout,
+                                                        gid0);
+        } else if (ag.scale || p0 != 1.0)
           beam_static_kernel<true><<<nblk(G.nele, c->elem_block), c->elem_block, 0, c->stream>>>(
               G.nele, G.idx, G.uidx, G.cdata, G.aidx, c->Avec, ag, rout, kout, gid0);
         else
