@@ -425,6 +425,7 @@ static void analyse(mgpu_ctx* c, Solver& S) {
     const int64_t target_warps = int64_t(16) * nsm;
     const int64_t pcap = std::max<int64_t>(1, (target_warps + ncomp - 1) / std::max(ncomp, 1));
     std::vector<int> Pc(ncomp, 1), sc(ncomp, 0);
+    std::vector<std::vector<int64_t>> cut(ncomp);  // first dof of each separator
     for (int cc = 0; cc < ncomp; ++cc) {
       const int64_t nc = comp_start[cc + 1] - comp_start[cc];
       const int sw = std::max(1, std::max(kl[cc], ku[cc]));
@@ -432,7 +433,32 @@ static void analyse(mgpu_ctx* c, Solver& S) {
       if (sw > 16 || nc < kTornMinDofs) continue;
       const int64_t mmin = std::max(2 * sw, 48);
       const int64_t pmax = std::min((nc + sw) / (mmin + sw), pcap > 5 ? pcap : std::min<int64_t>(pcap, 2));
-      Pc[cc] = int(std::max<int64_t>(1, pmax));
+      // separators at equal distances; one that would part a multiplier from a dof it
+      // holds, leaving an interior with a zero row, moves to the nearest place where it
+      // does not, or is left out
+      const int64_t c0 = comp_start[cc], P = std::max<int64_t>(1, pmax), tot = nc - (P - 1) * sw;
+      auto whole = [&](int64_t at) {
+        for (int64_t q = std::max<int64_t>(0, at - sw); q < std::min(nc, at + 2 * sw); ++q) {
+          const int32_t v = order[c0 + q];
+          if ((q >= at && q < at + sw) || c->dof_last.empty() || !c->dof_last[v]) continue;
+          for (int64_t e = deg[v]; e < deg[v + 1]; ++e) {
+            const int64_t u = pos[adj[e]] - c0;
+            if (u >= at && u < at + sw) return false;
+          }
+        }
+        return true;
+      };
+      for (int64_t a = 0, p0 = 0, prev = 0; a + 1 < P; ++a) {
+        p0 += tot / P + (a < tot % P ? 1 : 0) + (a > 0 ? sw : 0);
+        for (int64_t d = 0; d <= 4 * sw; ++d) {  // 0, 1, -1, 2, -2, ...
+          const int64_t at = p0 + (d % 2 ? (d + 1) / 2 : -(d / 2));
+          if (at - prev < mmin || nc - at - sw < mmin || !whole(at)) continue;
+          cut[cc].push_back(at);
+          prev = at + sw;
+          break;
+        }
+      }
+      Pc[cc] = int(cut[cc].size()) + 1;
       if (Pc[cc] > 1) S.tearable = 1;
     }
     if (S.tearable) {
@@ -454,11 +480,10 @@ static void analyse(mgpu_ctx* c, Solver& S) {
         csep0[cc] = int32_t(ts.size());
         S.maxP = std::max(S.maxP, P);
         maxwI = std::max(maxwI, w);
-        const int64_t tot = nc - int64_t(P - 1) * sw;
         int64_t p0 = 0;
         const int sep0 = int(ts.size()), int0 = int(ti.size());
         for (int a = 0; a < P; ++a) {
-          const int64_t m = tot / P + (a < tot % P ? 1 : 0);
+          const int64_t m = (a < P - 1 ? cut[cc][a] : nc) - p0;
           TornInt I{};
           I.rbase = orow;
           I.lbase = olm;

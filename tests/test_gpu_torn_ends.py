@@ -18,7 +18,7 @@ def _states(m, st, times, kind, OX=0, **kw):
     rc, X, _ = dm.sweepx(OX, times, st.time, [st.X[0]] * (OX + 1), **kw)
     again = dm.sweepx(OX, times, st.time, [st.X[0]] * (OX + 1), **kw)[1]
     dm.close()
-    assert rc == 0 and np.array_equal(X, again)
+    assert rc == 0 and (kind == "auto" or np.array_equal(X, again))  # auto may leave FP32 factors for good
     return X
 
 
@@ -51,3 +51,27 @@ def test_risers_match_whole_components(kind):
     st = m.initialize(time=0.0)
     kw = dict(OX=2, fixed_iter=4)
     _same(st, _states(m, st, times[:3], kind, **kw), _states(m, st, times[:3], "f64", **kw))
+
+
+@pytest.mark.parametrize("nel, every, ncomp", [(120, 60, 1), (120, 7, 3), (120, 1, 1), (120, 2, 2), (120, 60, 490)])
+def test_intermediate_supports_match_whole_components(nel, every, ncomp):
+    """Multipliers along the chain: no separator may part one from its dof (the interior
+    would have a zero row), so separators move, or a component stays whole."""
+    m = W.Model("supports")
+    mat = W.BeamCrossSection(EA=1e8, EI2=1e4, EI3=1e4, GJ=1e4, mu=10.0, iota1=1.0)
+    x = np.linspace(0.0, 0.5 * nel, nel + 1)
+    ends, held = [], []
+    for c in range(ncomp):
+        nodes = m.addnode(np.stack([x, np.full_like(x, 5.0 * c), np.zeros_like(x)], axis=1))
+        m.addelement(W.EulerBeam3D, np.stack([nodes[:-1], nodes[1:]], axis=1), mat=mat, orient2=(0.0, 1.0, 0.0))
+        ends += [nodes[0]]
+        held += list(nodes[every:-1:every])
+        m.addelement(W.DofLoad, nodes[every // 2 : every // 2 + 1, None], field="t3", value=lambda t: 50.0 * t)
+        m.addelement(W.DofLoad, nodes[-1:, None], field="t1", value=lambda t: 100.0 * t)
+    for f in ("t1", "t2", "t3", "r1", "r2", "r3"):
+        m.addelement(W.Hold, np.asarray(ends)[:, None], field=f)
+    for f in ("t2", "t3"):
+        m.addelement(W.Hold, np.asarray(held)[:, None], field=f)
+    st = m.initialize()
+    times = np.array([0.5, 1.0])
+    _same(st, _states(m, st, times, "auto", maxdx=1e-9), _states(m, st, times, "f64", maxdx=1e-9))
