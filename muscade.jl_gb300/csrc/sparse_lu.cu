@@ -1674,17 +1674,38 @@ __global__ void sp_start(int64_t n, const int32_t* __restrict__ perm, const doub
   w[k] = r[d] = D[d] * b[d];
 }
 
-// z = w, and D z in model order
-__global__ void sp_direction(int64_t n, const int32_t* __restrict__ perm, const double* __restrict__ D,
-                             const double* __restrict__ w, double* __restrict__ z, double* __restrict__ dz,
-                             const int* __restrict__ conv) {
+// |v| as ordered bits (non-negative doubles order like their bit patterns); NaN wins:
+// the block's largest to dst
+__device__ __forceinline__ void max_bits(unsigned long long* dst, double v) {
+  __shared__ double smax[kThreads / 32];
+  v = isnan(v) ? INFINITY : fabs(v);
+  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  if ((threadIdx.x & 31) == 0) smax[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int q = 1; q < kThreads / 32; ++q) v = fmax(v, smax[q]);
+    atomicMax(dst, (unsigned long long)__double_as_longlong(v));
+  }
+}
+
+// z = w, and D z in model order; the largest |w| of the sweep, the error that the
+// factors see before its step, decides convergence (not the step: a step along a
+// direction that does not reduce the residual is short without being right)
+__global__ void __launch_bounds__(kThreads) sp_direction(int64_t n, const int32_t* __restrict__ perm,
+                                                         const double* __restrict__ D, const double* __restrict__ w,
+                                                         double* __restrict__ z, double* __restrict__ dz,
+                                                         unsigned long long* __restrict__ nrm,
+                                                         const int* __restrict__ conv) {
   if (*conv) return;
   const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  const int32_t d = perm[k];
-  const double v = w[k];
-  z[k] = v;
-  dz[d] = D[d] * v;
+  double v = 0.0;
+  if (k < n) {
+    const int32_t d = perm[k];
+    v = w[k];
+    z[k] = v;
+    dz[d] = D[d] * v;
+  }
+  max_bits(nrm, v);
 }
 
 // Sums over all blocks of acc[0..NV), nv of them: each block's to part, and the block
@@ -1786,13 +1807,8 @@ __global__ void __launch_bounds__(kThreads) sp_conjugate(int64_t n, int it, cons
   }
   if (sp_sums(acc, 2, part, done, sum) && threadIdx.x == 0) {
     *qq = sum[0];
-    *alpha = sum[0] == 0.0 ? 0.0 : sum[1] / sum[0];  // zero only with a zero residual
+    *alpha = sum[0] > 0.0 ? sum[1] / sum[0] : 1.0;  // 1: no residual left, or a refinement step as it is
   }
-}
-
-__device__ __forceinline__ void max_bits(unsigned long long* dst, double v) {
-  // |v| as ordered bits (non-negative doubles order like their bit patterns); NaN wins
-  atomicMax(dst, (unsigned long long)__double_as_longlong(isnan(v) ? INFINITY : fabs(v)));
 }
 
 // y += alpha z, x = D y, r -= alpha q; w: the new residual in elimination order
@@ -1804,43 +1820,24 @@ __global__ void __launch_bounds__(kThreads) sp_step(int64_t n, int first, const 
                                                     unsigned long long* __restrict__ nrm,
                                                     const int* __restrict__ conv) {
   if (*conv) return;
-  __shared__ double smax[2][kThreads / 32];
   const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  double mw = 0.0, my = 0.0;
+  double y = 0.0;
   if (k < n) {
     const double al = *alpha, z = al * zv[k];
-    const double y = first ? z : yacc[k] + z;
+    y = first ? z : yacc[k] + z;
     yacc[k] = y;
     const int32_t d = perm[k];
     x[d] = D[d] * y;
     w[k] = r[d] = fma(-al, q[d], r[d]);
-    mw = isnan(z) ? INFINITY : fabs(z);
-    my = isnan(y) ? INFINITY : fabs(y);
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    mw = fmax(mw, __shfl_xor_sync(0xffffffffu, mw, o));
-    my = fmax(my, __shfl_xor_sync(0xffffffffu, my, o));
-  }
-  if ((threadIdx.x & 31) == 0) {
-    smax[0][threadIdx.x >> 5] = mw;
-    smax[1][threadIdx.x >> 5] = my;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int q = 1; q < kThreads / 32; ++q) {
-      mw = fmax(mw, smax[0][q]);
-      my = fmax(my, smax[1][q]);
-    }
-    max_bits(nrm, mw);
-    max_bits(nrm + 1, my);
-  }
+  max_bits(nrm + 1, y);
 }
 
-// Converged when the scaled correction is below tol of the scaled solution, or the
-// next one would be, by a factor of ten, at the rate of the last two (the rate only
-// improves from sweep to sweep), or when it has stopped shrinking (no better than half the previous one)
-// while below stall of the solution: the attainable accuracy of the FP64
-// residual is then reached.  prev holds the previous correction's norm.
+// Converged when the scaled correction M^-1 r is below tol of the scaled solution, or
+// the next one would be, by a factor of ten, at the rate of the last two (the rate only
+// improves from sweep to sweep), or when it has stopped shrinking (no better than half
+// the previous one) while below stall of the solution: the attainable accuracy of the
+// FP64 residual is then reached.  prev holds the previous correction's norm.
 __global__ void sp_check(unsigned long long* nrm, double* prev, int* flags, double tol, double stall) {
   if (flags[0]) return;
   const double nw = __longlong_as_double((long long)nrm[0]), ny = __longlong_as_double((long long)nrm[1]);
@@ -2109,7 +2106,8 @@ cudaError_t refine(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, int 
     }
     double *z = sp.dirz + it * n, *q = sp.dirq + it * n;
     const unsigned gd = std::max(1u, std::min(unsigned(kDotBlocks), unsigned(nblocks(n, kThreads))));
-    sp_direction<<<nblocks(n, kThreads), kThreads, 0, st>>>(n, sp.d_perm, sp.D, sp.w, z, sp.dz, sp.flags);
+    sp_direction<<<nblocks(n, kThreads), kThreads, 0, st>>>(n, sp.d_perm, sp.D, sp.w, z, sp.dz, sp.nrm,
+                                                             sp.flags);
     sp_apply<<<gd, kThreads, 0, st>>>(n, it, sp.d_rptr, sp.d_rq, sp.d_rcol, c->nzval, sp.D, sp.dz, sp.dirq, q, sp.part,
                                       sp.done, sp.coef, sp.coef + kSparseSweeps, sp.flags);
     sp_conjugate<<<gd, kThreads, 0, st>>>(n, it, sp.dirq, sp.dirz, q, z, sp.r, sp.coef + kSparseSweeps, sp.part,
