@@ -66,13 +66,14 @@ static int lu_class(int s, int w) {
 // (dofs with one neighbour) set aside, dofs of equal closed neighbourhood grouped,
 // the groups in reverse Cuthill-McKee order, and each group's leaves before it at
 // the start of the order, else behind it.  The narrower of the two is kept.
-static void narrow_by_nodes(int64_t n, const std::vector<int64_t>& deg, const std::vector<int32_t>& adj,
-                            const std::vector<std::vector<int32_t>>& members, const std::vector<int32_t>& comp_start,
-                            std::vector<int32_t>& order, std::vector<int32_t>& pos) {
+static void narrow_by_nodes(const Pattern& P, const std::vector<std::vector<int32_t>>& members,
+                            const std::vector<int32_t>& comp_start, std::vector<int32_t>& order,
+                            std::vector<int32_t>& pos) {
+  const int64_t n = int64_t(pos.size());
   auto width = [&](const std::vector<int32_t>& M) {
     int32_t w = 0;
     for (int32_t v : M)
-      for (int64_t q = deg[v]; q < deg[v + 1]; ++q) w = std::max(w, std::abs(pos[adj[q]] - pos[v]));
+      for (int64_t q = P.colptr[v]; q < P.colptr[v + 1]; ++q) w = std::max(w, std::abs(pos[P.rowval[q]] - pos[v]));
     return w;
   };
   std::vector<int32_t> todo, wid(members.size());
@@ -82,25 +83,26 @@ static void narrow_by_nodes(int64_t n, const std::vector<int64_t>& deg, const st
   for (size_t cc = 0; cc < members.size(); ++cc)
     if (wid[cc] > 11 && wid[cc] <= 48 && members[cc].size() > 2) todo.push_back(int32_t(cc));
   if (todo.empty()) return;
-  std::vector<int32_t> nb(adj.size()), cnt(n, 0), grp(n, -1), host(n, -1);  // sorted neighbours, each once
+  std::vector<int32_t> nb(P.nnz), cnt(n, 0), grp(n, -1), host(n, -1);  // neighbours: a column's rows but its own
 #pragma omp parallel for schedule(dynamic, 16) if (n > 50000)
   for (int64_t t = 0; t < int64_t(todo.size()); ++t) {
     const auto& M = members[todo[t]];
     const int32_t c0 = comp_start[todo[t]], w0 = wid[todo[t]];
     for (int32_t v : M) {
-      std::copy(adj.begin() + deg[v], adj.begin() + deg[v + 1], nb.begin() + deg[v]);
-      std::sort(nb.begin() + deg[v], nb.begin() + deg[v + 1]);
-      cnt[v] = int32_t(std::unique(nb.begin() + deg[v], nb.begin() + deg[v + 1]) - (nb.begin() + deg[v]));
+      int32_t* to = nb.data() + P.colptr[v];
+      for (int64_t q = P.colptr[v]; q < P.colptr[v + 1]; ++q)
+        if (P.rowval[q] != v) *to++ = int32_t(P.rowval[q]);
+      cnt[v] = int32_t(to - (nb.data() + P.colptr[v]));
     }
     for (int32_t v : M) {
-      const int32_t u = cnt[v] == 1 ? nb[deg[v]] : -1;
+      const int32_t u = cnt[v] == 1 ? nb[P.colptr[v]] : -1;
       host[v] = u >= 0 && cnt[u] > 1 ? u : -1;
     }
     // groups of equal closed neighbourhood (leaves left out), by a hash of the list
     auto closed = [&](int32_t v, std::vector<int32_t>& k) {
       k.clear();
       for (int32_t q = 0; q < cnt[v]; ++q)
-        if (host[nb[deg[v] + q]] < 0) k.push_back(nb[deg[v] + q]);
+        if (host[nb[P.colptr[v] + q]] < 0) k.push_back(nb[P.colptr[v] + q]);
       k.insert(std::lower_bound(k.begin(), k.end(), v), v);
     };
     std::vector<std::pair<uint64_t, int32_t>> key;
@@ -132,7 +134,7 @@ static void narrow_by_nodes(int64_t n, const std::vector<int64_t>& deg, const st
     std::vector<std::vector<int32_t>> ga(ng);
     for (int g = 0; g < ng; ++g) {
       for (int32_t q = 0, v = G[g][0]; q < cnt[v]; ++q) {
-        const int32_t u = nb[deg[v] + q];
+        const int32_t u = nb[P.colptr[v] + q];
         if (host[u] < 0 && grp[u] != g) ga[g].push_back(grp[u]);
       }
       std::sort(ga[g].begin(), ga[g].end());
@@ -299,7 +301,7 @@ static void analyse(mgpu_ctx* c, Solver& S) {
   comp_start[ncomp] = int32_t(order.size());
   std::vector<int32_t> pos(n);
   for (int64_t k = 0; k < n; ++k) pos[order[k]] = int32_t(k);
-  narrow_by_nodes(n, deg, adj, members, comp_start, order, pos);
+  narrow_by_nodes(P, members, comp_start, order, pos);
   // bandwidths per component
   std::vector<int32_t> kl(ncomp, 0), ku(ncomp, 0);
   for (int64_t j = 0; j < n; ++j)
