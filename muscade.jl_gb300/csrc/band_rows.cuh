@@ -24,7 +24,7 @@
 // computed instead of dividing by the pivot: an FP64 division is a chain of
 // about ten dependent FP64 instructions, on the critical path of every column.
 // With T = double the factors and the solution are bitwise those of the block
-// kernels in solver.cu, which do the same.
+// kernels in band_block.cuh, which do the same.
 //
 // Storage per component (offsets rbase, lbase, dof0 from the host analysis):
 //   A  (FP64, unfactorised rows)  A[i*w + (j - i + kl)],   w = kv + 1
@@ -111,7 +111,7 @@ struct TornInt {
   int64_t yL, yR;          // offsets of Y^L, Y^R (m x s), -1 if absent
   int32_t sepL, sepR;      // global index of the left / right separator, -1 if absent
   int32_t comp;            // connected component it belongs to
-  int32_t end;             // 1: an end of its component, held as [factors | coupling] (tb_end)
+  int32_t end;             // 1: an end of its component, without a spike (tb_end)
 };
 
 struct RbComp {

@@ -53,12 +53,16 @@ __device__ __forceinline__ bool tb_skip(const int* only, int comp) { return only
 // An interior with one separator needs no spike: with the separator after its last
 // row (the last interior of a component is numbered backwards for that), the
 // separator is only the next rows of the same elimination,
-//     T_kk -= G Z,   r_k -= G z,   x_a = U^-1 (z - Z x_S),   z = L^-1 P b_a,
-// with Z = L^-1 P E^R, nonzero in the last s + kl rows, and G = F^R U^-1, from the
-// last s rows of U alone.  Both come from the last s + kl pivot steps, where the
-// spikes cost kl + kv FMAs a row over the whole interior, half as much again as its
-// LU (512 frame chains of 60 to 2,400 dofs, five interiors each: 1.7 of 3.9 ms).  Y^R's room holds G (rows 0..s) and Z (its own rows); n >= 2 s + kl, since
-// interiors have at least 48 rows and s <= 16.
+//     T_kk -= F^R U^-1 Z,   r_k -= F^R U^-1 z,   x_a = U^-1 (z - Z x_S),   z = L^-1 P b_a,
+// with Z = L^-1 P E^R, nonzero in the last s + kl rows, and U^-1 Z, U^-1 z wanted in the
+// last s rows only, which the last s rows of U give.  So the coupling comes from the
+// last s + kl pivot steps, where the spikes cost kl + kv FMAs a row over the whole
+// interior, half as much again as its LU (512 frame chains of 60 to 2,400 dofs, five
+// interiors each: 1.7 of 3.9 ms).  The last interior is numbered backwards only where
+// components are cut in two: FP32 factors of 200 risers in 13 interiors, eliminated
+// from the driven end too, fell short of their refinement within 20 steps and left the
+// rest to FP64 (6.0 -> 6.7 ms a step).  Y^R's room holds U^-1 Z (rows 0..s) and Z (its
+// own rows); n >= 2 s + kl, since interiors have at least 48 rows and s <= 16.
 template <typename T, int KLW>
 __device__ void tb_end(const TornInt& I, const T* __restrict__ U, const T* __restrict__ L,
                        const int32_t* __restrict__ piv, const T* __restrict__ blk, T* __restrict__ Y, T* sU, T* sL,
@@ -97,39 +101,72 @@ __device__ void tb_end(const TornInt& I, const T* __restrict__ U, const T* __res
 #pragma unroll
     for (int p = 0; p < KLW; ++p) yw[p] = p < kl ? yw[min(p + 1, KLW - 1)] : p == kl ? nx : yw[p];
   }
-  // G, a row per lane
+  // U^-1 Z in the last s rows
   T g[16];
 #pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    if (j < s) {
-      T v = blk[I.fR + lane * s + j];
+  for (int j = 0; j < 16; ++j) g[j] = j < s ? Yr[int64_t(m - s + j) * s] : T(0);
 #pragma unroll
-      for (int q = 0; q < j; ++q) v = fma(-sU[j * w + j - q], g[q], v);
-      g[j] = v * sU[j * w];  // 1/U(j,j)
-      Y[I.yR + lane * s + j] = g[j];
+  for (int j = 15; j >= 0; --j) {
+    if (j < s) {
+      const T x = g[j] * sU[j * w];  // 1/U(j,j)
+      Yr[int64_t(j) * s] = x;
+#pragma unroll
+      for (int q = 0; q < j; ++q) g[q] = fma(-sU[j * w + j - q], x, g[q]);
     }
   }
 }
 
-// F^R (or G) of a separator's left interior and the rows it meets, and the same of its
-// right interior (F^L, or G of one numbered backwards)
+// F^R of a separator's left interior and the rows it meets, and the same of its right
+// interior (F^L, or F^R of one numbered backwards)
 template <typename T>
 struct TornSides {
   const T *fl, *fr;  // s x s
-  int64_t yl, yr;    // offsets in Y of the s rows next to the separator
+  int64_t yl, yr;    // offsets in Y of the spikes' s rows next to the separator
   int32_t pl, pr;    // band positions of these rows
 };
 template <typename T>
-__device__ __forceinline__ TornSides<T> tb_sides(const TornInt& IL, const TornInt& IR, const T* blk, const T* Y) {
+__device__ __forceinline__ TornSides<T> tb_sides(const TornInt& IL, const TornInt& IR, const T* blk) {
   TornSides<T> r;
   const int s = IL.s;
-  r.fl = IL.end ? Y + IL.yR : blk + IL.fR;
-  r.yl = IL.yR + int64_t(IL.n - s) * s;
+  r.fl = blk + IL.fR;
+  r.yl = IL.yR + (IL.end ? 0 : int64_t(IL.n - s) * s);
   r.pl = IL.dof0 + IL.n - s;
-  r.fr = IR.end ? Y + IR.yR : blk + IR.fL;
-  r.yr = IR.end ? IR.yR + int64_t(IR.n - s) * s : IR.yL;
+  r.fr = blk + (IR.end ? IR.fR : IR.fL);
+  r.yr = IR.end ? IR.yR : IR.yL;
   r.pr = IR.end ? IR.dof0 + IR.n - s : IR.dof0;
   return r;
+}
+
+// row `lane` < s of b_S - F^R_{left} ỹ_{left}[last s] - F^L_{right} ỹ_{right}[first s].
+// v: this lane's entry of the left (lanes 0..s) or the right (lanes 16..16+s) interior's
+// rows next to the separator; of an end interior z, whose backward substitution's first
+// s steps are done here.
+template <typename T>
+__device__ __forceinline__ T tb_sep_row(const TornSides<T>& sd, const TornInt& IL, const TornInt& IR,
+                                        const T* __restrict__ UC, T v, T b, int lane) {
+  const int s = IL.s, l = lane & 15;
+  const bool end = lane < 16 ? IL.end : IR.end;
+  if (IL.end || IR.end) {
+    const int w = lane < 16 ? IL.kl + IL.ku + 1 : IR.kl + IR.ku + 1;
+    const T* U = UC + (lane < 16 ? IL.rbase + int64_t(IL.n - s) * w : IR.rbase + int64_t(IR.n - s) * w);
+    T u[16];  // U(l, j) of this lane's row, 1/U(l, l)
+#pragma unroll
+    for (int j = 0; j < 16; ++j) u[j] = end && j < s && l <= j ? U[j * w + j - l] : T(0);
+#pragma unroll
+    for (int j = 15; j >= 0; --j) {
+      if (j >= s) continue;
+      const T x = __shfl_sync(RB_FULL, v, j, 16) * __shfl_sync(RB_FULL, u[j], j, 16);
+      if (end) v = l == j ? x : l < j ? fma(-u[j], x, v) : v;
+    }
+  }
+  for (int q = 0; q < s; ++q) {
+    const T yl = __shfl_sync(RB_FULL, v, q), yr = __shfl_sync(RB_FULL, v, 16 + q);
+    if (lane < s) {
+      b -= sd.fl[lane * s + q] * yl;
+      b -= sd.fr[lane * s + q] * yr;
+    }
+  }
+  return b;
 }
 
 // ---------------------------------------------------------------- spikes
@@ -268,7 +305,7 @@ __global__ void __launch_bounds__(32) tb_schur(int nsep, const TornSep* __restri
   if (tb_skip(only, S.comp)) return;
   const int s = S.s;
   const TornInt IL = ti[S.intL], IR = ti[S.intR];
-  const TornSides<T> sd = tb_sides<T>(IL, IR, blk, Y);
+  const TornSides<T> sd = tb_sides<T>(IL, IR, blk);
   T* Dk = DLU + 3 * int64_t(k) * BCR_SS;
   T* Uk = Dk + 2 * BCR_SS;
   T* Lk1 = DLU + (3 * int64_t(k + 1) + 1) * BCR_SS;  // L of the next separator (only when !S.last)
@@ -303,43 +340,32 @@ __global__ void __launch_bounds__(32) tb_schur(int nsep, const TornSep* __restri
 
 // ---------------------------------------------------------------- solve
 // separator right-hand sides: r = b_S - F^R_{left} ỹ_{left}[last s] - F^L_{right} ỹ_{right}[first s]
-// (b and ỹ in model order; ỹ of the interiors is already in x); arithmetic in
-// the factors' type, stored in FP64.  One warp; yl, yr: s entries of scratch.
+// (b and ỹ in model order; ỹ of the interiors, z of the end ones, is already in x);
+// arithmetic in the factors' type, stored in FP64.  One warp.
 template <typename T>
 __device__ void tb_sep_rhs_warp(const TornSep& S, const TornInt* __restrict__ ti, const T* __restrict__ blk,
-                                const T* __restrict__ Y, const int32_t* __restrict__ perm, const double* b, const double* x, double* tr,
-                                T* yl, T* yr, int lane) {
-  const int s = S.s;
-  const TornSides<T> sd = tb_sides<T>(ti[S.intL], ti[S.intR], blk, Y);
-  if (lane < s) {
-    yl[lane] = T(x[perm[sd.pl + lane]]);
-    yr[lane] = T(x[perm[sd.pr + lane]]);
-  }
-  __syncwarp();
-  if (lane < s) {
-    T v = T(b[perm[S.dof0 + lane]]);
-    for (int q = 0; q < s; ++q) {
-      v -= sd.fl[lane * s + q] * yl[q];
-      v -= sd.fr[lane * s + q] * yr[q];
-    }
-    tr[S.trow + lane] = double(v);
-  }
-  __syncwarp();
+                                const T* __restrict__ UC, const int32_t* __restrict__ perm, const double* b,
+                                const double* x, double* tr, int lane) {
+  const int s = S.s, l = lane & 15;
+  const TornInt IL = ti[S.intL], IR = ti[S.intR];
+  const TornSides<T> sd = tb_sides<T>(IL, IR, blk);
+  const T y = l < s ? T(x[perm[(lane < 16 ? sd.pl : sd.pr) + l]]) : T(0);
+  const T v = tb_sep_row(sd, IL, IR, UC, y, lane < s ? T(b[perm[S.dof0 + lane]]) : T(0), lane);
+  if (lane < s) tr[S.trow + lane] = double(v);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(32) tb_sep_rhs(int nsep, const TornSep* __restrict__ ts,
                                                  const TornInt* __restrict__ ti, const T* __restrict__ blk,
-                                                 const T* __restrict__ Y, const int32_t* __restrict__ perm,
+                                                 const T* __restrict__ UC, const int32_t* __restrict__ perm,
                                                  const double* __restrict__ b,
                                                  const double* __restrict__ x, double* __restrict__ tr,
                                                  const int* __restrict__ only) {
-  __shared__ T yl[BCR_S], yr[BCR_S];
   const int k = blockIdx.x;
   if (k >= nsep) return;
   const TornSep S = ts[k];
   if (tb_skip(only, S.comp)) return;
-  tb_sep_rhs_warp(S, ti, blk, Y, perm, b, x, tr, yl, yr, threadIdx.x);
+  tb_sep_rhs_warp(S, ti, blk, UC, perm, b, x, tr, threadIdx.x);
 }
 
 // x_a -= Y^L_a x_S_a + Y^R_a x_S_a+1 (interior dofs), x_S = T solution (separator dofs);
@@ -461,22 +487,15 @@ __host__ __device__ constexpr int tb_fused_warp_bytes() {
 }
 
 // separator right-hand side in band order: r_S = b_S - F^R_{left} t_{left}[last s] - F^L_{right} t_{right}[first s]
-// (G and z of an end interior in their place)
 template <typename T>
 __device__ void tb_sep_rhs_band(const TornSep& S, const TornInt* __restrict__ ti, const T* __restrict__ blk,
-                                const T* __restrict__ Y, const double* b, const T* t, double* tr, int lane) {
-  const int s = S.s;
-  if (lane < s) {
-    const TornSides<T> sd = tb_sides<T>(ti[S.intL], ti[S.intR], blk, Y);
-    const T* yl = t + sd.pl;
-    const T* yr = t + sd.pr;
-    T v = T(b[S.dof0 + lane]);
-    for (int q = 0; q < s; ++q) {
-      v -= sd.fl[lane * s + q] * yl[q];
-      v -= sd.fr[lane * s + q] * yr[q];
-    }
-    tr[S.trow + lane] = double(v);
-  }
+                                const T* __restrict__ UC, const double* b, const T* t, double* tr, int lane) {
+  const int s = S.s, l = lane & 15;
+  const TornInt IL = ti[S.intL], IR = ti[S.intR];
+  const TornSides<T> sd = tb_sides<T>(IL, IR, blk);
+  const T y = l < s ? t[(lane < 16 ? sd.pl : sd.pr) + l] : T(0);
+  const T v = tb_sep_row(sd, IL, IR, UC, y, lane < s ? T(b[S.dof0 + lane]) : T(0), lane);
+  if (lane < s) tr[S.trow + lane] = double(v);
 }
 
 // back-substitution in band order: t_a -= Y^L_a x_S_a + Y^R_a x_S_a+1, t_S = x_S.
@@ -576,7 +595,7 @@ __global__ void __launch_bounds__(kTbFusedMaxThreads, 2) tb_fused(TbFusedArgs A,
     }
     __syncthreads();
     if (k1 > k0) {
-      for (int k = k0 + w; k < k1; k += W) tb_sep_rhs_band(A.ts[k], A.ti, F.blk, F.Y, in, t, A.trhs, lane);
+      for (int k = k0 + w; k < k1; k += W) tb_sep_rhs_band(A.ts[k], A.ti, F.blk, F.UC, in, t, A.trhs, lane);
       __syncthreads();
       for (int l = 0; l < nlev; ++l) {
         for (int k = k0 + w; k < k1; k += W) {

@@ -498,7 +498,7 @@ static void analyse(mgpu_ctx* c, Solver& S) {
           I.sepL = a > 0 ? sep0 + a - 1 : -1;
           I.sepR = a < P - 1 ? sep0 + a : -1;
           I.comp = cc;
-          I.end = P > 1 && (a == 0 || a == P - 1);
+          I.end = P > 1 && (a == 0 || (a == 1 && P == 2 && pcap <= 5));
           const bool back = I.end && a > 0;  // numbered backwards, its separator after its last row
           if (back) {
             std::swap(I.sepL, I.sepR);
@@ -1199,7 +1199,7 @@ static void torn_apply(mgpu_ctx* c, bool tr, const double* rhs, double* out, con
     rb_solve<T, 64><<<S.nint, 32, 0, st>>>(cpI, S.tperm, S.TALL, B.uc, B.lm, S.tpiv, rhs, S.bw, S.xw, S.rw, tw, out, 0,
                                            mode, S.iflag, nullptr, ti);
   if (S.nsep == 0) return;
-  tb_sep_rhs<T><<<S.nsep, 32, 0, st>>>(S.nsep, S.d_ts, ti, blk, B.y, S.tperm, rhs, out, S.trhs, cflag);
+  tb_sep_rhs<T><<<S.nsep, 32, 0, st>>>(S.nsep, S.d_ts, ti, blk, B.uc, S.tperm, rhs, out, S.trhs, cflag);
   // separators: block cyclic reduction (trhs reduced in place, txs receives z and then x)
   for (int l = 0; l < S.bcr_levels; ++l) {
     bcr_fwd_elim<T><<<S.nsep, 32, 0, st>>>(S.nsep, S.d_bsep, l, B.fa, S.PV, S.d_brow, S.trhs, S.txs, cflag);

@@ -75,3 +75,15 @@ def test_intermediate_supports_match_whole_components(nel, every, ncomp):
     st = m.initialize()
     times = np.array([0.5, 1.0])
     _same(st, _states(m, st, times, "auto", maxdx=1e-9), _states(m, st, times, "f64", maxdx=1e-9))
+
+
+def test_driven_risers_keep_their_fp32_factors():
+    """Elimination from the driven end too left the FP32 factors short of their
+    refinement within these 20 steps, and the rest of the sweep to FP64 factors."""
+    m, times = W.risers()
+    st = m.initialize(time=0.0)
+    dm = DeviceModel(m, st.dis)
+    rc, _, _ = dm.sweepx(2, times[:20], st.time, [st.X[0]] * 3, fixed_iter=3)
+    info = dm.linear_solver_info()
+    dm.close()
+    assert rc == 0 and info["kind"] == "torn32" and info["last_fallback"] == 0
