@@ -309,7 +309,7 @@ def main():
         dm.close()
         return
     ngroup = len(model.groups)
-    launches_per_step = ngroup + 2 + 1  # element kernels, two scatters, L2 flush
+    launches_per_step = ngroup + 1 + 1  # element kernels (timed group by group), gather-sum, L2 flush
     # roofline of the beam element kernel (FP64-pipe bound)
     tbeam = float(tg[0])
     flops = None
@@ -323,7 +323,7 @@ def main():
         traffic = tr["dram_bytes_per_beam"] * nbeam
     except (OSError, KeyError, ValueError):
         pass
-    roof = {"bound": "fp64", "unit": "TFLOP/s", "kernel": "beam_kernel<false>", "ms_per_launch": tbeam,
+    roof = {"bound": "fp64", "unit": "TFLOP/s", "kernel": "beam_static_kernel<false>", "ms_per_launch": tbeam,
             "peak_source": "measured on this GPU: DFMA throughput of independent FMA chains (mgpu_measure_fp64_peak)", "peak": fp64_peak,
             "traffic": traffic, "traffic_unit": "bytes per launch"}
     if flops:
@@ -683,7 +683,7 @@ def bench_batched(args, rank, local_rank, ws, dist):
     value = len(allp) / dt  # all ranks' models over the slowest rank's time
     h2d = 8 * (model.ndof["X"] + len(times) * dm.ntval + len(times))
     d2h = 8 * model.ndof["X"] * len(times)
-    launches_per_iter = len(model.groups) + 2 + 9  # element kernels, scatters, solver, decrement, convergence
+    launches_per_iter = 1 + 1 + 1 + 8  # beams, small groups, gather-sum, solver, decrement, convergence
     line = {"metric": "models/s (SweepX{0}, 8 load steps per model, per-model convergence)", "value": value,
             "unit": "models/s", "n_gpus": ws, "steps": args.steps, "warmup": args.warmup, "ms_per_step": dt * 1e3,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f64",
