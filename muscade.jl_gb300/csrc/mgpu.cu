@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(256) beam_kernel(int64_t nele, const int32_t* 
 //   mass only   328/168  314/133    309/211   310/318    312/420    564/723
 //   with drag   508/228  498/189    494/303   495/459    497/609    933/1064
 constexpr int64_t kSplitMaxBeams = 9000;
-constexpr int kSplitEntries = 144 + 78 + 12 + 3 * 13;  // columns, symmetric part, direction, its sums
+constexpr int kSplitEntries = 144 + 78 + 12 + 2 * 13;  // columns, symmetric part, direction, two warps' sums of it
 constexpr size_t kSplitSmem = size_t(kSplitEntries) * 32 * sizeof(double);
 
 template <bool STEP>
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(128) beam_split_kernel(int64_t nele, const int
   double* col = sh + lane;                // entry q of this lane's beam at 32 q
   double* sym = col + 32 * 144;           // (i, j), i <= j at i + j (j + 1)/2
   double* dir = sym + 32 * 78;
-  double* dsum = dir + 32 * 12;           // [part − 1][13]
+  double* dsum = dir + 32 * 12;           // [part − 2][13]
   const int64_t e0 = int64_t(blockIdx.x) * 32 + lane;
   const bool live = e0 < nele;
   const int64_t e = live ? e0 : nele - 1;  // the last block's spare lanes repeat a beam and store nothing
@@ -311,20 +311,27 @@ __global__ void __launch_bounds__(128) beam_split_kernel(int64_t nele, const int
   auto put = [&](int i, int j, double v) { col[32 * (i + 12 * j)] = v; };
   auto puts = [&](int i, int j, double v) { sym[32 * (i + j * (j + 1) / 2)] = v; };
   auto nosum = [](BeamDirSums&) { return false; };
-  // the three column warps' sums of the direction; the first goes on with the total
+  // The three column warps' sums of the direction; the first goes on with the total.
+  // They meet at a barrier of their own with a stated count (the last two arrive, the
+  // first waits), whose sites may differ: these are in three different functions, and
+  // __syncthreads() has to be reached by the whole block at one.
   auto sum = [&](BeamDirSums& r) {
     double* p = reinterpret_cast<double*>(&r);
+    if (part != 1) {
 #pragma unroll
-    for (int q = 0; q < 13; ++q) dsum[32 * (13 * (part - 1) + q)] = p[q];
-    __syncthreads();
-    if (part != 1) return false;
+      for (int q = 0; q < 13; ++q) dsum[32 * (13 * (part - 2) + q)] = p[q];
+      __syncwarp();
+      asm volatile("barrier.cta.arrive 1, 96;" ::: "memory");
+      return false;
+    }
+    __syncwarp();
+    asm volatile("barrier.cta.sync 1, 96;" ::: "memory");
 #pragma unroll
-    for (int q = 0; q < 13; ++q) p[q] = (p[q] + dsum[32 * (13 + q)]) + dsum[32 * (26 + q)];
+    for (int q = 0; q < 13; ++q) p[q] = (p[q] + dsum[32 * q]) + dsum[32 * (13 + q)];
     return true;
   };
   if (part == 0) {
     beam_newmark_part<1>(bc, X0, X1, X2, u, pt, av, bv, R, puts, nosum, nullptr, nullptr);
-    if constexpr (STEP) __syncthreads();  // the sums'
   } else if (part == 1) {
     beam_newmark_part<2>(bc, X0, X1, X2, u, pt, av, bv, R, put, sum, STEP ? rd : nullptr, nullptr);
     if constexpr (STEP)
