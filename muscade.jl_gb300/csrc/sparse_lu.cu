@@ -1659,19 +1659,30 @@ __global__ void sp_bwdb_fin(const SpFrontDev* __restrict__ fr, const int32_t* __
 // factors' error E = I − M^-1 A is large in a few soft modes of the structure only;
 // plain refinement carries each at its own rate, |E| a sweep, here each direction
 // takes one of them out.  A and r are scaled, A = D Lλx D; z in elimination order, q
-// and r in model order.  The directions of all sweeps are kept (kSparseSweeps at most).
+// and r in model order.  The directions of all sweeps are kept (kSparseSweeps at most),
+// the residual is that of the solution itself in every sweep (sp_residual).
 //   60 x 60 x 20 lattice: 11 -> 8 sweeps a solve; 12 x 12 x 6: 8 -> 5
 constexpr int kDotBlocks = 304;
 
-// r = D b, w = r in elimination order
-__global__ void sp_start(int64_t n, const int32_t* __restrict__ perm, const double* __restrict__ D,
-                         const double* __restrict__ b, double* __restrict__ r, double* __restrict__ w,
-                         const int* __restrict__ conv) {
+// r = D (b − Lλx x), w = r in elimination order; x: the solution so far, none in the
+// first sweep.  The recursion r − alpha q, a product less, loses the rounding of y, x
+// and the conjugated q: it goes on falling where the residual does not.
+__global__ void __launch_bounds__(kThreads) sp_residual(int64_t n, const int32_t* __restrict__ perm,
+                                                        const int64_t* __restrict__ rptr,
+                                                        const int32_t* __restrict__ rq,
+                                                        const int32_t* __restrict__ rcol,
+                                                        const double* __restrict__ nzval,
+                                                        const double* __restrict__ D, const double* __restrict__ x,
+                                                        const double* __restrict__ b, double* __restrict__ r,
+                                                        double* __restrict__ w, const int* __restrict__ conv) {
   if (*conv) return;
   const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const int32_t d = perm[k];
-  w[k] = r[d] = D[d] * b[d];
+  double s = b[d];
+  if (x)
+    for (int64_t t = rptr[d]; t < rptr[d + 1]; ++t) s = fma(-nzval[rq[t]], x[rcol[t]], s);
+  w[k] = r[d] = D[d] * s;
 }
 
 // |v| as ordered bits (non-negative doubles order like their bit patterns); NaN wins:
@@ -1811,24 +1822,21 @@ __global__ void __launch_bounds__(kThreads) sp_conjugate(int64_t n, int it, cons
   }
 }
 
-// y += alpha z, x = D y, r -= alpha q; w: the new residual in elimination order
+// y += alpha z, x = D y
 __global__ void __launch_bounds__(kThreads) sp_step(int64_t n, int first, const int32_t* __restrict__ perm,
                                                     const double* __restrict__ D, const double* __restrict__ alpha,
-                                                    const double* __restrict__ zv, const double* __restrict__ q,
-                                                    double* __restrict__ yacc, double* __restrict__ x,
-                                                    double* __restrict__ r, double* __restrict__ w,
-                                                    unsigned long long* __restrict__ nrm,
+                                                    const double* __restrict__ zv, double* __restrict__ yacc,
+                                                    double* __restrict__ x, unsigned long long* __restrict__ nrm,
                                                     const int* __restrict__ conv) {
   if (*conv) return;
   const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   double y = 0.0;
   if (k < n) {
-    const double al = *alpha, z = al * zv[k];
+    const double z = *alpha * zv[k];
     y = first ? z : yacc[k] + z;
     yacc[k] = y;
     const int32_t d = perm[k];
     x[d] = D[d] * y;
-    w[k] = r[d] = fma(-al, q[d], r[d]);
   }
   max_bits(nrm + 1, y);
 }
@@ -2000,10 +2008,9 @@ cudaError_t refine(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, int 
       const cudaError_t e = cudaMemsetAsync(sp.chain, 0, (2 * size_t(sp.nheight) + 1) * sizeof(int), st);
       if (e != cudaSuccess) return e;
     }
-    if (it == 0) {
-      sp_start<<<nblocks(n, kThreads), kThreads, 0, st>>>(n, sp.d_perm, sp.D, b, sp.r, sp.w, sp.flags);
-      ++c->launches;
-    }
+    sp_residual<<<nblocks(n, kThreads), kThreads, 0, st>>>(n, sp.d_perm, sp.d_rptr, sp.d_rq, sp.d_rcol, c->nzval, sp.D,
+                                                           it > 0 ? sp.xs : nullptr, b, sp.r, sp.w, sp.flags);
+    ++c->launches;
     for (int h = 0; h < sp.nheight; ++h) {
       if (!sp.h_nlf[h]) continue;
       const int32_t* fl = sp.d_lf + sp.h_lf0[h];
@@ -2112,8 +2119,8 @@ cudaError_t refine(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, int 
                                       sp.done, sp.coef, sp.coef + kSparseSweeps, sp.flags);
     sp_conjugate<<<gd, kThreads, 0, st>>>(n, it, sp.dirq, sp.dirz, q, z, sp.r, sp.coef + kSparseSweeps, sp.part,
                                           sp.done, sp.coef + it, sp.coef + 2 * kSparseSweeps, sp.flags);
-    sp_step<<<nblocks(n, kThreads), kThreads, 0, st>>>(n, it == 0, sp.d_perm, sp.D, sp.coef + 2 * kSparseSweeps, z, q,
-                                                       sp.yacc, sp.xs, sp.r, sp.w, sp.nrm, sp.flags);
+    sp_step<<<nblocks(n, kThreads), kThreads, 0, st>>>(n, it == 0, sp.d_perm, sp.D, sp.coef + 2 * kSparseSweeps, z,
+                                                       sp.yacc, sp.xs, sp.nrm, sp.flags);
     c->launches += 4;
     sp_check<<<1, 1, 0, st>>>(sp.nrm, sp.prev, sp.flags, kRefineTol, kRefineStall);
     ++c->launches;

@@ -1,0 +1,45 @@
+"""What the multifrontal solver says about its solutions (csrc/sparse_lu.cu): a solve
+counts as converged only where the residual b − Lλx x of the solution itself does."""
+import numpy as np
+import pytest
+
+from muscade_gpu import workloads as W
+from muscade_gpu.device import DeviceModel
+from muscade_gpu.model import Model
+
+pytestmark = pytest.mark.gpu
+
+
+def tower(nx, ny, nz, decades, seed=0):
+    """A space frame whose members' stiffnesses are spread over some decades, the nodes
+    up to 1 % out of place, held at its base and pushed at the top."""
+    rng = np.random.default_rng(seed)
+    m = Model("tower")
+    ix, iy, iz = [a.ravel() for a in np.meshgrid(range(nx + 1), range(ny + 1), range(nz + 1), indexing="ij")]
+    at = {p: k for k, p in enumerate(zip(ix, iy, iz))}
+    nodes = m.addnode(np.stack([4.0 * ix, 4.0 * iy, 3.0 * iz], axis=1) + 0.01 * rng.normal(size=(len(ix), 3)))
+    for step, orient in (((1, 0, 0), (0.0, 1.0, 0.0)), ((0, 1, 0), (0.0, 0.0, 1.0)), ((0, 0, 1), (1.0, 0.0, 0.0))):
+        pairs = [(k, at[q]) for p, k in at.items()
+                 if (q := tuple(np.add(p, step))) in at and (step == (0, 0, 1) or p[2] > 0)]
+        f = 10.0 ** (decades * (rng.random(len(pairs)) - 0.5))
+        mat = W.BeamCrossSection(EA=4.2e9 * f, EI2=1e8 * f, EI3=1e8 * f, GJ=8e7 * f, mu=100.0, iota1=1.0)
+        m.addelement(W.EulerBeam3D, nodes[np.asarray(pairs)], mat=mat, orient2=orient)
+    for f in ("t1", "t2", "t3", "r1", "r2", "r3"):
+        m.addelement(W.Hold, nodes[iz == 0][:, None], field=f)
+    m.addelement(W.DofLoad, nodes[iz == nz][:, None], field="t1", value=lambda t: 1e5 * t)
+    m.addelement(W.DofLoad, nodes[iz == nz][:, None], field="t2", value=lambda t: 2e4 * t)
+    return m
+
+
+def test_factors_that_cannot_converge_give_way_to_fp64():
+    """Forty storeys with stiffnesses over six decades: the corrections of the residuals
+    formed from the solution level off at 5e-10 of it or more, above the 1e-10 at which a
+    solve may stop short, whatever a recursion for the residual says (it went to 1e-14
+    in nine sweeps)."""
+    m = tower(3, 3, 40, 6.0)
+    st = m.initialize()
+    dm = DeviceModel(m, st.dis, linsolve="sparse")
+    rc, _, _ = dm.sweepx(0, np.array([1.0]), st.time, list(st.X), fixed_iter=1)
+    info = dm.sparse_info()
+    dm.close()
+    assert rc == 0 and info["last_fallback"] == 1
