@@ -1,6 +1,7 @@
 // Device sparse direct solver: multifrontal LU over nested-dissection fronts
 // (see sparse_lu.hpp and sparse_analysis.hpp).
 #include "sparse_lu.hpp"
+#include "sparse_stop.hpp"
 
 #include <algorithm>
 #include <chrono>
@@ -40,8 +41,6 @@ __device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) {
 }
 
 constexpr size_t kUpd32Smem = size_t(2) * 64 * (128 + 4) * sizeof(float);  // sp_update_f32<64> tiles
-constexpr double kRefineTol = 1e-14;   // scaled correction / scaled solution: converged
-constexpr double kRefineStall = 1e-10;  // ... or stalled below this
 
 // f(0), f(1), .., f(N − 1) with constant arguments
 template <class F, int... K>
@@ -1661,29 +1660,8 @@ __global__ void sp_bwdb_fin(const SpFrontDev* __restrict__ fr, const int32_t* __
 // takes one of them out.  A and r are scaled, A = D Lλx D; z in elimination order, q
 // and r in model order.  The directions of all sweeps are kept (kSparseSweeps at most),
 // the residual is that of the solution itself in every sweep (sp_residual).
-//   60 x 60 x 20 lattice: 11 -> 8 sweeps a solve; 12 x 12 x 6: 8 -> 5
+//   60 x 60 x 20 lattice: 11 -> 9 sweeps a solve; 12 x 12 x 6: 8 -> 5
 constexpr int kDotBlocks = 304;
-
-// r = D (b − Lλx x), w = r in elimination order; x: the solution so far, none in the
-// first sweep.  The recursion r − alpha q, a product less, loses the rounding of y, x
-// and the conjugated q: it goes on falling where the residual does not.
-__global__ void __launch_bounds__(kThreads) sp_residual(int64_t n, const int32_t* __restrict__ perm,
-                                                        const int64_t* __restrict__ rptr,
-                                                        const int32_t* __restrict__ rq,
-                                                        const int32_t* __restrict__ rcol,
-                                                        const double* __restrict__ nzval,
-                                                        const double* __restrict__ D, const double* __restrict__ x,
-                                                        const double* __restrict__ b, double* __restrict__ r,
-                                                        double* __restrict__ w, const int* __restrict__ conv) {
-  if (*conv) return;
-  const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  const int32_t d = perm[k];
-  double s = b[d];
-  if (x)
-    for (int64_t t = rptr[d]; t < rptr[d + 1]; ++t) s = fma(-nzval[rq[t]], x[rcol[t]], s);
-  w[k] = r[d] = D[d] * s;
-}
 
 // |v| as ordered bits (non-negative doubles order like their bit patterns); NaN wins:
 // the block's largest to dst
@@ -1691,12 +1669,48 @@ __device__ __forceinline__ void max_bits(unsigned long long* dst, double v) {
   __shared__ double smax[kThreads / 32];
   v = isnan(v) ? INFINITY : fabs(v);
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  __syncthreads();  // a kernel may take two
   if ((threadIdx.x & 31) == 0) smax[threadIdx.x >> 5] = v;
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int q = 1; q < kThreads / 32; ++q) v = fmax(v, smax[q]);
     atomicMax(dst, (unsigned long long)__double_as_longlong(v));
   }
+}
+
+// r = D (b − Lλx x), w = r in elimination order; x: the solution so far, none in the
+// first sweep.  The recursion r − alpha q, a product less, loses the rounding of y, x
+// and the conjugated q: it goes on falling where the residual does not.  nrm[2], nrm[3]:
+// the largest |r| and the largest of its rows' |A||y| + |D b|, whose rounding bounds what
+// of r can be told from zero.
+__global__ void __launch_bounds__(kThreads) sp_residual(int64_t n, const int32_t* __restrict__ perm,
+                                                        const int64_t* __restrict__ rptr,
+                                                        const int32_t* __restrict__ rq,
+                                                        const int32_t* __restrict__ rcol,
+                                                        const double* __restrict__ nzval,
+                                                        const double* __restrict__ D, const double* __restrict__ x,
+                                                        const double* __restrict__ b, double* __restrict__ r,
+                                                        double* __restrict__ w, unsigned long long* __restrict__ nrm,
+                                                        const int* __restrict__ conv) {
+  if (*conv) return;
+  const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  double s = 0.0, a = 0.0;
+  if (k < n) {
+    const int32_t d = perm[k];
+    s = b[d];
+    a = fabs(s);
+    if (x)
+      for (int64_t t = rptr[d]; t < rptr[d + 1]; ++t) {
+        const double v = nzval[rq[t]], u = x[rcol[t]];
+        s = fma(-v, u, s);
+        a = fma(fabs(v), fabs(u), a);
+      }
+    s *= D[d];
+    a *= D[d];
+    w[k] = r[d] = s;
+  }
+  max_bits(nrm + 2, s);
+  max_bits(nrm + 3, a);
 }
 
 // z = w, and D z in model order; the largest |w| of the sweep, the error that the
@@ -1841,22 +1855,15 @@ __global__ void __launch_bounds__(kThreads) sp_step(int64_t n, int first, const 
   max_bits(nrm + 1, y);
 }
 
-// Converged when the scaled correction M^-1 r is below tol of the scaled solution, or
-// the next one would be, by a factor of ten, at the rate of the last two (the rate only
-// improves from sweep to sweep), or when it has stopped shrinking (no better than half
-// the previous one) while below stall of the solution: the attainable accuracy of the
-// FP64 residual is then reached.  prev holds the previous correction's norm.
-__global__ void sp_check(unsigned long long* nrm, double* prev, int* flags, double tol, double stall) {
+// flags[0] when the sweep was the last that is needed (sp_stop)
+__global__ void sp_check(unsigned long long* nrm, double* last, int nrow, int* flags) {
   if (flags[0]) return;
-  const double nw = __longlong_as_double((long long)nrm[0]), ny = __longlong_as_double((long long)nrm[1]);
-  flags[1] += 1;
-  const bool again = flags[1] > 1;
-  if (nw <= tol * ny || (again && nw < *prev && nw * (nw / *prev) <= 0.1 * tol * ny) ||
-      (again && nw >= 0.5 * *prev && nw <= stall * ny))
-    flags[0] = 1;
-  *prev = nw;
-  nrm[0] = 0ull;
-  nrm[1] = 0ull;
+  double v[4];
+  for (int q = 0; q < 4; ++q) {
+    v[q] = __longlong_as_double((long long)nrm[q]);
+    nrm[q] = 0ull;
+  }
+  if (sp_stop(++flags[1], v[0], v[1], v[2], v[3], nrow, last) == SP_CONVERGED) flags[0] = 1;
 }
 
 template <class T>
@@ -2009,7 +2016,7 @@ cudaError_t refine(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, int 
       if (e != cudaSuccess) return e;
     }
     sp_residual<<<nblocks(n, kThreads), kThreads, 0, st>>>(n, sp.d_perm, sp.d_rptr, sp.d_rq, sp.d_rcol, c->nzval, sp.D,
-                                                           it > 0 ? sp.xs : nullptr, b, sp.r, sp.w, sp.flags);
+                                                           it > 0 ? sp.xs : nullptr, b, sp.r, sp.w, sp.nrm, sp.flags);
     ++c->launches;
     for (int h = 0; h < sp.nheight; ++h) {
       if (!sp.h_nlf[h]) continue;
@@ -2122,7 +2129,7 @@ cudaError_t refine(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, int 
     sp_step<<<nblocks(n, kThreads), kThreads, 0, st>>>(n, it == 0, sp.d_perm, sp.D, sp.coef + 2 * kSparseSweeps, z,
                                                        sp.yacc, sp.xs, sp.nrm, sp.flags);
     c->launches += 4;
-    sp_check<<<1, 1, 0, st>>>(sp.nrm, sp.prev, sp.flags, kRefineTol, kRefineStall);
+    sp_check<<<1, 1, 0, st>>>(sp.nrm, sp.last, sp.nrow, sp.flags);
     ++c->launches;
   }
   return cudaGetLastError();
@@ -2304,6 +2311,7 @@ int sparse_create(mgpu_ctx* c, SparseDev*& spp, const double* dof_xyz, const uin
   }
   std::vector<int64_t> rptr(A.n + 1, 0);
   for (int64_t q = 0; q < A.nnz; ++q) rptr[P.rowval[q] + 1]++;
+  for (int64_t i = 0; i < A.n; ++i) sp.nrow = std::max(sp.nrow, int(rptr[i + 1]));
   for (int64_t i = 0; i < A.n; ++i) rptr[i + 1] += rptr[i];
   std::vector<int32_t> rq(A.nnz), rcol(A.nnz);
   {
@@ -2354,8 +2362,8 @@ int sparse_create(mgpu_ctx* c, SparseDev*& spp, const double* dof_xyz, const uin
   ok(cudaMalloc(&sp.part, size_t(kDotBlocks) * kSparseSweeps * sizeof(double)));
   ok(cudaMalloc(&sp.coef, (2 * kSparseSweeps + 2) * sizeof(double)));  // q·q, beta, alpha, done
   ok(cudaMalloc(&sp.xs, n * sizeof(double)));
-  ok(cudaMalloc(&sp.nrm, 2 * sizeof(unsigned long long)));
-  ok(cudaMalloc(&sp.prev, sizeof(double)));
+  ok(cudaMalloc(&sp.nrm, 4 * sizeof(unsigned long long)));
+  ok(cudaMalloc(&sp.last, 2 * sizeof(double)));
   ok(cudaMalloc(&sp.flags, 4 * sizeof(int)));
   ok(cudaMallocHost(&sp.hflags, 4 * sizeof(int)));
   sp.ntflag = int64_t(A.fidx.size()) / 64 + 2 * int64_t(sp.nfront) + 64;
@@ -2374,7 +2382,7 @@ int sparse_create(mgpu_ctx* c, SparseDev*& spp, const double* dof_xyz, const uin
     sp.chain_grid64 = std::max(1, nsm * std::max(1, std::min(f64, b64)));
   }
   if (const char* ev = getenv("MGPU_SPARSE_CHAINED")) sp.chained = atoi(ev) != 0;
-  ok(cudaMemset(sp.nrm, 0, 2 * sizeof(unsigned long long)));
+  ok(cudaMemset(sp.nrm, 0, 4 * sizeof(unsigned long long)));
   ok(cudaMemsetAsync(sp.coef, 0, (2 * kSparseSweeps + 2) * sizeof(double), c->stream));
   sp.done = reinterpret_cast<unsigned*>(sp.coef + 2 * kSparseSweeps + 1);
   for (cudaEvent_t& ev : sp.ev) ok(cudaEventCreate(&ev));
@@ -2423,7 +2431,7 @@ void sparse_destroy(SparseDev*& sp) {
   if (!sp) return;
   void* ps[] = {sp->d_fr, sp->d_lf, sp->d_ea, sp->d_clist, sp->d_fidx, sp->d_emap, sp->d_amap, sp->d_aq,
                 sp->d_acol, sp->d_perm, sp->d_diag, sp->d_colptr, sp->d_rowval, sp->d_rptr, sp->d_rq, sp->d_rcol,
-                sp->F32, sp->F64, sp->prev,
+                sp->F32, sp->F64, sp->last,
                 sp->D, sp->cvec, sp->w, sp->V, sp->P, sp->d_poff, sp->tw, sp->yacc, sp->r,
                 sp->dirz, sp->dirq, sp->pack, sp->dz, sp->part, sp->coef, sp->xs, sp->nrm,
                 sp->flags, sp->tflag, sp->chain};

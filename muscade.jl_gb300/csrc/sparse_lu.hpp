@@ -14,12 +14,11 @@
 //     of NB columns: one kernel factors the diagonal block and solves the
 //     block's L and U panels, one updates the trailing block;
 //   * FP32 factors inside FP64 sweeps of the conjugate residual method (residuals
-//     of the FP64 Lλx), until the scaled correction, or the next one at the rate
-//     of the last two and ten times over, is below 1e-14 of the scaled solution
-//     or stops shrinking below 1e-10 of it (the FP64 residual's attainable
-//     accuracy), at most kSparseSweeps sweeps; when that fails the same
-//     kernels factorise in FP64 (MGPU_LINSOLVE_SPARSE), or FP64 throughout
-//     (_SPARSE64).
+//     of the FP64 Lλx and the solution so far), until the scaled correction is
+//     below 1e-14 of the scaled solution, or as good as that, or at the accuracy
+//     that FP64 attains (sparse_stop.hpp), at most kSparseSweeps sweeps; when that
+//     fails the same kernels factorise in FP64 (MGPU_LINSOLVE_SPARSE), or FP64
+//     throughout (_SPARSE64).
 // Every sum runs in a fixed order: results are bitwise repeatable.
 #pragma once
 #include <cuda_runtime.h>
@@ -94,8 +93,9 @@ struct SparseDev {
   unsigned* done = nullptr;                 // blocks that have added theirs
   double* r = nullptr;          // [n] residual (model order)
   double* xs = nullptr;         // [n] current solution (model order)
-  unsigned long long* nrm = nullptr;  // [2] max |correction|, max |solution| (as ordered bits)
-  double* prev = nullptr;       // the previous sweep's max |correction|
+  unsigned long long* nrm = nullptr;  // [4] max |correction|, |solution|, |residual|, |A||y| + |D b| (as ordered bits)
+  double* last = nullptr;       // [2] the previous sweep's max |correction|, the worst rate so far
+  int nrow = 0;                 // most entries in a row
   int* flags = nullptr;         // [0] converged, [1] sweeps done, [2] perturbed pivots, [3] non-finite pivot
                                 // (bit 1: a chained substitution's wait ran out, bit 2: a tensor-core tile's)
   unsigned* tflag = nullptr;    // [ntflag] per blocked front and pivot tile: epoch of the launch that solved it
