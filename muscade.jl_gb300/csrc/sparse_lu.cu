@@ -1855,7 +1855,8 @@ __global__ void __launch_bounds__(kThreads) sp_step(int64_t n, int first, const 
   max_bits(nrm + 1, y);
 }
 
-// flags[0] when the sweep was the last that is needed (sp_stop)
+// flags[0] when the sweep was the last that is needed (sp_stop); flags[3] bit 3 where a
+// norm is not finite
 __global__ void sp_check(unsigned long long* nrm, double* last, int nrow, int* flags) {
   if (flags[0]) return;
   double v[4];
@@ -1863,7 +1864,9 @@ __global__ void sp_check(unsigned long long* nrm, double* last, int nrow, int* f
     v[q] = __longlong_as_double((long long)nrm[q]);
     nrm[q] = 0ull;
   }
-  if (sp_stop(++flags[1], v[0], v[1], v[2], v[3], nrow, last) == SP_CONVERGED) flags[0] = 1;
+  const SpStop s = sp_stop(++flags[1], v[0], v[1], v[2], v[3], nrow, last);
+  if (s == SP_CONVERGED) flags[0] = 1;
+  if (s == SP_NOT_FINITE) flags[3] |= 8;
 }
 
 template <class T>
@@ -2501,7 +2504,7 @@ int sparse_factor_solve(mgpu_ctx* c, SparseDev& sp, const double* rhs, double* o
     sp.last_sweeps = sp.hflags[1];
     sp.last_perturbed = sp.hflags[2];
     if (sp.hflags[3] & 6) return set_err(c, MGPU_ERR_CUDA, "sparse solve: a bounded wait on the device ran out");
-    if (sp.hflags[3] != 0) {  // a zero or non-finite pivot in FP64: the matrix is singular
+    if (sp.hflags[3] & 1) {  // a zero or non-finite pivot in FP64: the matrix is singular
       const int one = 1;
       MG_CUDA(cudaMemcpy(info, &one, sizeof(int), cudaMemcpyHostToDevice));
     }

@@ -17,8 +17,8 @@
 //     of the FP64 Lλx and the solution so far), until the scaled correction is
 //     below 1e-14 of the scaled solution, or as good as that, or at the accuracy
 //     that FP64 attains (sparse_stop.hpp), at most kSparseSweeps sweeps; when that
-//     fails the same kernels factorise in FP64 (MGPU_LINSOLVE_SPARSE), or FP64
-//     throughout (_SPARSE64).
+//     fails, or a norm is not finite, the same kernels factorise in FP64
+//     (MGPU_LINSOLVE_SPARSE), or FP64 throughout (_SPARSE64).
 // Every sum runs in a fixed order: results are bitwise repeatable.
 #pragma once
 #include <cuda_runtime.h>
@@ -97,7 +97,8 @@ struct SparseDev {
   double* last = nullptr;       // [2] the previous sweep's max |correction|, the worst rate so far
   int nrow = 0;                 // most entries in a row
   int* flags = nullptr;         // [0] converged, [1] sweeps done, [2] perturbed pivots, [3] non-finite pivot
-                                // (bit 1: a chained substitution's wait ran out, bit 2: a tensor-core tile's)
+                                // (bit 1: a chained substitution's wait ran out, bit 2: a tensor-core tile's,
+                                // bit 3: a norm of the sweeps is not finite)
   unsigned* tflag = nullptr;    // [ntflag] per blocked front and pivot tile: epoch of the launch that solved it
   int64_t ntflag = 0;
   int* chain = nullptr;         // [2·nheight + 1] work counters of the chained substitutions, abort word

@@ -19,7 +19,7 @@ constexpr double kRefineTol = 1e-14;    // correction / solution: converged
 constexpr double kRefineNear = 1e-11;   // ... or below this with the next one 0.1 kRefineTol
 constexpr double kRefineStall = 1e-10;  // ... or no longer shrinking below this
 
-enum SpStop : int { SP_GO_ON = 0, SP_CONVERGED = 1 };
+enum SpStop : int { SP_GO_ON = 0, SP_CONVERGED = 1, SP_NOT_FINITE = 2 };
 
 // The largest entries of a sweep's correction (c) and of the solution with it (y), the
 // largest residual that the correction came from (r) and the largest of its rows'
@@ -37,6 +37,7 @@ enum SpStop : int { SP_GO_ON = 0, SP_CONVERGED = 1 };
 // is conditioned well: 12 x 12 x 6 lattice 5 -> 6 sweeps a solve, 44.7 -> 52.8 ms for its
 // three load steps; 60 x 60 x 20 ends by the third after 9 either way.
 SP_HD SpStop sp_stop(int sweep, double c, double y, double r, double a, int nrow, double last[2]) {
+  if (!(c <= 1.7e308) || !(y <= 1.7e308)) return SP_NOT_FINITE;
   const bool again = sweep > 1;
   const double prev = last[0], rate = again ? fmax(last[1], c / prev) : 0.0;
   last[0] = c;

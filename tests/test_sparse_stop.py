@@ -54,3 +54,9 @@ def test_a_plateau_counts_only_where_the_residual_is_rounding(stop):
     assert stop(c, r=45 * U) == 0
     assert stop([1.0, 1e-6, 2e-10, 1.9e-10], r=0.0) == 0  # too far off to stop at all
 
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_what_is_not_finite_never_converges(stop, bad):
+    assert stop([bad], y=[bad]) == -1
+    assert stop([1.0, bad], y=[1.0, bad]) == -2
+    assert stop([1.0, 1e-5], y=[1.0, bad]) == -2
