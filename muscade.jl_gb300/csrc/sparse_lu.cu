@@ -2158,11 +2158,16 @@ cudaError_t refine_batches(mgpu_ctx* c, SparseDev& sp, const T* F, const double*
   return cudaSuccess;
 }
 
+// Room for a front's vector in the one-block substitutions: the limit of what they take,
+// whatever the model needs.  It is a setting of the process's kernels, not of a model's,
+// so a smaller model's must not lower it; and the 48 KB that need no setting hold the
+// kernels' static shared memory too (up to 13 KB).
+constexpr int kSubstSmem = 200 * 1024;
 template <class T>
-cudaError_t set_smem(int bytes) {
+cudaError_t set_smem() {
   for (const void* k : {reinterpret_cast<const void*>(sp_fwd_tri<T>), reinterpret_cast<const void*>(sp_bwd_tri<T>),
                         reinterpret_cast<const void*>(sp_fwd_gemv<T>), reinterpret_cast<const void*>(sp_bwd_gemv<T>)}) {
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSubstSmem);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -2191,7 +2196,7 @@ int sparse_create(mgpu_ctx* c, SparseDev*& spp, const double* dof_xyz, const uin
   if (const char* ev = getenv("MGPU_SPARSE_BLOCKED_PIVOTS")) sp.big_pivots = std::max(1, atoi(ev));
   for (const SparseFront& S : A.fronts)
     if (S.p < sp.big_pivots) sp.max_m_small = std::max(sp.max_m_small, int(S.m));
-  if (int64_t(sp.max_m_small) * 8 > 200 * 1024) {
+  if (int64_t(sp.max_m_small) * 8 > kSubstSmem) {
     sp.why = "front of " + std::to_string(sp.max_m_small) + " dofs exceeds the substitution kernels' shared memory";
     return MGPU_OK;
   }
@@ -2389,11 +2394,8 @@ int sparse_create(mgpu_ctx* c, SparseDev*& spp, const double* dof_xyz, const uin
   ok(cudaMemsetAsync(sp.coef, 0, (2 * kSparseSweeps + 2) * sizeof(double), c->stream));
   sp.done = reinterpret_cast<unsigned*>(sp.coef + 2 * kSparseSweeps + 1);
   for (cudaEvent_t& ev : sp.ev) ok(cudaEventCreate(&ev));
-  const int smem = int(sp.max_m_small * sizeof(double));
-  if (smem > 48 * 1024) {
-    ok(set_smem<float>(smem));
-    ok(set_smem<double>(smem));
-  }
+  ok(set_smem<float>());
+  ok(set_smem<double>());
   ok(cudaFuncSetAttribute(sp_update_f32<kNB32>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kUpd32Smem)));
   ok(cudaFuncSetAttribute(sp_update_tc<kNB32>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tc::kTcSmem)));
   ok(cudaFuncSetAttribute(sp_rect_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kUpd32Smem)));

@@ -1,5 +1,6 @@
-"""What the multifrontal solver says about its solutions (csrc/sparse_lu.cu): a solve
-counts as converged only where the residual b − Lλx x of the solution itself does."""
+"""The multifrontal solver (csrc/sparse_lu.cu) where it was wrong or refused: a solve counts
+as converged only where the residual b − Lλx x of the solution itself does, and fronts of
+every size have their substitutions."""
 import numpy as np
 import pytest
 
@@ -43,3 +44,24 @@ def test_factors_that_cannot_converge_give_way_to_fp64():
     info = dm.sparse_info()
     dm.close()
     assert rc == 0 and info["last_fallback"] == 1
+
+
+def test_one_block_substitutions_of_a_front_near_48_kb(monkeypatch):
+    """Fronts whose vector fits the 48 KB of shared memory that need no opt-in, but not
+    beside the substitution kernels' own tables, against the blocked substitutions."""
+    m, times = W.lattice(23, 23, 23)
+    st = m.initialize()
+    out = {}
+    for threshold in ("128", "100000"):
+        monkeypatch.setenv("MGPU_SPARSE_BLOCKED_PIVOTS", threshold)
+        dm = DeviceModel(m, st.dis, linsolve="sparse")
+        rc, X, _ = dm.sweepx(0, times[:1], st.time, list(st.X), fixed_iter=1)
+        info = dm.sparse_info()
+        dm.close()
+        assert rc == 0 and info["last_fallback"] == 0
+        assert 36 * 1024 < 8 * info["max_front"] <= 48 * 1024
+        out[threshold] = X
+    a, b = out.values()
+    lam = np.array([str(f).startswith("λ") for f in st.dis.fieldX])
+    for sel in (lam, ~lam):
+        assert np.max(np.abs(a[0, 0][sel] - b[0, 0][sel])) <= 1e-9 * np.max(np.abs(b[0, 0][sel]))
