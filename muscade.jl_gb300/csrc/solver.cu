@@ -584,12 +584,13 @@ static void analyse(mgpu_ctx* c, Solver& S) {
         if (allow && S.maxP <= kFusedMaxP) {
           S.fuseW32 = std::max(1, std::min({S.maxP, budget / b32, kFusedMaxW}));
           S.fuseW64 = std::max(1, std::min({S.maxP, budget / b64, kFusedMaxW}));
+          // a setting of the process's kernels: the same for every model
           if (S.twmI == 32) {
-            cudaFuncSetAttribute(tb_fused<float, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, S.fuseW32 * b32);
-            cudaFuncSetAttribute(tb_fused<double, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, S.fuseW64 * b64);
+            cudaFuncSetAttribute(tb_fused<float, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, budget);
+            cudaFuncSetAttribute(tb_fused<double, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, budget);
           } else {
-            cudaFuncSetAttribute(tb_fused<float, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, S.fuseW32 * b32);
-            cudaFuncSetAttribute(tb_fused<double, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, S.fuseW64 * b64);
+            cudaFuncSetAttribute(tb_fused<float, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, budget);
+            cudaFuncSetAttribute(tb_fused<double, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, budget);
           }
         }
       }

@@ -87,3 +87,21 @@ def test_driven_risers_keep_their_fp32_factors():
     info = dm.linear_solver_info()
     dm.close()
     assert rc == 0 and info["kind"] == "torn32" and info["last_fallback"] == 0
+
+
+def test_a_second_model_leaves_the_first_ones_solver_alone():
+    """Models in one process: the shared memory of the fused solve is a setting of its
+    kernels, and a later model of fewer interiors must not lower it for an earlier one."""
+    m, times = W.risers(nriser=3, nel=200)
+    st = m.initialize(time=0.0)
+    few, ftimes = W.cantilever(nel=85, length=42.5)
+    fst = few.initialize()
+    kw = dict(fixed_iter=3)
+    alone = _states(m, st, times[:2], "torn32", OX=2, **kw)
+    first = DeviceModel(m, st.dis, linsolve="torn32")
+    second = DeviceModel(few, fst.dis, linsolve="torn32")
+    rc, X, _ = first.sweepx(2, times[:2], st.time, [st.X[0]] * 3, **kw)
+    rc2, _, _ = second.sweepx(0, ftimes[:1], fst.time, [fst.X[0]], **kw)
+    first.close()
+    second.close()
+    assert rc == 0 and rc2 == 0 and np.array_equal(X, alone)
