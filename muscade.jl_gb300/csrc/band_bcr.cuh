@@ -50,7 +50,7 @@ __device__ __forceinline__ int bcr_role(int kloc, int N, int l) {
 }
 
 // 1/pivot in the factors' type
-__device__ __forceinline__ double bcr_rcp(double p) { return rb_rcp(p); }
+__device__ __forceinline__ double bcr_rcp(double p) { return __drcp_rn(p); }
 __device__ __forceinline__ float bcr_rcp(float p) { return __frcp_rn(p); }
 
 // The dense work of one block, one warp, a matrix row per lane in registers:

@@ -11,9 +11,9 @@
 // stands on either side.  Multipliers, interchanges and updates are those of
 // LAPACK gbtf2, each entry updated in the order of the pivots, so the factors are
 // bitwise those of the row-band kernels (band_rows.cuh).  Measured on that frame:
-// 2.4 ms a factorisation, of which two thirds are the panels' pivot steps (2,300
-// cycles each: two block barriers, the reciprocal, up to 15 multiply-adds for a
-// warp's rows); 64 ms with one block working on the band in global memory.
+// 1.93 ms a factorisation, most of it the panels' pivot steps (two block barriers,
+// the reciprocal, up to 15 multiply-adds for a warp's rows each); 64 ms with one
+// block working on the band in global memory.
 //
 // Storage: LAPACK's, A(i, j) at base[kv + i − j + ld j], ld = 2kl + ku + 1.
 #pragma once
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(kBlkThreads) band_lu(const int64_t* cbase, con
         const unsigned fl = __reduce_max_sync(RB_FULL, h2 == fh ? l2 : 0u);
         const int pr = int(__reduce_min_sync(RB_FULL, h2 == fh && l2 == fl ? i2 : 0xffffffffu));
         if (tid == pr) {
-          const double p = a[c], rp = p != 0.0 ? rb_rcp(p) : 0.0;
+          const double p = a[c], rp = p != 0.0 ? __drcp_rn(p) : 0.0;
           s_rp[par] = rp;
 #pragma unroll
           for (int j = c + 1; j < kBlkNB; ++j) prow[par][j] = a[j];

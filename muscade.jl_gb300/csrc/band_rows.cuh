@@ -80,20 +80,6 @@ __device__ __forceinline__ void rb_cp_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
-// 1/p for a pivot: the hardware's reciprocal approximation (PTX rcp.approx.ftz.f64,
-// 20 bits) and two Newton steps r += r(1 − p r), to rounding.  Four FP64
-// instructions on the chain from one column to the next, against about ten of a
-// correctly rounded division (a warp's FP64 instruction holds its sub-partition for
-// 64 cycles).  Pivots near the ends of the exponent range take the division.
-__device__ __forceinline__ double rb_rcp(double p) {
-  const unsigned e = (unsigned(__double2hiint(p)) >> 20) & 0x7ffu;
-  if (e - 24u > 1998u) return 1.0 / p;
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(p));
-  r = fma(r, fma(-p, r, 1.0), r);
-  return fma(r, fma(-p, r, 1.0), r);
-}
-
 // What a launch does with the per-component flag array:
 enum RbMode : int {
   RB_PRIMARY = 0,   // all components; a zero pivot or a failed refinement sets flag[c]
@@ -178,10 +164,10 @@ __global__ void __launch_bounds__(32) rb_lu(RbComp cp, const T* __restrict__ Aro
       pos = jp;
     const bool zero = (pv == T(0));
     singular = singular || zero;
-    T rp = T(0);
+    T rp = T(0);  // correctly rounded 1/pv (the value of T(1)/pv, without the general division)
     if (!zero) {
       if constexpr (sizeof(T) == 8)
-        rp = rb_rcp(pv);
+        rp = __drcp_rn(pv);
       else
         rp = __frcp_rn(pv);
     }
@@ -282,10 +268,10 @@ __global__ void __launch_bounds__(32) rb_lu_half(RbComp cp, const T* __restrict_
       pos = jp;
     const bool zero = (pv == T(0));
     singular = singular || zero;
-    T rp = T(0);
+    T rp = T(0);  // correctly rounded 1/pv (the value of T(1)/pv, without the general division)
     if (!zero) {
       if constexpr (sizeof(T) == 8)
-        rp = rb_rcp(pv);
+        rp = __drcp_rn(pv);
       else
         rp = __frcp_rn(pv);
     }
