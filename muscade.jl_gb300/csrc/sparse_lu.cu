@@ -1658,8 +1658,9 @@ __global__ void sp_bwdb_fin(const SpFrontDev* __restrict__ fr, const int32_t* __
 // factors' error E = I − M^-1 A is large in a few soft modes of the structure only;
 // plain refinement carries each at its own rate, |E| a sweep, here each direction
 // takes one of them out.  A and r are scaled, A = D Lλx D; z in elimination order, q
-// and r in model order.  The directions of all sweeps are kept (kSparseSweeps at most),
-// the residual is that of the solution itself in every sweep (sp_residual).
+// and r in model order.  The directions of all sweeps are kept (kSparseSweeps at most;
+// where there is no room for them fewer, and the conjugation starts again when these are
+// full), the residual is that of the solution itself in every sweep (sp_residual).
 //   60 x 60 x 20 lattice: 11 -> 9 sweeps a solve; 12 x 12 x 6: 8 -> 5
 constexpr int kDotBlocks = 304;
 
@@ -2121,14 +2122,15 @@ cudaError_t refine(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, int 
         }
       }
     }
-    double *z = sp.dirz + it * n, *q = sp.dirq + it * n;
+    const int kept = it % sp.ndir;  // earlier directions that this one is made conjugate to
+    double *z = sp.dirz + kept * n, *q = sp.dirq + kept * n;
     const unsigned gd = std::max(1u, std::min(unsigned(kDotBlocks), unsigned(nblocks(n, kThreads))));
     sp_direction<<<nblocks(n, kThreads), kThreads, 0, st>>>(n, sp.d_perm, sp.D, sp.w, z, sp.dz, sp.nrm,
                                                              sp.flags);
-    sp_apply<<<gd, kThreads, 0, st>>>(n, it, sp.d_rptr, sp.d_rq, sp.d_rcol, c->nzval, sp.D, sp.dz, sp.dirq, q, sp.part,
-                                      sp.done, sp.coef, sp.coef + kSparseSweeps, sp.flags);
-    sp_conjugate<<<gd, kThreads, 0, st>>>(n, it, sp.dirq, sp.dirz, q, z, sp.r, sp.coef + kSparseSweeps, sp.part,
-                                          sp.done, sp.coef + it, sp.coef + 2 * kSparseSweeps, sp.flags);
+    sp_apply<<<gd, kThreads, 0, st>>>(n, kept, sp.d_rptr, sp.d_rq, sp.d_rcol, c->nzval, sp.D, sp.dz, sp.dirq, q,
+                                      sp.part, sp.done, sp.coef, sp.coef + kSparseSweeps, sp.flags);
+    sp_conjugate<<<gd, kThreads, 0, st>>>(n, kept, sp.dirq, sp.dirz, q, z, sp.r, sp.coef + kSparseSweeps, sp.part,
+                                          sp.done, sp.coef + kept, sp.coef + 2 * kSparseSweeps, sp.flags);
     sp_step<<<nblocks(n, kThreads), kThreads, 0, st>>>(n, it == 0, sp.d_perm, sp.D, sp.coef + 2 * kSparseSweeps, z,
                                                        sp.yacc, sp.xs, sp.nrm, sp.flags);
     c->launches += 4;
@@ -2364,8 +2366,6 @@ int sparse_create(mgpu_ctx* c, SparseDev*& spp, const double* dof_xyz, const uin
   ok(cudaMalloc(&sp.tw, n * sizeof(double)));
   ok(cudaMalloc(&sp.yacc, n * sizeof(double)));
   ok(cudaMalloc(&sp.r, n * sizeof(double)));
-  ok(cudaMalloc(&sp.dirz, size_t(kSparseSweeps) * n * sizeof(double)));
-  ok(cudaMalloc(&sp.dirq, size_t(kSparseSweeps) * n * sizeof(double)));
   ok(cudaMalloc(&sp.dz, n * sizeof(double)));
   ok(cudaMalloc(&sp.part, size_t(kDotBlocks) * kSparseSweeps * sizeof(double)));
   ok(cudaMalloc(&sp.coef, (2 * kSparseSweeps + 2) * sizeof(double)));  // q·q, beta, alpha, done
@@ -2405,6 +2405,19 @@ int sparse_create(mgpu_ctx* c, SparseDev*& spp, const double* dof_xyz, const uin
   if (const char* ev = getenv("MGPU_SPARSE_TC_LEFT")) sp.tc_left = atoi(ev) != 0;
   if (const char* ev = getenv("MGPU_SPARSE_SUPER")) sp.super_panels = atoi(ev) != 0;
   if (const char* ev = getenv("MGPU_SPARSE_TC")) sp.tensor_cores = atoi(ev) != 0;
+  // directions of the sweeps: 24 vectors, or as many as there is room for, two at least
+  // (MGPU_SPARSE_DIRECTIONS: at most that many pairs)
+  const char* de = getenv("MGPU_SPARSE_DIRECTIONS");
+  for (int nd = de ? std::clamp(atoi(de), 1, kSparseSweeps) : kSparseSweeps; e == cudaSuccess; nd = (nd + 1) / 2) {
+    sp.ndir = nd;
+    cudaError_t x = cudaMalloc(&sp.dirz, size_t(nd) * n * sizeof(double));
+    if (x == cudaSuccess) x = cudaMalloc(&sp.dirq, size_t(nd) * n * sizeof(double));
+    if (x == cudaSuccess) break;
+    cudaGetLastError();
+    cudaFree(sp.dirz);
+    sp.dirz = sp.dirq = nullptr;
+    if (nd == 1) e = x;
+  }
   // workspace of the packed trailing updates; without it (MGPU_SPARSE_PACK=0, or no
   // room) the trailing blocks take their operands from the fronts
   const char* pe = getenv("MGPU_SPARSE_PACK");
@@ -2488,6 +2501,12 @@ int sparse_factor_solve(mgpu_ctx* c, SparseDev& sp, const double* rhs, double* o
   if (use64) {
     if (!sp.F64) {
       cudaError_t e = cudaMalloc(&sp.F64, std::max<int64_t>(sp.fsize, 1) * sizeof(double));
+      if (e != cudaSuccess && sp.pack) {  // the FP32 factors do without their workspace
+        cudaGetLastError();
+        cudaFree(sp.pack);
+        sp.pack = nullptr;
+        e = cudaMalloc(&sp.F64, std::max<int64_t>(sp.fsize, 1) * sizeof(double));
+      }
       if (e != cudaSuccess) {
         sp.F64 = nullptr;
         return set_err(c, MGPU_ERR_NOMEM, std::string("FP64 factors of the sparse solver: ") + cudaGetErrorString(e));

@@ -88,7 +88,8 @@ struct SparseDev {
   int64_t* d_poff = nullptr;    // [nfront] offset of each blocked front's partials in P
   double* tw = nullptr;         // [n] U₁₂ x_u of each pivot (backward substitution)
   double* yacc = nullptr;       // [n] accumulated scaled solution (elimination order)
-  double *dirz = nullptr, *dirq = nullptr;  // [kSparseSweeps][n] directions of the sweeps and A times them
+  int ndir = 0;                             // directions kept
+  double *dirz = nullptr, *dirq = nullptr;  // [ndir][n] directions of the sweeps and A times them
   double *dz = nullptr, *part = nullptr, *coef = nullptr;  // D z, blocks' sums, the sweeps' coefficients
   unsigned* done = nullptr;                 // blocks that have added theirs
   double* r = nullptr;          // [n] residual (model order)

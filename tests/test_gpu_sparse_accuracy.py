@@ -65,3 +65,24 @@ def test_one_block_substitutions_of_a_front_near_48_kb(monkeypatch):
     lam = np.array([str(f).startswith("λ") for f in st.dis.fieldX])
     for sel in (lam, ~lam):
         assert np.max(np.abs(a[0, 0][sel] - b[0, 0][sel])) <= 1e-9 * np.max(np.abs(b[0, 0][sel]))
+
+
+@pytest.mark.parametrize("kind", ["sparse", "sparse64"])
+@pytest.mark.parametrize("kept", ["1", "2", "3"])
+def test_sweeps_with_fewer_directions_reach_the_same_solution(monkeypatch, kind, kept):
+    """Where there is no room for the directions of all sweeps, the conjugation starts
+    again after fewer; a solve is as accurate, after some sweeps more perhaps."""
+    m, times = W.lattice(12, 12, 6)
+    st = m.initialize()
+    out = {}
+    for n in ("12", kept):
+        monkeypatch.setenv("MGPU_SPARSE_DIRECTIONS", n)
+        dm = DeviceModel(m, st.dis, linsolve=kind)
+        rc, out[n], _ = dm.sweepx(0, times[:2], st.time, list(st.X), maxdx=1e-8, maxLl=1e-3)
+        info = dm.sparse_info()
+        dm.close()
+        assert rc == 0 and info["last_fallback"] == 0
+    lam = np.array([str(f).startswith("λ") for f in st.dis.fieldX])
+    a, b = out[kept][:, 0], out["12"][:, 0]
+    for sel in (lam, ~lam):
+        assert np.max(np.abs(a[:, sel] - b[:, sel])) <= 1e-9 * np.max(np.abs(b[:, sel]))
