@@ -280,10 +280,11 @@ class DeviceModel:
         arrays are overwritten by the next reuse call."""
         X = [np.ascontiguousarray(x, dtype=np.float64) for x in X]
         nXder = len(X)
-        if not X or any(v.size != self.nX for v in X):
+        if not X or any(v.shape != (self.nX,) for v in X):
             flat = np.concatenate(X)
-            if flat.size < nXder * self.nX or (reuse and flat.size > nXder * self.nX):
-                raise ValueError(f"a state of {flat.size} values for {nXder} times {self.nX} dofs")
+            if flat.size < nXder * self.nX or (reuse and flat.shape != (nXder * self.nX,)):
+                raise ValueError(f"a state of shape {flat.shape} for {nXder} times {self.nX} dofs")
+            flat = flat.reshape(-1)
             X = [flat[k * self.nX:] for k in range(nXder)]
         x = (ctypes.POINTER(ctypes.c_double) * nXder)(*[L.ptr(v) for v in X])
         u = np.ascontiguousarray(U if U is not None else np.zeros(self.nU), dtype=np.float64)
