@@ -1147,16 +1147,18 @@ extern "C" int mgpu_get_asm(const mgpu_ctx* cc, int32_t g, int64_t* asm1, int64_
   return MGPU_OK;
 }
 
-// the state's nXder parts, each nX long
-static int upload_parts(mgpu_ctx* c, int32_t nXder, const double* const* x, const double* u, const double* tvals) {
+// The state's nXder derivatives, each nX long, at x[0], or (parts) each at its own x[k].
+// Those are copied one by one even where they lie one after the other: a copy must not
+// span memory that is page-locked and memory that is not.
+static int upload_state(mgpu_ctx* c, int32_t nXder, const double* const* x, bool parts, const double* u,
+                        const double* tvals) {
   MG_CUDA(cudaSetDevice(c->device));
   const size_t nb = size_t(c->nX) * sizeof(double);
-  for (int32_t k = 0; k < nXder;) {
-    int32_t m = 1;  // parts that lie one after the other are one copy
-    while (k + m < nXder && x[k + m] == x[k] + m * c->nX) ++m;
-    MG_CUDA(cudaMemcpyAsync(c->x + k * c->nX, x[k], m * nb, cudaMemcpyHostToDevice, c->stream));
-    k += m;
-  }
+  if (!parts)
+    MG_CUDA(cudaMemcpyAsync(c->x, x[0], nXder * nb, cudaMemcpyHostToDevice, c->stream));
+  else
+    for (int32_t k = 0; k < nXder; ++k)
+      MG_CUDA(cudaMemcpyAsync(c->x + k * c->nX, x[k], nb, cudaMemcpyHostToDevice, c->stream));
   if (nXder < 3) MG_CUDA(cudaMemsetAsync(c->x + nXder * c->nX, 0, (3 - nXder) * nb, c->stream));
   if (c->nU > 0 && u) MG_CUDA(cudaMemcpyAsync(c->u, u, c->nU * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   if (c->ntval > 0 && tvals)
@@ -1167,8 +1169,7 @@ static int upload_parts(mgpu_ctx* c, int32_t nXder, const double* const* x, cons
 
 extern "C" int mgpu_upload_state(mgpu_ctx* c, int32_t nXder, const double* x, const double* u, const double* tvals) {
   if (!c || !x || nXder < 1 || nXder > 3) return set_err(c, MGPU_ERR_ARG, "mgpu_upload_state: bad arguments");
-  const double* part[3] = {x, x + c->nX, x + 2 * c->nX};
-  return upload_parts(c, nXder, part, u, tvals);
+  return upload_state(c, nXder, &x, false, u, tvals);
 }
 
 static int assemble_resident(mgpu_ctx* c, int32_t mission, double t, const mgpu_newmark* nm, double* host_nz) {
@@ -1194,15 +1195,15 @@ extern "C" int mgpu_download(mgpu_ctx* c, double* Ll, double* nzval) {
   return nan_error(c, *c->herr);
 }
 
-static int assemble_parts(mgpu_ctx* c, int32_t mission, int32_t nXder, const double* const* x, const double* u,
-                          double t, const double* tvals, const mgpu_newmark* nm, double* Ll, double* nzval) {
+static int assemble(mgpu_ctx* c, int32_t mission, int32_t nXder, const double* const* x, bool parts, const double* u,
+                    double t, const double* tvals, const mgpu_newmark* nm, double* Ll, double* nzval) {
   MG_CUDA(cudaSetDevice(c->device));
   if (nzval && c->pat.nnz >= kDownMin && !c->dstream) {
     for (cudaEvent_t& e : c->down_ev) MG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     MG_CUDA(cudaStreamCreateWithFlags(&c->dstream, cudaStreamNonBlocking));
   }
   MG_TRY(reset_errflag(c));
-  MG_TRY(upload_parts(c, nXder, x, u, tvals));
+  MG_TRY(upload_state(c, nXder, x, parts, u, tvals));
   double* own = nzval && c->pat.nnz >= kDownMin ? nzval : nullptr;  // copied beside the gather-sum
   const int rc = assemble_resident(c, mission, t, nm, own);
   if (own && cudaStreamSynchronize(c->dstream) != cudaSuccess && rc == MGPU_OK)
@@ -1215,8 +1216,7 @@ extern "C" int mgpu_assemble(mgpu_ctx* c, int32_t mission, int32_t nXder, const 
                              const double* tvals, const mgpu_newmark* nm, double* Ll, double* nzval) {
   if (!c) return MGPU_ERR_ARG;
   if (!x || nXder < 1 || nXder > 3) return set_err(c, MGPU_ERR_ARG, "mgpu_upload_state: bad arguments");
-  const double* part[3] = {x, x + c->nX, x + 2 * c->nX};
-  return assemble_parts(c, mission, nXder, part, u, t, tvals, nm, Ll, nzval);
+  return assemble(c, mission, nXder, &x, false, u, t, tvals, nm, Ll, nzval);
 }
 
 extern "C" int mgpu_assemble_parts(mgpu_ctx* c, int32_t mission, int32_t nXder, const double* const* x,
@@ -1226,7 +1226,7 @@ extern "C" int mgpu_assemble_parts(mgpu_ctx* c, int32_t mission, int32_t nXder, 
   bool bad = !x || nXder < 1 || nXder > 3;
   for (int32_t k = 0; !bad && k < nXder; ++k) bad = !x[k];
   if (bad) return set_err(c, MGPU_ERR_ARG, "mgpu_upload_state: bad arguments");
-  return assemble_parts(c, mission, nXder, x, u, t, tvals, nm, Ll, nzval);
+  return assemble(c, mission, nXder, x, true, u, t, tvals, nm, Ll, nzval);
 }
 
 // Pipelined assembly.  Slot s = ticket mod 2 owns a device copy of the outputs
