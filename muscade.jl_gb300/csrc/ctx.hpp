@@ -72,7 +72,7 @@ struct mgpu_ctx {
   size_t flush_bytes = 0;
   int nXder_resident = 1;
   double* res_work = nullptr;  // mgpu_beam_results: states and results of a call
-  size_t res_bytes = 0;
+  size_t res_bytes = 0, res_fields = 0;  // bytes of it, and of the groups' records
   std::mutex res_lock;  // its owner
   // host: coordinates of each X-dof's node from the beam and bar elements'
   // geometry (NaN where no element gives one) and the constraint multipliers;

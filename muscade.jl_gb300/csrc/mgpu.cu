@@ -1474,7 +1474,8 @@ extern "C" int mgpu_beam_results(mgpu_ctx* c, int32_t g, int64_t nstate, const d
   if (n == 0) return MGPU_OK;
   MG_CUDA(cudaSetDevice(c->device));
   std::lock_guard<std::mutex> own(c->res_lock);
-  // workspace [X | results], kept for the next call up to kResKeep bytes
+  // workspace [X | results] and the groups' records, kept for the next call up to
+  // kResKeep bytes of a model, the workspace giving way first
   constexpr size_t kResKeep = size_t(256) << 20;
   const size_t nx = size_t(nstate) * c->nX, bytes = (nx + size_t(n) * kRes) * sizeof(double);
   cudaError_t e = cudaSuccess;
@@ -1482,21 +1483,37 @@ extern "C" int mgpu_beam_results(mgpu_ctx* c, int32_t g, int64_t nstate, const d
     cudaGetLastError();
     return set_err(c, MGPU_ERR_NOMEM, std::string("mgpu_beam_results: ") + cudaGetErrorString(e));
   };
+  const size_t nf = G.h_edata.size() * sizeof(double);
+  auto drop_fields = [&] {
+    cudaFree(G.fields);
+    G.fields = nullptr;
+    c->res_fields -= nf;
+  };
+  auto drop_work = [&] {
+    cudaFree(c->res_work);
+    c->res_work = nullptr;
+    c->res_bytes = 0;
+  };
   if (!G.fields) {
-    const size_t nf = G.h_edata.size() * sizeof(double);
-    if ((e = cudaMalloc(&G.fields, nf)) != cudaSuccess) return nomem();
+    if ((e = cudaMalloc(&G.fields, nf)) != cudaSuccess) {
+      G.fields = nullptr;
+      return nomem();
+    }
+    c->res_fields += nf;
     e = cudaMemcpyAsync(G.fields, G.h_edata.data(), nf, cudaMemcpyHostToDevice, c->stream);
     if (e != cudaSuccess) {
-      cudaFree(G.fields);
-      G.fields = nullptr;
+      drop_fields();
       return set_err(c, MGPU_ERR_CUDA, std::string("mgpu_beam_results: ") + cudaGetErrorString(e));
     }
   }
   if (bytes > c->res_bytes) {
-    cudaFree(c->res_work);
-    c->res_work = nullptr;
-    c->res_bytes = 0;
-    if ((e = cudaMalloc(&c->res_work, bytes)) != cudaSuccess) return nomem();
+    drop_work();
+    if ((e = cudaMalloc(&c->res_work, bytes)) != cudaSuccess) {
+      c->res_work = nullptr;
+      cudaStreamSynchronize(c->stream);  // the records' copy
+      drop_fields();
+      return nomem();
+    }
     c->res_bytes = bytes;
   }
   double *dX = c->res_work, *dout = dX + nx;
@@ -1509,11 +1526,8 @@ extern "C" int mgpu_beam_results(mgpu_ctx* c, int32_t g, int64_t nstate, const d
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(out, dout, size_t(n) * kRes * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
   const cudaError_t es = cudaStreamSynchronize(c->stream);
-  if (c->res_bytes > kResKeep) {
-    cudaFree(c->res_work);
-    c->res_work = nullptr;
-    c->res_bytes = 0;
-  }
+  if (c->res_fields + c->res_bytes > kResKeep) drop_work();
+  if (c->res_fields > kResKeep) drop_fields();
   if (e == cudaSuccess) e = es;
   if (e != cudaSuccess) return set_err(c, MGPU_ERR_CUDA, std::string("mgpu_beam_results: ") + cudaGetErrorString(e));
   return MGPU_OK;

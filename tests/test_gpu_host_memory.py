@@ -1,4 +1,5 @@
-"""Memory at the edges of the calls: states in arrays of which some are page-locked."""
+"""Memory at the edges of the calls: states in arrays of which some are page-locked, and
+what a model keeps on the device between calls for results."""
 import ctypes
 
 import numpy as np
@@ -44,3 +45,24 @@ def test_a_state_of_which_a_part_is_page_locked():
         dm.lib.mgpu_host_unregister(first)
         dm.close()
     assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1])
+
+
+def test_results_hold_no_more_than_their_allowance():
+    """The records of 600,000 beams are 330 MB, above the 256 MB that a model keeps for
+    its next results: neither they nor the workspace stay."""
+    torch = pytest.importorskip("torch")
+    m, st = _chain(600_000, "t1")
+    dm = DeviceModel(m, st.dis)
+    x = np.random.default_rng(1).normal(size=m.ndof["X"]) * 1e-3
+    few = _chain(3)
+    small = DeviceModel(few[0], few[1].dis)  # the library's own first allocations
+    small.beam_results(0, [np.zeros(few[0].ndof["X"])])
+    free = torch.cuda.mem_get_info()[0]
+    a = dm.beam_results(0, [x])
+    held = free - torch.cuda.mem_get_info()[0]
+    b = dm.beam_results(0, [x])
+    dm.close()
+    small.close()
+    assert held <= 256 << 20
+    for p, q in zip(a.values(), b.values()):
+        assert np.array_equal(p, q)
