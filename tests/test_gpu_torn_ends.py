@@ -105,3 +105,40 @@ def test_a_second_model_leaves_the_first_ones_solver_alone():
     first.close()
     second.close()
     assert rc == 0 and rc2 == 0 and np.array_equal(X, alone)
+
+
+@pytest.mark.parametrize("kind", ["torn", "torn32"])
+@pytest.mark.parametrize("nel, ncomp", [(85, 1), (200, 3), (85, 490)])
+def test_transposed_solves_match_whole_components(nel, ncomp, kind):
+    """Gradients by the adjoint, whose solves are of Lλx's transpose: one first end
+    without a spike, many interiors, and (490 components) a last end numbered
+    backwards.  Chains swaying with drag: Lλx and its transpose differ by up to 1,150
+    where the lateral stiffnesses are 8e5.  To 1e-6 of the largest component, the bar of
+    the adjoint tests."""
+    m = W.Model("swaying chains")
+    x = np.linspace(0.0, 0.5 * nel, nel + 1)
+    mat = W.BeamCrossSection(EA=1e8, EI2=1e4, EI3=1e4, GJ=1e4, mu=10.0, iota1=1.0, Ca2=5.0, Cq2=400.0, Ca3=6.0, Cq3=500.0)
+    ends, sense = [], []
+    for c in range(ncomp):
+        nodes = m.addnode(np.stack([x, np.full_like(x, 5.0 * c), np.zeros_like(x)], axis=1))
+        own = m.addnode(np.stack([0.5 * (x[1:] + x[:-1]), np.full(nel, 5.0 * c + 1.0), np.zeros(nel)], axis=1))
+        m.addelement(W.EulerBeam3D, np.stack([nodes[:-1], nodes[1:], own], axis=1), mat=mat, orient2=(0.0, 1.0, 0.0), adof=True)
+        ends.append(nodes[0])
+        sense += [nodes[nel // 2], nodes[-1]]
+        m.addelement(W.DofLoad, nodes[nel // 2 : nel // 2 + 1, None], field="t3", value=lambda t: 3e4 * t)
+        m.addelement(W.DofLoad, nodes[-1:, None], field="t2", value=lambda t: 2e4 * t)
+    for f in ("t1", "t2", "t3", "r1", "r2", "r3"):
+        m.addelement(W.Hold, np.asarray(ends)[:, None], field=f)
+    st = m.initialize(time=0.0)
+    times = np.array([0.1, 0.2, 0.3])
+    dofs = np.sort(W.node_dofs(m, np.asarray(sense))[:, 1:3].reshape(-1)) + 1
+    out = {}
+    for k in (kind, "f64"):
+        dm = DeviceModel(m, st.dis, linsolve=k)
+        dm.set_A(np.linspace(0.8, 1.25, dm.nA))
+        C, g, _, _ = dm.adjoint(2, times, st.time, list(st.X), dofs, 1.0, np.zeros((len(times), len(dofs))), maxdx=1e-9)
+        out[k] = (C, g)
+        dm.close()
+    (C, g), (Cr, gr) = out[kind], out["f64"]
+    assert C == pytest.approx(Cr, rel=1e-9)
+    assert np.max(np.abs(g - gr)) <= 1e-6 * np.max(np.abs(gr)) and np.max(np.abs(gr)) > 0.0
