@@ -83,62 +83,95 @@ static void narrow_by_nodes(const Pattern& P, const std::vector<std::vector<int3
   for (size_t cc = 0; cc < members.size(); ++cc)
     if (wid[cc] > 11 && wid[cc] <= 48 && members[cc].size() > 2) todo.push_back(int32_t(cc));
   if (todo.empty()) return;
-  std::vector<int32_t> nb(P.nnz), cnt(n, 0), grp(n, -1), host(n, -1);  // neighbours: a column's rows but its own
+  std::vector<int32_t> host(n, -1), grp(n, -1);  // a leaf's dof, the others' group
+  std::vector<uint64_t> hash(n, 0);
 #pragma omp parallel for schedule(dynamic, 16) if (n > 50000)
   for (int64_t t = 0; t < int64_t(todo.size()); ++t) {
     const auto& M = members[todo[t]];
     const int32_t c0 = comp_start[todo[t]], w0 = wid[todo[t]];
-    for (int32_t v : M) {
-      int32_t* to = nb.data() + P.colptr[v];
+    // neighbours: a column's rows but its own
+    auto neighbours = [&](int32_t v, auto&& f) {
       for (int64_t q = P.colptr[v]; q < P.colptr[v + 1]; ++q)
-        if (P.rowval[q] != v) *to++ = int32_t(P.rowval[q]);
-      cnt[v] = int32_t(to - (nb.data() + P.colptr[v]));
-    }
-    for (int32_t v : M) {
-      const int32_t u = cnt[v] == 1 ? nb[P.colptr[v]] : -1;
-      host[v] = u >= 0 && cnt[u] > 1 ? u : -1;
-    }
-    // groups of equal closed neighbourhood (leaves left out), by a hash of the list
-    auto closed = [&](int32_t v, std::vector<int32_t>& k) {
-      k.clear();
-      for (int32_t q = 0; q < cnt[v]; ++q)
-        if (host[nb[P.colptr[v] + q]] < 0) k.push_back(nb[P.colptr[v] + q]);
-      k.insert(std::lower_bound(k.begin(), k.end(), v), v);
+        if (P.rowval[q] != v) f(P.rowval[q]);
     };
-    std::vector<std::pair<uint64_t, int32_t>> key;
-    std::vector<int32_t> ka, kb;
+    auto several = [&](int32_t v) {
+      int32_t k = 0;
+      neighbours(v, [&](int32_t) { ++k; });
+      return k > 1;
+    };
     for (int32_t v : M)
-      if (host[v] < 0) {
-        closed(v, ka);
+      if (P.colptr[v + 1] - P.colptr[v] <= 2 && !several(v))
+        neighbours(v, [&](int32_t u) {
+          if (several(u)) host[v] = u;
+        });
+    auto leaf = [&](int32_t v) { return host[v] >= 0; };
+    // Groups of equal closed neighbourhood (leaves left out), numbered by their first
+    // dof, so that a model orders alike alone and among others.  The dofs of a group
+    // are neighbours of each other: a dof's group is that of the first neighbour of
+    // the same hash and list.
+    auto closed = [&](int32_t v, auto&& f) {  // in increasing order, until f returns false
+      bool self = false;
+      for (int64_t q = P.colptr[v]; q < P.colptr[v + 1]; ++q) {
+        const int32_t u = P.rowval[q];
+        if (u > v && !self && !f(v)) return;
+        self = self || u >= v;
+        if ((u == v || !leaf(u)) && !f(u)) return;
+      }
+      if (!self) f(v);
+    };
+    for (int32_t v : M)
+      if (!leaf(v)) {
         uint64_t h = 1469598103934665603ull;
-        for (int32_t u : ka) h = (h ^ uint64_t(uint32_t(u))) * 1099511628211ull;
-        key.push_back({h, v});
+        closed(v, [&](int32_t u) {
+          h = (h ^ uint64_t(uint32_t(u))) * 1099511628211ull;
+          return true;
+        });
+        hash[v] = h;
       }
-    std::sort(key.begin(), key.end());
-    std::vector<std::vector<int32_t>> G;  // dofs of each group
-    for (size_t q = 0; q < key.size(); ++q) {
-      bool same = q > 0 && key[q].first == key[q - 1].first;
-      if (same) {
-        closed(key[q].second, ka);
-        closed(G.back()[0], kb);
-        same = ka == kb;
+    std::vector<int32_t> ka, kb, first;  // first: each group's first dof
+    auto list = [&](int32_t v, std::vector<int32_t>& k) {
+      k.clear();
+      closed(v, [&](int32_t u) {
+        k.push_back(u);
+        return true;
+      });
+    };
+    for (int32_t v : M) {
+      if (leaf(v)) continue;
+      int32_t& g = grp[v];
+      closed(v, [&](int32_t u) {
+        if (u >= v) return false;
+        if (hash[u] != hash[v]) return true;
+        list(u, ka);
+        list(v, kb);
+        if (ka == kb) g = grp[u];
+        return g < 0;
+      });
+      if (g < 0) {
+        g = int32_t(first.size());
+        first.push_back(v);
       }
-      if (!same) G.push_back({});
-      G.back().push_back(key[q].second);
     }
-    // numbered by their first dof, so that a model orders alike alone and among others
-    std::sort(G.begin(), G.end());
-    const int ng = int(G.size());
-    for (int g = 0; g < ng; ++g)
-      for (int32_t v : G[g]) grp[v] = g;
-    std::vector<std::vector<int32_t>> ga(ng);
+    const int ng = int(first.size());
+    // the groups' dofs, leaves and neighbouring groups
+    std::vector<int32_t> g0(ng + 1, 0), l0(ng + 1, 0), a0(1, 0), gd(M.size()), ld(M.size()), ga;
+    for (int32_t v : M) ++(leaf(v) ? l0[grp[host[v]] + 1] : g0[grp[v] + 1]);
+    for (int g = 0; g < ng; ++g) g0[g + 1] += g0[g], l0[g + 1] += l0[g];
+    {
+      std::vector<int32_t> gf(g0.begin(), g0.end() - 1), lf(l0.begin(), l0.end() - 1);
+      for (int32_t v : M)
+        if (leaf(v))
+          ld[lf[grp[host[v]]]++] = v;
+        else
+          gd[gf[grp[v]]++] = v;
+    }
     for (int g = 0; g < ng; ++g) {
-      for (int32_t q = 0, v = G[g][0]; q < cnt[v]; ++q) {
-        const int32_t u = nb[P.colptr[v] + q];
-        if (host[u] < 0 && grp[u] != g) ga[g].push_back(grp[u]);
-      }
-      std::sort(ga[g].begin(), ga[g].end());
-      ga[g].erase(std::unique(ga[g].begin(), ga[g].end()), ga[g].end());
+      neighbours(first[g], [&](int32_t u) {
+        if (!leaf(u) && grp[u] != g) ga.push_back(grp[u]);
+      });
+      std::sort(ga.begin() + a0[g], ga.end());
+      ga.erase(std::unique(ga.begin() + a0[g], ga.end()), ga.end());
+      a0.push_back(int32_t(ga.size()));
     }
     // breadth-first order from an end of the group graph (the farthest group, three times)
     std::vector<int32_t> seen(ng, -1), bfs;
@@ -147,10 +180,11 @@ static void narrow_by_nodes(const Pattern& P, const std::vector<std::vector<int3
       seen[s0] = tag;
       for (size_t h = 0; h < bfs.size(); ++h) {
         const size_t from = bfs.size();
-        for (int32_t u : ga[bfs[h]])
-          if (seen[u] != tag) seen[u] = tag, bfs.push_back(u);
+        for (int32_t q = a0[bfs[h]], end = a0[bfs[h] + 1]; q < end; ++q)
+          if (seen[ga[q]] != tag) seen[ga[q]] = tag, bfs.push_back(ga[q]);
         std::sort(bfs.begin() + from, bfs.end(), [&](int32_t x, int32_t y) {
-          return ga[x].size() != ga[y].size() ? ga[x].size() < ga[y].size() : x < y;
+          const int32_t dx = a0[x + 1] - a0[x], dy = a0[y + 1] - a0[y];
+          return dx != dy ? dx < dy : x < y;
         });
       }
     };
@@ -161,18 +195,17 @@ static void narrow_by_nodes(const Pattern& P, const std::vector<std::vector<int3
     }
     sweep(start, 3);
     if (int(bfs.size()) != ng) continue;
-    std::vector<std::vector<int32_t>> leaves(ng);
-    for (int32_t v : M)
-      if (host[v] >= 0) leaves[grp[host[v]]].push_back(v);
     std::vector<int32_t> ord;
     ord.reserve(M.size());
     for (size_t h = 0; h < bfs.size(); ++h) {
       const int32_t g = bfs[bfs.size() - 1 - h];
-      auto& lv = leaves[g];
-      std::sort(lv.begin(), lv.end(), [&](int32_t x, int32_t y) { return host[x] != host[y] ? host[x] < host[y] : x < y; });
-      if (h == 0) ord.insert(ord.end(), lv.begin(), lv.end());
-      ord.insert(ord.end(), G[g].begin(), G[g].end());
-      if (h > 0) ord.insert(ord.end(), lv.begin(), lv.end());
+      const auto la = ld.begin() + l0[g], lb = ld.begin() + l0[g + 1];
+      std::sort(la, lb, [&](int32_t x, int32_t y) {
+        return host[x] != host[y] ? host[x] < host[y] : x < y;
+      });
+      if (h == 0) ord.insert(ord.end(), la, lb);
+      ord.insert(ord.end(), gd.begin() + g0[g], gd.begin() + g0[g + 1]);
+      if (h > 0) ord.insert(ord.end(), la, lb);
     }
     const std::vector<int32_t> keep(order.begin() + c0, order.begin() + c0 + M.size());
     for (size_t k = 0; k < ord.size(); ++k) {
