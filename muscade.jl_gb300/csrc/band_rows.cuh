@@ -213,11 +213,12 @@ __global__ void __launch_bounds__(32) rb_lu(RbComp cp, const T* __restrict__ Aro
 }
 
 // The same for kl <= 15 and kv + 2 <= 2 NC (chains of 6-dof nodes: kl = ku = 11, NC =
-// 12; at an odd step column k + 2 NC - 1 has no slot): rb_lu leaves lanes kl+1..31 idle in every FP64 instruction, so here 16 lanes
-// hold a row each and the half-warps share its columns, half h those of parity h
-// (slot s of half h: column 2(⌊k/2⌋ + s) + h), which needs a shift only every
-// second step.  12 instead of 22 multiply-adds a column; 132 dofs of one cantilever
-// 218 -> 139 us.  The arithmetic of an entry is that of rb_lu.
+// 12; at an odd step k column k + 2 NC - 1 has no slot): rb_lu leaves lanes kl+1..31
+// idle in every FP64 instruction, so here 16 lanes hold a row each and the half-warps
+// share its columns, half h those of parity h (slot s of half h: column
+// 2(⌊k/2⌋ + s) + h), which needs a shift only every second step.  12 instead of 22
+// multiply-adds a column; 132 dofs of one cantilever 218 -> 141 us.  The arithmetic of
+// an entry is that of rb_lu.
 template <typename T, int NC>
 __global__ void __launch_bounds__(32) rb_lu_half(RbComp cp, const T* __restrict__ Arows, T* __restrict__ UC,
                                                  T* __restrict__ LM, int32_t* __restrict__ ipiv, int mode,

@@ -61,7 +61,8 @@ __device__ __forceinline__ bool tb_skip(const int* only, int comp) { return only
 // interiors each: 1.7 of 3.9 ms).  The last interior is numbered backwards only where
 // components are cut in two: FP32 factors of 200 risers in 13 interiors, eliminated
 // from the driven end too, fell short of their refinement within 20 steps and left the
-// rest to FP64 (6.0 -> 6.7 ms a step).  Y^R's room holds U^-1 Z (rows 0..s) and Z (its
+// rest to FP64 (6.0 -> 6.7 ms a step); in two interiors that comes after 30 to 60 steps
+// (500 risers of 250 beams: 12.8 ms a step in FP32, 15 to 18 in FP64).  Y^R's room holds U^-1 Z (rows 0..s) and Z (its
 // own rows); n >= 2 s + kl, since interiors have at least 48 rows and s <= 16.
 template <typename T, int KLW>
 __device__ void tb_end(const TornInt& I, const T* __restrict__ U, const T* __restrict__ L,
