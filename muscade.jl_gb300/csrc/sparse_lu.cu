@@ -2371,7 +2371,7 @@ int sparse_create(mgpu_ctx* c, SparseDev*& spp, const double* dof_xyz, const uin
   ok(cudaMalloc(&sp.coef, (2 * kSparseSweeps + 2) * sizeof(double)));  // q·q, beta, alpha, done
   ok(cudaMalloc(&sp.xs, n * sizeof(double)));
   ok(cudaMalloc(&sp.nrm, 4 * sizeof(unsigned long long)));
-  ok(cudaMalloc(&sp.last, 2 * sizeof(double)));
+  ok(cudaMalloc(&sp.last, 3 * sizeof(double)));
   ok(cudaMalloc(&sp.flags, 4 * sizeof(int)));
   ok(cudaMallocHost(&sp.hflags, 4 * sizeof(int)));
   sp.ntflag = int64_t(A.fidx.size()) / 64 + 2 * int64_t(sp.nfront) + 64;

@@ -95,7 +95,7 @@ struct SparseDev {
   double* r = nullptr;          // [n] residual (model order)
   double* xs = nullptr;         // [n] current solution (model order)
   unsigned long long* nrm = nullptr;  // [4] max |correction|, |solution|, |residual|, |A||y| + |D b| (as ordered bits)
-  double* last = nullptr;       // [2] the previous sweep's max |correction|, the worst rate so far
+  double* last = nullptr;       // [3] of the previous sweep (sp_stop)
   int nrow = 0;                 // most entries in a row
   int* flags = nullptr;         // [0] converged, [1] sweeps done, [2] perturbed pivots, [3] non-finite pivot
                                 // (bit 1: a chained substitution's wait ran out, bit 2: a tensor-core tile's,

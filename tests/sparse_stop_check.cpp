@@ -3,7 +3,7 @@
 #include "sparse_stop.hpp"
 
 extern "C" int sparse_stop_check(int n, const double* c, const double* y, const double* r, const double* a, int nrow) {
-  double last[2] = {0.0, 0.0};
+  double last[3] = {0.0, 0.0, 0.0};
   for (int k = 0; k < n; ++k) {
     const int s = mgpu::sp_stop(k + 1, c[k], y[k], r[k], a[k], nrow, last);
     if (s != mgpu::SP_GO_ON) return s == mgpu::SP_CONVERGED ? k + 1 : -(k + 1);

@@ -47,12 +47,13 @@ def test_corrections_that_shrink(stop, c, at):
     assert stop(c, r=1.0) == at
 
 
-def test_a_plateau_counts_only_where_the_residual_is_rounding(stop):
+def test_a_plateau_counts_where_the_residual_is_rounding_or_it_lasts(stop):
     c = [1.0, 1e-2, 5e-11, 4e-11, 3.5e-11, 1e-12]
     assert stop(c, r=44 * U) == 4
     assert stop(c, r=[1.0, 1e-4, 1e-9, 1e-10, 44 * U, 44 * U]) == 5  # two orders above it in the fourth
-    assert stop(c, r=45 * U) == 0
-    assert stop([1.0, 1e-6, 2e-10, 1.9e-10], r=0.0) == 0  # too far off to stop at all
+    assert stop(c, r=1e-12) == 5  # the second time in a row
+    assert stop([1.0, 1e-2, 5e-11, 4e-11, 1e-13, 9e-14], r=1e-12) == 0  # it did not last
+    assert stop([1.0, 1e-6, 2e-10, 1.9e-10, 1.8e-10], r=0.0) == 0  # too far off to stop at all
 
 
 @pytest.mark.parametrize("bad", [np.nan, np.inf])
