@@ -1651,17 +1651,22 @@ __global__ void sp_bwdb_fin(const SpFrontDev* __restrict__ fr, const int32_t* __
 }
 
 // ---------------------------------------------------------------- refinement
-// Sweeps of the generalised conjugate residual method (Eisenstat, Elman, Schultz
-// 1983), preconditioned by the factors M and in FP64 throughout: a sweep's direction
-// z = M^-1 r, q = A z, is made conjugate to the earlier ones (q orthogonal to their
-// q), and the step along it leaves the smallest residual over all of them.  The
-// factors' error E = I − M^-1 A is large in a few soft modes of the structure only;
-// plain refinement carries each at its own rate, |E| a sweep, here each direction
-// takes one of them out.  A and r are scaled, A = D Lλx D; z in elimination order, q
-// and r in model order.  The directions of all sweeps are kept (kSparseSweeps at most;
-// where there is no room for them fewer, and the conjugation starts again when these are
-// full), the residual is that of the solution itself in every sweep (sp_residual).
-//   60 x 60 x 20 lattice: 11 -> 9 sweeps a solve; 12 x 12 x 6: 8 -> 5
+// Sweeps of iterative refinement, y += f with f = M^-1 r and r the residual of y itself,
+// accelerated by Anderson's mixing (Anderson 1965, Walker and Ni 2011) in FP64: the
+// factors' error E = I − M^-1 A is large in a few soft modes of the structure only, plain
+// refinement carries each at its own rate, |E| a sweep, and the mixture of the sweeps so
+// far that makes f smallest takes one of them out a sweep.  f is the error as the factors
+// see it, and plain refinement's is one of the mixtures, so a sweep gains whatever |r|
+// does meanwhile: the conjugate residual method, which lessens |r|, took steps of next to
+// nothing along corrections that first raise it (factors of raised or grown pivots), and
+// left solutions 1e-4 off that plain refinement brings to 1e-9.
+// With the differences of successive f and y, df and dy, orthogonalised to q_j and z_j,
+//     y += f − sum_j c_j (z_j + q_j),   c_j = q_j·f / q_j·q_j.
+// A and r are scaled, A = D Lλx D; all vectors in elimination order.  The pairs of all
+// sweeps are kept (where there is no room for them fewer, and the mixing starts again
+// when these are full).
+//   60 x 60 x 20 lattice: 11 -> 8 or 9 sweeps a solve; 12 x 12 x 6: 8 -> 5
+constexpr double kDependent = 1e-12;  // q·q of df·df: a difference that tells nothing new
 constexpr int kDotBlocks = 304;
 
 // |v| as ordered bits (non-negative doubles order like their bit patterns); NaN wins:
@@ -1679,9 +1684,8 @@ __device__ __forceinline__ void max_bits(unsigned long long* dst, double v) {
   }
 }
 
-// r = D (b − Lλx x), w = r in elimination order; x: the solution so far, none in the
-// first sweep.  The recursion r − alpha q, a product less, loses the rounding of y, x
-// and the conjugated q: it goes on falling where the residual does not.  nrm[2], nrm[3]:
+// w = r = D (b − Lλx x); x: the solution so far, none in the first sweep.  (A recursion
+// for r, a product less, goes on falling where the residual does not.)  nrm[2], nrm[3]:
 // the largest |r| and the largest of its rows' |A||y| + |D b|, whose rounding bounds what
 // of r can be told from zero.
 __global__ void __launch_bounds__(kThreads) sp_residual(int64_t n, const int32_t* __restrict__ perm,
@@ -1690,8 +1694,8 @@ __global__ void __launch_bounds__(kThreads) sp_residual(int64_t n, const int32_t
                                                         const int32_t* __restrict__ rcol,
                                                         const double* __restrict__ nzval,
                                                         const double* __restrict__ D, const double* __restrict__ x,
-                                                        const double* __restrict__ b, double* __restrict__ r,
-                                                        double* __restrict__ w, unsigned long long* __restrict__ nrm,
+                                                        const double* __restrict__ b, double* __restrict__ w,
+                                                        unsigned long long* __restrict__ nrm,
                                                         const int* __restrict__ conv) {
   if (*conv) return;
   const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -1708,30 +1712,10 @@ __global__ void __launch_bounds__(kThreads) sp_residual(int64_t n, const int32_t
       }
     s *= D[d];
     a *= D[d];
-    w[k] = r[d] = s;
+    w[k] = s;
   }
   max_bits(nrm + 2, s);
   max_bits(nrm + 3, a);
-}
-
-// z = w, and D z in model order; the largest |w| of the sweep, the error that the
-// factors see before its step, decides convergence (not the step: a step along a
-// direction that does not reduce the residual is short without being right)
-__global__ void __launch_bounds__(kThreads) sp_direction(int64_t n, const int32_t* __restrict__ perm,
-                                                         const double* __restrict__ D, const double* __restrict__ w,
-                                                         double* __restrict__ z, double* __restrict__ dz,
-                                                         unsigned long long* __restrict__ nrm,
-                                                         const int* __restrict__ conv) {
-  if (*conv) return;
-  const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  double v = 0.0;
-  if (k < n) {
-    const int32_t d = perm[k];
-    v = w[k];
-    z[k] = v;
-    dz[d] = D[d] * v;
-  }
-  max_bits(nrm, v);
 }
 
 // Sums over all blocks of acc[0..NV), nv of them: each block's to part, and the block
@@ -1778,81 +1762,104 @@ __device__ __forceinline__ bool sp_sums(double (&acc)[NV], int nv, double* __res
   return true;
 }
 
-// q = D Lλx dz, and beta_j = q·q_j / q_j·q_j for the it earlier directions (Q: [it][n])
-__global__ void __launch_bounds__(kThreads) sp_apply(int64_t n, int it, const int64_t* __restrict__ rptr,
-                                                     const int32_t* __restrict__ rq, const int32_t* __restrict__ rcol,
-                                                     const double* __restrict__ nzval, const double* __restrict__ D,
-                                                     const double* __restrict__ dz, const double* __restrict__ Q,
-                                                     double* __restrict__ q, double* __restrict__ part,
-                                                     unsigned* __restrict__ done, const double* __restrict__ qq,
-                                                     double* __restrict__ beta, const int* __restrict__ conv) {
+// q = f − fprev, z = dy, and beta_j = q·q_j / q_j·q_j for the nk earlier pairs (Q: [nk][n]);
+// beta[nk] = q·q
+__global__ void __launch_bounds__(kThreads) sp_difference(int64_t n, int nk, const double* __restrict__ f,
+                                                          const double* __restrict__ fprev,
+                                                          const double* __restrict__ dy, const double* __restrict__ Q,
+                                                          double* __restrict__ q, double* __restrict__ z,
+                                                          double* __restrict__ part, unsigned* __restrict__ done,
+                                                          const double* __restrict__ qq, double* __restrict__ beta,
+                                                          const int* __restrict__ conv) {
   if (*conv) return;
   __shared__ double sum[kSparseSweeps];
   double acc[kSparseSweeps];
 #pragma unroll
   for (int j = 0; j < kSparseSweeps; ++j) acc[j] = 0.0;
   for (int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x; i < n; i += int64_t(gridDim.x) * kThreads) {
-    double s = 0.0;
-    for (int64_t t = rptr[i]; t < rptr[i + 1]; ++t) s = fma(nzval[rq[t]], dz[rcol[t]], s);
-    s *= D[i];
-    q[i] = s;
+    const double d = f[i] - fprev[i];
+    q[i] = d;
+    z[i] = dy[i];
 #pragma unroll
     for (int j = 0; j < kSparseSweeps; ++j)
-      if (j < it) acc[j] = fma(s, Q[j * n + i], acc[j]);
+      if (j <= nk) acc[j] = fma(d, j < nk ? Q[j * n + i] : d, acc[j]);
   }
-  if (it > 0 && sp_sums(acc, it, part, done, sum) && threadIdx.x < it)
-    beta[threadIdx.x] = qq[threadIdx.x] > 0.0 ? sum[threadIdx.x] / qq[threadIdx.x] : 0.0;
+  if (sp_sums(acc, nk + 1, part, done, sum) && threadIdx.x <= nk)
+    beta[threadIdx.x] = threadIdx.x == nk                ? sum[nk]
+                        : qq[threadIdx.x] > 0.0 ? sum[threadIdx.x] / qq[threadIdx.x]
+                                                : 0.0;
 }
 
-// q -= Σ beta_j q_j, z -= Σ beta_j z_j; qq = q·q, alpha = q·r / q·q
-__global__ void __launch_bounds__(kThreads) sp_conjugate(int64_t n, int it, const double* __restrict__ Q,
+// q −= Σ beta_j q_j, z −= Σ beta_j z_j; qq[nk] = q·q, c_j = q_j·f / q_j·q_j for all pairs
+__global__ void __launch_bounds__(kThreads) sp_conjugate(int64_t n, int nk, const double* __restrict__ Q,
                                                          const double* __restrict__ Z, double* __restrict__ q,
-                                                         double* __restrict__ z, const double* __restrict__ r,
+                                                         double* __restrict__ z, const double* __restrict__ f,
                                                          const double* __restrict__ beta, double* __restrict__ part,
                                                          unsigned* __restrict__ done, double* __restrict__ qq,
-                                                         double* __restrict__ alpha, const int* __restrict__ conv) {
+                                                         double* __restrict__ coef, const int* __restrict__ conv) {
   if (*conv) return;
-  __shared__ double sum[2];
-  double acc[2] = {0.0, 0.0}, be[kSparseSweeps];
+  __shared__ double sum[kSparseSweeps];
+  double acc[kSparseSweeps], be[kSparseSweeps];
 #pragma unroll
-  for (int j = 0; j < kSparseSweeps; ++j) be[j] = j < it ? beta[j] : 0.0;
+  for (int j = 0; j < kSparseSweeps; ++j) {
+    acc[j] = 0.0;
+    be[j] = j < nk ? beta[j] : 0.0;
+  }
   for (int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x; i < n; i += int64_t(gridDim.x) * kThreads) {
     double a = q[i], b = z[i];
+    const double v = f[i];
 #pragma unroll
-    for (int j = 0; j < kSparseSweeps; ++j)
-      if (j < it) {
-        a = fma(-be[j], Q[j * n + i], a);
+    for (int j = 0; j < kSparseSweeps - 2; ++j)
+      if (j < nk) {
+        const double u = Q[j * n + i];
+        acc[j + 2] = fma(u, v, acc[j + 2]);
+        a = fma(-be[j], u, a);
         b = fma(-be[j], Z[j * n + i], b);
       }
-    if (it > 0) {
+    if (nk > 0) {
       q[i] = a;
       z[i] = b;
     }
     acc[0] = fma(a, a, acc[0]);
-    acc[1] = fma(a, r[i], acc[1]);
+    acc[1] = fma(a, v, acc[1]);
   }
-  if (sp_sums(acc, 2, part, done, sum) && threadIdx.x == 0) {
-    *qq = sum[0];
-    *alpha = sum[0] > 0.0 ? sum[1] / sum[0] : 1.0;  // 1: no residual left, or a refinement step as it is
+  if (sp_sums(acc, nk + 2, part, done, sum)) {
+    const bool fresh = sum[0] > kDependent * beta[nk];
+    if (threadIdx.x == 0) {
+      qq[nk] = fresh ? sum[0] : 0.0;
+      coef[nk] = fresh ? sum[1] / sum[0] : 0.0;
+    } else if (threadIdx.x <= nk) {
+      coef[threadIdx.x - 1] = qq[threadIdx.x - 1] > 0.0 ? sum[threadIdx.x + 1] / qq[threadIdx.x - 1] : 0.0;
+    }
   }
 }
 
-// y += alpha z, x = D y
-__global__ void __launch_bounds__(kThreads) sp_step(int64_t n, int first, const int32_t* __restrict__ perm,
-                                                    const double* __restrict__ D, const double* __restrict__ alpha,
-                                                    const double* __restrict__ zv, double* __restrict__ yacc,
+// dy = f − Σ c_j (z_j + q_j) over np pairs, y += dy, x = D y, fprev = f; the largest
+// |f|, the error that the factors see before the step, and |y|
+__global__ void __launch_bounds__(kThreads) sp_step(int64_t n, int first, int np, const int32_t* __restrict__ perm,
+                                                    const double* __restrict__ D, const double* __restrict__ coef,
+                                                    const double* __restrict__ Q, const double* __restrict__ Z,
+                                                    const double* __restrict__ f, double* __restrict__ fprev,
+                                                    double* __restrict__ dy, double* __restrict__ yacc,
                                                     double* __restrict__ x, unsigned long long* __restrict__ nrm,
                                                     const int* __restrict__ conv) {
   if (*conv) return;
   const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  double y = 0.0;
+  double v = 0.0, y = 0.0;
   if (k < n) {
-    const double z = *alpha * zv[k];
-    y = first ? z : yacc[k] + z;
+    v = f[k];
+    double s = v;
+#pragma unroll
+    for (int j = 0; j < kSparseSweeps; ++j)
+      if (j < np) s = fma(-coef[j], Z[j * n + k] + Q[j * n + k], s);
+    y = first ? s : yacc[k] + s;
     yacc[k] = y;
+    dy[k] = s;
+    fprev[k] = v;
     const int32_t d = perm[k];
     x[d] = D[d] * y;
   }
+  max_bits(nrm, v);
   max_bits(nrm + 1, y);
 }
 
@@ -2005,11 +2012,11 @@ unsigned next_epoch(SparseDev& sp, cudaStream_t st) {
   return sp.epoch;
 }
 
-// refinement sweeps with the factors F: x = Lλx⁻¹ b.  Per height, the fronts
+// refinement sweeps with the factors F, mixed or plain: x = Lλx⁻¹ b.  Per height, the fronts
 // with fewer than sp.big_pivots pivots (the tail of the height's list) take
 // the one-block-per-front kernels, the others the blocked ones.
 template <class T>
-cudaError_t refine(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, int it0, int it1) {
+cudaError_t refine(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, bool mix, int it0, int it1) {
   cudaStream_t st = c->stream;
   const int64_t n = sp.n;
   const size_t smem = size_t(std::max(sp.max_m_small, 1)) * sizeof(double);
@@ -2020,7 +2027,7 @@ cudaError_t refine(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, int 
       if (e != cudaSuccess) return e;
     }
     sp_residual<<<nblocks(n, kThreads), kThreads, 0, st>>>(n, sp.d_perm, sp.d_rptr, sp.d_rq, sp.d_rcol, c->nzval, sp.D,
-                                                           it > 0 ? sp.xs : nullptr, b, sp.r, sp.w, sp.nrm, sp.flags);
+                                                           it > 0 ? sp.xs : nullptr, b, sp.w, sp.nrm, sp.flags);
     ++c->launches;
     for (int h = 0; h < sp.nheight; ++h) {
       if (!sp.h_nlf[h]) continue;
@@ -2122,18 +2129,20 @@ cudaError_t refine(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, int 
         }
       }
     }
-    const int kept = it % sp.ndir;  // earlier directions that this one is made conjugate to
-    double *z = sp.dirz + kept * n, *q = sp.dirq + kept * n;
-    const unsigned gd = std::max(1u, std::min(unsigned(kDotBlocks), unsigned(nblocks(n, kThreads))));
-    sp_direction<<<nblocks(n, kThreads), kThreads, 0, st>>>(n, sp.d_perm, sp.D, sp.w, z, sp.dz, sp.nrm,
-                                                             sp.flags);
-    sp_apply<<<gd, kThreads, 0, st>>>(n, kept, sp.d_rptr, sp.d_rq, sp.d_rcol, c->nzval, sp.D, sp.dz, sp.dirq, q,
-                                      sp.part, sp.done, sp.coef, sp.coef + kSparseSweeps, sp.flags);
-    sp_conjugate<<<gd, kThreads, 0, st>>>(n, kept, sp.dirq, sp.dirz, q, z, sp.r, sp.coef + kSparseSweeps, sp.part,
-                                          sp.done, sp.coef + kept, sp.coef + 2 * kSparseSweeps, sp.flags);
-    sp_step<<<nblocks(n, kThreads), kThreads, 0, st>>>(n, it == 0, sp.d_perm, sp.D, sp.coef + 2 * kSparseSweeps, z,
-                                                       sp.yacc, sp.xs, sp.nrm, sp.flags);
-    c->launches += 4;
+    // the pairs of differences: one more a sweep from the second on, after ndir from the start
+    const int nk = it > 0 ? (it - 1) % sp.ndir : 0;
+    if (mix && it > 0) {
+      double *z = sp.dirz + nk * n, *q = sp.dirq + nk * n;
+      const unsigned gd = std::max(1u, std::min(unsigned(kDotBlocks), unsigned(nblocks(n, kThreads))));
+      sp_difference<<<gd, kThreads, 0, st>>>(n, nk, sp.w, sp.fprev, sp.dy, sp.dirq, q, z, sp.part, sp.done, sp.qq,
+                                             sp.beta, sp.flags);
+      sp_conjugate<<<gd, kThreads, 0, st>>>(n, nk, sp.dirq, sp.dirz, q, z, sp.w, sp.beta, sp.part, sp.done, sp.qq,
+                                            sp.mix, sp.flags);
+      c->launches += 2;
+    }
+    sp_step<<<nblocks(n, kThreads), kThreads, 0, st>>>(n, it == 0, mix && it > 0 ? nk + 1 : 0, sp.d_perm, sp.D, sp.mix, sp.dirq,
+                                                       sp.dirz, sp.w, sp.fprev, sp.dy, sp.yacc, sp.xs, sp.nrm, sp.flags);
+    ++c->launches;
     sp_check<<<1, 1, 0, st>>>(sp.nrm, sp.last, sp.nrow, sp.flags);
     ++c->launches;
   }
@@ -2144,20 +2153,32 @@ cudaError_t refine(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, int 
 // convergence flag, so that few sweeps are enqueued after convergence
 // (every kernel of a converged sweep returns at once, but is still launched)
 template <class T>
-cudaError_t refine_batches(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, int sweeps, int first) {
-  int done = 0;
-  while (done < sweeps) {
+cudaError_t refine_batches(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, bool mix, int sweeps, int first) {
+  for (int done = 0; done < sweeps;) {
     const int nb_ = done == 0 ? std::min(first, sweeps) : 1;
-    cudaError_t e = refine<T>(c, sp, F, b, done, done + nb_);
+    cudaError_t e = refine<T>(c, sp, F, b, mix, done, done + nb_);
     if (e != cudaSuccess) return e;
     done += nb_;
-    if (done >= sweeps) break;
     e = cudaMemcpyAsync(sp.hflags, sp.flags, 4 * sizeof(int), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return e;
     if (sp.hflags[0] != 0 || sp.hflags[3] != 0) break;
   }
   return cudaSuccess;
+}
+
+// The solution by mixed sweeps, or where these don't converge by plain ones from the
+// start: factors that hold little but rounding in some directions (a component that
+// floats until its last multiplier is eliminated) answer to no mixture, as f there is no
+// function of y, and plain sweeps may still settle.  Their last state is the answer
+// where neither does.  hflags holds the flags of the last sweep.
+template <class T>
+cudaError_t refine_solve(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, int sweeps, int first) {
+  cudaError_t e = refine_batches<T>(c, sp, F, b, true, sweeps, first);
+  if (e != cudaSuccess || sp.hflags[0] != 0 || (sp.hflags[3] & 7)) return e;
+  e = cudaMemsetAsync(sp.flags, 0, 2 * sizeof(int), c->stream);  // converged, sweeps
+  if (e == cudaSuccess) e = cudaMemsetAsync(sp.flags + 3, 0, sizeof(int), c->stream);
+  return e == cudaSuccess ? refine_batches<T>(c, sp, F, b, false, sweeps, first) : e;
 }
 
 // Room for a front's vector in the one-block substitutions: the limit of what they take,
@@ -2365,10 +2386,10 @@ int sparse_create(mgpu_ctx* c, SparseDev*& spp, const double* dof_xyz, const uin
   ok(upload(&sp.d_poff, poff));
   ok(cudaMalloc(&sp.tw, n * sizeof(double)));
   ok(cudaMalloc(&sp.yacc, n * sizeof(double)));
-  ok(cudaMalloc(&sp.r, n * sizeof(double)));
-  ok(cudaMalloc(&sp.dz, n * sizeof(double)));
+  ok(cudaMalloc(&sp.fprev, n * sizeof(double)));
+  ok(cudaMalloc(&sp.dy, n * sizeof(double)));
   ok(cudaMalloc(&sp.part, size_t(kDotBlocks) * kSparseSweeps * sizeof(double)));
-  ok(cudaMalloc(&sp.coef, (2 * kSparseSweeps + 2) * sizeof(double)));  // q·q, beta, alpha, done
+  ok(cudaMalloc(&sp.coef, (3 * kSparseSweeps + 1) * sizeof(double)));  // q·q, beta, c, blocks done
   ok(cudaMalloc(&sp.xs, n * sizeof(double)));
   ok(cudaMalloc(&sp.nrm, 4 * sizeof(unsigned long long)));
   ok(cudaMalloc(&sp.last, 3 * sizeof(double)));
@@ -2391,8 +2412,11 @@ int sparse_create(mgpu_ctx* c, SparseDev*& spp, const double* dof_xyz, const uin
   }
   if (const char* ev = getenv("MGPU_SPARSE_CHAINED")) sp.chained = atoi(ev) != 0;
   ok(cudaMemset(sp.nrm, 0, 4 * sizeof(unsigned long long)));
-  ok(cudaMemsetAsync(sp.coef, 0, (2 * kSparseSweeps + 2) * sizeof(double), c->stream));
-  sp.done = reinterpret_cast<unsigned*>(sp.coef + 2 * kSparseSweeps + 1);
+  ok(cudaMemsetAsync(sp.coef, 0, (3 * kSparseSweeps + 1) * sizeof(double), c->stream));
+  sp.qq = sp.coef;
+  sp.beta = sp.coef + kSparseSweeps;
+  sp.mix = sp.coef + 2 * kSparseSweeps;
+  sp.done = reinterpret_cast<unsigned*>(sp.coef + 3 * kSparseSweeps);
   for (cudaEvent_t& ev : sp.ev) ok(cudaEventCreate(&ev));
   ok(set_smem<float>());
   ok(set_smem<double>());
@@ -2405,10 +2429,11 @@ int sparse_create(mgpu_ctx* c, SparseDev*& spp, const double* dof_xyz, const uin
   if (const char* ev = getenv("MGPU_SPARSE_TC_LEFT")) sp.tc_left = atoi(ev) != 0;
   if (const char* ev = getenv("MGPU_SPARSE_SUPER")) sp.super_panels = atoi(ev) != 0;
   if (const char* ev = getenv("MGPU_SPARSE_TC")) sp.tensor_cores = atoi(ev) != 0;
-  // directions of the sweeps: 24 vectors, or as many as there is room for, two at least
-  // (MGPU_SPARSE_DIRECTIONS: at most that many pairs)
+  // the sweeps' pairs of differences: 22 vectors, or as many as there is room for, two at
+  // least (MGPU_SPARSE_DIRECTIONS: at most that many pairs)
   const char* de = getenv("MGPU_SPARSE_DIRECTIONS");
-  for (int nd = de ? std::clamp(atoi(de), 1, kSparseSweeps) : kSparseSweeps; e == cudaSuccess; nd = (nd + 1) / 2) {
+  for (int nd = de ? std::clamp(atoi(de), 1, kSparseSweeps - 1) : kSparseSweeps - 1; e == cudaSuccess;
+       nd = (nd + 1) / 2) {
     sp.ndir = nd;
     cudaError_t x = cudaMalloc(&sp.dirz, size_t(nd) * n * sizeof(double));
     if (x == cudaSuccess) x = cudaMalloc(&sp.dirq, size_t(nd) * n * sizeof(double));
@@ -2450,8 +2475,8 @@ void sparse_destroy(SparseDev*& sp) {
   void* ps[] = {sp->d_fr, sp->d_lf, sp->d_ea, sp->d_clist, sp->d_fidx, sp->d_emap, sp->d_amap, sp->d_aq,
                 sp->d_acol, sp->d_perm, sp->d_diag, sp->d_colptr, sp->d_rowval, sp->d_rptr, sp->d_rq, sp->d_rcol,
                 sp->F32, sp->F64, sp->last,
-                sp->D, sp->cvec, sp->w, sp->V, sp->P, sp->d_poff, sp->tw, sp->yacc, sp->r,
-                sp->dirz, sp->dirq, sp->pack, sp->dz, sp->part, sp->coef, sp->xs, sp->nrm,
+                sp->D, sp->cvec, sp->w, sp->V, sp->P, sp->d_poff, sp->tw, sp->yacc, sp->fprev,
+                sp->dirz, sp->dirq, sp->pack, sp->dy, sp->part, sp->coef, sp->xs, sp->nrm,
                 sp->flags, sp->tflag, sp->chain};
   for (void* p : ps) cudaFree(p);
   if (sp->hflags) cudaFreeHost(sp->hflags);
@@ -2482,7 +2507,7 @@ int sparse_factor_solve(mgpu_ctx* c, SparseDev& sp, const double* rhs, double* o
     MG_CUDA(cudaEventRecord(sp.ev[0], st));
     MG_CUDA((factorise<float, kNB32>(c, sp, sp.F32, 1e-10f)));
     MG_CUDA(cudaEventRecord(sp.ev[1], st));
-    MG_CUDA(refine_batches<float>(c, sp, sp.F32, rhs, kSparseSweeps, 4));
+    MG_CUDA(refine_solve<float>(c, sp, sp.F32, rhs, kSparseSweeps, 4));
     MG_CUDA(cudaEventRecord(sp.ev[2], st));
     MG_CUDA(cudaMemcpyAsync(sp.hflags, sp.flags, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
     MG_CUDA(cudaStreamSynchronize(st));
@@ -2516,7 +2541,7 @@ int sparse_factor_solve(mgpu_ctx* c, SparseDev& sp, const double* rhs, double* o
     MG_CUDA(cudaEventRecord(sp.ev[0], st));
     MG_CUDA((factorise<double, kNB64>(c, sp, sp.F64, 0.0)));
     MG_CUDA(cudaEventRecord(sp.ev[1], st));
-    MG_CUDA(refine_batches<double>(c, sp, sp.F64, rhs, kSparseSweeps64, 2));
+    MG_CUDA(refine_solve<double>(c, sp, sp.F64, rhs, kSparseSweeps64, 2));
     MG_CUDA(cudaEventRecord(sp.ev[2], st));
     MG_CUDA(cudaMemcpyAsync(sp.hflags, sp.flags, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
     MG_CUDA(cudaStreamSynchronize(st));

@@ -13,11 +13,11 @@
 //     dofs they constrain, so their zero diagonal is never a pivot) in blocks
 //     of NB columns: one kernel factors the diagonal block and solves the
 //     block's L and U panels, one updates the trailing block;
-//   * FP32 factors inside FP64 sweeps of the conjugate residual method (residuals
-//     of the FP64 Lλx and the solution so far), until the scaled correction is
-//     below 1e-14 of the scaled solution, or as good as that, or at the accuracy
-//     that FP64 attains (sparse_stop.hpp), at most kSparseSweeps sweeps; when that
-//     fails, or a norm is not finite, the same kernels factorise in FP64
+//   * FP32 factors inside FP64 sweeps of iterative refinement with Anderson's mixing
+//     (residuals of the FP64 Lλx and the solution so far), until the scaled
+//     correction is below 1e-14 of the scaled solution, or as good as that, or at
+//     the accuracy that FP64 attains (sparse_stop.hpp), at most kSparseSweeps sweeps;
+//     when that fails, or a norm is not finite, the same kernels factorise in FP64
 //     (MGPU_LINSOLVE_SPARSE), or FP64 throughout (_SPARSE64).
 // Every sum runs in a fixed order: results are bitwise repeatable.
 #pragma once
@@ -88,11 +88,12 @@ struct SparseDev {
   int64_t* d_poff = nullptr;    // [nfront] offset of each blocked front's partials in P
   double* tw = nullptr;         // [n] U₁₂ x_u of each pivot (backward substitution)
   double* yacc = nullptr;       // [n] accumulated scaled solution (elimination order)
-  int ndir = 0;                             // directions kept
-  double *dirz = nullptr, *dirq = nullptr;  // [ndir][n] directions of the sweeps and A times them
-  double *dz = nullptr, *part = nullptr, *coef = nullptr;  // D z, blocks' sums, the sweeps' coefficients
+  int ndir = 0;                             // pairs of differences kept by the sweeps
+  double *dirz = nullptr, *dirq = nullptr;  // [ndir][n] differences of the solutions and of the corrections
+  double *fprev = nullptr, *dy = nullptr;   // [n] the last sweep's correction, and its step
+  double *part = nullptr, *coef = nullptr;  // blocks' sums, the sweeps' coefficients:
+  double *qq = nullptr, *beta = nullptr, *mix = nullptr;
   unsigned* done = nullptr;                 // blocks that have added theirs
-  double* r = nullptr;          // [n] residual (model order)
   double* xs = nullptr;         // [n] current solution (model order)
   unsigned long long* nrm = nullptr;  // [4] max |correction|, |solution|, |residual|, |A||y| + |D b| (as ordered bits)
   double* last = nullptr;       // [3] of the previous sweep (sp_stop)

@@ -30,7 +30,8 @@ enum SpStop : int { SP_GO_ON = 0, SP_CONVERGED = 1, SP_NOT_FINITE = 2 };
 //  * c <= 1e-14 y;
 //  * from the third sweep on, c <= 1e-11 y and the next correction below 1e-15 y at the
 //    worst rate so far (not the last: the rate may worsen again, the method lessens
-//    |r|₂, not |M⁻¹r|; a rate a thousand times the worst still leaves 1e-12);
+//    |M⁻¹r|₂ over the sweeps so far, not its largest entry; a rate a thousand times the
+//    worst still leaves 1e-12);
 //  * c <= 1e-10 y and no better than half the last one, with r down at its own rounding,
 //    (nrow + 4) 2⁻⁵³ a, or for the second time in a row: with neither it may be a plateau
 //    of the method instead of the accuracy attained.  (Factors of raised pivots add

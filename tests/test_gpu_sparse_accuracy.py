@@ -86,3 +86,51 @@ def test_sweeps_with_fewer_directions_reach_the_same_solution(monkeypatch, kind,
     a, b = out[kept][:, 0], out["12"][:, 0]
     for sel in (lam, ~lam):
         assert np.max(np.abs(a[:, sel] - b[:, sel])) <= 1e-9 * np.max(np.abs(b[:, sel]))
+
+
+def stubs(nels, axis, hold=0, seed=0):
+    """Clamped beams of a few elements side by side, each floating until the multipliers
+    of its one support are eliminated."""
+    rng = np.random.default_rng(seed)
+    m = Model("stubs")
+    held, tip = [], []
+    for c, nel in enumerate(nels):
+        xyz = np.zeros((nel + 1, 3))
+        xyz[:, axis] = np.arange(nel + 1.0)
+        nodes = m.addnode(xyz + [0.0, 0.0, 50.0 * c] + 0.02 * rng.normal(size=xyz.shape))
+        EA, EI2, EI3, GJ = (v * np.exp(rng.normal(0.0, 0.5, nel)) for v in (1e7, 1e4, 1e4, 1e4))
+        mat = W.BeamCrossSection(EA=EA, EI2=EI2, EI3=EI3, GJ=GJ, mu=10.0, iota1=1.0)
+        m.addelement(W.EulerBeam3D, np.stack([nodes[:-1], nodes[1:]], axis=1), mat=mat,
+                     orient2=[(0.0, 1.0, 0.0), (0.0, 0.0, 1.0), (1.0, 0.0, 0.0)][axis])
+        held.append(nodes[hold])
+        tip.append(nodes[-1])
+    for f in ("t1", "t2", "t3", "r1", "r2", "r3"):
+        m.addelement(W.Hold, np.asarray(held)[:, None], field=f)
+    m.addelement(W.DofLoad, np.asarray(tip)[:, None], field="t1", value=lambda t: 10.0 * t)
+    m.addelement(W.DofLoad, np.asarray(tip)[:1, None], field="t2", value=lambda t: 13.0 * t)
+    return m
+
+
+STUBS = [((3,) * 9, 0, 0, 1e-9), ((3,) * 9, 0, 1, 1e-9), ((2, 3, 4), 2, 0, 1e-9), ((2, 60), 0, 1, 1e-6)]
+
+
+@pytest.mark.parametrize("nels, axis, hold, tol, kind", [(*s, k) for k in ("sparse", "sparse64") for s in STUBS]
+                         + [((1, 2), 0, 0, 1e-9, "sparse")])  # FP64 without row exchanges meets a zero pivot there
+def test_short_clamped_beams(nels, axis, hold, tol, kind):
+    """One solve against the banded FP64 solver, which pivots: the factors are as good as
+    rounding in the direction in which a component floats, so the first corrections are
+    large and raise the residual, and steps that may only lessen it came to nothing
+    (states wholly wrong, or FP32 factors given up for singular FP64 ones).  A component
+    of 60 beams has a condition of some 1e10."""
+    m = stubs(nels, axis, hold)
+    st = m.initialize()
+    out = {}
+    for k in (kind, "f64"):
+        dm = DeviceModel(m, st.dis, linsolve=k)
+        rc, X, _ = dm.sweepx(0, np.array([1.0]), st.time, list(st.X), fixed_iter=1)
+        dm.close()
+        assert rc == 0
+        out[k] = X[0, 0]
+    lam = np.array([str(f).startswith("λ") for f in st.dis.fieldX])
+    for sel in (lam, ~lam):
+        assert np.max(np.abs(out[kind][sel] - out["f64"][sel])) <= tol * np.max(np.abs(out["f64"][sel]))
