@@ -1865,14 +1865,14 @@ __global__ void __launch_bounds__(kThreads) sp_step(int64_t n, int first, int np
 
 // flags[0] when the sweep was the last that is needed (sp_stop); flags[3] bit 3 where a
 // norm is not finite
-__global__ void sp_check(unsigned long long* nrm, double* last, int nrow, int* flags) {
+__global__ void sp_check(unsigned long long* nrm, double* last, int nrow, bool mixed, int* flags) {
   if (flags[0]) return;
   double v[4];
   for (int q = 0; q < 4; ++q) {
     v[q] = __longlong_as_double((long long)nrm[q]);
     nrm[q] = 0ull;
   }
-  const SpStop s = sp_stop(++flags[1], v[0], v[1], v[2], v[3], nrow, last);
+  const SpStop s = sp_stop(mixed, ++flags[1], v[0], v[1], v[2], v[3], nrow, last);
   if (s == SP_CONVERGED) flags[0] = 1;
   if (s == SP_NOT_FINITE) flags[3] |= 8;
 }
@@ -2143,7 +2143,7 @@ cudaError_t refine(mgpu_ctx* c, SparseDev& sp, const T* F, const double* b, bool
     sp_step<<<nblocks(n, kThreads), kThreads, 0, st>>>(n, it == 0, mix && it > 0 ? nk + 1 : 0, sp.d_perm, sp.D, sp.mix, sp.dirq,
                                                        sp.dirz, sp.w, sp.fprev, sp.dy, sp.yacc, sp.xs, sp.nrm, sp.flags);
     ++c->launches;
-    sp_check<<<1, 1, 0, st>>>(sp.nrm, sp.last, sp.nrow, sp.flags);
+    sp_check<<<1, 1, 0, st>>>(sp.nrm, sp.last, sp.nrow, mix, sp.flags);
     ++c->launches;
   }
   return cudaGetLastError();

@@ -32,14 +32,14 @@ enum SpStop : int { SP_GO_ON = 0, SP_CONVERGED = 1, SP_NOT_FINITE = 2 };
 //    worst rate so far (not the last: the rate may worsen again, the method lessens
 //    |M⁻¹r|₂ over the sweeps so far, not its largest entry; a rate a thousand times the
 //    worst still leaves 1e-12);
-//  * c <= 1e-10 y and no better than half the last one, with r down at its own rounding,
-//    (nrow + 4) 2⁻⁵³ a, or for the second time in a row: with neither it may be a plateau
-//    of the method instead of the accuracy attained.  (Factors of raised pivots add
-//    rounding of their own, and r stays a hundred times higher.)
+//  * c <= 1e-10 y and no better than half the last one, after mixed sweeps with r down at
+//    its own rounding, (nrow + 4) 2⁻⁵³ a, or for the second time in a row: with neither it
+//    may be a plateau of the method instead of the accuracy attained.  (Factors of raised
+//    pivots add rounding of their own, and r stays a hundred times higher.)
 // Without the second rule a sweep or two at the rounding level follow where the matrix
 // is conditioned well: 12 x 12 x 6 lattice 5 -> 6 sweeps a solve, 44.7 -> 52.8 ms for its
 // three load steps; 60 x 60 x 20 ends by the third after 9 either way.
-SP_HD SpStop sp_stop(int sweep, double c, double y, double r, double a, int nrow, double last[3]) {
+SP_HD SpStop sp_stop(bool mixed, int sweep, double c, double y, double r, double a, int nrow, double last[3]) {
   if (!(c <= 1.7e308) || !(y <= 1.7e308)) return SP_NOT_FINITE;
   const bool again = sweep > 1;
   const double prev = last[0], rate = again ? fmax(last[1], c / prev) : 0.0;
@@ -49,7 +49,7 @@ SP_HD SpStop sp_stop(int sweep, double c, double y, double r, double a, int nrow
   last[2] = still ? 1.0 : 0.0;
   if (c <= kRefineTol * y) return SP_CONVERGED;
   if (sweep >= 3 && c <= kRefineNear * y && c * rate <= 0.1 * kRefineTol * y) return SP_CONVERGED;
-  if (still && c <= kRefineStall * y && (before || r <= (nrow + 4) * 0x1p-53 * a)) return SP_CONVERGED;
+  if (still && c <= kRefineStall * y && (!mixed || before || r <= (nrow + 4) * 0x1p-53 * a)) return SP_CONVERGED;
   return SP_GO_ON;
 }
 

@@ -115,7 +115,7 @@ STUBS = [((3,) * 9, 0, 0, 1e-9), ((3,) * 9, 0, 1, 1e-9), ((2, 3, 4), 2, 0, 1e-9)
 
 
 @pytest.mark.parametrize("nels, axis, hold, tol, kind", [(*s, k) for k in ("sparse", "sparse64") for s in STUBS]
-                         + [((1, 2), 0, 0, 1e-9, "sparse")])  # FP64 without row exchanges meets a zero pivot there
+                         + [((1, 2), 0, 0, 1e-9, "sparse"), ((1,), 1, 0, 1e-9, "sparse")])  # FP64 without row exchanges meets a zero pivot there
 def test_short_clamped_beams(nels, axis, hold, tol, kind):
     """One solve against the banded FP64 solver, which pivots: the factors are as good as
     rounding in the direction in which a component floats, so the first corrections are

@@ -21,13 +21,13 @@ def stop():
                     os.path.join(HERE, "sparse_stop_check.cpp")], check=True)
     os.replace(so + ".tmp", so)
     f = ctypes.CDLL(so).sparse_stop_check
-    f.argtypes = [ctypes.c_int] + [ctypes.c_void_p] * 4 + [ctypes.c_int]
+    f.argtypes = [ctypes.c_int] * 2 + [ctypes.c_void_p] * 4 + [ctypes.c_int]
 
-    def run(c, r=None, y=None, a=None, nrow=40):
+    def run(c, r=None, y=None, a=None, nrow=40, mixed=True):
         n = len(c)
         v = [np.ascontiguousarray(np.broadcast_to(np.asarray(q, dtype=np.float64), (n,)).copy())
              for q in (c, 1.0 if y is None else y, 0.0 if r is None else r, 1.0 if a is None else a)]
-        return f(n, *[q.ctypes.data for q in v], nrow)
+        return f(int(mixed), n, *[q.ctypes.data for q in v], nrow)
 
     return run
 
@@ -53,6 +53,7 @@ def test_a_plateau_counts_where_the_residual_is_rounding_or_it_lasts(stop):
     assert stop(c, r=[1.0, 1e-4, 1e-9, 1e-10, 44 * U, 44 * U]) == 5  # two orders above it in the fourth
     assert stop(c, r=1e-12) == 5  # the second time in a row
     assert stop([1.0, 1e-2, 5e-11, 4e-11, 1e-13, 9e-14], r=1e-12) == 0  # it did not last
+    assert stop(c, r=1e-12, mixed=False) == 4  # plain sweeps have none of their own
     assert stop([1.0, 1e-6, 2e-10, 1.9e-10, 1.8e-10], r=0.0) == 0  # too far off to stop at all
 
 
