@@ -1665,7 +1665,7 @@ __global__ void sp_bwdb_fin(const SpFrontDev* __restrict__ fr, const int32_t* __
 // A and r are scaled, A = D Lλx D; all vectors in elimination order.  The pairs of all
 // sweeps are kept (where there is no room for them fewer, and the mixing starts again
 // when these are full).
-//   60 x 60 x 20 lattice: 11 -> 8 or 9 sweeps a solve; 12 x 12 x 6: 8 -> 5
+//   60 x 60 x 20 lattice: 11 -> 9 sweeps a solve; 12 x 12 x 6: 8 -> 6
 constexpr double kDependent = 1e-12;  // q·q of df·df: a difference that tells nothing new
 constexpr int kDotBlocks = 304;
 

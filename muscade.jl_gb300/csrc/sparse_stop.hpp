@@ -32,13 +32,14 @@ enum SpStop : int { SP_GO_ON = 0, SP_CONVERGED = 1, SP_NOT_FINITE = 2 };
 //    worst rate so far (not the last: the rate may worsen again, the method lessens
 //    |M⁻¹r|₂ over the sweeps so far, not its largest entry; a rate a thousand times the
 //    worst still leaves 1e-12);
-//  * c <= 1e-10 y and no better than half the last one, after mixed sweeps with r down at
-//    its own rounding, (nrow + 4) 2⁻⁵³ a, or for the second time in a row: with neither it
-//    may be a plateau of the method instead of the accuracy attained.  (Factors of raised
-//    pivots add rounding of their own, and r stays a hundred times higher.)
+//  * c <= 1e-10 y and no better than half the last one: after plain sweeps at once; after
+//    mixed ones with r down at its own rounding, (nrow + 4) 2⁻⁵³ a, or for the second time
+//    in a row: with neither it may be a plateau of the method instead of the accuracy
+//    attained.  (Factors of raised pivots add rounding of their own, and r stays a
+//    hundred times higher.)
 // Without the second rule a sweep or two at the rounding level follow where the matrix
-// is conditioned well: 12 x 12 x 6 lattice 5 -> 6 sweeps a solve, 44.7 -> 52.8 ms for its
-// three load steps; 60 x 60 x 20 ends by the third after 9 either way.
+// is conditioned well: 12 x 12 x 6 lattice 44.6 -> 51.7 ms for its three load steps;
+// 60 x 60 x 20 takes 9 sweeps a solve either way (491 ms).
 SP_HD SpStop sp_stop(bool mixed, int sweep, double c, double y, double r, double a, int nrow, double last[3]) {
   if (!(c <= 1.7e308) || !(y <= 1.7e308)) return SP_NOT_FINITE;
   const bool again = sweep > 1;
