@@ -313,7 +313,8 @@ int mgpu_sensitivity_sweepx(mgpu_ctx *ctx, int32_t OX, int64_t nstep, const doub
  *                        matrix, FP32 factors inside FP64 iterative refinement
  *                        until the scaled correction is below 1e-14 of the
  *                        scaled solution or stops shrinking below 1e-10 of it
- *                        (at most 12 sweeps), else the FP64 factors, which then
+ *                        (at most 12 sweeps with Anderson's mixing, then at
+ *                        most 12 plain ones), else the FP64 factors, which then
  *                        stay in use for the context
  *   MGPU_LINSOLVE_SPARSE64 the multifrontal LU in FP64 throughout
  * F64 and BLOCK give bitwise the same Δx.  Returns MGPU_ERR_UNSUPPORTED when
